@@ -1,32 +1,41 @@
 // mgpu_device.cu - sm_103a kernels of the loop-extrusion epoch engine.
 //
-// One warp simulates one cell (Simulation::simulate_one_cell, src/libmodle/cpu/
-// simulation.cpp:1056-1152).  The cell's state is structure-of-arrays of 32-bit words; the
-// host plans which per-LEF arrays fit in the cell's shared memory and places the rest in a
-// per-cell global scratch slot (large chromosomes).  The barrier track and its integer
+// One thread block simulates one cell (Simulation::simulate_one_cell, src/libmodle/cpu/
+// simulation.cpp:1056-1152): 4, 8 or 16 worker warps by the number of LEFs, and one or two producer
+// warps that generate the cell's random numbers.  The cell's state is structure-of-arrays of
+// 32-bit words; the host plans which per-LEF arrays fit in the cell's shared memory and places
+// the rest in a per-cell global scratch slot (large chromosomes).  The barrier track and its integer
 // thresholds are read-only in global memory and shared by every cell of the chromosome.
-// The kernel is persistent: each warp pulls cell indices from a global work counter.
+// The kernel is persistent: each block pulls cell indices from a global work counter.
+//
+// Why a block per cell.  An epoch is about twenty dependent sweeps over the LEFs or barriers.  With one
+// warp per cell a sweep of 2,000 LEFs is 63 dependent rounds of loads, shared memory holds at most a
+// dozen such warps per SM, and an instruction issued on 10 % of cycles.  With 16 warps a sweep is
+// two or four rounds, the arrays stay in shared memory, and a sweep costs about one barrier.
 //
 // Draw order.  Every random number of the reference comes from one sequential
-// Xoshiro256++ stream per cell, consumed in a data-dependent order.  The warp keeps a ring of
-// pre-generated draws in shared memory: all 32 lanes generate RNG_S consecutive draws each per
-// refill and then advance their private state by 31 * RNG_S steps with a GF(2) jump table (the
-// state transition of xoshiro is linear), so the ring always holds the exact stream.
+// Xoshiro256++ stream per cell, consumed in a data-dependent order.  The producer warps keep a
+// ring of draws in shared memory filled ahead of the workers: each of their P lanes generates
+// RNG_S consecutive draws per refill and then advances its private state by (P - 1) * RNG_S steps with
+// a GF(2) jump table (the state transition of xoshiro is linear), so the ring always holds the
+// exact stream.  A jump costs as much as 50 draws and has a long latency, which is why it runs
+// beside the epoch loop instead of inside it.  The workers acquire the ring's fill position
+// (rng_ensure) and release the draws they are done with after a barrier (rng_publish); every wait
+// is bounded and ends the cell with a status.
 //
-// Every step of the epoch runs warp-parallel with the exact draw order:
-//  * steps whose items take one draw each (binding, barrier steps, moves, release, LEF-BAR
-//    and LEF-LEF trials) give lane k the draw at offset popc(ballot & lanemask_lt);
+// Every step of the epoch runs block-parallel with the exact draw order:
+//  * steps whose items take one draw each (binding, barrier steps, release, LEF-BAR and LEF-LEF
+//    trials) give every item the draw at its offset from a block-wide scan;
 //  * items that may take more draws (ziggurat wedges and tails, rejected contact attempts,
 //    failed bypass trials in a chain of secondary collisions) are evaluated speculatively at
-//    the offsets they would have if every earlier item took its usual count; the first item
-//    that deviates is resolved exactly and the warp resumes after it;
-//  * sequential sweeps are replaced by closed forms: rank_lefs by a merge of the units bound
-//    this epoch into the still-sorted order of the others, adjust_moves by segmented min/max
-//    scans, the LEF-BAR and primary LEF-LEF sweeps by binary searches over the ranked
-//    positions.
+//    the offsets they would have if every earlier item took its usual count; the offsets are then
+//    corrected from the items that deviate, or the workers resume after the first of them;
+//  * sequential sweeps are replaced by closed forms: rank_lefs by a merge of the units that moved
+//    into the still-sorted order of the others, adjust_moves by walks from the units that push a
+//    neighbour, the LEF-BAR and primary LEF-LEF sweeps by searches over the ranked positions.
 // Where a closed form's precondition does not hold (full ties in the ranking, a chain that
-// reaches a chromosome end, unsorted caller input), the step falls back to a line-by-line
-// serial restatement run by lane 0, so results never depend on the fast path.
+// reaches a chromosome end, unsorted caller input), the step falls back to an exact restatement run
+// by one warp or one thread, so results never depend on the fast path.
 //
 // Floating point.  The file is compiled with --fmad=false so every double multiply and add
 // is rounded separately, like the reference's x86-64 build; bernoulli and
@@ -45,15 +54,6 @@ namespace mgpu {
 
 #define MGPU_ITER_LIMIT 100000000ull
 #define FULL 0xFFFFFFFFu
-
-// Items per lane in the chunked sweeps: the per-LEF arrays of large cells live in global
-// memory, where every dependent load waits for L2; a lane that carries MLP independent items
-// through each stage of a sweep keeps MLP loads in flight instead of one.
-#ifndef MGPU_MLP
-#define MGPU_MLP 2
-#endif
-constexpr unsigned MLP = MGPU_MLP;
-
 
 __device__ __forceinline__ u64 rotl64(u64 x, int k) { return (x << k) | (x >> (64 - k)); }
 
@@ -91,20 +91,23 @@ __device__ __forceinline__ u32 warp_excl_scan(u32 v, u32* total) {
   return x - v;
 }
 
-// Cell scalars (warp-uniform, kept in shared memory so lane 0's serial code can update them).
+// Cell scalars (the same for every thread, kept in shared memory so thread 0's serial code can update
+// them; a value thread 0 writes is read by the others only after a barrier).
 // Per-launch profile counters (cycles per step and fallback counts), summed over cells.
 enum : u32 {
   PF_BURNIN = 0, PF_BIND, PF_RANK, PF_CONTACTS, PF_MOVES, PF_ADJUST, PF_BARRIERS, PF_BOUNDARIES,
   PF_LEF_BAR, PF_PRIMARY, PF_CORRECT, PF_SECONDARY, PF_FIX, PF_EXTRUDE_RELEASE, PF_TRACE, PF_TOTAL,
   PF_RANK_FALLBACK, PF_ADJUST_FALLBACK, PF_CHAIN_SERIAL, PF_CONTACT_SERIAL, PF_FIX_FALLBACK,
   PF_REFILLS, PF_STALE_REFILLS, PF_EPOCHS, PF_RANK_PDQ, PF_RANK_PASS, PF_RANK_BLOCK, PF_RANK_MERGE,
-  PF_RANK_SERIAL, PF_COUNT = 32
+  PF_RANK_SERIAL, PF_RANK_SPLIT, PF_COUNT = 32
 };
 
 struct Scalars {
-  u64 rpos, gpos;  // next draw to consume / to generate (stream indices)
-  u64 canon[4];    // xoshiro state at gpos
-  u32 lanes_stale; // lanes must re-derive their states from canon before the next refill
+  u64 rpos;        // next draw to consume (stream index)
+  u64 canon[4];    // xoshiro state at the start of the stream
+  u32 gpos;        // draws generated so far (modulo 2^32): producers release, workers acquire
+  u32 rpub;        // draws the workers are done with (modulo 2^32): thread 0 releases
+  u32 stop, pgo;   // end of the cell; the producers' decision to refill
   u32 status;
   u64 epoch, num_burnin_epochs, num_active, num_contacts;
   u32 burnin_completed, flag;
@@ -117,10 +120,27 @@ struct Scalars {
 };
 static_assert(sizeof(Scalars) <= CELL_HEADER_BYTES, "scalars do not fit the cell header");
 
-// Pointers of one cell (lives in shared memory; identical for every lane).
+// Scratch of the block-wide steps.
+struct BlockTmp {
+  u32 cnt[2][32];       // scan2
+  u32 tab[16][32];      // gen_moves_dir: per warp and entry lane, leaving position | normals << 16
+  u64 wmax[16];         // rank_dir_block
+  u32 rem[16], rembase[16];
+  u32 nrem, tie, tie2;
+  u32 dev[16], okm[16], dus[16];  // sample_contacts
+  u32 used, qend, nr, nf, released, missed, flag;
+  u64 sum;
+  ulonglong2 zt[128];   // normal ziggurat per layer: {draws below this are accepted, width * 2^60}
+};
+
+// Pointers of one cell (lives in shared memory; identical for every thread).
 struct Cell {
   Scalars* sc;
+  BlockTmp* bt;
   u64* ring;
+  u32 T;      // worker threads (0: no producers, one thread generates its own draws)
+  u32 rmask;  // ring capacity - 1
+  u32 lim;    // draws the producers always provide beyond the last published position
   u32 *rev, *fwd, *rr, *fr, *rm, *fm, *rc, *fc, *sr, *sf, *tmp, *bep;
   u32* bst;
   double *hcfx, *havg;
@@ -140,6 +160,40 @@ __device__ __forceinline__ u32 bar_flags(const Cell& c, u32 i) { return __ldg(&c
 // ---------------------------------------------------------------------------------------
 // PRNG ring
 // ---------------------------------------------------------------------------------------
+__device__ __forceinline__ u32 ld_acquire(const u32* p) {
+  u32 v;
+  asm volatile("ld.acquire.cta.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release(u32* p, u32 v) {
+  asm volatile("st.release.cta.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ u64 global_ns() {
+  u64 t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Barrier of the cell's worker warps (the producer warps do not take part).
+__device__ __forceinline__ void wsync(const Cell& c) { asm volatile("barrier.sync 1, %0;" ::"r"(c.T) : "memory"); }
+// The same, returning whether any worker thread passed a true predicate.
+__device__ __forceinline__ bool wsync_or(const Cell& c, bool p) {
+  u32 r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.red.or.pred q, 1, %2, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((u32)p), "r"(c.T)
+      : "memory");
+  return r != 0;
+}
+
+__device__ __forceinline__ void set_status(Cell& c, u32 st) {
+  if (c.sc->status == DEV_OK) c.sc->status = st;
+}
+
 __device__ __forceinline__ void xo_jump(u64* s, const ulonglong2* jt) {
   u64 n0 = 0, n1 = 0, n2 = 0, n3 = 0;
 #pragma unroll 8
@@ -158,63 +212,106 @@ __device__ __forceinline__ void xo_jump(u64* s, const ulonglong2* jt) {
   s[3] = n3;
 }
 
-// Collective: append RNG_BLOCK draws to the ring.  s is this lane's private stream state.
-__device__ __noinline__ void rng_refill(Cell& c, u64* s) {
+// Body of the producer warps for one cell: whenever a refill fits beside the unconsumed draws,
+// each lane writes its next RNG_S draws and jumps over the other lanes' (see the file header).
+// Returns when the workers set sc->stop, or after 20 s without a consumer (which then runs into
+// its own limit in rng_wait).
+__device__ __noinline__ void rng_produce(Cell& c) {
   Scalars* sc = c.sc;
-  const u32 lane = ln();
-  const bool stale = sc->lanes_stale != 0;
-  if (stale) {
-    for (int k = 0; k < 4; ++k) s[k] = sc->canon[k];
-    for (u32 t = 0; t < lane * RNG_S; ++t) xo_next(s);
-  }
-  if (lane == 0 && sc->prof) {
-    atomicAdd((unsigned long long*)&sc->prof[PF_REFILLS], 1ull);
-    if (stale) atomicAdd((unsigned long long*)&sc->prof[PF_STALE_REFILLS], 1ull);
-  }
-  const u64 g = sc->gpos;
+  const u32 pl = threadIdx.x - c.T, P = blockDim.x - c.T;
+  const u32 block = P * RNG_S, mask = c.rmask;
+  u64 s[4];
+  for (int k = 0; k < 4; ++k) s[k] = sc->canon[k];
+  for (u32 t = 0; t < pl * RNG_S; ++t) xo_next(s);
+  u64* ring = c.ring;
+  const ulonglong2* jt = c.jt;
+  u32 g = 0;
+  for (;;) {
+    if (pl == 0) {
+      u32 go = 1;
+      u64 t0 = 0;
+      for (;;) {
+        if (ld_acquire(&sc->stop)) {
+          go = 0;
+          break;
+        }
+        if (g - ld_acquire(&sc->rpub) <= block) break;
+        __nanosleep(100);
+        const u64 t = global_ns();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > 20000000000ull) {
+          go = 0;
+          break;
+        }
+      }
+      sc->pgo = go;
+    }
+    asm volatile("barrier.sync 2, %0;" ::"r"(P) : "memory");
+    if (!sc->pgo) return;
+    const u32 at = g + pl * RNG_S;
 #pragma unroll 4
-  for (int k = 0; k < RNG_S; ++k) c.ring[(g + (u64)lane * RNG_S + k) & (RING - 1)] = xo_next(s);
-  xo_jump(s, c.jt);
-  __syncwarp();
-  if (lane == 0) {
-    sc->gpos = g + RNG_BLOCK;
-    for (int k = 0; k < 4; ++k) sc->canon[k] = s[k];
-    sc->lanes_stale = 0;
+    for (u32 k = 0; k < (u32)RNG_S; ++k) ring[(at + k) & mask] = xo_next(s);
+    g += block;
+    asm volatile("barrier.sync 2, %0;" ::"r"(P) : "memory");
+    if (pl == 0) st_release(&sc->gpos, g);
+    xo_jump(s, jt);  // overlaps with the consumers
   }
-  __syncwarp();
 }
 
-// Collective: make at least n (<= RNG_BLOCK) unconsumed draws available.
-__device__ __forceinline__ void rng_ensure(Cell& c, u64* s, u32 n) {
-  while (c.sc->gpos - c.sc->rpos < n) rng_refill(c, s);
+// Wait for the producers (at most 2 s, then the cell is abandoned with a status).
+__device__ __noinline__ void rng_wait(Cell& c, u32 rp, u32 n) {
+  const u64 t0 = global_ns();
+  while (ld_acquire(&c.sc->gpos) - rp < n) {
+    if (*(volatile u32*)&c.sc->status == DEV_ERR_RNG) return;
+    __nanosleep(20);
+    if (global_ns() - t0 > 2000000000ull) {
+      c.sc->status = DEV_ERR_RNG;
+      return;
+    }
+  }
 }
 
-__device__ __forceinline__ u64 ring_at(const Cell& c, u64 k) { return c.ring[k & (RING - 1)]; }
+// Every worker thread that reads draws [rp, rp + n) calls this first (n <= c.lim minus the draws
+// consumed since the last rng_publish).
+__device__ __forceinline__ void rng_ensure(Cell& c, u64 rp, u32 n) {
+  if (ld_acquire(&c.sc->gpos) - (u32)rp < n) rng_wait(c, (u32)rp, n);
+}
 
-// Lane 0 only: next draw of the stream, generated serially when the ring is dry.
+// Thread 0, after a wsync that follows every read of the draws before rp: record the position
+// and hand the ring space back to the producers.
+__device__ __forceinline__ void rng_publish(Cell& c, u64 rp) {
+  if (threadIdx.x == 0) {
+    c.sc->rpos = rp;
+    st_release(&c.sc->rpub, (u32)rp);
+  }
+}
+
+__device__ __forceinline__ u64 ring_at(const Cell& c, u64 k) { return c.ring[(u32)k & c.rmask]; }
+
+// Thread 0 only (the other workers wait at a barrier): next draw of the stream.  Without
+// producer warps (c.T == 0, the sampler probe) the thread generates it itself.
 __device__ __noinline__ u64 rng_serial(Cell& c) {
   Scalars* sc = c.sc;
-  if (sc->rpos == sc->gpos) {
-    const u64 v = xo_next(sc->canon);
-    c.ring[sc->gpos & (RING - 1)] = v;
-    sc->gpos++;
-    sc->lanes_stale = 1;
+  if ((u32)sc->rpos == ld_acquire(&sc->gpos)) {
+    if (c.T == 0) {
+      c.ring[sc->gpos & c.rmask] = xo_next(sc->canon);
+      sc->gpos++;
+    } else {
+      rng_wait(c, (u32)sc->rpos, 1);
+    }
   }
-  const u64 v = c.ring[sc->rpos & (RING - 1)];
+  const u64 v = ring_at(c, sc->rpos);
   sc->rpos++;
+  if (c.T) st_release(&sc->rpub, (u32)sc->rpos);
   return v;
 }
 
 __device__ __forceinline__ void prof_add(Cell& c, u32 k, u64 v) {
-  if (ln() == 0 && c.sc->prof) atomicAdd((unsigned long long*)&c.sc->prof[k], (unsigned long long)v);
-}
-
-__device__ __forceinline__ void set_status(Cell& c, u32 st) {
-  if (c.sc->status == DEV_OK) c.sc->status = st;
+  if (threadIdx.x == 0 && c.sc->prof) atomicAdd((unsigned long long*)&c.sc->prof[k], (unsigned long long)v);
 }
 
 // ---------------------------------------------------------------------------------------
-// Serial distributions (lane 0).  Boost.Random 1.79 semantics, see the oracle for the
+// Serial distributions (thread 0).  Boost.Random 1.79 semantics, see the oracle for the
 // line-by-line restatement; thresholds replace bernoulli / canonical comparisons.
 // ---------------------------------------------------------------------------------------
 
@@ -261,7 +358,7 @@ __device__ __forceinline__ double ifp_fraction(u64 u) {
   return (double)(u >> 8) * (1.0 / 72057594037927936.0);
 }
 
-// Draw sources of the samplers below.  SerialSrc is lane 0's view of the cell's stream; RingSrc
+// Draw sources of the samplers below.  SerialSrc is thread 0's view of the cell's stream; RingSrc
 // is one lane's view of the pre-generated ring starting at a given stream position, which
 // reports exhaustion instead of generating.
 struct SerialSrc {
@@ -276,11 +373,11 @@ struct SerialSrc {
 
 struct RingSrc {
   const u64* ring;
-  u64 pos, end;
+  u32 mask, pos, end;
   u32 n;
   __device__ bool next(u64& u) {
-    if (pos >= end) return false;
-    u = ring[pos & (RING - 1)];
+    if (pos == end) return false;
+    u = ring[pos & mask];
     ++pos;
     ++n;
     return true;
@@ -588,7 +685,7 @@ __device__ __noinline__ double s_gev(Cell& c, const KParams& P) {
 
 
 // ---------------------------------------------------------------------------------------
-// Serial restatements (lane 0): the exact fallbacks of the warp-parallel steps.  They and the
+// Serial restatements (thread 0): the exact fallbacks of the warp-parallel steps.  They and the
 // serial samplers are kept out of line: the epoch loop's code is large enough that, with eight
 // or more cells per SM, instruction fetch stalls grow with its size.
 // ---------------------------------------------------------------------------------------
@@ -933,120 +1030,146 @@ __device__ __noinline__ void fix_secondary_serial(Cell& c, const KParams& P, u32
 
 
 // ---------------------------------------------------------------------------------------
-// Warp-parallel steps (all 32 lanes, uniform control flow)
+// Block-parallel steps (the cell's worker threads, uniform control flow).  Each step takes the
+// stream position rp and returns the position after it; every step ends with a wsync after which
+// the state it wrote is visible to all workers.
 // ---------------------------------------------------------------------------------------
 
-// ExtrusionBarriers::init_states (extrusion_barriers.cpp:220-231)
-__device__ void barriers_init(Cell& c, u64* s) {
-  for (u32 base = 0; base < c.nb; base += 32) {
-    rng_ensure(c, s, 32);
-    const u32 i = base + ln();
-    const bool need = i < c.nb && (bar_flags(c, i) & BF_OCC_DRAWS);
-    const unsigned m = __ballot_sync(FULL, need);
-    const u32 off = __popc(m & lanemask_lt());
-    bool occ = false;
-    if (need) occ = ring_at(c, c.sc->rpos + off) <= c.bar[i].t_occ;
-    const unsigned om = __ballot_sync(FULL, occ);
-    __syncwarp();
-    if (ln() == 0) {
-      c.bst[base >> 5] = om;
-      c.sc->rpos += __popc(m);
-    }
-    __syncwarp();
+// Exclusive counts of two flags per thread over the window's items in order (item h of thread t is
+// item h * T + t): where this thread's flags fall, and how many there are.  One wsync; successive
+// calls alternate buf.
+struct Scan2 {
+  u32 off0, off1, total;
+};
+__device__ __forceinline__ Scan2 scan2(Cell& c, u32 buf, bool f0, bool f1) {
+  const unsigned m0 = __ballot_sync(FULL, f0), m1 = __ballot_sync(FULL, f1);
+  const u32 w = threadIdx.x >> 5, l = ln();
+  u32* cnt = c.bt->cnt[buf];
+  if (l == 0) {
+    cnt[w] = __popc(m0);
+    cnt[16 + w] = __popc(m1);
   }
+  wsync(c);
+  const u32 v = (l & 15u) < (c.T >> 5) ? cnt[l] : 0u;
+  const u32 before = (l & 15u) < w ? v : 0u;
+  const u32 b0 = __reduce_add_sync(FULL, l < 16 ? before : 0u);
+  const u32 b1 = __reduce_add_sync(FULL, l < 16 ? v : before);
+  Scan2 r;
+  r.total = __reduce_add_sync(FULL, v);
+  r.off0 = b0 + __popc(m0 & lanemask_lt());
+  r.off1 = b1 + __popc(m1 & lanemask_lt());
+  return r;
+}
+
+// ExtrusionBarriers::init_states (extrusion_barriers.cpp:220-231)
+__device__ __noinline__ u64 barriers_init(Cell& c, u64 rp) {
+  const u32 T = c.T;
+  u32 buf = 0;
+  for (u32 base = 0; base < c.nb; base += T) {
+    const u32 i = base + threadIdx.x;
+    const bool need = i < c.nb && (bar_flags(c, i) & BF_OCC_DRAWS);
+    const Scan2 sc2 = scan2(c, buf, need, false);
+    rng_publish(c, rp);
+    buf ^= 1;
+    rng_ensure(c, rp, T);
+    const bool occ = need && ring_at(c, rp + sc2.off0) <= c.bar[i].t_occ;
+    const unsigned om = __ballot_sync(FULL, occ);
+    if (ln() == 0 && i < c.nb) c.bst[i >> 5] = om;
+    rp += sc2.total;
+  }
+  wsync(c);
+  rng_publish(c, rp);
+  return rp;
 }
 
 // ExtrusionBarriers::next_state (extrusion_barriers.cpp:145-161): one draw per barrier.
-__device__ void barriers_next(Cell& c, u64* s) {
-  const u32 nwords = (c.nb + 31) / 32;
-  for (u32 base = 0; base < c.nb; base += 32 * MLP) {
-    rng_ensure(c, s, 32 * MLP);
-    const u64 r0 = c.sc->rpos;
-    u32 word[MLP], f[MLP];
-    u64 thr[MLP], u[MLP];
-    bool st[MLP], valid[MLP];
+__device__ __noinline__ u64 barriers_next(Cell& c, u64 rp) {
+  const u32 T = c.T, nb = c.nb;
+  const uint2* __restrict__ bpf = c.bpf;
+  const DevBarrier* __restrict__ bar = c.bar;
+  for (u32 base = 0; base < nb; base += 2 * T) {
+    rng_ensure(c, rp, 2 * T);
+    u32 f[2];
+    u64 thr[2];
+    bool st[2];
 #pragma unroll
-    for (u32 h = 0; h < MLP; ++h) {
-      const u32 i = base + 32 * h + ln();
-      valid[h] = i < c.nb;
-      const u32 w = (base >> 5) + h;
-      word[h] = w < nwords ? c.bst[w] : 0u;
-      st[h] = (word[h] >> ln()) & 1u;
-      const u32 ic = valid[h] ? i : 0u;
-      f[h] = bar_flags(c, ic);
-      thr[h] = st[h] ? c.bar[ic].t_act : c.bar[ic].t_ina;
-      u[h] = ring_at(c, r0 + 32 * h + ln());
-    }
-    unsigned nm[MLP];
-#pragma unroll
-    for (u32 h = 0; h < MLP; ++h) {
-      bool nst = st[h];
-      if (valid[h]) {
-        if (!st[h]) {
-          nst = !(f[h] & BF_INA_NEVER) && u[h] >= thr[h];
-        } else {
-          nst = !(!(f[h] & BF_ACT_NEVER) && u[h] >= thr[h]);
-        }
-      }
-      nm[h] = __ballot_sync(FULL, valid[h] && nst);
+    for (u32 h = 0; h < 2; ++h) {
+      const u32 i = base + h * T + threadIdx.x, ic = i < nb ? i : 0u;
+      st[h] = i < nb && ((c.bst[i >> 5] >> ln()) & 1u);
+      f[h] = __ldg(&bpf[ic].y);
+      thr[h] = st[h] ? __ldg(&bar[ic].t_act) : __ldg(&bar[ic].t_ina);
     }
     __syncwarp();
-    if (ln() == 0) {
 #pragma unroll
-      for (u32 h = 0; h < MLP; ++h)
-        if ((base >> 5) + h < nwords) c.bst[(base >> 5) + h] = nm[h];
-      c.sc->rpos = r0 + min(32u * MLP, c.nb - base);
+    for (u32 h = 0; h < 2; ++h) {
+      const u32 k = h * T + threadIdx.x, i = base + k;
+      const bool above = ring_at(c, rp + k) >= thr[h];
+      const bool nst = st[h] ? !(!(f[h] & BF_ACT_NEVER) && above) : !(f[h] & BF_INA_NEVER) && above;
+      const unsigned m = __ballot_sync(FULL, i < nb && nst);
+      if (ln() == 0 && i < nb) c.bst[i >> 5] = m;
     }
-    __syncwarp();
+    rp += min(2 * T, nb - base);
+    wsync(c);
+    rng_publish(c, rp);
   }
+  return rp;
 }
 
 // select_lefs_to_bind + bind_lefs (simulation_impl.hpp:28-89): one uniform_int draw per
 // selected LEF in index order.  Selection: mode 0 = unbound LEFs (the epoch loop), 1 =
-// nonzero entries of mask, 2 = every LEF (an empty mask in the reference).
-__device__ __forceinline__ bool bind_selected(const Cell& c, u32 i, int mode, const u64* mask) {
-  return mode == 0 ? c.bep[i] == UNBOUND : (mode == 1 ? mask[i] != 0 : true);
-}
-
-__device__ void bind_lefs(Cell& c, u64* s, const KParams& P, u32 n, u32 epoch, int mode,
-                          const u64* mask) {
-  for (u32 i0 = 0; i0 < n; i0 += 32) {
-    rng_ensure(c, s, 32);
-    const u32 i = i0 + ln();
-    const bool need = i < n && bind_selected(c, i, mode, mask);
-    const unsigned m = __ballot_sync(FULL, need);
-    const u32 off = __popc(m & lanemask_lt());
+// nonzero entries of mask, 2 = every LEF (an empty mask in the reference).  The selected LEFs are
+// compacted first: they are a few per cent of all, and each takes a 64-bit division.
+__device__ __noinline__ u64 bind_lefs(Cell& c, const KParams& P, u64 rp, u32 n, u32 epoch, int mode,
+                                      const u64* mask) {
+  const u32 T = c.T;
+  u32* list = c.tmp;
+  u32 nsel = 0, buf = 0;
+  for (u32 base = 0; base < n; base += 2 * T) {
+    const u32 i0 = base + threadIdx.x, i1 = i0 + T;
+    const bool f0 = i0 < n && (mode == 0 ? c.bep[i0] == UNBOUND : (mode == 1 ? mask[i0] != 0 : true));
+    const bool f1 = i1 < n && (mode == 0 ? c.bep[i1] == UNBOUND : (mode == 1 ? mask[i1] != 0 : true));
+    const Scan2 s = scan2(c, buf, f0, f1);
+    buf ^= 1;
+    if (f0) list[nsel + s.off0] = i0;
+    if (f1) list[nsel + s.off1] = i1;
+    nsel += s.total;
+  }
+  wsync(c);
+  for (u32 q = 0; q < nsel; q += T) {
+    const u32 cnt = min(T, nsel - q);
+    rng_ensure(c, rp, cnt);
+    const bool mine = threadIdx.x < cnt;
     u64 r = 0;
     bool ok = true;
-    if (need) {
-      r = ring_at(c, c.sc->rpos + off) / P.pos_bucket;
+    if (mine) {
+      r = ring_at(c, rp + threadIdx.x) / P.pos_bucket;
       ok = r <= P.pos_range;
     }
-    const unsigned bad = __ballot_sync(FULL, need && !ok);
-    const u32 f = bad ? (u32)(__ffs(bad) - 1) : 32u;
-    if (need && ln() < f) {
-      const u32 pos = (u32)(P.wstart + r);
+    if (wsync_or(c, !ok)) {
+      // a bucket rejection: the rest one by one with the exact number of draws
+      if (threadIdx.x == 0) {
+        for (u32 j = q; j < nsel; ++j) {
+          const u64 pos = s_uniform_int(c, P.wstart, (u64)P.wend - 1);
+          c.rev[list[j]] = (u32)pos;
+          c.fwd[list[j]] = (u32)pos;
+          c.bep[list[j]] = epoch;
+        }
+      }
+      wsync(c);
+      return c.sc->rpos;
+    }
+    rp += cnt;
+    rng_publish(c, rp);
+    if (mine) {
+      const u32 i = list[q + threadIdx.x], pos = (u32)(P.wstart + r);
       c.rev[i] = pos;
       c.fwd[i] = pos;
       c.bep[i] = epoch;
     }
-    __syncwarp();
-    if (ln() == 0) {
-      c.sc->rpos += __popc(m & (f == 32 ? FULL : ((1u << f) - 1)));
-      if (f < 32) {  // finish this chunk serially from the rejecting LEF
-        for (u32 k = i0 + f; k < min(i0 + 32, n); ++k) {
-          if (!bind_selected(c, k, mode, mask)) continue;
-          const u64 pos = s_uniform_int(c, P.wstart, (u64)P.wend - 1);
-          c.rev[k] = (u32)pos;
-          c.fwd[k] = (u32)pos;
-          c.bep[k] = epoch;
-        }
-      }
-    }
-    __syncwarp();
   }
+  wsync(c);
+  return rp;
 }
-
 // Ranking key of a unit: position, then binding epoch ascending (rev) or descending (fwd).
 __device__ __forceinline__ u64 rank_key(const Cell& c, u32 dir, u32 idx) {
   const u32 p = dir ? c.fwd[idx] : c.rev[idx];
@@ -1131,7 +1254,7 @@ __device__ __noinline__ u32 tie_fix_run(const Cell& c, u32 dir, u32* a, u32 t, u
 // rm, fm and sf.  The move arrays are dead from binding until the moves are generated (the
 // callers that keep them restore them), and every event removes one input element, so n
 // entries per list always suffice.
-__device__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
+__device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
   if (n < 2 || n > 0xFFFFu) return false;
   u32* R = dir ? c.fr : c.rr;
   const u32* pos = dir ? c.fwd : c.rev;
@@ -1344,24 +1467,239 @@ __device__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
   return true;
 }
 
-__device__ void rank_lefs(Cell& c, const KParams& P, u32 n, u32 epoch, bool partially_sorted) {
+__device__ __forceinline__ u64 max64(u64 a, u64 b) { return a > b ? a : b; }
+
+// rank_lefs for one direction with the previous order reused, by all workers.
+//
+// Unless two units share position and binding epoch (a full tie), the reference's order (split_sort,
+// then the tie fix) is simply the order by that key, whatever the way it is sorted.  So the units are
+// split into those that still form a non-decreasing sequence and the few that do not: the units bound
+// this epoch and every other one below the running maximum of the rest.  The few are sorted by key
+// (runs of 32 in registers, then each finds its place in the other runs by binary search) and merged
+// back by rank.  Returns false with R untouched when a full tie turns up or when too many units moved:
+// the caller then takes rank_dir_split, the exact restatement.
+//
+// Phases, each ended by a wsync; warp w owns a contiguous range of the ranks:
+//  1 keys in rank order to rm / fm, and their maximum per warp;
+//  2 running maximum; the removed units' keys to the 64-bit array in sr / sf, with index and
+//    rank packed in tmp; a bit mask of the kept ranks at the end of sf;
+//  3 runs of 32 removed units sorted in registers;
+//  4 each removed unit's place among the removed (pairwise searches) and among the kept;
+//  5 the new order, written to rm; 6 copied to R.
+__device__ __noinline__ bool rank_dir_block(Cell& c, u32 dir, u32 n, u32 epoch) {
+  if (n < 2 || n > 0xFFFFu) return false;
+  const u32 T = c.T, W = T >> 5, w = threadIdx.x >> 5, lane = ln();
+  u32* R = dir ? c.fr : c.rr;
+  const u32* pos = dir ? c.fwd : c.rev;
+  const u32* bep = c.bep;
+  u32* kh = c.rm;
+  u32* kl = c.fm;
+  u64* bk = reinterpret_cast<u64*>(c.sr);
+  const u32 nch = (n + 31) >> 5;
+  u32* kmask = c.sf + (n - nch);
+  const u32 maxb = n / 3;
+  u32 *bp = c.tmp, *sr0 = c.tmp + maxb, *sfin = c.tmp + 2 * maxb;
+  BlockTmp* bt = c.bt;
+  const u32 ch0 = w * nch / W, ch1 = (w + 1) * nch / W;
+  const u32 newlo = dir ? ~epoch : epoch;
+  u64 mx = 0;
+  for (u32 ch = ch0; ch < ch1; ++ch) {
+    const u32 r = ch * 32 + lane;
+    if (r < n) {
+      const u32 idx = R[r];
+      const u32 p = pos[idx], e = bep[idx], lo = dir ? ~e : e;
+      kh[r] = p;
+      kl[r] = lo;
+      if (lo != newlo) mx = max64(mx, ((u64)p << 32) | lo);
+    }
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) mx = max64(mx, __shfl_xor_sync(FULL, mx, d));
+  if (lane == 0) bt->wmax[w] = mx;
+  if (threadIdx.x == 0) {
+    bt->nrem = 0;
+    bt->tie = 0;
+    bt->tie2 = 0;
+  }
+  wsync(c);
+  u64 carry = lane < w ? bt->wmax[lane] : 0;
+#pragma unroll
+  for (int d = 8; d > 0; d >>= 1) carry = max64(carry, __shfl_xor_sync(FULL, carry, d));
+  carry = __shfl_sync(FULL, carry, 0);
+  bool tie = false;
+  u32 removed = 0;
+  for (u32 ch = ch0; ch < ch1; ++ch) {
+    const u32 r = ch * 32 + lane;
+    const bool valid = r < n;
+    const u32 hi = valid ? kh[r] : 0u, lo = valid ? kl[r] : 0u;
+    const u64 key = ((u64)hi << 32) | lo;
+    const bool old = valid && lo != newlo;
+    u64 x = old ? key : 0;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const u64 y = __shfl_up_sync(FULL, x, d);
+      if ((int)lane >= d) x = max64(x, y);
+    }
+    u64 excl = __shfl_up_sync(FULL, x, 1);
+    excl = lane == 0 ? carry : max64(excl, carry);
+    const bool keep = old && key >= excl;
+    tie |= keep && key == excl;
+    const bool rem = valid && !keep;
+    const unsigned km = __ballot_sync(FULL, keep), rmk = __ballot_sync(FULL, rem);
+    if (lane == 0) kmask[ch] = km;
+    if (rmk) {
+      u32 q = 0;
+      if (lane == 0) q = atomicAdd(&bt->nrem, (u32)__popc(rmk));
+      q = __shfl_sync(FULL, q, 0) + __popc(rmk & lanemask_lt());
+      if (rem) {
+        kh[r] = (u32)(excl >> 32);
+        kl[r] = (u32)excl;
+        if (q < maxb) {
+          bk[q] = key;
+          bp[q] = R[r] | (r << 16);
+        }
+      }
+      removed += __popc(rmk);
+    }
+    carry = max64(carry, __shfl_sync(FULL, x, 31));
+  }
+  if (lane == 0) bt->rem[w] = removed;
+  if (tie) bt->tie = 1;
+  wsync(c);
+  const u32 m = bt->nrem;
+  if (m > maxb || bt->tie) return false;
+  // 3: runs of 32
+  if (w == W - 1) {  // removed units before each warp's range
+    u32 v = lane < W ? bt->rem[lane] : 0u;
+    const u32 ex = warp_excl_scan(v, nullptr);
+    if (lane < W) bt->rembase[lane] = ex;
+  }
+  for (u32 run = w; run * 32 < m; run += W) {
+    const u32 q = run * 32 + lane;
+    u64 key = q < m ? bk[q] : ~0ull;
+    u32 pl = q < m ? bp[q] : 0u;
+#pragma unroll
+    for (int k = 2; k <= 32; k <<= 1) {
+#pragma unroll
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        const u64 ok = __shfl_xor_sync(FULL, key, j);
+        const u32 op = __shfl_xor_sync(FULL, pl, j);
+        const bool up = (lane & k) == 0 || k == 32;
+        const bool lower = (lane & j) == 0;
+        const bool take = (lower == up) ? ok < key : ok > key;
+        if (take) {
+          key = ok;
+          pl = op;
+        }
+      }
+    }
+    const u64 prev = __shfl_up_sync(FULL, key, 1);
+    if (q < m) {
+      bk[q] = key;
+      bp[q] = pl;
+      if (lane > 0 && prev == key) bt->tie2 = 1;
+    }
+  }
+  wsync(c);
+  // 4: places
+  for (u32 q = threadIdx.x; q < m; q += T) {
+    const u64 key = bk[q];
+    const u32 my = q >> 5;
+    u32 rank = q & 31u;
+    for (u32 s0 = 0; s0 < m; s0 += 32) {
+      if ((s0 >> 5) == my) continue;
+      const u32 len = min(32u, m - s0);
+      u32 lo = 0, hi = len;
+      while (lo < hi) {
+        const u32 mid = (lo + hi) >> 1;
+        if (bk[s0 + mid] < key) lo = mid + 1; else hi = mid;
+      }
+      if (lo < len && bk[s0 + lo] == key) bt->tie2 = 1;
+      rank += lo;
+    }
+    const u32 khi = (u32)(key >> 32), klo = (u32)key;
+    u32 lo = 0, hi = n;  // first rank whose running maximum is >= key
+    while (lo < hi) {
+      const u32 mid = (lo + hi) >> 1;
+      const u32 h = kh[mid];
+      if (h < khi || (h == khi && kl[mid] < klo)) lo = mid + 1; else hi = mid;
+    }
+    u32 before = m;  // removed units at ranks below lo
+    if (lo < n) {
+      if (kh[lo] == khi && kl[lo] == klo) bt->tie2 = 1;
+      const u32 ch = lo >> 5, ow = ((ch + 1) * W - 1) / nch;
+      before = bt->rembase[ow];
+      for (u32 k = ow * nch / W; k < ch; ++k) before += 32 - __popc(kmask[k]);
+      before += (lo & 31u) - __popc(kmask[ch] & ((1u << (lo & 31u)) - 1u));
+    }
+    sr0[rank] = lo;
+    sfin[rank] = (bp[q] & 0xFFFFu) | ((rank + lo - before) << 16);
+  }
+  wsync(c);
+  if (bt->tie2) return false;
+  // 5: the new order
+  u32* O = c.rm;
+  for (u32 q = threadIdx.x; q < m; q += T) {
+    const u32 v = sfin[q];
+    O[v >> 16] = v & 0xFFFFu;
+  }
+  {
+    u32 j;  // removed units that go before this warp's range
+    {
+      const u32 r0 = ch0 * 32;
+      u32 lo = 0, hi = m;
+      while (lo < hi) {
+        const u32 mid = (lo + hi) >> 1;
+        if (sr0[mid] < r0) lo = mid + 1; else hi = mid;
+      }
+      j = lo;
+    }
+    u32 rb = bt->rembase[w];
+    for (u32 ch = ch0; ch < ch1; ++ch) {
+      const u32 r = ch * 32 + lane;
+      const u32 km = kmask[ch];
+      u32 ins = j;
+      for (; j < m; ++j) {
+        const u32 at = sr0[j];
+        if (at >= ch * 32 + 32) break;
+        ins += at <= r ? 1u : 0u;
+      }
+      if ((km >> lane) & 1u) O[r - rb - (lane - __popc(km & lanemask_lt())) + ins] = R[r];
+      rb += 32 - __popc(km);
+    }
+  }
+  wsync(c);
+  for (u32 r = threadIdx.x; r < n; r += T) R[r] = O[r];
+  wsync(c);
+  return true;
+}
+
+// Full ties, many moved units (a young cell binds most of its units in one epoch) or a small n:
+// one warp's exact emulation; the first epoch and unsorted callers: the serial restatement.
+__device__ __noinline__ void rank_lefs(Cell& c, const KParams& P, u32 n, u32 epoch, bool partially_sorted) {
+  const bool fast = partially_sorted && !(P.debug_flags & DBG_SERIAL_RANK) && n >= 2 && n <= 0xFFFFu;
   for (u32 dir = 0; dir < 2; ++dir) {
-    const bool ok = partially_sorted && !(P.debug_flags & DBG_SERIAL_RANK) && rank_dir_split(c, dir, n);
-    if (!ok) {
+    if (fast) {
+      if (rank_dir_block(c, dir, n, epoch)) continue;
+      const u64 t0 = clock64();
+      if (threadIdx.x < 32) rank_dir_split(c, dir, n);
+      wsync(c);
+      prof_add(c, PF_RANK_SPLIT, clock64() - t0);
+    } else {
       const u64 t0 = clock64();
       prof_add(c, PF_RANK_FALLBACK, 1);
-      if (ln() == 0) {
+      if (threadIdx.x == 0) {
         rank_dir_serial(c, dir, n, partially_sorted);
         c.sc->sort_fallbacks++;
       }
-      __syncwarp();
+      wsync(c);
       prof_add(c, PF_RANK_SERIAL, clock64() - t0);
     }
   }
 }
 
 // positions in rank order: sr[k] = rev[rr[k]], sf[k] = fwd[fr[k]]
-__device__ void gather_ranked(Cell& c, u32 n) {
+__device__ __noinline__ void gather_ranked(Cell& c, u32 n) {
   const u32* __restrict__ rr = c.rr;
   const u32* __restrict__ fr = c.fr;
   const u32* __restrict__ rev = c.rev;
@@ -1369,253 +1707,282 @@ __device__ void gather_ranked(Cell& c, u32 n) {
   u32* __restrict__ sr = c.sr;
   u32* __restrict__ sf = c.sf;
 #pragma unroll 4
-  for (u32 k = ln(); k < n; k += 32) {
+  for (u32 k = threadIdx.x; k < n; k += c.T) {
     sr[k] = rev[rr[k]];
     sf[k] = fwd[fr[k]];
   }
-  __syncwarp();
+  wsync(c);
+}
+
+// One draw of the moves' normal distribution and the move it gives: v = round(max(0, z * sd + mean)).
+// The reference evaluates this in doubles; here the ziggurat's comparison is an integer threshold on
+// the draw (zt[i].x) and the move is computed in 32.32 fixed point from the layer's width (zt[i].y =
+// x_i * 2^60) and sd * 2^36.  Both the doubles' rounding and the fixed point's are below 8 units of
+// 2^-32 for the parameters MoveSpec accepts, so the rounded move is the reference's unless the value
+// lies within 16 units of a half: then, for the tail layer, and where the wedge test is closer than
+// the single-precision estimate resolves, the draw is evaluated in doubles by unit_normal_t.
+// The FP64 pipe of sm_103a runs at 1/64 of the FP32 rate: with doubles alone the moves of a
+// 2,500-LEF cell kept it busy for about a third of the epoch.
+struct MoveSpec {
+  double mean, sd;
+  u64 sdq;    // sd * 2^36
+  i64 meanq;  // mean * 2^32
+  bool fixed; // fixed-point evaluation allowed
+};
+__device__ __forceinline__ MoveSpec move_spec(double mean, double sd) {
+  MoveSpec m{mean, sd, 0, 0, false};
+  // integer speeds below 2^19 with sd below 2^14: |z * sd + mean| < 2^20
+  m.fixed = mean >= 0.0 && mean < 524288.0 && sd < 16384.0 && mean == floor(mean);
+  if (m.fixed) {
+    m.sdq = (u64)(sd * 68719476736.0);
+    m.meanq = (i64)mean << 32;
+  }
+  return m;
+}
+
+__device__ __noinline__ int move_exact(RingSrc& g, const MoveSpec& ms, u32* v, bool* range) {
+  double z = 0.0;
+  const int st = unit_normal_t(g, z);
+  const double d = round(fmax(0.0, z * ms.sd + ms.mean));
+  *range = d > 4294967295.0;
+  *v = (u32)(u64)d;
+  return st;
+}
+
+__device__ __forceinline__ int move_sample(const ulonglong2* zt, RingSrc& g, const MoveSpec& ms, u32* v, bool* range) {
+  *range = false;
+  if (ms.fixed) {
+    for (int it = 0; it < 64; ++it) {
+      const RingSrc here = g;  // an attempt of the sampler carries nothing from the one before
+      u64 u;
+      if (!g.next(u)) return SMP_DRY;
+      const u32 ii = (u32)u & 0xFFu, i = ii >> 1;
+      const u64 m = (u & ~(1ull << 11)) >> 8;
+      const ulonglong2 e = zt[i];
+      const u64 t = __umul64hi(m << 8, e.y);  // x * 2^60
+      bool acc = m < e.x, exact = false;
+      if (!acc) {
+        u64 u2 = 0;
+        if (i == 0) {
+          exact = true;
+        } else if (!g.next(u2)) {
+          return SMP_DRY;
+        } else if (u2 >= ~0ull << 12) {
+          exact = true;  // uniform_01 may round to 1 and be drawn again
+        } else {
+          const float x = (float)t * 0x1p-60f;
+          const float ef = expf(-0.5f * x * x);
+          const float y0 = (float)mgpu_zig_normal_y[i], y1 = (float)mgpu_zig_normal_y[i + 1];
+          const float d = y0 + (float)u2 * 0x1p-64f * (y1 - y0) - ef;
+          exact = fabsf(d) <= 2e-5f * ef;
+          acc = d < 0.0f;
+        }
+      }
+      if (acc && !exact) {
+        const i64 wq = (i64)__umul64hi(t, ms.sdq);
+        const i64 q = (ii & 1u) ? ms.meanq + wq : ms.meanq - wq;
+        if (q <= -16) {
+          *v = 0;
+          return SMP_OK;
+        }
+        const u32 frac = (u32)q - 0x80000000u;
+        exact = frac + 16u <= 32u;
+        if (!exact) {
+          *v = (u32)((q + 0x80000000ll) >> 32);
+          return SMP_OK;
+        }
+      }
+      if (exact) {
+        g = here;
+        return move_exact(g, ms, v, range);
+      }
+    }
+  }
+  return move_exact(g, ms, v, range);
 }
 
 // generate_moves_helper (simulation.cpp:264-290) for one direction: move = round(max(0,
 // normal(mean, sd))) for every bound LEF in index order, unbound ones get 0.
 //
 // The normals are variable-length (a ziggurat wedge takes a second draw, the tail takes
-// exponentials), so the warp evaluates a window of 32 candidate starts at once: lane k runs the
-// whole sampler as if a normal started at stream position rpos + k.  The real starts form the
-// chain s0 = 0, s(j+1) = s(j) + len(s(j)); lane j finds s(j) by binary lifting over the
-// lanes' next-start pointers.  A window serves the normals whose start lies inside it (31 or
-// 32 of them in the common case), in stream order, to the next LEFs in index order.
-// Kept out of line: inlined into the epoch loop it shares the kernel's register allocation,
-// and the batched genome launch took 13 % longer that way.
-__device__ __noinline__ void gen_moves_dir(Cell& c, u64* s, u32* mv, u32 n, double mean, double sd, u64 move_int) {
+// exponentials), so the workers evaluate a window of T candidate starts at once: thread k runs the
+// whole sampler as if a normal started at stream position rp + k.  The real starts form the chain
+// s0 = 0, s(j+1) = s(j) + len(s(j)).  Each warp tabulates, for every lane it could be entered at, the
+// number of normals starting inside it and where the chain leaves it (pointer doubling over the lanes'
+// next-start pointers); after one wsync every warp follows the few table entries before its own and
+// marks its starts.  A window serves about T normals, in stream order, to the next LEFs in index order.
+__device__ __noinline__ u64 gen_moves_dir(Cell& c, u64 rp, u32* mv, u32 n, double mean, double sd, u64 move_int) {
+  const u32 T = c.T, W = T >> 5, w = threadIdx.x >> 5, lane = ln();
   if (sd == 0.0) {
-    for (u32 i = ln(); i < n; i += 32) mv[i] = c.bep[i] == UNBOUND ? 0u : (u32)move_int;
-    __syncwarp();
-    return;
+    for (u32 i = threadIdx.x; i < n; i += T) mv[i] = c.bep[i] == UNBOUND ? 0u : (u32)move_int;
+    wsync(c);
+    return rp;
   }
   // items: the bound LEFs in index order (a compacted list only when some are unbound)
-  u32 nb = 0;
-  for (u32 base = 0; base < n; base += 32) {
-    const u32 i = base + ln();
-    const bool need = i < n && c.bep[i] != UNBOUND;
-    const unsigned m = __ballot_sync(FULL, need);
-    if (i < n && !need) mv[i] = 0;
-    if (need) c.tmp[nb + __popc(m & lanemask_lt())] = i;
-    nb += __popc(m);
+  u32 nb = n;
+  bool unb = false;
+  for (u32 i = threadIdx.x; i < n; i += T) unb |= c.bep[i] == UNBOUND;
+  const bool all = !wsync_or(c, unb);
+  if (!all) {
+    nb = 0;
+    u32 buf = 0;
+    for (u32 base = 0; base < n; base += T) {
+      const u32 i = base + threadIdx.x;
+      const bool need = i < n && c.bep[i] != UNBOUND;
+      const Scan2 s = scan2(c, buf, need, false);
+      buf ^= 1;
+      if (i < n && !need) mv[i] = 0;
+      if (need) c.tmp[nb + s.off0] = i;
+      nb += s.total;
+    }
+    wsync(c);
   }
-  const bool all = nb == n;
-  __syncwarp();
+  const MoveSpec ms = move_spec(mean, sd);
+  BlockTmp* bt = c.bt;
+  const u32 DRY = 0x4000u;
   u32 t0 = 0;
   while (t0 < nb) {
-    rng_ensure(c, s, 96);
-    const u64 r0 = c.sc->rpos;
-    RingSrc g{c.ring, r0 + ln(), c.sc->gpos, 0};
-    double z = 0.0;
-    const int st = unit_normal_t(g, z);
+    rng_ensure(c, rp, T + 64);
+    RingSrc g{c.ring, c.rmask, (u32)rp + threadIdx.x, (u32)rp + T + 64, 0};
+    u32 v = 0;
+    bool range = false;
+    const int st = move_sample(bt->zt, g, ms, &v, &range);
     const u32 len = g.n;
-    // next-start pointers: 32 = beyond the window, 33 = unknown (the sampler ran dry)
-    u32 J[5];
-    J[0] = st == SMP_OK ? min(ln() + len, 32u) : 33u;
-#pragma unroll
-    for (int b = 1; b < 5; ++b) {
-      const u32 prev = J[b - 1];
-      const u32 v = __shfl_sync(FULL, prev, prev < 32 ? prev : 0);
-      J[b] = prev < 32 ? v : prev;
-    }
-    u32 p = 0;  // start of the ln()-th normal of the window
+    // next-start pointers relative to the warp's first lane; DRY + lane: this sampler ran dry
+    u32 J[5], ptr = st == SMP_OK ? lane + len : DRY + lane, cnt = st == SMP_OK ? 1u : 0u;
 #pragma unroll
     for (int b = 0; b < 5; ++b) {
-      const u32 v = __shfl_sync(FULL, J[b], p < 32 ? p : 0);
-      if (((ln() >> b) & 1) && p < 32) p = v;
-    }
-    // the ln()-th normal is usable when it starts inside the window and its sampler finished
-    const u32 jn = __shfl_sync(FULL, J[0], p < 32 ? p : 0);
-    const u32 m = __popc(__ballot_sync(FULL, p < 32 && jn != 33u));
-    const u32 served = min(m, nb - t0);
-    if (served == 0) {
-      // the first normal needs more draws than the ring holds: take it serially
-      if (ln() == 0) {
-        const double zz = s_unit_normal(c);
-        const double v = round(fmax(0.0, zz * sd + mean));
-        if (v > 4294967295.0) set_status(c, DEV_ERR_MOVE_RANGE);
-        mv[all ? t0 : c.tmp[t0]] = (u32)(u64)v;
+      J[b] = ptr;
+      const u32 p2 = __shfl_sync(FULL, ptr, ptr & 31u), c2 = __shfl_sync(FULL, cnt, ptr & 31u);
+      if (ptr < 32) {
+        cnt += c2;
+        ptr = p2;
       }
-      __syncwarp();
+    }
+    bt->tab[w][lane] = ptr | (cnt << 16);
+    wsync(c);
+    u32 e = 0, base = 0, my_e = 64, my_base = 0;
+    bool dry = false;
+    for (u32 k = 0; k < W; ++k) {
+      if (e >= 32) {
+        e -= 32;
+        continue;
+      }
+      if (k == w) {
+        my_e = e;
+        my_base = base;
+      }
+      const u32 t = bt->tab[k][e];
+      base += t >> 16;
+      const u32 p = t & 0xFFFFu;
+      if (p & DRY) {
+        dry = true;
+        e = k * 32 + (p & 31u);  // the window ends before the sampler that ran dry
+        break;
+      }
+      e = p - 32;
+    }
+    const u32 served = min(base, nb - t0);
+    u32 used = dry ? e : T + e;  // draws taken when every start of the window is served
+    if (my_e < 32) {
+      u32 vis = 1u << my_e;
+#pragma unroll
+      for (int b = 0; b < 5; ++b)
+        vis |= __reduce_or_sync(FULL, ((vis >> lane) & 1u) && J[b] < 32 ? 1u << J[b] : 0u);
+      const u32 ord = my_base + __popc(vis & lanemask_lt());
+      if (((vis >> lane) & 1u) && st == SMP_OK && ord < served) {
+        if (range) set_status(c, DEV_ERR_MOVE_RANGE);
+        mv[all ? t0 + ord : c.tmp[t0 + ord]] = v;
+        if (ord == served - 1) bt->used = threadIdx.x + len;
+      }
+    }
+    wsync(c);
+    if (served == 0) {
+      // the first normal needs more draws than the window holds: take it serially
+      if (threadIdx.x == 0) {
+        c.sc->rpos = rp;
+        const double zz = s_unit_normal(c);
+        const double d = round(fmax(0.0, zz * sd + mean));
+        if (d > 4294967295.0) set_status(c, DEV_ERR_MOVE_RANGE);
+        mv[all ? t0 : c.tmp[t0]] = (u32)(u64)d;
+      }
+      wsync(c);
+      rp = c.sc->rpos;
       ++t0;
       continue;
     }
-    const double zj = __shfl_sync(FULL, z, p < 32 ? p : 0);
-    if (ln() < served) {
-      const double v = round(fmax(0.0, zj * sd + mean));
-      if (v > 4294967295.0) set_status(c, DEV_ERR_MOVE_RANGE);
-      mv[all ? t0 + ln() : c.tmp[t0 + ln()]] = (u32)(u64)v;
-    }
-    const u32 plast = __shfl_sync(FULL, p, served - 1);
-    const u32 llast = __shfl_sync(FULL, len, plast);
-    __syncwarp();
-    if (ln() == 0) c.sc->rpos = r0 + plast + llast;
-    __syncwarp();
+    if (served < base) used = bt->used;
+    rp += used;
+    rng_publish(c, rp);
     t0 += served;
   }
+  wsync(c);
+  return rp;
 }
 
-// adjust_moves_of_consecutive_extr_units, rev units: pairs (k, k+1) from the top rank down.
-// With t_k = pos_k - move_k the reference computes T_k = min(t_k, T_{k+1} - 1) when the pair
-// links (both bound, t_k > start, T_{k+1} > start), else T_k = t_k.  In U_k = T_k - k this is
-// a segmented suffix minimum.  The scan takes the static part of the link condition; the
-// dynamic part (T_{k+1} > start) is checked afterwards and a failure anywhere rejects the
-// result (serial fallback).  New moves go to tmp first and are copied only on success.
-__device__ bool adjust_rev_fast(Cell& c, const KParams& P, u32 n) {
-  const i64 start = P.start;
-  u32* out = c.tmp;
-  i64 carry_u = 0;       // U of element kb + 32
-  bool carry_b = false;  // bound flag of element kb + 32
-  bool bad = false;
-  {
-  // the chunk below is loaded while this one is scanned (the scan writes only tmp)
-  const u32* __restrict__ rr = c.rr;
-  const u32* __restrict__ sr = c.sr;
+// adjust_moves_of_consecutive_extr_units (simulation.cpp:343-399), one direction.
+// rev: with t_k = pos_k - move_k the reference goes down the ranks and sets T_k = min(t_k, T_{k+1} - 1)
+// when the pair links (both bound, t_k > start, T_{k+1} > start), else T_k = t_k.  Every unit whose lower
+// neighbour it pushes starts a walk down the ranks that carries its target, one less per rank, until a
+// unit is clear of it; the walks meet in an atomic maximum of the moves, so each unit ends with the
+// smallest target that reaches it.  Pushed units are few and their walks short, so almost all threads
+// only compare two neighbours.  fwd units mirror this upwards.  A linked pair whose pushing target lies
+// beyond the chromosome end is skipped by the reference: that rejects the result (serial restatement).
+__device__ __noinline__ bool adjust_dir_block(Cell& c, const KParams& P, u32 dir, u32 n) {
+  const u32* __restrict__ R = dir ? c.fr : c.rr;
+  const u32* __restrict__ S = dir ? c.sf : c.sr;
   const u32* __restrict__ bep = c.bep;
-  const u32* __restrict__ rm = c.rm;
-  i64 kb = ((i64)n - 1) / 32 * 32;
-  u32 idx_n = 0, sp_n = 0, be_n = UNBOUND, m_n = 0;
-  {
-    const i64 k = kb + ln();
-    const bool valid = k < (i64)n;
-    idx_n = valid ? rr[k] : 0u;
-    sp_n = valid ? sr[k] : 0u;
-    be_n = valid ? bep[idx_n] : UNBOUND;
-    m_n = valid ? rm[idx_n] : 0u;
-  }
-  for (; kb >= 0; kb -= 32) {
-    const i64 k = kb + ln();
-    const bool valid = k < (i64)n;
-    const bool b = valid && be_n != UNBOUND;
-    const i64 p = valid ? (i64)sp_n : 0;
-    const i64 t = valid ? p - (i64)m_n : 0;
-    if (kb >= 32) {
-      const i64 k2 = kb - 32 + ln();
-      idx_n = rr[k2];
-      sp_n = sr[k2];
-      be_n = bep[idx_n];
-      m_n = rm[idx_n];
-    }
-    bool b_next = __shfl_down_sync(FULL, b, 1);
-    if (ln() == 31) b_next = carry_b;
-    const bool link_next = valid && k + 1 < (i64)n && b && b_next && t > start;
-    i64 v = t - k;
-    bool stop = !link_next;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const i64 vr = __shfl_down_sync(FULL, v, d);
-      const bool sr_ = __shfl_down_sync(FULL, stop, d);
-      if ((int)ln() + d < 32 && !stop) {
-        v = min(v, vr);
-        stop = sr_;
-      }
-    }
-    if (valid && !stop) v = min(v, carry_u);  // linked through lane 31 to element kb + 32
-    const i64 T = v + k;
-    i64 T_next = __shfl_down_sync(FULL, T, 1);
-    if (ln() == 31) T_next = carry_u + kb + 32;
-    if (link_next && T_next <= start) bad = true;  // the reference would skip this pair
-    if (valid) out[k] = (u32)(p - T);
-    carry_u = __shfl_sync(FULL, v, 0);
-    carry_b = __shfl_sync(FULL, b, 0);
-  }
-  }
-  if (__any_sync(FULL, bad)) return false;
-  __syncwarp();
-#pragma unroll 4
-  for (u32 k = ln(); k < n; k += 32) c.rm[c.rr[k]] = out[k];
-  __syncwarp();
-  return true;
-}
-
-// fwd units: pairs (k-1, k) from the bottom rank up; T_k = max(t_k, T_{k-1} + 1) when linked
-// (both bound, t_k <= end - 1, T_{k-1} <= end - 1); V_k = T_k - k is a segmented prefix max.
-__device__ bool adjust_fwd_fast(Cell& c, const KParams& P, u32 n) {
-  const i64 endm1 = (i64)P.end - 1;
+  u32* M = dir ? c.fm : c.rm;
   u32* out = c.tmp;
-  i64 carry_v = 0;       // V of element kb - 1
-  bool carry_b = false;  // bound flag of element kb - 1
-  bool bad = false;
-  {
-  // the next chunk is loaded while this one is scanned (the scan writes only tmp)
-  const u32* __restrict__ fr = c.fr;
-  const u32* __restrict__ sf = c.sf;
-  const u32* __restrict__ bep = c.bep;
-  const u32* __restrict__ fm = c.fm;
-  u32 idx_n = 0, sp_n = 0, be_n = UNBOUND, m_n = 0;
-  if (ln() < n) {
-    idx_n = fr[ln()];
-    sp_n = sf[ln()];
-    be_n = bep[idx_n];
-    m_n = fm[idx_n];
-  }
-  for (u32 kb = 0; kb < n; kb += 32) {
-    const i64 k = (i64)kb + ln();
-    const bool valid = k < (i64)n;
-    const bool b = valid && be_n != UNBOUND;
-    const i64 p = valid ? (i64)sp_n : 0;
-    const i64 t = valid ? p + (i64)m_n : 0;
-    {
-      const u32 k2 = kb + 32 + ln();
-      if (k2 < n) {
-        idx_n = fr[k2];
-        sp_n = sf[k2];
-        be_n = bep[idx_n];
-        m_n = fm[idx_n];
-      }
-    }
-    bool b_prev = __shfl_up_sync(FULL, b, 1);
-    if (ln() == 0) b_prev = carry_b;
-    const bool link_prev = valid && k > 0 && b && b_prev && t <= endm1;
-    i64 v = t - k;
-    bool stop = !link_prev;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const i64 vl = __shfl_up_sync(FULL, v, d);
-      const bool sl = __shfl_up_sync(FULL, stop, d);
-      if ((int)ln() >= d && !stop) {
-        v = max(v, vl);
-        stop = sl;
-      }
-    }
-    if (valid && !stop) v = max(v, carry_v);  // linked through lane 0 to element kb - 1
-    const i64 T = v + k;
-    i64 T_prev = __shfl_up_sync(FULL, T, 1);
-    if (ln() == 0) T_prev = carry_v + (i64)kb - 1;
-    if (link_prev && T_prev > endm1) bad = true;
-    if (valid) out[k] = (u32)(T - p);
-    carry_v = __shfl_sync(FULL, v, 31);
-    carry_b = __shfl_sync(FULL, b, 31);
-  }
-  }
-  if (__any_sync(FULL, bad)) return false;
-  __syncwarp();
+  const i64 lim = dir ? (i64)P.end - 1 : (i64)P.start;
 #pragma unroll 4
-  for (u32 k = ln(); k < n; k += 32) c.fm[c.fr[k]] = out[k];
-  __syncwarp();
+  for (u32 k = threadIdx.x; k < n; k += c.T) out[k] = M[R[k]];
+  wsync(c);
+  bool bad = false;
+  for (u32 k = threadIdx.x; k < n; k += c.T) {
+    // source k, pushed unit i = k - 1 (rev) or k + 1 (fwd)
+    if (dir ? k + 1 >= n : k == 0) continue;
+    const u32 src = R[k];
+    if (bep[src] == UNBOUND) continue;
+    i64 T = dir ? (i64)pos64(S[k]) + M[src] : (i64)pos64(S[k]) - M[src];
+    u32 i = dir ? k + 1 : k - 1;
+    for (;;) {
+      const u32 u = R[i];
+      if (bep[u] == UNBOUND) break;
+      const i64 p = (i64)pos64(S[i]);
+      const i64 t = dir ? p + M[u] : p - M[u];
+      if (dir ? t > lim : t <= lim) break;
+      if (dir ? T > lim : T <= lim) {
+        bad = true;
+        break;
+      }
+      if (dir ? T < t : T > t) break;
+      T += dir ? 1 : -1;
+      atomicMax(&out[i], (u32)(dir ? T - p : p - T));
+      if (dir ? i + 1 >= n : i == 0) break;
+      i += dir ? 1u : ~0u;
+    }
+  }
+  if (wsync_or(c, bad)) return false;
+#pragma unroll 4
+  for (u32 k = threadIdx.x; k < n; k += c.T) M[R[k]] = out[k];
+  wsync(c);
   return true;
 }
 
 __device__ void adjust_moves(Cell& c, const KParams& P, u32 n) {
   const bool serial = P.debug_flags & DBG_SERIAL_ADJUST;
-  if (serial || !adjust_rev_fast(c, P, n)) {
-    prof_add(c, PF_ADJUST_FALLBACK, 1);
-    if (ln() == 0) adjust_dir_serial(c, P, 0, n);
-    __syncwarp();
-  }
-  if (serial || !adjust_fwd_fast(c, P, n)) {
-    prof_add(c, PF_ADJUST_FALLBACK, 1);
-    if (ln() == 0) adjust_dir_serial(c, P, 1, n);
-    __syncwarp();
+  for (u32 dir = 0; dir < 2; ++dir) {
+    if (serial || !adjust_dir_block(c, P, dir, n)) {
+      prof_add(c, PF_ADJUST_FALLBACK, 1);
+      if (threadIdx.x == 0) adjust_dir_serial(c, P, dir, n);
+      wsync(c);
+    }
   }
 }
 
 // clamp_moves (simulation.cpp:325-340)
-__device__ void clamp_moves(Cell& c, const KParams& P, u32 n) {
+__device__ __noinline__ void clamp_moves(Cell& c, const KParams& P, u32 n) {
   const u32* __restrict__ bep = c.bep;
   const u32* __restrict__ rev = c.rev;
   const u32* __restrict__ fwd = c.fwd;
@@ -1623,34 +1990,22 @@ __device__ void clamp_moves(Cell& c, const KParams& P, u32 n) {
   u32* __restrict__ fm = c.fm;
   const u64 start = P.start, end = P.end;
 #pragma unroll 4
-  for (u32 i = ln(); i < n; i += 32) {
+  for (u32 i = threadIdx.x; i < n; i += c.T) {
     if (bep[i] == UNBOUND) continue;
     const u64 rmv = min((u64)rm[i], pos64(rev[i]) - start);
     const u64 fmv = min((u64)fm[i], end - pos64(fwd[i]) - 1);
     rm[i] = (u32)rmv;
     fm[i] = (u32)fmv;
   }
-  __syncwarp();
+  wsync(c);
 }
 
 // ranked positions sorted (non-decreasing)?  Needed by the closed forms below; the epoch loop
 // always satisfies it, caller-provided ranks may not.
-__device__ bool ranked_sorted(const Cell& c, u32 n) {
+__device__ __noinline__ bool ranked_sorted(const Cell& c, u32 n) {
   bool bad = false;
-  u32 pr = 0, pf = 0;  // last values of the previous chunk
-  for (u32 base = 0; base < n; base += 32) {
-    const u32 k = base + ln();
-    const u32 r = k < n ? c.sr[k] : UNBOUND, f = k < n ? c.sf[k] : UNBOUND;
-    u32 r0 = __shfl_up_sync(FULL, r, 1), f0 = __shfl_up_sync(FULL, f, 1);
-    if (ln() == 0) {
-      r0 = pr;
-      f0 = pf;
-    }
-    if (k < n && k > 0 && (r0 > r || f0 > f)) bad = true;
-    pr = __shfl_sync(FULL, r, 31);
-    pf = __shfl_sync(FULL, f, 31);
-  }
-  return !__any_sync(FULL, bad);
+  for (u32 k = threadIdx.x + 1; k < n; k += c.T) bad |= c.sr[k - 1] > c.sr[k] || c.sf[k - 1] > c.sf[k];
+  return !wsync_or(c, bad);
 }
 
 // Bucket index over a sorted array of ranked positions (unbound units, UNBOUND, at the tail):
@@ -1661,7 +2016,16 @@ struct BucketIndex {
   const u32* key;
   const u32* T;
   u32 n, start, shift, nbk;
+  // first k in [0, n) with key[k] >= x
   __device__ u32 lower_bound(u32 x) const {
+    if (!T) {  // n too small for a table
+      u32 lo = 0, hi = n;
+      while (lo < hi) {
+        const u32 mid = (lo + hi) >> 1;
+        if (key[mid] >= x) hi = mid; else lo = mid + 1;
+      }
+      return lo;
+    }
     if (x <= start) return 0;
     u32 b = (x - start) >> shift;
     if (b > nbk) b = nbk;
@@ -1671,16 +2035,22 @@ struct BucketIndex {
   }
 };
 
-// Collective; T needs n entries.  Returns an index with T == nullptr (binary-search fallback)
-// when n is too small for a table.
-__device__ BucketIndex build_bucket_index(const u32* key, u32 n, u32 start, u32 end, u32* T) {
+// Collective; T needs n entries.
+__device__ __forceinline__ BucketIndex build_bucket_index(const Cell& c, const u32* key, u32 n, u32 start, u32 end,
+                                                          u32* T) {
   BucketIndex ix{key, nullptr, n, start, 0, 0};
   if (n < 8 || end <= start) return ix;
   const u32 range = end - start;
+  // smallest shift with (range >> shift) + 2 <= n
   u32 shift = 0;
-  while ((range >> shift) + 2 > n) ++shift;
+  {
+    const int d = __clz(n - 2) - __clz(range);
+    shift = d > 0 ? (u32)d : 0u;
+    if (shift && (range >> (shift - 1)) + 2 <= n) --shift;
+    while ((range >> shift) + 2 > n) ++shift;
+  }
   const u32 nbk = range >> shift;
-  for (u32 k = ln(); k <= n; k += 32) {
+  for (u32 k = threadIdx.x; k <= n; k += c.T) {
     u32 bmin = 0, bmax = nbk;
     if (k > 0) {
       const u32 lo = key[k - 1];
@@ -1692,25 +2062,14 @@ __device__ BucketIndex build_bucket_index(const u32* key, u32 n, u32 start, u32 
     }
     for (u32 b = bmin; b <= bmax; ++b) T[b] = k;
   }
-  __syncwarp();
+  wsync(c);
   ix.T = T;
   ix.shift = shift;
   ix.nbk = nbk;
   return ix;
 }
 
-// first k in [0, n) with key[k] >= x
-__device__ __forceinline__ u32 ranked_lower_bound(const BucketIndex& ix, u32 x) {
-  if (ix.T) return ix.lower_bound(x);
-  u32 lo = 0, hi = ix.n;
-  while (lo < hi) {
-    const u32 mid = (lo + hi) >> 1;
-    if (ix.key[mid] >= x) hi = mid; else lo = mid + 1;
-  }
-  return lo;
-}
-
-// Bernoulli trial of one lane with the draw at its offset (or none).
+// Bernoulli trial of one thread with the draw at its offset (or none).
 __device__ __forceinline__ bool trial_needs_draw(const Trial& t) { return !t.always && t.draws; }
 __device__ __forceinline__ bool trial_outcome(const Trial& t, u64 u) {
   if (t.always) return true;
@@ -1718,170 +2077,163 @@ __device__ __forceinline__ bool trial_outcome(const Trial& t, u64 u) {
   return u <= t.thr;
 }
 
-// ranked_lower_bound of MLP queries at once: the bucket loads and the scans of all queries are
-// issued together.
-__device__ __forceinline__ void ranked_lower_bounds(const BucketIndex& ix, const u32* x, u32* out) {
-  if (!ix.T) {
-#pragma unroll
-    for (u32 h = 0; h < MLP; ++h) out[h] = ranked_lower_bound(ix, x[h]);
-    return;
-  }
-#pragma unroll
-  for (u32 h = 0; h < MLP; ++h) {
-    const u32 b = x[h] <= ix.start ? 0u : min((x[h] - ix.start) >> ix.shift, ix.nbk);
-    out[h] = x[h] <= ix.start ? 0u : ix.T[b];
-  }
-  for (;;) {
-    bool more = false;
-#pragma unroll
-    for (u32 h = 0; h < MLP; ++h) {
-      const bool a = out[h] < ix.n && ix.key[out[h]] < x[h];
-      out[h] += a ? 1u : 0u;
-      more |= a;
-    }
-    if (!more) break;
-  }
-}
-
-// detect_lef_bar_collisions (simulation_detect_collisions.cpp:128-252), warp-parallel.  For
+// detect_lef_bar_collisions (simulation_detect_collisions.cpp:128-252) for one direction.  For
 // an occupied barrier the reference's sweep tests the first rev unit (in rank order, from
 // index max(n5 - 1, 0)) strictly downstream of it and the last fwd unit strictly upstream of
-// it (up to index n - max(n3 - 1, 0) - 1): binary searches over the ranked positions.
-// Trials draw in barrier order (ascending for rev units, descending for fwd units); a unit
-// hit by several barriers keeps the last successful one in that order.
-__device__ void detect_lef_bar_fast(Cell& c, u64* s, const KParams& P, u32 n, u64 n5, u64 n3) {
-  const u32* __restrict__ rr = c.rr;
-  const u32* __restrict__ fr = c.fr;
-  const u32* __restrict__ sr = c.sr;
-  const u32* __restrict__ sf = c.sf;
+// it (up to index n - max(n3 - 1, 0) - 1): searches over the ranked positions.  Trials draw in
+// barrier order (ascending for rev units, descending for fwd units), and a unit hit by several
+// barriers keeps the last successful one in that order: the largest barrier index for rev units,
+// the smallest for fwd units, which an atomic maximum on the unit's word resolves.  Until the
+// closing sweep of detect_lef_bar_block a hit is stored under an event code above every other
+// (EV_HIT), fwd units with the complemented index.
+constexpr u32 EV_HIT = EV_COLLISION | EV_CHROM_BOUNDARY | EV_LEF_BAR;
+
+__device__ __noinline__ u64 detect_lef_bar_dir(Cell& c, const KParams& P, u64 rp, u32 dir, u32 n, u64 n5, u64 n3) {
+  const u32 T = c.T;
+  const u32* __restrict__ R = dir ? c.fr : c.rr;
+  const u32* __restrict__ S = dir ? c.sf : c.sr;
   const u32* __restrict__ bep = c.bep;
-  const u32* __restrict__ rm = c.rm;
-  const u32* __restrict__ fm = c.fm;
-  for (u32 dir = 0; dir < 2; ++dir) {
-    // rev: first k >= j0 with sr[k] > bpos; fwd: last k <= jtop with sf[k] < bpos
-    const u32 j0 = (u32)min(n5, n5 - 1);
-    const u32 jtop = (u32)(n - min(n3, n3 - 1)) - 1;
-    const BucketIndex ix = build_bucket_index(dir ? sf : sr, n, (u32)P.start, (u32)P.end, c.tmp);
-    const u32 nchunks = (c.nb + 32 * MLP - 1) / (32 * MLP);
-    for (u32 ch = 0; ch < nchunks; ++ch) {
-      rng_ensure(c, s, 32 * MLP);
-      u32 bi[MLP], bpos[MLP], x[MLP], lo[MLP], k[MLP], unit[MLP], kpos[MLP], be[MLP], mv[MLP];
-      bool act[MLP];
-      int ti[MLP];
+  const u32* __restrict__ M = dir ? c.fm : c.rm;
+  u32* C = dir ? c.fc : c.rc;
+  // rev: first k >= j0 with S[k] > bpos; fwd: last k <= jtop with S[k] < bpos
+  const u32 j0 = (u32)min(n5, n5 - 1);
+  const u32 jtop = (u32)(n - min(n3, n3 - 1)) - 1;
+  const BucketIndex ix = build_bucket_index(c, S, n, (u32)P.start, (u32)P.end, c.tmp);
+  u32 buf = 0;
+  for (u32 base = 0; base < c.nb; base += 2 * T) {
+    rng_ensure(c, rp, 2 * T);
+    u32 bi[2], unit[2];
+    int ti[2];
+    bool cand[2], drawn[2];
 #pragma unroll
-      for (u32 h = 0; h < MLP; ++h) {
-        const i64 i = dir ? (i64)c.nb - 1 - (i64)(ch * 32 * MLP + 32 * h + ln()) : (i64)(ch * 32 * MLP + 32 * h + ln());
-        act[h] = i >= 0 && i < (i64)c.nb && bar_active(c, (u32)i);
-        bi[h] = act[h] ? (u32)i : 0u;
-        const uint2 pf = act[h] ? __ldg(&c.bpf[bi[h]]) : make_uint2(0u, 0u);
-        bpos[h] = pf.x;
-        const u32 bdir = pf.y & BF_DIR_MASK;
-        ti[h] = dir ? (bdir == MGPU_DIR_FWD ? 0 : 1) : (bdir == MGPU_DIR_REV ? 0 : 1);
-        x[h] = act[h] ? (dir ? pf.x : pf.x + 1) : 0u;
-      }
-      ranked_lower_bounds(ix, x, lo);
-#pragma unroll
-      for (u32 h = 0; h < MLP; ++h) {
-        bool ok;
-        if (dir == 0) {
-          lo[h] = max(j0, lo[h]);
-          ok = lo[h] < n;
-          k[h] = ok ? lo[h] : 0u;
-        } else {
-          lo[h] = min(jtop + 1, lo[h]);
-          ok = lo[h] > 0;
-          k[h] = ok ? lo[h] - 1 : 0u;
-        }
-        act[h] = act[h] && ok;
-        unit[h] = dir ? fr[k[h]] : rr[k[h]];
-        kpos[h] = dir ? sf[k[h]] : sr[k[h]];
-      }
-#pragma unroll
-      for (u32 h = 0; h < MLP; ++h) {
-        be[h] = bep[unit[h]];
-        mv[h] = dir ? fm[unit[h]] : rm[unit[h]];
-      }
-      u32 used = 0;
-#pragma unroll
-      for (u32 h = 0; h < MLP; ++h) {
-        bool cand = false, drawn = false;
-        if (act[h] && be[h] != UNBOUND) {
-          const u64 delta = dir ? (u64)bpos[h] - kpos[h] : (u64)kpos[h] - bpos[h];
-          if (delta > 0 && delta <= mv[h]) {
-            cand = true;
-            drawn = trial_needs_draw(P.lef_bar[ti[h]]);
+    for (u32 h = 0; h < 2; ++h) {
+      const u32 o = base + h * T + threadIdx.x;
+      cand[h] = drawn[h] = false;
+      bi[h] = unit[h] = 0;
+      ti[h] = 0;
+      if (o < c.nb) {
+        const u32 i = dir ? c.nb - 1 - o : o;
+        if (bar_active(c, i)) {
+          const uint2 pf = __ldg(&c.bpf[i]);
+          const u32 bdir = pf.y & BF_DIR_MASK;
+          u32 k = ix.lower_bound(dir ? pf.x : pf.x + 1);
+          bool ok;
+          if (dir == 0) {
+            k = max(j0, k);
+            ok = k < n;
+          } else {
+            k = min(jtop + 1, k);
+            ok = k > 0;
+            --k;
+          }
+          if (ok) {
+            const u32 u = R[k], kpos = S[k];
+            if (bep[u] != UNBOUND) {
+              const u64 delta = dir ? (u64)pf.x - kpos : (u64)kpos - pf.x;
+              if (delta > 0 && delta <= M[u]) {
+                cand[h] = true;
+                bi[h] = i;
+                unit[h] = u;
+                ti[h] = dir ? (bdir == MGPU_DIR_FWD ? 0 : 1) : (bdir == MGPU_DIR_REV ? 0 : 1);
+                drawn[h] = trial_needs_draw(P.lef_bar[ti[h]]);
+              }
+            }
           }
         }
-        const unsigned dm = __ballot_sync(FULL, drawn);
-        bool hit = false;
-        if (cand) {
-          const u64 u = drawn ? ring_at(c, c.sc->rpos + used + __popc(dm & lanemask_lt())) : 0;
-          hit = trial_outcome(P.lef_bar[ti[h]], u);
-        }
-        used += __popc(dm);
-        // within an item the highest lane is the last barrier in sweep order; later items
-        // overwrite earlier ones
-        const unsigned hm = __ballot_sync(FULL, hit);
-        const unsigned same = __match_any_sync(FULL, hit ? unit[h] : 0xFFFFFFFFu);
-        if (hit && (31 - __clz(same & hm)) == (int)ln()) {
-          const u32 w = cw_make(bi[h], EV_COLLISION | EV_LEF_BAR);
-          if (dir) c.fc[unit[h]] = w; else c.rc[unit[h]] = w;
-        }
-        __syncwarp();
       }
-      if (ln() == 0) c.sc->rpos += used;
-      __syncwarp();
     }
+    const Scan2 s = scan2(c, buf, drawn[0], drawn[1]);
+    rng_publish(c, rp);  // the draws of the windows before
+    buf ^= 1;
+#pragma unroll
+    for (u32 h = 0; h < 2; ++h) {
+      if (cand[h]) {
+        const u64 u = drawn[h] ? ring_at(c, rp + (h ? s.off1 : s.off0)) : 0;
+        if (trial_outcome(P.lef_bar[ti[h]], u))
+          atomicMax(&C[unit[h]], cw_make(dir ? CW_IDX_MASK - bi[h] : bi[h], EV_HIT));
+      }
+    }
+    rp += s.total;
   }
+  wsync(c);
+  rng_publish(c, rp);
+  return rp;
 }
 
-// detect_primary_lef_lef_collisions (simulation_detect_collisions.cpp:255-401), warp-parallel.
+__device__ __noinline__ u64 detect_lef_bar_block(Cell& c, const KParams& P, u64 rp, u32 n, u64 n5, u64 n3) {
+  rp = detect_lef_bar_dir(c, P, rp, 0, n, n5, n3);
+  rp = detect_lef_bar_dir(c, P, rp, 1, n, n5, n3);
+  for (u32 i = threadIdx.x; i < n; i += c.T) {
+    const u32 r = c.rc[i], f = c.fc[i];
+    if (cw_event(r) == EV_HIT) c.rc[i] = cw_make(cw_idx(r), EV_COLLISION | EV_LEF_BAR);
+    if (cw_event(f) == EV_HIT) c.fc[i] = cw_make(CW_IDX_MASK - cw_idx(f), EV_COLLISION | EV_LEF_BAR);
+  }
+  wsync(c);
+  return rp;
+}
+
+// No caller-provided collision word uses the sweep's own code (the epoch loop writes none).
+__device__ __noinline__ bool words_plain(const Cell& c, u32 n) {
+  bool bad = false;
+  for (u32 i = threadIdx.x; i < n; i += c.T) bad |= cw_event(c.rc[i]) == EV_HIT || cw_event(c.fc[i]) == EV_HIT;
+  return !wsync_or(c, bad);
+}
+
+// detect_primary_lef_lef_collisions (simulation_detect_collisions.cpp:255-401).
 // With cnt(j) = number of fwd units (rank < i2) strictly before rev unit j, the sweep tests
 // exactly the rev units j >= n5 with cnt(j) > cnt(j - 1) (cnt(n5 - 1) := 0) and cnt(j) < i2,
 // each against the fwd unit of rank cnt(j) - 1.  Tested pairs are disjoint, so their
 // collision words are updated independently; trials draw in ascending j.
-__device__ void detect_primary_fast(Cell& c, u64* s, const KParams& P, u32 n, u64 n5, u64 n3) {
-  if (n5 == n || n3 == n) return;
+__device__ __noinline__ u64 detect_primary_block(Cell& c, const KParams& P, u64 rp, u32 n, u64 n5, u64 n3) {
+  if (n5 == n || n3 == n) return rp;
+  const u32 T = c.T;
   const u32 i2 = (u32)(n - min(n3, n3 - 1));
   // bucket index over the fwd ranked positions (this step can also run on its own)
-  const BucketIndex ixf = build_bucket_index(c.sf, n, (u32)P.start, (u32)P.end, c.tmp);
-  u32 carry = 0;  // cnt of the element before the chunk
-  for (u32 base = (u32)n5; base < n; base += 32) {
-    rng_ensure(c, s, 32);
-    const u32 j = base + ln();
-    const bool valid = j < n;
-    u32 cnt = 0;
-    if (valid) cnt = min(i2, ranked_lower_bound(ixf, c.sr[j]));  // first i < i2 with sf[i] >= rp
-    u32 prev = __shfl_up_sync(FULL, cnt, 1);
-    if (ln() == 0) prev = carry;
-    const bool tested = valid && cnt > prev && cnt < i2;
-    u32 rev_idx = 0, fwd_idx = 0;
-    u64 rmv = 0, fmv = 0, rp = 0, fp = 0;
-    bool cand = false;
-    if (tested) {
-      rev_idx = c.rr[j];
-      fwd_idx = c.fr[cnt - 1];
-      rp = pos64(c.sr[j]);
-      fp = pos64(c.sf[cnt - 1]);
-      rmv = c.rm[rev_idx];
-      fmv = c.fm[fwd_idx];
-      const u64 delta = rp - fp;
-      cand = delta > 0 && delta < rmv + fmv;
+  const BucketIndex ixf = build_bucket_index(c, c.sf, n, (u32)P.start, (u32)P.end, c.tmp);
+  u32 buf = 0;
+  for (u32 base = (u32)n5; base < n; base += 2 * T) {
+    rng_ensure(c, rp, 2 * T);
+    u32 ru[2], fu[2], rp_[2], fp_[2], rmv[2], fmv[2];
+    bool cand[2], drawn[2];
+#pragma unroll
+    for (u32 h = 0; h < 2; ++h) {
+      const u32 j = base + h * T + threadIdx.x;
+      const bool valid = j < n;
+      u32 cnt = 0;
+      if (valid) cnt = min(i2, ixf.lower_bound(c.sr[j]));  // first i < i2 with sf[i] >= rev position
+      u32 prev = __shfl_up_sync(FULL, cnt, 1);
+      if (ln() == 0 && valid) prev = j == (u32)n5 ? 0u : min(i2, ixf.lower_bound(c.sr[j - 1]));
+      cand[h] = drawn[h] = false;
+      ru[h] = fu[h] = rp_[h] = fp_[h] = rmv[h] = fmv[h] = 0;
+      if (valid && cnt > prev && cnt < i2) {
+        ru[h] = c.rr[j];
+        fu[h] = c.fr[cnt - 1];
+        rp_[h] = c.sr[j];
+        fp_[h] = c.sf[cnt - 1];
+        rmv[h] = c.rm[ru[h]];
+        fmv[h] = c.fm[fu[h]];
+        const u64 delta = pos64(rp_[h]) - pos64(fp_[h]);
+        cand[h] = delta > 0 && delta < (u64)rmv[h] + fmv[h];
+        drawn[h] = cand[h] && trial_needs_draw(P.lef_lef);
+      }
     }
-    const bool drawn = cand && trial_needs_draw(P.lef_lef);
-    const unsigned dm = __ballot_sync(FULL, drawn);
-    bool hit = false;
-    if (cand) hit = trial_outcome(P.lef_lef, drawn ? ring_at(c, c.sc->rpos + __popc(dm & lanemask_lt())) : 0);
-    if (hit) primary_pair_update(c, rev_idx, fwd_idx, rp, fp, rmv, fmv);
-    carry = __shfl_sync(FULL, cnt, 31);
-    __syncwarp();
-    if (ln() == 0) c.sc->rpos += __popc(dm);
-    __syncwarp();
+    const Scan2 s = scan2(c, buf, drawn[0], drawn[1]);
+    rng_publish(c, rp);
+    buf ^= 1;
+#pragma unroll
+    for (u32 h = 0; h < 2; ++h) {
+      if (cand[h] && trial_outcome(P.lef_lef, drawn[h] ? ring_at(c, rp + (h ? s.off1 : s.off0)) : 0))
+        primary_pair_update(c, ru[h], fu[h], pos64(rp_[h]), pos64(fp_[h]), rmv[h], fmv[h]);
+    }
+    rp += s.total;
   }
+  wsync(c);
+  rng_publish(c, rp);
+  return rp;
 }
 
 // correct_moves_for_lef_bar_collisions (simulation_correct_moves.cpp:20-51)
-__device__ void correct_lef_bar(Cell& c, u32 n) {
+__device__ __noinline__ void correct_lef_bar(Cell& c, u32 n) {
   const u32* __restrict__ rc = c.rc;
   const u32* __restrict__ fc = c.fc;
   const u32* __restrict__ rev = c.rev;
@@ -1889,20 +2241,20 @@ __device__ void correct_lef_bar(Cell& c, u32 n) {
   u32* __restrict__ rm = c.rm;
   u32* __restrict__ fm = c.fm;
 #pragma unroll 4
-  for (u32 i = ln(); i < n; i += 32) {
+  for (u32 i = threadIdx.x; i < n; i += c.T) {
     const u32 r = rc[i], f = fc[i];
     if (cw_occurred_as(r, EV_LEF_BAR)) rm[i] = (u32)(pos64(rev[i]) - bar_pos(c, cw_idx(r)) - 1);
     if (cw_occurred_as(f, EV_LEF_BAR)) fm[i] = (u32)(bar_pos(c, cw_idx(f)) - pos64(fwd[i]) - 1);
   }
-  __syncwarp();
+  wsync(c);
 }
 
 // correct_moves_for_primary_lef_lef_collisions (simulation_correct_moves.cpp:54-122): the
-// pairs it visits are disjoint, so both passes are warp-parallel.
-__device__ void correct_primary(Cell& c, u32 n) {
+// pairs it visits are disjoint, so both passes are parallel.
+__device__ __noinline__ void correct_primary(Cell& c, u32 n) {
   // detect_primary pairs each fwd unit with at most one rev unit, so visiting the units in
   // index order instead of rank order changes nothing
-  for (u32 rev_idx = ln(); rev_idx < n; rev_idx += 32) {
+  for (u32 rev_idx = threadIdx.x; rev_idx < n; rev_idx += c.T) {
     const u32 r = c.rc[rev_idx];
     if (!cw_occurred_as(r, EV_PRIMARY)) continue;
     const u32 fwd_idx = cw_idx(r);
@@ -1917,8 +2269,8 @@ __device__ void correct_primary(Cell& c, u32 n) {
       c.rm[rev_idx] = (u32)(pos64(c.rev[rev_idx]) - (pos64(c.fwd[fwd_idx]) + c.fm[fwd_idx]) - 1);
     }
   }
-  __syncwarp();
-  for (u32 fwd_idx = ln(); fwd_idx < n; fwd_idx += 32) {
+  wsync(c);
+  for (u32 fwd_idx = threadIdx.x; fwd_idx < n; fwd_idx += c.T) {
     const u32 f = c.fc[fwd_idx];
     if (!cw_occurred_as(f, EV_PRIMARY)) continue;
     const u32 rev_idx = cw_idx(f);
@@ -1926,22 +2278,22 @@ __device__ void correct_primary(Cell& c, u32 n) {
       c.fm[fwd_idx] = (u32)((pos64(c.rev[rev_idx]) - c.rm[rev_idx]) - pos64(c.fwd[fwd_idx]) - 1);
     }
   }
-  __syncwarp();
+  wsync(c);
 }
 
-// process_secondary_lef_lef_collisions (simulation_detect_collisions.cpp:404-518), warp-parallel.
+// process_secondary_lef_lef_collisions (simulation_detect_collisions.cpp:404-518).
 // A stalled unit followed (rev: in rank order; fwd: in reverse rank order) by free units
 // starts a chain: each free unit whose target passes its stalled predecessor's target draws a
 // bypass trial; success stalls it one bp behind (extending the chain), failure marks it
 // avoided and ends the chain.  Chains lie between units that were stalled on entry, so they
-// are disjoint and one lane walks one chain.  Draw offsets assume every trial succeeds; the
-// first chain whose trial fails shifts the later ones, so the warp commits up to it and
-// resumes after it.  dir 0: rev units (chains ascend), dir 1: fwd units (chains descend).
+// are disjoint and one thread walks one chain.  A chain of at most one trial always takes the
+// same number of draws, so only a longer chain that fails before its last trial shifts the chains
+// after it: one warp settles the offsets of all chains of a round from those few, then every
+// chain is walked with its draws.
 enum ChainMode { CHAIN_COUNT = 0, CHAIN_RING = 1, CHAIN_SERIAL = 2 };
 
 template <int MODE>
-__device__ __forceinline__ u32 chain_walk(Cell& c, const KParams& P, u32 dir, u32 n, i64 k,
-                                          u64 off, u32* used_out) {
+__device__ __forceinline__ u32 chain_walk(Cell& c, const KParams& P, u32 dir, u32 n, i64 k, u64 at) {
   const Trial& tr = P.lef_lef;
   const u32* R = dir ? c.fr : c.rr;
   u32* M = dir ? c.fm : c.rm;
@@ -1951,7 +2303,7 @@ __device__ __forceinline__ u32 chain_walk(Cell& c, const KParams& P, u32 dir, u3
   const i64 stop = dir ? -1 : (i64)n;
   u32 idx_prev = R[k - step];
   u64 tprev = dir ? pos64(S[k - step]) + M[idx_prev] : pos64(S[k - step]) - M[idx_prev];
-  u32 used = 0, trials = 0;
+  u32 trials = 0;
   for (; k != stop; k += step) {
     const u32 idx = R[k];
     if (cw_occurred(C[idx])) break;  // stalled on entry: the next chain starts after it
@@ -1965,10 +2317,9 @@ __device__ __forceinline__ u32 chain_walk(Cell& c, const KParams& P, u32 dir, u3
       ok = false;
     } else {
       u64 u = 0;
-      if (MODE == CHAIN_RING) u = ring_at(c, c.sc->rpos + off + used);
+      if (MODE == CHAIN_RING) u = ring_at(c, at++);
       if (MODE == CHAIN_SERIAL) u = rng_serial(c);
       ok = MODE == CHAIN_COUNT || u <= tr.thr;
-      ++used;
     }
     ++trials;
     if (!ok) {
@@ -1984,180 +2335,182 @@ __device__ __forceinline__ u32 chain_walk(Cell& c, const KParams& P, u32 dir, u3
     tprev = dir ? p + m2 : p - m2;
     idx_prev = idx;
   }
-  *used_out = used;
   return trials;
 }
 
-__device__ void secondary_dir_fast(Cell& c, u64* s, const KParams& P, u32 dir, u32 n, u64 n5, u64 n3) {
+__device__ __noinline__ u64 secondary_dir_block(Cell& c, const KParams& P, u64 rp, u32 dir, u32 n, u64 n5, u64 n3) {
+  const u32 T = c.T;
   const u32* R = dir ? c.fr : c.rr;
   const u32* C = dir ? c.fc : c.rc;
   // chain starts (index of the first free unit): rev: k in [max(1, n5), n) with R[k-1]
   // stalled and R[k] free, ascending; fwd: k = i - 1 for i in [1, itop] with R[i] stalled
-  // and R[k] free, in descending i
+  // and R[k] free, in descending i.  Each start pairs with its own stalled unit: at most n / 2.
   u32* starts = c.tmp;
-  u32 nst = 0;
-  // stalled(k) = the unit of rank k collided; each unit's word is read once and its neighbour's
-  // flag comes from the adjacent lane (or the previous chunk)
-  if (dir == 0) {
-    const u32 k0 = (u32)max((u64)1, n5);
-    bool prev = k0 - 1 < n && cw_occurred(C[R[k0 - 1]]);
-    for (u32 base = k0; base < n; base += 32) {
-      const u32 k = base + ln();
-      const bool cur = k < n && cw_occurred(C[R[k]]);
-      bool before = __shfl_up_sync(FULL, cur, 1);
-      if (ln() == 0) before = prev;
-      const bool st = k < n && before && !cur;
-      const unsigned m = __ballot_sync(FULL, st);
-      if (st) starts[nst + __popc(m & lanemask_lt())] = k;
-      nst += __popc(m);
-      prev = __shfl_sync(FULL, cur, 31);
-    }
-  } else {
-    const i64 itop = (i64)(n - min(n3, n3 - 1)) - 1;
-    for (i64 top = itop; top >= 1; top -= 32) {
-      // lane l holds i = top - l and needs stalled(i) and stalled(i - 1): the latter is the
-      // next lane's flag, read directly by lane 31
-      const i64 i = top - (i64)ln();
-      const bool stalled = i >= 0 && cw_occurred(C[R[i]]);
-      bool below = __shfl_down_sync(FULL, stalled, 1);
-      if (ln() == 31) below = i - 1 >= 0 && cw_occurred(C[R[i - 1]]);
-      const bool st = i >= 1 && stalled && !below;
-      const unsigned m = __ballot_sync(FULL, st);
-      if (st) starts[nst + __popc(m & lanemask_lt())] = (u32)(i - 1);
-      nst += __popc(m);
-    }
-  }
-  __syncwarp();
-  const bool draws = trial_needs_draw(P.lef_lef);
-  u32 q = 0;
-  while (q < nst) {
-    rng_ensure(c, s, RNG_BLOCK);
-    const u32 ci = q + ln();
-    u32 L = 0, unused;
-    if (ci < nst) L = chain_walk<CHAIN_COUNT>(c, P, dir, n, starts[ci], 0, &unused);
-    const u32 Ld = draws ? L : 0;
-    u32 tot;
-    const u32 off = warp_excl_scan(Ld, &tot);
-    // lanes whose speculative window would run past the draws known to be in the ring
-    const unsigned over = __ballot_sync(FULL, ci < nst && off + Ld > RNG_BLOCK);
-    const u32 fb = over ? (u32)(__ffs(over) - 1) : 32u;
-    if (fb == 0) {  // a single chain longer than the ring window: walk it serially
-      prof_add(c, PF_CHAIN_SERIAL, 1);
-      if (ln() == 0) {
-        u32 used;
-        chain_walk<CHAIN_SERIAL>(c, P, dir, n, starts[q], 0, &used);
+  BlockTmp* bt = c.bt;
+  const i64 itop = (i64)(n - min(n3, n3 - 1)) - 1;
+  const u32 k0 = (u32)max((u64)1, n5);
+  const u32 items = dir ? (itop > 0 ? (u32)itop : 0u) : (n > k0 ? n - k0 : 0u);
+  u32 nst = 0, buf = 0;
+  for (u32 base = 0; base < items; base += 2 * T) {
+    bool st[2];
+    u32 at[2];
+#pragma unroll
+    for (u32 h = 0; h < 2; ++h) {
+      const u32 o = base + h * T + threadIdx.x;
+      st[h] = false;
+      at[h] = 0;
+      if (o < items) {
+        const u32 k = dir ? (u32)itop - o - 1 : k0 + o;      // the free unit
+        const u32 kp = dir ? k + 1 : k - 1;                  // the stalled one
+        st[h] = cw_occurred(C[R[kp]]) && !cw_occurred(C[R[k]]);
+        at[h] = k;
       }
-      __syncwarp();
-      q += 1;
+    }
+    const Scan2 s = scan2(c, buf, st[0], st[1]);
+    buf ^= 1;
+    if (st[0]) starts[nst + s.off0] = at[0];
+    if (st[1]) starts[nst + s.off1] = at[1];
+    nst += s.total;
+  }
+  wsync(c);
+  if (nst == 0) return rp;
+  u32* lens = c.tmp + nst;  // trials of each chain if all succeed, then its first draw's offset
+  for (u32 q = threadIdx.x; q < nst; q += T) lens[q] = chain_walk<CHAIN_COUNT>(c, P, dir, n, starts[q], 0);
+  wsync(c);
+  const bool draws = trial_needs_draw(P.lef_lef);
+  const u64 thr = P.lef_lef.thr;
+  const u32 lim = c.lim;  // draws of one round at most
+  u32 q0 = 0;
+  while (q0 < nst) {
+    if (threadIdx.x < 32) {
+      u32 off = 0, q = q0;
+      for (; q < nst; q += 32) {
+        const u32 ci = q + ln();
+        const u32 L = ci < nst && draws ? lens[ci] : 0u;
+        u32 tot;
+        u32 o = off + warp_excl_scan(L, &tot);
+        if (off + tot > lim) break;
+        rng_ensure(c, rp, off + tot);
+        u32 fixed = 0;  // lanes whose offset is settled
+        for (;;) {
+          bool dev = false;
+          u32 used = L;
+          if (L >= 2 && ln() >= fixed) {
+            u32 k = 0;
+            while (k + 1 < L && ring_at(c, rp + o + k) <= thr) ++k;
+            used = k + 1;
+            dev = used < L;
+          }
+          const unsigned dm = __ballot_sync(FULL, dev);
+          if (!dm) break;
+          const u32 f = (u32)(__ffs(dm) - 1);
+          const u32 d = __shfl_sync(FULL, L - used, f);
+          if (ln() > f) o -= d;
+          tot -= d;
+          fixed = f + 1;
+        }
+        if (ci < nst) lens[ci] = o;
+        off += tot;
+      }
+      if (ln() == 0) {
+        bt->qend = min(q, nst);
+        bt->used = off;
+      }
+    }
+    wsync(c);
+    const u32 q1 = bt->qend, used = bt->used;
+    if (q1 == q0) {
+      // 32 chains that might outrun the ring: walk them one by one
+      prof_add(c, PF_CHAIN_SERIAL, 1);
+      const u32 qe = min(q0 + 32, nst);
+      if (threadIdx.x == 0) {
+        for (u32 q = q0; q < qe; ++q) chain_walk<CHAIN_SERIAL>(c, P, dir, n, starts[q], 0);
+      }
+      wsync(c);
+      rp = c.sc->rpos;
+      q0 = qe;
       continue;
     }
-    // evaluate each chain's trials at its speculative offset
-    u32 used = 0;
-    bool fails = false;
-    if (ci < nst && ln() < fb && Ld > 0) {
-      u32 k = 0;
-      while (k < Ld && ring_at(c, c.sc->rpos + off + k) <= P.lef_lef.thr) ++k;
-      fails = k < Ld;
-      used = fails ? k + 1 : Ld;
-    } else {
-      used = Ld;
-    }
-    const unsigned fm_ = __ballot_sync(FULL, fails);
-    const u32 f = fm_ ? (u32)(__ffs(fm_) - 1) : 32u;  // first chain whose trial fails
-    const u32 last = min(f == 32 ? 31u : f, fb - 1);   // commit chains q .. q + last
-    if (ci < nst && ln() <= last) {
-      u32 u2;
-      chain_walk<CHAIN_RING>(c, P, dir, n, starts[ci], off, &u2);
-    }
-    const u32 consumed = __shfl_sync(FULL, off + used, last);
-    __syncwarp();
-    if (ln() == 0) c.sc->rpos += consumed;
-    __syncwarp();
-    q += last + 1;
+    rng_ensure(c, rp, used);
+    for (u32 q = q0 + threadIdx.x; q < q1; q += T)
+      chain_walk<CHAIN_RING>(c, P, dir, n, starts[q], rp + lens[q]);
+    rp += used;
+    q0 = q1;
+    wsync(c);
+    rng_publish(c, rp);
   }
+  wsync(c);
+  return rp;
 }
 
-// fix_secondary_lef_lef_collisions, warp-parallel: candidates (units marked avoided) are never
+// fix_secondary_lef_lef_collisions: candidates (units marked avoided) are never
 // adjacent in rank order (the unit before a rev candidate, after a fwd candidate, is stalled),
 // so each is an independent swap of two neighbours.
-__device__ bool fix_secondary_fast(Cell& c, const KParams& P, u32 n, u64 n5, u64 n3) {
+__device__ __noinline__ bool fix_secondary_block(Cell& c, const KParams& P, u32 n, u64 n5, u64 n3) {
+  const u32 T = c.T;
   const u32 k0 = (u32)max((u64)1, n5);
   const u32 naf = (u32)(n - min(n3, n3 - 1));
+  BlockTmp* bt = c.bt;
+  if (threadIdx.x == 0) bt->nr = bt->nf = 0;
+  wsync(c);
+  // candidate ranks: rev [k0, n), fwd [0, naf - 1); rev list from the front of tmp, fwd list from its end
   u32* list = c.tmp;
-  u32 nr = 0, nf = 0;
   bool adj = false;
-  for (u32 dir = 0; dir < 2; ++dir) {
-    const u32* __restrict__ R = dir ? c.fr : c.rr;
-    const u32* __restrict__ W = dir ? c.fc : c.rc;
-    // candidate ranks: rev [k0, n), fwd [0, naf - 1)
-    const u32 lo = dir ? 0u : k0, hi = dir ? (naf > 0 ? naf - 1 : 0u) : n;
-    bool prev = false;  // avoided flag of the rank before the item
-    u32& cnt = dir ? nf : nr;
-    for (u32 base = lo; base < hi; base += 32 * MLP) {
-      u32 idx[MLP], w[MLP];
-#pragma unroll
-      for (u32 h = 0; h < MLP; ++h) {
-        const u32 k = base + 32 * h + ln();
-        idx[h] = k < hi ? R[k] : 0u;
-      }
-#pragma unroll
-      for (u32 h = 0; h < MLP; ++h) w[h] = W[idx[h]];
-#pragma unroll
-      for (u32 h = 0; h < MLP; ++h) {
-        const u32 k = base + 32 * h + ln();
-        const bool av = k < hi && cw_avoided_as(w[h], EV_SECONDARY);
-        bool before = __shfl_up_sync(FULL, av, 1);
-        if (ln() == 0) before = prev;
-        if (av && before) adj = true;
-        const unsigned m = __ballot_sync(FULL, av);
-        const u32 slot = (dir ? nr + nf : nr) + __popc(m & lanemask_lt());
-        if (av && slot < n) list[slot] = k;
-        cnt += __popc(m);
-        prev = __shfl_sync(FULL, av, 31);
-      }
-    }
+  for (u32 k = k0 + threadIdx.x; k < n; k += T) {
+    if (!cw_avoided_as(c.rc[c.rr[k]], EV_SECONDARY)) continue;
+    if (k > k0 && cw_avoided_as(c.rc[c.rr[k - 1]], EV_SECONDARY)) adj = true;
+    const u32 s = atomicAdd(&bt->nr, 1u);
+    if (s < n) list[s] = k;
   }
-  if (__any_sync(FULL, adj) || nr + nf > n) return false;
-  __syncwarp();
-  for (u32 t = ln(); t < nr; t += 32) fix_rev_at(c, P.start, list[t]);
-  __syncwarp();
-  for (u32 t = ln(); t < nf; t += 32) fix_fwd_at(c, P.end, list[nr + t]);
-  __syncwarp();
+  wsync(c);
+  const u32 nr = bt->nr;
+  for (u32 k = threadIdx.x; k + 1 < naf; k += T) {
+    if (!cw_avoided_as(c.fc[c.fr[k]], EV_SECONDARY)) continue;
+    if (k > 0 && cw_avoided_as(c.fc[c.fr[k - 1]], EV_SECONDARY)) adj = true;
+    const u32 s = atomicAdd(&bt->nf, 1u);
+    if (nr + s < n) list[nr + s] = k;
+  }
+  if (wsync_or(c, adj)) return false;
+  const u32 nf = bt->nf;
+  if (nr + nf > n) return false;
+  for (u32 t = threadIdx.x; t < nr; t += T) fix_rev_at(c, P.start, list[t]);
+  wsync(c);
+  for (u32 t = threadIdx.x; t < nf; t += T) fix_fwd_at(c, P.end, list[nr + t]);
+  wsync(c);
   return true;
 }
 
 // process_collisions (simulation.cpp:925-955) in the reference's order.
 // sorted_ranks: the ranked positions are known to be sorted (the epoch loop ranks them itself);
 // otherwise (caller state) they are checked and unsorted ones take the serial restatement.
-__device__ void process_collisions(Cell& c, u64* s, const KParams& P, u32 n, bool fix,
-                                   bool sorted_ranks = false) {
+__device__ __noinline__ u64 process_collisions(Cell& c, const KParams& P, u64 rp, u32 n, bool fix,
+                                               bool sorted_ranks = false) {
   Scalars* sc = c.sc;
   u64 t0 = clock64();
-  const bool serial = (P.debug_flags & DBG_SERIAL_COLLISIONS) || !(sorted_ranks || ranked_sorted(c, n));
-  __syncwarp();
-  if (ln() == 0) {
+  const bool serial = (P.debug_flags & DBG_SERIAL_COLLISIONS) || !(sorted_ranks || (ranked_sorted(c, n) && words_plain(c, n)));
+  if (threadIdx.x == 0) {
     u64 n5, n3;
     detect_boundaries_serial(c, P, n, n5, n3);
     sc->n5 = n5;
     sc->n3 = n3;
   }
-  __syncwarp();
+  wsync(c);
   u64 t1 = clock64();
   prof_add(c, PF_BOUNDARIES, t1 - t0);
   const u64 n5 = sc->n5, n3 = sc->n3;
   if (serial) {
-    rng_ensure(c, s, RNG_BLOCK);
-    if (ln() == 0) {
+    if (threadIdx.x == 0) {
       detect_lef_bar_serial(c, P, n, n5, n3);
       detect_primary_serial(c, P, n, n5, n3);
     }
-    __syncwarp();
+    wsync(c);
+    rp = sc->rpos;
   } else {
-    detect_lef_bar_fast(c, s, P, n, n5, n3);
+    rp = detect_lef_bar_block(c, P, rp, n, n5, n3);
     t0 = clock64();
     prof_add(c, PF_LEF_BAR, t0 - t1);
     t1 = t0;
-    detect_primary_fast(c, s, P, n, n5, n3);
+    rp = detect_primary_block(c, P, rp, n, n5, n3);
   }
   t0 = clock64();
   prof_add(c, PF_PRIMARY, t0 - t1);
@@ -2166,197 +2519,264 @@ __device__ void process_collisions(Cell& c, u64* s, const KParams& P, u32 n, boo
   t1 = clock64();
   prof_add(c, PF_CORRECT, t1 - t0);
   if (serial) {
-    rng_ensure(c, s, RNG_BLOCK);
-    if (ln() == 0) process_secondary_serial(c, P, n, n5, n3);
-    __syncwarp();
+    if (threadIdx.x == 0) process_secondary_serial(c, P, n, n5, n3);
+    wsync(c);
+    rp = sc->rpos;
   } else {
     // chains read ranked positions; secondary moves only change moves and words
-    secondary_dir_fast(c, s, P, 0, n, n5, n3);
-    secondary_dir_fast(c, s, P, 1, n, n5, n3);
+    rp = secondary_dir_block(c, P, rp, 0, n, n5, n3);
+    rp = secondary_dir_block(c, P, rp, 1, n, n5, n3);
   }
   t0 = clock64();
   prof_add(c, PF_SECONDARY, t0 - t1);
   if (fix) {
-    if (serial || !fix_secondary_fast(c, P, n, n5, n3)) {
+    if (serial || !fix_secondary_block(c, P, n, n5, n3)) {
       prof_add(c, PF_FIX_FALLBACK, 1);
-      if (ln() == 0) fix_secondary_serial(c, P, n, n5, n3);
-      __syncwarp();
+      if (threadIdx.x == 0) fix_secondary_serial(c, P, n, n5, n3);
+      wsync(c);
     }
   }
   prof_add(c, PF_FIX, clock64() - t0);
+  return rp;
 }
 
 // extrude (simulation.cpp:489-512)
-__device__ void extrude(Cell& c, u32 n) {
+__device__ __noinline__ void extrude(Cell& c, u32 n) {
   const u32* __restrict__ bep = c.bep;
   const u32* __restrict__ rm = c.rm;
   const u32* __restrict__ fm = c.fm;
   u32* __restrict__ rev = c.rev;
   u32* __restrict__ fwd = c.fwd;
 #pragma unroll 4
-  for (u32 i = ln(); i < n; i += 32) {
+  for (u32 i = threadIdx.x; i < n; i += c.T) {
     if (bep[i] == UNBOUND) continue;
     rev[i] -= rm[i];
     fwd[i] += fm[i];
   }
-  __syncwarp();
+  wsync(c);
 }
 
-// release_lefs (simulation.cpp:544-592): one draw per bound LEF with p > 0.
-__device__ u32 release_lefs(Cell& c, u64* s, const KParams& P, u32 n, bool completed) {
-  u32 released = 0;
-  for (u32 base = 0; base < n; base += 32 * MLP) {
-    rng_ensure(c, s, 32 * MLP);
-    u32 r[MLP], f[MLP], be[MLP], fr_[MLP], ff[MLP];
+// release_lefs (simulation.cpp:544-592): one draw per bound LEF with p > 0.  bt->released counts
+// the released units (reset by the caller that wants it).
+__device__ __noinline__ u64 release_lefs(Cell& c, const KParams& P, u64 rp, u32 n, bool completed) {
+  const u32 T = c.T;
+  u32 buf = 0;
+  for (u32 base = 0; base < n; base += 2 * T) {
+    rng_ensure(c, rp, 2 * T);
+    u64 thr[2];
+    bool need[2];
 #pragma unroll
-    for (u32 h = 0; h < MLP; ++h) {
-      const u32 i = base + 32 * h + ln();
-      const u32 ic = i < n ? i : 0u;
-      be[h] = i < n ? c.bep[ic] : UNBOUND;
-      r[h] = c.rc[ic];
-      f[h] = c.fc[ic];
-    }
-#pragma unroll
-    for (u32 h = 0; h < MLP; ++h) {
-      const bool rb = be[h] != UNBOUND && cw_occurred_as(r[h], EV_LEF_BAR);
-      const bool fb = be[h] != UNBOUND && cw_occurred_as(f[h], EV_LEF_BAR);
-      fr_[h] = rb ? bar_flags(c, cw_idx(r[h])) : 0u;
-      ff[h] = fb ? bar_flags(c, cw_idx(f[h])) : 0u;
-    }
-    u32 used = 0;
-#pragma unroll
-    for (u32 h = 0; h < MLP; ++h) {
-      const u32 i = base + 32 * h + ln();
-      const bool bound = be[h] != UNBOUND;
-      Trial tr{0, 0, 0};
-      if (bound) {
+    for (u32 h = 0; h < 2; ++h) {
+      const u32 i = base + h * T + threadIdx.x;
+      need[h] = false;
+      thr[h] = 0;
+      if (i < n && c.bep[i] != UNBOUND) {
+        const u32 r = c.rc[i], f = c.fc[i];
         u32 nh = 0;
-        if (cw_occurred_as(r[h], EV_LEF_BAR) && (fr_[h] & BF_DIR_MASK) == MGPU_DIR_REV) ++nh;
-        if (cw_occurred_as(f[h], EV_LEF_BAR) && (ff[h] & BF_DIR_MASK) == MGPU_DIR_FWD) ++nh;
-        tr = P.release[completed ? 1 : 0][nh];
+        if (cw_occurred_as(r, EV_LEF_BAR) && (bar_flags(c, cw_idx(r)) & BF_DIR_MASK) == MGPU_DIR_REV) ++nh;
+        if (cw_occurred_as(f, EV_LEF_BAR) && (bar_flags(c, cw_idx(f)) & BF_DIR_MASK) == MGPU_DIR_FWD) ++nh;
+        const Trial& tr = P.release[completed ? 1 : 0][nh];
+        need[h] = tr.draws;
+        thr[h] = tr.thr;
       }
-      const bool need = bound && tr.draws;
-      const unsigned m = __ballot_sync(FULL, need);
-      const bool rel = need && ring_at(c, c.sc->rpos + used + __popc(m & lanemask_lt())) <= tr.thr;
-      used += __popc(m);
+    }
+    const Scan2 s = scan2(c, buf, need[0], need[1]);
+    rng_publish(c, rp);
+    buf ^= 1;
+#pragma unroll
+    for (u32 h = 0; h < 2; ++h) {
+      const u32 i = base + h * T + threadIdx.x;
+      const bool rel = need[h] && ring_at(c, rp + (h ? s.off1 : s.off0)) <= thr[h];
       if (rel) {
         c.rev[i] = UNBOUND;
         c.fwd[i] = UNBOUND;
         c.bep[i] = UNBOUND;
       }
-      released += __popc(__ballot_sync(FULL, rel));
+      const unsigned m = __ballot_sync(FULL, rel);
+      if (m && ln() == 0) atomicAdd(&c.bt->released, (u32)__popc(m));
     }
-    __syncwarp();
-    if (ln() == 0) c.sc->rpos += used;
-    __syncwarp();
+    rp += s.total;
   }
-  return released;
+  wsync(c);
+  rng_publish(c, rp);
+  return rp;
+}
+
+// Sum of n non-negative doubles with the rounding of the loop s = s + t[i], by one warp.
+// While s stays inside one binade, adding t rounds to a multiple of that binade's unit in the last
+// place: s + ulp * rint(t / ulp), unless t / ulp lies exactly halfway between two integers (then the
+// parity of s decides).  So a group of terms adds as integers; terms that would carry s out of the
+// binade, and exact halves, are added one at a time in double precision.
+__device__ __noinline__ double ordered_sum(const double* t, u32 n) {
+  const u32 lane = ln();
+  double s = 0.0;
+  u32 i = 0;
+  // s grows through most of its binades in the first terms
+  const u32 head = min(n, 32u);
+  {
+    const double mine = lane < head ? t[lane] : 0.0;
+    for (u32 k = 0; k < head; ++k) s = s + __shfl_sync(FULL, mine, k);
+    i = head;
+  }
+  while (i < n) {
+    const u64 sb = (u64)__double_as_longlong(s);
+    const u32 e = (u32)(sb >> 52) & 0x7FFu;
+    const u32 cnt = min(n - i, 128u);
+    bool done = false;
+    if (e > 60 && e < 1900) {
+      // t / ulp by an exact scaling with 2^(1075 - e)
+      const double scale = __longlong_as_double((i64)(2098 - e) << 52);
+      i64 part = 0;
+      bool stop = false;
+#pragma unroll
+      for (u32 h = 0; h < 4; ++h) {
+        const u32 k = 32 * h + lane;
+        const double q = k < cnt ? t[i + k] * scale : 0.0;
+        stop |= !(q < 9007199254740992.0);
+        const double r = rint(q);
+        stop |= fabs(q - r) == 0.5;
+        part += stop ? 0 : (i64)r;
+      }
+      if (!__any_sync(FULL, stop)) {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(FULL, part, d);
+        const u64 mant = (sb & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+        if (mant + (u64)part < (1ull << 53)) {
+          s = __longlong_as_double((i64)((sb & ~0xFFFFFFFFFFFFFull) | ((mant + (u64)part) & 0xFFFFFFFFFFFFFull)));
+          done = true;
+        }
+      }
+    }
+    if (!done) {
+#pragma unroll
+      for (u32 h = 0; h < 4; ++h) {
+        const u32 k0 = 32 * h;
+        if (k0 < cnt) {
+          const double mine = k0 + lane < cnt ? t[i + k0 + lane] : 0.0;
+          const u32 m = min(32u, cnt - k0);
+          for (u32 k = 0; k < m; ++k) s = s + __shfl_sync(FULL, mine, k);
+        }
+      }
+    }
+    i += cnt;
+  }
+  return s;
 }
 
 // compute_loop_size_stats + evaluate_burnin (simulation.cpp:957-1025).  Loop sizes are
-// integers below 2^32, so the reference's double sum is exact and the mean is computed from a
-// warp sum; the sum of squared deviations keeps the reference's left-to-right rounding (the
-// terms are computed by all lanes, the accumulation by lane 0).
-__device__ bool burnin_stats(Cell& c, const KParams& P, u32 n) {
+// integers below 2^32, so the reference's double sum is exact and the mean is computed from an
+// integer sum; the sum of squared deviations keeps the reference's left-to-right rounding
+// (ordered_sum).
+__device__ __noinline__ bool burnin_stats(Cell& c, const KParams& P, u32 n) {
   Scalars* sc = c.sc;
+  BlockTmp* bt = c.bt;
   const u32 cap = P.hist_cap;
   if (n == 0) {
-    if (ln() == 0) {
+    if (threadIdx.x == 0) {
       sc->hist_size = 0;
       sc->hist_head = 0;
     }
-    __syncwarp();
+    wsync(c);
     return false;
   }
+  if (threadIdx.x == 0) bt->sum = 0;
+  wsync(c);
   u64 part = 0;
 #pragma unroll 4
-  for (u32 i = ln(); i < n; i += 32) part += pos64(c.fwd[i]) - pos64(c.rev[i]);
+  for (u32 i = threadIdx.x; i < n; i += c.T) part += pos64(c.fwd[i]) - pos64(c.rev[i]);
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(FULL, part, d);
-  const double mean = (double)part / (double)n;
+  if (ln() == 0) atomicAdd((unsigned long long*)&bt->sum, (unsigned long long)part);
+  wsync(c);
+  const double mean = (double)bt->sum / (double)n;
   double* terms = reinterpret_cast<double*>(c.sr);  // sr and sf are adjacent: n doubles
-  for (u32 i = ln(); i < n; i += 32) {
+  for (u32 i = threadIdx.x; i < n; i += c.T) {
     const double d = (double)(pos64(c.fwd[i]) - pos64(c.rev[i])) - mean;
     terms[i] = d * d;
   }
-  __syncwarp();
-  if (ln() == 0) {
-    double ssd = 0.0;
-    for (u32 i = 0; i < n; ++i) ssd = ssd + terms[i];
-    const double sd = sqrt(ssd / (double)n);
-    if (sc->hist_size == cap) {
-      sc->hist_head = (sc->hist_head + 1) % cap;
-      sc->hist_size--;
-    }
-    const u32 slot = (sc->hist_head + sc->hist_size) % cap;
-    c.havg[slot] = mean;
-    c.hcfx[slot] = sd / mean;
-    sc->hist_size++;
-  }
-  __syncwarp();
-  bool done = false;
-  if (sc->hist_size == cap) {
-    // evaluate_burnin's smoothed-dip ratio: window pairs (i1, i2) = (k + 1, k + 1 + w) for
-    // k < cap - w - 1, one window per lane, each window summed in the reference's order
-    const u32 w = P.smooth_w;
-    const u32 head = sc->hist_head;
-    auto ratio = [&](const double* d) {
-      u32 nd = 0;
-      for (u32 i1 = 1 + ln(); i1 + w < cap; i1 += 32) {
-        const u32 i2 = i1 + w;
-        double a1 = 0.0, a2 = 0.0;
-        u32 k = head + i1 - 1;
-        if (k >= cap) k -= cap;
-        for (u32 t = 0; t < w; ++t) {
-          a1 = a1 + d[k];
-          if (++k == cap) k = 0;
-        }
-        k = head + i1;
-        if (k >= cap) k -= cap;
-        for (u32 t = 0; t < w; ++t) {
-          a2 = a2 + d[k];
-          if (++k == cap) k = 0;
-        }
-        const double n1 = a1 / (double)(i2 - i1), n2 = a2 / (double)(i2 - i1);
-        nd += (n1 > n2) ? 1u : 0u;
+  wsync(c);
+  if (threadIdx.x < 32) {
+    const double ssd = ordered_sum(terms, n);
+    if (ln() == 0) {
+      const double sd = sqrt(ssd / (double)n);
+      if (sc->hist_size == cap) {
+        sc->hist_head = (sc->hist_head + 1) % cap;
+        sc->hist_size--;
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) nd += __shfl_xor_sync(FULL, nd, o);
-      return (double)nd / (double)((u64)cap - w - nd);
-    };
-    const double r1 = ratio(c.hcfx);
-    if (r1 >= 0.95 && r1 <= 1.05) {
-      const double r2 = ratio(c.havg);
-      done = r2 >= 0.95 && r2 <= 1.05;
+      const u32 slot = (sc->hist_head + sc->hist_size) % cap;
+      c.havg[slot] = mean;
+      c.hcfx[slot] = sd / mean;
+      sc->hist_size++;
     }
+    __syncwarp();
+    bool done = false;
+    if (sc->hist_size == cap) {
+      // evaluate_burnin's smoothed-dip ratio: window pairs (i1, i2) = (k + 1, k + 1 + w) for
+      // k < cap - w - 1, one window per lane, each window summed in the reference's order
+      const u32 w = P.smooth_w;
+      const u32 head = sc->hist_head;
+      auto ratio = [&](const double* d) {
+        u32 nd = 0;
+        for (u32 i1 = 1 + ln(); i1 + w < cap; i1 += 32) {
+          const u32 i2 = i1 + w;
+          double a1 = 0.0, a2 = 0.0;
+          u32 k = head + i1 - 1;
+          if (k >= cap) k -= cap;
+          for (u32 t = 0; t < w; ++t) {
+            a1 = a1 + d[k];
+            if (++k == cap) k = 0;
+          }
+          k = head + i1;
+          if (k >= cap) k -= cap;
+          for (u32 t = 0; t < w; ++t) {
+            a2 = a2 + d[k];
+            if (++k == cap) k = 0;
+          }
+          const double n1 = a1 / (double)(i2 - i1), n2 = a2 / (double)(i2 - i1);
+          nd += (n1 > n2) ? 1u : 0u;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) nd += __shfl_xor_sync(FULL, nd, o);
+        return (double)nd / (double)((u64)cap - w - nd);
+      };
+      const double r1 = ratio(c.hcfx);
+      if (r1 >= 0.95 && r1 <= 1.05) {
+        const double r2 = ratio(c.havg);
+        done = r2 >= 0.95 && r2 <= 1.05;
+      }
+    }
+    if (ln() == 0) bt->flag = done ? 1 : 0;
   }
-  return done;
+  wsync(c);
+  return bt->flag != 0;
 }
 
 // run_burnin (simulation.cpp:1027-1054)
-__device__ void run_burnin(Cell& c, u64* s, const KParams& P) {
+__device__ __noinline__ u64 run_burnin(Cell& c, const KParams& P, u64 rp) {
   Scalars* sc = c.sc;
   for (u64 it = 0; it < MGPU_ITER_LIMIT; ++it) {
-    if (ln() == 0) ++sc->num_burnin_epochs;
-    __syncwarp();
-    if (sc->num_active != P.nlefs) {
-      rng_ensure(c, s, 64);
-      if (ln() == 0) {
+    const bool active = sc->num_active == P.nlefs;
+    wsync(c);  // thread 0 changes num_active below
+    bool done = false;
+    if (active) done = burnin_stats(c, P, P.nlefs);
+    if (threadIdx.x == 0) {
+      ++sc->num_burnin_epochs;
+      if (!active) {
         const u64 k = s_poisson(c, P);
         sc->num_active = min(sc->num_active + k, (u64)P.nlefs);
+      } else {
+        done = done && (sc->epoch > P.min_burnin);
+        if (!done && sc->epoch >= P.max_burnin) done = true;
+        sc->burnin_completed = done ? 1 : 0;
       }
-      __syncwarp();
-    } else {
-      bool done = burnin_stats(c, P, (u32)sc->num_active);
-      done = done && (sc->epoch > P.min_burnin);
-      if (!done && sc->epoch >= P.max_burnin) done = true;
-      if (ln() == 0) sc->burnin_completed = done ? 1 : 0;
-      __syncwarp();
     }
-    if (sc->num_active != 0) return;
+    wsync(c);
+    rp = sc->rpos;
+    if (sc->num_active != 0) return rp;
   }
-  if (ln() == 0) set_status(c, DEV_ERR_ITER_LIMIT);
-  __syncwarp();
+  if (threadIdx.x == 0) set_status(c, DEV_ERR_ITER_LIMIT);
+  wsync(c);
+  return rp;
 }
 
 // ContactMatrixDense::increment (contact_matrix_dense_safe_impl.hpp:52-87); returns whether
@@ -2375,22 +2795,17 @@ __device__ __forceinline__ bool band_increment(Cell& c, const KParams& P, u64 ro
   return false;
 }
 
-__device__ u64 s_uniform_int(Cell& c, u64 a, u64 b);
-__device__ double s_gev(Cell& c, const KParams& P);
-__device__ i64 s_binomial(Cell& c, const KParams& P, i64 t_, double p_);
-__device__ __forceinline__ double canonical_of(u64 u);
-
-// One contact attempt read from draws at `off` (register_contacts.cpp:129-198).  Returns the
+// One contact attempt read from draws at `at` (register_contacts.cpp:129-198).  Returns the
 // draws it takes; *ok tells whether it registers a contact; *regular is false when the attempt
 // hit a bucket rejection (exact handling needs the serial path).
-__device__ __forceinline__ u32 contact_attempt(const Cell& c, const KParams& P, u64 off, bool tad,
+__device__ __forceinline__ u32 contact_attempt(const Cell& c, const KParams& P, u64 at, bool tad,
                                                u64 na, u64 lbucket, bool* ok, bool* regular,
                                                u64* row, u64* col) {
   *ok = false;
   *regular = true;
   const u64 start = (u64)P.wstart + 1, end = (u64)P.wend - 1;
   u32 used = 0;
-  const u64 li = ring_at(c, c.sc->rpos + off + used++) / lbucket;
+  const u64 li = ring_at(c, at + used++) / lbucket;
   if (li > na - 1) {
     *regular = false;
     return used;
@@ -2400,13 +2815,13 @@ __device__ __forceinline__ u32 contact_attempt(const Cell& c, const KParams& P, 
   if (!(rp > start && rp < end && fp > start && fp < end)) return used;
   double n1 = 0.0, n2 = 0.0;
   if (P.noisify) {
-    const double u1 = canonical_of(ring_at(c, c.sc->rpos + off + used++));
+    const double u1 = canonical_of(ring_at(c, at + used++));
     n1 = (P.gev_xi == 0.0) ? (P.gev_mu - P.gev_sigma) * log(-log(u1))
                            : P.gev_mu + (P.gev_sigma * (1.0 - pow(-log(u1), P.gev_xi))) / P.gev_xi;
   }
   const double a = (double)rp - n1;
   if (P.noisify) {
-    const double u2 = canonical_of(ring_at(c, c.sc->rpos + off + used++));
+    const double u2 = canonical_of(ring_at(c, at + used++));
     n2 = (P.gev_xi == 0.0) ? (P.gev_mu - P.gev_sigma) * log(-log(u2))
                            : P.gev_mu + (P.gev_sigma * (1.0 - pow(-log(u2), P.gev_xi))) / P.gev_xi;
   }
@@ -2426,12 +2841,12 @@ __device__ __forceinline__ u32 contact_attempt(const Cell& c, const KParams& P, 
   if (range != 0) {
     u64 bucket = ~0ull / (range + 1);
     if (~0ull % (range + 1) == range) ++bucket;
-    const u64 r1 = ring_at(c, c.sc->rpos + off + used++) / bucket;
+    const u64 r1 = ring_at(c, at + used++) / bucket;
     if (r1 > range) {
       *regular = false;
       return used;
     }
-    const u64 r2 = ring_at(c, c.sc->rpos + off + used++) / bucket;
+    const u64 r2 = ring_at(c, at + used++) / bucket;
     if (r2 > range) {
       *regular = false;
       return used;
@@ -2445,7 +2860,7 @@ __device__ __forceinline__ u32 contact_attempt(const Cell& c, const KParams& P, 
   return used;
 }
 
-// Lane 0: one contact attempt with serial draws (the exact path for rejections).
+// Thread 0: one contact attempt with serial draws (the exact path for rejections).
 // register_1d_lef_occupancy (register_contacts.cpp:200-232): one count in each of the two bins
 __device__ __forceinline__ void occ_increment(const KParams& P, u64 i1, u64 i2) {
   if (!P.occ) return;
@@ -2454,7 +2869,7 @@ __device__ __forceinline__ void occ_increment(const KParams& P, u64 i1, u64 i2) 
 }
 
 // One attempt of register_contacts_loop / _tad (register_contacts.cpp:129-198) or, with occ, of
-// register_1d_lef_occupancy (the loop attempt with the 1D counters as its sink); lane 0.
+// register_1d_lef_occupancy (the loop attempt with the 1D counters as its sink); thread 0.
 __device__ __noinline__ void contact_attempt_serial(Cell& c, const KParams& P, bool tad, u64 na, bool* ok, bool* miss,
                                        bool occ = false) {
   *ok = false;
@@ -2482,18 +2897,19 @@ __device__ __noinline__ void contact_attempt_serial(Cell& c, const KParams& P, b
   *ok = true;
 }
 
-// sample_and_register_contacts (register_contacts.cpp:94-198): attempts are evaluated 32 at a
+// sample_and_register_contacts (register_contacts.cpp:94-198): attempts are evaluated up to T at a
 // time at the offsets they would have if each took the usual number of draws (1 for the LEF,
-// 2 for the noise, 2 more for a TAD contact).  The warp commits up to the first attempt that
+// 2 for the noise, 2 more for a TAD contact).  The workers commit up to the first attempt that
 // took a different number (a LEF or position outside the bounds, a zero-width TAD range) and
-// resumes after it; an attempt that hit a uniform_int bucket rejection is redone serially.
-__device__ void sample_contacts(Cell& c, u64* s, const KParams& P, u64 target) {
+// resume after it; an attempt that hit a uniform_int bucket rejection is redone serially.
+__device__ __noinline__ u64 sample_contacts(Cell& c, const KParams& P, u64 rp, u64 target) {
   Scalars* sc = c.sc;
+  BlockTmp* bt = c.bt;
+  const u32 T = c.T, W = T >> 5, w = threadIdx.x >> 5, lane = ln();
   u64 num = P.spe;
   if (P.density_positive) num = min(num, target - sc->num_contacts);
-  if (num == 0) return;
-  rng_ensure(c, s, 64);
-  if (ln() == 0) {
+  if (num == 0) return rp;
+  if (threadIdx.x == 0) {
     u64 n_loop;
     if (P.ratio_mode == 0) {
       n_loop = num;
@@ -2503,8 +2919,10 @@ __device__ void sample_contacts(Cell& c, u64* s, const KParams& P, u64 target) {
       n_loop = (u64)s_binomial(c, P, (i64)num, P.p_loop);
     }
     sc->bc0 = n_loop;
+    bt->missed = 0;
   }
-  __syncwarp();
+  wsync(c);
+  rp = sc->rpos;
   const u64 n_loop = sc->bc0;
   const u64 na = sc->num_active;
   u64 lbucket;
@@ -2513,7 +2931,6 @@ __device__ void sample_contacts(Cell& c, u64* s, const KParams& P, u64 target) {
     lbucket = ~0ull / (range + 1);
     if (~0ull % (range + 1) == range) ++lbucket;
   }
-  const bool serial = P.debug_flags & DBG_SERIAL_CONTACTS;
   u64 budget = 1000 * num + 1000000;  // attempts before giving up (see DEV_ERR_NO_BOUND_LEF)
   u32 missed = 0;
   const int passes = P.track_occ ? 3 : 2;  // loop, TAD, then the 1D occupancy
@@ -2521,65 +2938,101 @@ __device__ void sample_contacts(Cell& c, u64* s, const KParams& P, u64 target) {
     const bool tad = pass == 1, occ = pass == 2;
     u64 todo = occ ? num : (tad ? num - n_loop : n_loop);
     const u32 nominal = 1 + (P.noisify ? 2 : 0) + (tad ? 2 : 0);
+    const u32 most = min(T, c.lim / nominal);
     while (todo != 0) {
-      if (budget < 32) {
-        if (ln() == 0) set_status(c, DEV_ERR_NO_BOUND_LEF);
-        __syncwarp();
-        return;
+      if (budget < T) {
+        if (threadIdx.x == 0) {
+          rng_publish(c, rp);
+          set_status(c, DEV_ERR_NO_BOUND_LEF);
+        }
+        wsync(c);
+        return rp;
       }
-      budget -= 32;
-      rng_ensure(c, s, 32 * 5);
+      // a few attempts more than contacts are wanted, in whole warps
+      const u32 active = (u32)min((u64)most, (u64)((todo + todo / 16 + 32) & ~31ull));
+      budget -= active;
+      rng_ensure(c, rp, active * nominal);
       bool ok = false, regular = true;
       u64 row = 0, col = 0;
       u32 used = nominal;
-      if (!serial) used = contact_attempt(c, P, (u64)ln() * nominal, tad, na, lbucket, &ok, &regular, &row, &col);
-      const bool deviates = serial || !regular || used != nominal;
-      const unsigned dm = __ballot_sync(FULL, deviates);
-      const u32 f = dm ? (u32)(__ffs(dm) - 1) : 32u;
-      const bool f_regular = f < 32 && __shfl_sync(FULL, regular && !serial, f);
-      u32 lim = (f == 32) ? 32u : (f_regular ? f + 1 : f);  // lanes [0, lim) are exact
-      const unsigned okm = __ballot_sync(FULL, ok && ln() < lim);
-      if ((u64)__popc(okm) >= todo) {  // the todo-th success ends the pass
-        unsigned mm = okm;
-        for (u64 t = 1; t < todo; ++t) mm &= mm - 1;
-        lim = (u32)__ffs(mm);
+      if (threadIdx.x < active)
+        used = contact_attempt(c, P, rp + (u64)threadIdx.x * nominal, tad, na, lbucket, &ok, &regular, &row, &col);
+      const bool deviates = !regular || used != nominal;
+      const unsigned dm = __ballot_sync(FULL, deviates), om = __ballot_sync(FULL, ok);
+      const u32 fl = dm ? (u32)(__ffs(dm) - 1) : 0u;
+      const u32 fu = __shfl_sync(FULL, used | (regular ? 0x80000000u : 0u), fl);
+      if (lane == 0) {
+        bt->dev[w] = dm;
+        bt->okm[w] = om;
+        bt->dus[w] = fu;
       }
-      const unsigned lanes = lim >= 32 ? FULL : ((1u << lim) - 1);
-      if (ok && ((lanes >> ln()) & 1u)) {
+      wsync(c);
+      // first deviating attempt f, its draws, and the commit limit: attempts [0, lim) are exact
+      const u32 myd = lane < W ? bt->dev[lane] : 0u;
+      const unsigned dw = __ballot_sync(FULL, myd != 0);
+      u32 f = active, f_used = nominal;
+      bool f_regular = false;
+      if (dw) {
+        const u32 fw = (u32)(__ffs(dw) - 1);
+        f = fw * 32 + (u32)(__ffs(__shfl_sync(FULL, myd, fw)) - 1);
+        const u32 v = bt->dus[fw];
+        f_used = v & 0x7FFFFFFFu;
+        f_regular = (v & 0x80000000u) != 0;
+      }
+      u32 lim = f_regular ? f + 1 : f;
+      // contacts among them; the todo-th success ends the pass
+      u32 okw = lane < W ? bt->okm[lane] : 0u;
+      if (lim <= lane * 32) okw = 0;
+      else if (lim < lane * 32 + 32) okw &= (1u << (lim - lane * 32)) - 1u;
+      u32 total;
+      const u32 ex = warp_excl_scan(__popc(okw), &total);
+      if ((u64)total >= todo) {
+        const u32 want = (u32)todo;  // total <= T
+        const unsigned hit = __ballot_sync(FULL, ex < want && ex + __popc(okw) >= want);
+        const u32 hw = (u32)(__ffs(hit) - 1);
+        unsigned mm = __shfl_sync(FULL, okw, hw);
+        const u32 skip = want - 1 - __shfl_sync(FULL, ex, hw);
+        for (u32 t = 0; t < skip; ++t) mm &= mm - 1;
+        lim = hw * 32 + (u32)__ffs(mm);
+        total = want;
+      }
+      if (ok && threadIdx.x < lim) {
         if (occ) {
           occ_increment(P, row, col);
         } else if (band_increment(c, P, row, col)) {
           ++missed;
         }
       }
-      const u32 draws = lim == 0 ? 0 : (lim - 1) * nominal + __shfl_sync(FULL, used, lim == 0 ? 0 : lim - 1);
-      todo -= __popc(okm & lanes);
-      __syncwarp();
-      if (ln() == 0) sc->rpos += draws;
-      __syncwarp();
-      if (todo != 0 && lim == f && f < 32) {
+      if (lim) rp += (u64)(lim - 1) * nominal + (lim - 1 == f ? f_used : nominal);
+      todo -= total;
+      wsync(c);  // the draws are read and bt may be written again
+      rng_publish(c, rp);
+      if (todo != 0 && lim == f && f < active) {
         // attempt f could not be evaluated from the ring: run it serially
         prof_add(c, PF_CONTACT_SERIAL, 1);
-        if (ln() == 0) {
+        if (threadIdx.x == 0) {
           bool sok, smiss;
           contact_attempt_serial(c, P, tad, na, &sok, &smiss, occ);
           sc->bc1 = sok ? 1 : 0;
           if (smiss) sc->missed++;
         }
-        __syncwarp();
+        wsync(c);
+        rp = sc->rpos;
         if (sc->bc1) todo -= 1;
-        __syncwarp();
-        if (sc->status != DEV_OK) return;
+        wsync(c);
       }
     }
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) missed += __shfl_xor_sync(FULL, missed, d);
-  if (ln() == 0) {
-    sc->missed += missed;
+  if (lane == 0 && missed) atomicAdd(&bt->missed, missed);
+  wsync(c);
+  if (threadIdx.x == 0) {
+    sc->missed += bt->missed;
     sc->num_contacts += num;
   }
-  __syncwarp();
+  wsync(c);
+  return rp;
 }
 
 // sample_and_register_contacts with serial draws (lane 0): the exact path behind the
@@ -2632,7 +3085,9 @@ __device__ __noinline__ void trace_record(Cell& c, const KParams& P, const DevTr
   const u32 nl = P.nlefs;
   const bool full = rec < T.max_records;
   u64 part = 0;
-  for (u32 i = ln(); i < nl; i += 32) {
+  if (threadIdx.x == 0) c.bt->sum = 0;
+  wsync(c);
+  for (u32 i = threadIdx.x; i < nl; i += c.T) {
     const u64 v[9] = {pos64(c.rev[i]), pos64(c.fwd[i]), pos64(c.bep[i]), c.rr[i], c.fr[i],
                       c.rm[i], c.fm[i], cw_to_ref(c.rc[i]), cw_to_ref(c.fc[i])};
     u64 h = mix64((u64)i * 0x9E3779B97F4A7C15ull + 0x632BE59BD9B4E019ull);
@@ -2653,7 +3108,9 @@ __device__ __noinline__ void trace_record(Cell& c, const KParams& P, const DevTr
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(FULL, part, off);
-  if (ln() == 0) {
+  if (ln() == 0) atomicAdd((unsigned long long*)&c.bt->sum, (unsigned long long)part);
+  wsync(c);
+  if (threadIdx.x == 0) {
     const Scalars* sc = c.sc;
     mgpu_trace_header h;
     h.epoch = sc->epoch;
@@ -2664,45 +3121,49 @@ __device__ __noinline__ void trace_record(Cell& c, const KParams& P, const DevTr
     h.rng_draws = sc->rpos;
     h.n5prime = sc->n5;
     h.n3prime = sc->n3;
-    h.digest = part;
+    h.digest = c.bt->sum;
     if (T.all_headers && rec < T.max_epochs) T.all_headers[rec] = h;
     if (full && T.headers) T.headers[rec] = h;
   }
-  __syncwarp();
+  wsync(c);
 }
 
 // Lay out one cell: the header in shared memory, then each per-LEF array either in shared
-// memory or in the block's global scratch slot, as planned by the host.
-__device__ void carve(Cell& c, char* smem, char* gslot, const KParams& P, u32 nl, const DevChrom& ch,
+// memory or in the block's global scratch slot, as planned by the host.  Thread 0; the caller's
+// barrier follows.
+__device__ void carve(Cell& c, BlockTmp* bt, char* smem, char* gslot, const KParams& P, u32 nl, const DevChrom& ch,
                       const ulonglong2* jt, u32* band) {
-  if (ln() == 0) {
-    char* p = smem;
-    c.sc = reinterpret_cast<Scalars*>(p);
-    p += CELL_HEADER_BYTES;
-    c.ring = reinterpret_cast<u64*>(p);
-    p += (u64)RING * 8;
-    c.hcfx = reinterpret_cast<double*>(p);
-    p += (u64)P.hist_cap * 8;
-    c.havg = reinterpret_cast<double*>(p);
-    p += (u64)P.hist_cap * 8;
-    c.bst = reinterpret_cast<u32*>(p);
-    u32** arr[NARR] = {&c.rev, &c.fwd, &c.rr, &c.fr, &c.rm, &c.fm, &c.rc, &c.fc, &c.sr, &c.sf, &c.tmp, &c.bep};
-    for (u32 k = 0; k < NARR; ++k) {
-      char* base = ((P.arr_smem >> k) & 1u) ? smem : gslot;
-      *arr[k] = reinterpret_cast<u32*>(base + P.arr_off[k]);
-    }
-    c.bar = ch.barriers;
-    c.bpf = ch.pos_flags;
-    c.nb = ch.nbarriers;
-    c.nl = nl;
-    c.jt = jt;
-    c.band = band;
+  if (threadIdx.x != 0) return;
+  const u32 workers = P.workers, pw = producer_warps(workers);
+  c.sc = reinterpret_cast<Scalars*>(smem);
+  c.bt = bt;
+  c.T = workers * 32;
+  c.lim = pw * 32 * RNG_S;
+  c.rmask = 2 * c.lim - 1;
+  c.ring = reinterpret_cast<u64*>(smem + CELL_HEADER_BYTES);
+  c.hcfx = reinterpret_cast<double*>((P.hist_smem ? smem : gslot) + P.hist_off);
+  c.havg = c.hcfx + P.hist_cap;
+  c.bst = reinterpret_cast<u32*>((P.bst_smem ? smem : gslot) + P.bst_off);
+  u32** arr[NARR] = {&c.rev, &c.fwd, &c.rr, &c.fr, &c.rm, &c.fm, &c.rc, &c.fc, &c.sr, &c.sf, &c.tmp, &c.bep};
+  for (u32 k = 0; k < NARR; ++k) {
+    char* base = ((P.arr_smem >> k) & 1u) ? smem : gslot;
+    *arr[k] = reinterpret_cast<u32*>(base + P.arr_off[k]);
   }
-  __syncwarp();
+  c.bar = ch.barriers;
+  c.bpf = ch.pos_flags;
+  c.nb = ch.nbarriers;
+  c.nl = nl;
+  c.jt = jt + (u64)(pw - 1) * 2 * JUMP_TABLE_ENTRIES;
+  c.band = band;
 }
 
-__device__ void cell_reset(Cell& c, u32 nl, u64 seed) {
-  for (u32 i = ln(); i < nl; i += 32) {
+// The normal ziggurat's fixed-point layers (after the two jump tables) into the block's scratch.
+__device__ __forceinline__ void load_layers(BlockTmp* bt, const ulonglong2* jt) {
+  for (u32 i = threadIdx.x; i < 128; i += blockDim.x) bt->zt[i] = jt[4 * JUMP_TABLE_ENTRIES + i];
+}
+
+__device__ __noinline__ void cell_reset(Cell& c, u32 nl, u64 seed, u64* prof) {
+  for (u32 i = threadIdx.x; i < nl; i += blockDim.x) {
     c.rev[i] = UNBOUND;
     c.fwd[i] = UNBOUND;
     c.bep[i] = UNBOUND;
@@ -2713,8 +3174,8 @@ __device__ void cell_reset(Cell& c, u32 nl, u64 seed) {
     c.rc[i] = 0;
     c.fc[i] = 0;
   }
-  for (u32 w = ln(); w < (c.nb + 31) / 32; w += 32) c.bst[w] = 0;
-  if (ln() == 0) {
+  for (u32 w = threadIdx.x; w < (c.nb + 31) / 32; w += blockDim.x) c.bst[w] = 0;
+  if (threadIdx.x == 0) {
     Scalars* sc = c.sc;
     u64 st = seed;  // SplitMix64 seeding (random.hpp:26-30)
     for (int k = 0; k < 4; ++k) {
@@ -2724,9 +3185,9 @@ __device__ void cell_reset(Cell& c, u32 nl, u64 seed) {
       sc->canon[k] = z ^ (z >> 31);
     }
     sc->rpos = 0;
-    sc->gpos = 0;
+    sc->gpos = sc->rpub = 0;
+    sc->stop = 0;
     sc->nrec = 0;
-    sc->lanes_stale = 1;
     sc->status = DEV_OK;
     sc->epoch = 0;
     sc->num_burnin_epochs = 0;
@@ -2740,19 +3201,19 @@ __device__ void cell_reset(Cell& c, u32 nl, u64 seed) {
     sc->hist_size = 0;
     sc->hist_head = 0;
     sc->bc0 = sc->bc1 = sc->bc2 = 0;
-    sc->flag = 0;
+    sc->prof = prof;
   }
-  __syncwarp();
 }
 
 // Simulation::dump_stats (simulation.cpp:1166-1224): the epoch's model-state record, taken after
 // extrude and before release_lefs; the loop-size mean is exact (an integer sum below 2^53).
+// Warp 0; the caller's barrier follows.
 __device__ __noinline__ void log_model_state(Cell& c, const KParams& P, u32 n, u64 cell) {
   Scalars* sc = c.sc;
-  if (!P.records || sc->nrec >= P.rec_max) return;
+  if (!P.records || sc->nrec >= P.rec_max || threadIdx.x >= 32) return;
   u32 st_rev = 0, st_fwd = 0, st_both = 0, lb = 0, pri = 0, sec = 0;
   u64 loop = 0;
-  for (u32 i = ln(); i < n; i += 32) {
+  for (u32 i = threadIdx.x; i < n; i += 32) {
     const u32 r = c.rc[i], f = c.fc[i];
     const bool sr = cw_occurred(r), sf = cw_occurred(f);
     st_rev += sr;
@@ -2764,7 +3225,7 @@ __device__ __noinline__ void log_model_state(Cell& c, const KParams& P, u32 n, u
     loop += pos64(c.fwd[i]) - pos64(c.rev[i]);
   }
   u32 occ = 0;
-  for (u32 w = ln(); w < (c.nb + 31) / 32; w += 32) occ += __popc(c.bst[w]);
+  for (u32 w = threadIdx.x; w < (c.nb + 31) / 32; w += 32) occ += __popc(c.bst[w]);
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {
     st_rev += __shfl_xor_sync(FULL, st_rev, d);
@@ -2796,33 +3257,30 @@ __device__ __noinline__ void log_model_state(Cell& c, const KParams& P, u32 n, u
   __syncwarp();
 }
 
-__device__ void run_cell(Cell& c, u64* s, const KParams& P, const CellTask& task, u64 target_epochs,
-                         const DevTrace* trace, mgpu_cell_stats* stats, u64 cell) {
+// The epoch loop of one cell (simulation.cpp:1056-1152), run by the worker threads.
+__device__ __noinline__ void run_cell(Cell& c, const KParams& P, u64 target, u64 target_epochs, const DevTrace* trace,
+                                      mgpu_cell_stats* stats, u64 cell) {
   Scalars* sc = c.sc;
   const u32 nl = P.nlefs;
-  cell_reset(c, nl, task.seed);
-  if (ln() == 0) sc->prof = P.prof;
-  __syncwarp();
-  barriers_init(c, s);
-  if (P.skip_burnin && ln() == 0) {
+  u64 rp = barriers_init(c, 0);
+  if (P.skip_burnin && threadIdx.x == 0) {
     sc->num_active = nl;
     sc->burnin_completed = 1;
   }
-  __syncwarp();
-  const u64 target = task.target_contacts;
+  wsync(c);
   for (u64 guard = 0; guard < MGPU_ITER_LIMIT; ++guard) {
     const bool go = P.contact_mode ? (sc->num_contacts < target)
                                    : (sc->epoch - sc->num_burnin_epochs < target_epochs);
     if (!go) break;
     const u64 te0 = clock64();
-    if (!sc->burnin_completed) run_burnin(c, s, P);
+    if (!sc->burnin_completed) rp = run_burnin(c, P, rp);
     u64 ta = clock64();
     prof_add(c, PF_BURNIN, ta - te0);
     const u32 n = (u32)sc->num_active;
     const u32 epoch = (u32)sc->epoch;
     const bool completed = sc->burnin_completed != 0;
-    if (ln() == 0) sc->lef_epochs += n;
-    bind_lefs(c, s, P, n, epoch, 0, nullptr);
+    if (threadIdx.x == 0) sc->lef_epochs += n;
+    rp = bind_lefs(c, P, rp, n, epoch, 0, nullptr);
     u64 tb = clock64();
     prof_add(c, PF_BIND, tb - ta);
     rank_lefs(c, P, n, epoch, epoch != 0);
@@ -2830,11 +3288,11 @@ __device__ void run_cell(Cell& c, u64* s, const KParams& P, const CellTask& task
     prof_add(c, PF_RANK, ta - tb);
     if (completed) {
       if (P.debug_flags & DBG_SERIAL_CONTACTS) {
-        rng_ensure(c, s, RNG_BLOCK);
-        if (ln() == 0) sample_contacts_serial(c, P, target);
-        __syncwarp();
+        if (threadIdx.x == 0) sample_contacts_serial(c, P, target);
+        wsync(c);
+        rp = sc->rpos;
       } else {
-        sample_contacts(c, s, P, target);
+        rp = sample_contacts(c, P, rp, target);
       }
       tb = clock64();
       prof_add(c, PF_CONTACTS, tb - ta);
@@ -2844,9 +3302,10 @@ __device__ void run_cell(Cell& c, u64* s, const KParams& P, const CellTask& task
         break;
       }
       if (sc->status != DEV_OK) break;
+      wsync(c);  // no worker writes a status before all have read it
     }
-    gen_moves_dir(c, s, c.rm, n, P.rev_speed[completed], P.rev_std, P.rev_move_int[completed]);
-    gen_moves_dir(c, s, c.fm, n, P.fwd_speed[completed], P.fwd_std, P.fwd_move_int[completed]);
+    rp = gen_moves_dir(c, rp, c.rm, n, P.rev_speed[completed], P.rev_std, P.rev_move_int[completed]);
+    rp = gen_moves_dir(c, rp, c.fm, n, P.fwd_speed[completed], P.fwd_std, P.fwd_move_int[completed]);
     tb = clock64();
     prof_add(c, PF_MOVES, tb - ta);
     gather_ranked(c, n);
@@ -2854,31 +3313,35 @@ __device__ void run_cell(Cell& c, u64* s, const KParams& P, const CellTask& task
     clamp_moves(c, P, n);
     ta = clock64();
     prof_add(c, PF_ADJUST, ta - tb);
-    barriers_next(c, s);
-#pragma unroll 4
-    for (u32 i = ln(); i < n; i += 32) {
+    for (u32 i = threadIdx.x; i < n; i += c.T) {
       c.rc[i] = 0;
       c.fc[i] = 0;
     }
-    __syncwarp();
+    rp = barriers_next(c, rp);
+    wsync(c);
     tb = clock64();
     prof_add(c, PF_BARRIERS, tb - ta);
-    process_collisions(c, s, P, n, true, true);
+    rp = process_collisions(c, P, rp, n, true, true);
     ta = clock64();
     extrude(c, n);
-    if (P.log_state) log_model_state(c, P, n, cell);
-    release_lefs(c, s, P, n, completed);
+    if (P.log_state) {
+      log_model_state(c, P, n, cell);
+      wsync(c);
+    }
+    rp = release_lefs(c, P, rp, n, completed);
     tb = clock64();
     prof_add(c, PF_EXTRUDE_RELEASE, tb - ta);
     if (trace) trace_record(c, P, *trace, sc->epoch);
-    if (ln() == 0) sc->epoch++;
-    __syncwarp();
+    const bool failed = sc->status != DEV_OK;
+    wsync(c);
+    if (threadIdx.x == 0) sc->epoch++;
+    wsync(c);
     prof_add(c, PF_TRACE, clock64() - tb);
     prof_add(c, PF_TOTAL, clock64() - te0);
     prof_add(c, PF_EPOCHS, 1);
-    if (sc->status != DEV_OK) break;
+    if (failed) break;
   }
-  if (ln() == 0) {
+  if (threadIdx.x == 0) {
     if (P.rec_count) P.rec_count[cell] = sc->nrec;
     if (trace && trace->num_recorded) *trace->num_recorded = sc->epoch;
     if (stats) {
@@ -2887,72 +3350,97 @@ __device__ void run_cell(Cell& c, u64* s, const KParams& P, const CellTask& task
       stats->contacts = sc->num_contacts;
       stats->missed_updates = sc->missed;
       stats->lef_epochs = sc->lef_epochs;
-      stats->rng_draws = sc->rpos;
+      stats->rng_draws = rp;
       stats->sort_fallbacks = sc->sort_fallbacks;
       stats->status = sc->status;
     }
   }
-  __syncwarp();
 }
 
-__global__ void __launch_bounds__(32) simulate_kernel(const __grid_constant__ KParams P, DevChrom ch,
-                                                      const CellTask* tasks, u64 ncells,
-                                                      u64 target_epochs, u32* band, u64* missed,
-                                                      mgpu_cell_stats* stats, DevTrace trace,
-                                                      u32 tracing, const ulonglong2* jt, u32* work,
-                                                      char* gscratch) {
+// One cell on the whole block: reset, then the workers run the epoch loop while the producers
+// generate its draws.
+__device__ __forceinline__ void block_cell(Cell& c, const KParams& P, const CellTask& task, u64 target_epochs,
+                                           const DevTrace* trace, mgpu_cell_stats* stats, u64 cell) {
+  cell_reset(c, P.nlefs, task.seed, P.prof);
+  __syncthreads();
+  if (threadIdx.x < c.T) {
+    run_cell(c, P, task.target_contacts, target_epochs, trace, stats, cell);
+    wsync(c);
+    if (threadIdx.x == 0) st_release(&c.sc->stop, 1);
+  } else {
+    rng_produce(c);
+  }
+  __syncthreads();
+}
+
+// Next index of the launch's work queue, the same for the whole block.
+__device__ __forceinline__ u32 next_cell(u32* work, u32* slot) {
+  if (threadIdx.x == 0) *slot = atomicAdd(work, 1u);
+  __syncthreads();
+  const u32 cell = *slot;
+  __syncthreads();
+  return cell;
+}
+
+__global__ void __launch_bounds__(MAX_BLOCK_THREADS) simulate_kernel(const __grid_constant__ KParams P, DevChrom ch,
+                                                                     const CellTask* tasks, u64 ncells,
+                                                                     u64 target_epochs, u32* band, u64* missed,
+                                                                     mgpu_cell_stats* stats,
+                                                                     const __grid_constant__ DevTrace trace,
+                                                                     u32 tracing, const ulonglong2* jt, u32* work,
+                                                                     char* gscratch) {
   extern __shared__ __align__(16) char smem[];
   __shared__ Cell c;
-  u64 s[4] = {0, 0, 0, 0};
-  carve(c, smem, gscratch + (u64)blockIdx.x * P.slot_bytes, P, P.nlefs, ch, jt, band);
+  __shared__ BlockTmp bt;
+  __shared__ u32 slot;
+  load_layers(&bt, jt);
+  carve(c, &bt, smem, gscratch + (u64)blockIdx.x * P.slot_bytes, P, P.nlefs, ch, jt, band);
   for (;;) {
-    u32 cell = 0;
-    if (ln() == 0) cell = atomicAdd(work, 1u);
-    cell = __shfl_sync(FULL, cell, 0);
+    const u32 cell = next_cell(work, &slot);
     if (cell >= ncells) break;
-    run_cell(c, s, P, tasks[cell], target_epochs, tracing ? &trace : nullptr, stats ? stats + cell : nullptr, cell);
-    if (ln() == 0 && missed) atomicAdd((unsigned long long*)missed, (unsigned long long)c.sc->missed);
-    __syncwarp();
+    block_cell(c, P, tasks[cell], target_epochs, tracing ? &trace : nullptr, stats ? stats + cell : nullptr, cell);
+    if (threadIdx.x == 0 && missed) atomicAdd((unsigned long long*)missed, (unsigned long long)c.sc->missed);
   }
 }
 
 // Batched persistent kernel: cells of many chromosomes or windows in one work queue.  Each
-// task names its plan (parameters, layout, barrier track, band); a warp copies the plan's
+// task names its plan (parameters, layout, barrier track, band); a block copies the plan's
 // parameters into shared memory when its next cell belongs to another plan than the last.
-__global__ void __launch_bounds__(32) simulate_batch_kernel(const BatchPlan* plans, const BatchTask* tasks,
-                                                            u64 ntasks, u64 slot_bytes,
-                                                            mgpu_cell_stats* stats, const ulonglong2* jt,
-                                                            u32* work, char* gscratch) {
+__global__ void __launch_bounds__(MAX_BLOCK_THREADS) simulate_batch_kernel(const BatchPlan* plans,
+                                                                           const BatchTask* tasks, u64 ntasks,
+                                                                           u64 slot_bytes, mgpu_cell_stats* stats,
+                                                                           const ulonglong2* jt, u32* work,
+                                                                           char* gscratch) {
   extern __shared__ __align__(16) char smem[];
   __shared__ Cell c;
+  __shared__ BlockTmp bt;
   __shared__ __align__(16) KParams Psh;
-  u64 s[4] = {0, 0, 0, 0};
+  __shared__ u32 slot;
   char* gslot = gscratch + (u64)blockIdx.x * slot_bytes;
+  load_layers(&bt, jt);
   u32 cur = 0xFFFFFFFFu;
   for (;;) {
-    u32 cell = 0;
-    if (ln() == 0) cell = atomicAdd(work, 1u);
-    cell = __shfl_sync(FULL, cell, 0);
+    const u32 cell = next_cell(work, &slot);
     if (cell >= ntasks) break;
     const BatchTask t = tasks[cell];
     const BatchPlan& pl = plans[t.plan];
     if (t.plan != cur) {
       const u32* src = reinterpret_cast<const u32*>(&pl.P);
       u32* dst = reinterpret_cast<u32*>(&Psh);
-      for (u32 w = ln(); w < sizeof(KParams) / 4; w += 32) dst[w] = src[w];
-      __syncwarp();
-      carve(c, smem, gslot, Psh, Psh.nlefs, pl.ch, jt, pl.band);
+      for (u32 w = threadIdx.x; w < sizeof(KParams) / 4; w += blockDim.x) dst[w] = src[w];
+      __syncthreads();
+      carve(c, &bt, smem, gslot, Psh, Psh.nlefs, pl.ch, jt, pl.band);
+      __syncthreads();
       cur = t.plan;
     }
     const CellTask ct{t.seed, t.target_contacts};
-    run_cell(c, s, Psh, ct, pl.target_epochs, nullptr, stats ? stats + cell : nullptr, cell);
-    if (ln() == 0 && pl.missed) atomicAdd(pl.missed, (unsigned long long)c.sc->missed);
-    __syncwarp();
+    block_cell(c, Psh, ct, pl.target_epochs, nullptr, stats ? stats + cell : nullptr, cell);
+    if (threadIdx.x == 0 && pl.missed) atomicAdd(pl.missed, (unsigned long long)c.sc->missed);
   }
 }
 
 // One step of the epoch loop on caller state (mgpu_run_phase).
-__global__ void __launch_bounds__(32) phase_kernel(const __grid_constant__ KParams P, DevChrom ch, int phase,
+__global__ void __launch_bounds__(MAX_BLOCK_THREADS) phase_kernel(const __grid_constant__ KParams P, DevChrom ch, int phase,
                                                    u32 n, u64* arrays, u64* bind_mask,
                                                    uint8_t* barrier_state, u64 epoch,
                                                    u32 burnin_completed, u32 partially_sorted,
@@ -2960,11 +3448,13 @@ __global__ void __launch_bounds__(32) phase_kernel(const __grid_constant__ KPara
                                                    u64* outs, const ulonglong2* jt, char* gslot) {
   extern __shared__ __align__(16) char smem[];
   __shared__ Cell c;
-  u64 s[4] = {0, 0, 0, 0};
-  carve(c, smem, gslot, P, n, ch, jt, nullptr);
+  __shared__ BlockTmp bt;
+  load_layers(&bt, jt);
+  carve(c, &bt, smem, gslot, P, n, ch, jt, nullptr);
+  __syncthreads();
   u64* A[9];
   for (int k = 0; k < 9; ++k) A[k] = arrays + (u64)k * n;
-  for (u32 i = ln(); i < n; i += 32) {
+  for (u32 i = threadIdx.x; i < n; i += blockDim.x) {
     c.rev[i] = A[0][i] == ~0ull ? UNBOUND : (u32)A[0][i];
     c.fwd[i] = A[1][i] == ~0ull ? UNBOUND : (u32)A[1][i];
     c.bep[i] = A[2][i] == ~0ull ? UNBOUND : (u32)A[2][i];
@@ -2975,7 +3465,7 @@ __global__ void __launch_bounds__(32) phase_kernel(const __grid_constant__ KPara
     c.rc[i] = cw_from_ref(A[7][i]);
     c.fc[i] = cw_from_ref(A[8][i]);
   }
-  for (u32 w = ln(); w < (c.nb + 31) / 32; w += 32) {
+  for (u32 w = threadIdx.x; w < (c.nb + 31) / 32; w += blockDim.x) {
     u32 bits = 0;
     for (u32 b = 0; b < 32; ++b) {
       const u32 i = w * 32 + b;
@@ -2985,33 +3475,41 @@ __global__ void __launch_bounds__(32) phase_kernel(const __grid_constant__ KPara
   }
   u64 init_state[4];
   for (int k = 0; k < 4; ++k) init_state[k] = prng[k];
-  if (ln() == 0) {
+  if (threadIdx.x == 0) {
     Scalars* sc = c.sc;
     for (int k = 0; k < 4; ++k) sc->canon[k] = prng[k];
-    sc->rpos = sc->gpos = 0;
-    sc->lanes_stale = 1;
+    sc->rpos = 0;
+    sc->gpos = sc->rpub = 0;
+    sc->stop = 0;
     sc->status = DEV_OK;
     sc->epoch = epoch;
     sc->num_active = n;
     sc->burnin_completed = burnin_completed;
     sc->sort_fallbacks = 0;
+    sc->n5 = sc->n3 = 0;
     sc->prof = nullptr;
+    bt.released = 0;
   }
-  __syncwarp();
+  __syncthreads();
+  if (threadIdx.x >= c.T) {
+    rng_produce(c);
+    return;
+  }
   const bool completed = burnin_completed != 0;
-  u64 released = 0;
+  const bool fast = !(P.debug_flags & DBG_SERIAL_COLLISIONS);
+  u64 rp = 0;
   switch (phase) {
     case MGPU_PHASE_BIND:
-      bind_lefs(c, s, P, n, (u32)epoch, bind_mask ? 1 : 2, bind_mask);
+      rp = bind_lefs(c, P, rp, n, (u32)epoch, bind_mask ? 1 : 2, bind_mask);
       rank_lefs(c, P, n, (u32)epoch, epoch != 0);
       break;
     case MGPU_PHASE_RANK:
       if (init_ranks) {
-        for (u32 i = ln(); i < n; i += 32) {
+        for (u32 i = threadIdx.x; i < n; i += c.T) {
           c.rr[i] = i;
           c.fr[i] = i;
         }
-        __syncwarp();
+        wsync(c);
       }
       rank_lefs(c, P, n, (u32)epoch, partially_sorted != 0);
       break;
@@ -3021,8 +3519,8 @@ __global__ void __launch_bounds__(32) phase_kernel(const __grid_constant__ KPara
       clamp_moves(c, P, n);
       break;
     case MGPU_PHASE_GENERATE_MOVES:
-      gen_moves_dir(c, s, c.rm, n, P.rev_speed[completed], P.rev_std, P.rev_move_int[completed]);
-      gen_moves_dir(c, s, c.fm, n, P.fwd_speed[completed], P.fwd_std, P.fwd_move_int[completed]);
+      rp = gen_moves_dir(c, rp, c.rm, n, P.rev_speed[completed], P.rev_std, P.rev_move_int[completed]);
+      rp = gen_moves_dir(c, rp, c.fm, n, P.fwd_speed[completed], P.fwd_std, P.fwd_move_int[completed]);
       if (adjust) {
         gather_ranked(c, n);
         adjust_moves(c, P, n);
@@ -3031,46 +3529,43 @@ __global__ void __launch_bounds__(32) phase_kernel(const __grid_constant__ KPara
       break;
     case MGPU_PHASE_PROCESS_COLLISIONS:
       gather_ranked(c, n);
-      process_collisions(c, s, P, n, false);
+      rp = process_collisions(c, P, rp, n, false);
       break;
     case MGPU_PHASE_FIX_SECONDARY:
-      if (ln() == 0) fix_secondary_serial(c, P, n, 0, 0);
+      if (threadIdx.x == 0) fix_secondary_serial(c, P, n, 0, 0);
       break;
     case MGPU_PHASE_DETECT_LEF_BAR:
       gather_ranked(c, n);
-      if (ranked_sorted(c, n) && !(P.debug_flags & DBG_SERIAL_COLLISIONS)) {
-        detect_lef_bar_fast(c, s, P, n, 0, 0);
-      } else {
-        rng_ensure(c, s, RNG_BLOCK);
-        if (ln() == 0) detect_lef_bar_serial(c, P, n, 0, 0);
+      if (ranked_sorted(c, n) && words_plain(c, n) && fast) {
+        rp = detect_lef_bar_block(c, P, rp, n, 0, 0);
+      } else if (threadIdx.x == 0) {
+        detect_lef_bar_serial(c, P, n, 0, 0);
       }
       break;
     case MGPU_PHASE_LEF_LEF:
       gather_ranked(c, n);
-      if (ranked_sorted(c, n) && !(P.debug_flags & DBG_SERIAL_COLLISIONS)) {
-        detect_primary_fast(c, s, P, n, 0, 0);
+      if (ranked_sorted(c, n) && fast) {
+        rp = detect_primary_block(c, P, rp, n, 0, 0);
         correct_primary(c, n);
-        secondary_dir_fast(c, s, P, 0, n, 0, 0);
-        secondary_dir_fast(c, s, P, 1, n, 0, 0);
+        rp = secondary_dir_block(c, P, rp, 0, n, 0, 0);
+        rp = secondary_dir_block(c, P, rp, 1, n, 0, 0);
       } else {
-        rng_ensure(c, s, RNG_BLOCK);
-        if (ln() == 0) detect_primary_serial(c, P, n, 0, 0);
-        __syncwarp();
+        if (threadIdx.x == 0) detect_primary_serial(c, P, n, 0, 0);
+        wsync(c);
         correct_primary(c, n);
-        if (ln() == 0) process_secondary_serial(c, P, n, 0, 0);
+        if (threadIdx.x == 0) process_secondary_serial(c, P, n, 0, 0);
       }
       break;
     case MGPU_PHASE_DETECT_PRIMARY:
       gather_ranked(c, n);
-      if (ranked_sorted(c, n) && !(P.debug_flags & DBG_SERIAL_COLLISIONS)) {
-        detect_primary_fast(c, s, P, n, 0, 0);
-      } else {
-        rng_ensure(c, s, RNG_BLOCK);
-        if (ln() == 0) detect_primary_serial(c, P, n, 0, 0);
+      if (ranked_sorted(c, n) && fast) {
+        rp = detect_primary_block(c, P, rp, n, 0, 0);
+      } else if (threadIdx.x == 0) {
+        detect_primary_serial(c, P, n, 0, 0);
       }
       break;
     case MGPU_PHASE_DETECT_BOUNDARIES:
-      if (ln() == 0) {
+      if (threadIdx.x == 0) {
         u64 n5, n3;
         detect_boundaries_serial(c, P, n, n5, n3);
         c.sc->n5 = n5;
@@ -3087,21 +3582,21 @@ __global__ void __launch_bounds__(32) phase_kernel(const __grid_constant__ KPara
       extrude(c, n);
       break;
     case MGPU_PHASE_RELEASE:
-      released = release_lefs(c, s, P, n, completed);
+      rp = release_lefs(c, P, rp, n, completed);
       break;
     case MGPU_PHASE_BARRIER_NEXT:
-      barriers_next(c, s);
+      rp = barriers_next(c, rp);
       break;
     case MGPU_PHASE_BARRIER_INIT:
-      barriers_init(c, s);
+      rp = barriers_init(c, rp);
       break;
     default:
       break;
   }
-  __syncwarp();
+  wsync(c);
   // rank_lefs uses the move arrays as scratch: the caller's moves stay as they were
   const bool moves_kept = phase == MGPU_PHASE_BIND || phase == MGPU_PHASE_RANK;
-  for (u32 i = ln(); i < n; i += 32) {
+  for (u32 i = threadIdx.x; i < n; i += c.T) {
     A[0][i] = pos64(c.rev[i]);
     A[1][i] = pos64(c.fwd[i]);
     A[2][i] = pos64(c.bep[i]);
@@ -3114,17 +3609,18 @@ __global__ void __launch_bounds__(32) phase_kernel(const __grid_constant__ KPara
     A[7][i] = cw_to_ref(c.rc[i]);
     A[8][i] = cw_to_ref(c.fc[i]);
   }
-  for (u32 i = ln(); i < c.nb; i += 32) {
+  for (u32 i = threadIdx.x; i < c.nb; i += c.T) {
     if (barrier_state) barrier_state[i] = bar_active(c, i) ? 1 : 0;
   }
-  if (ln() == 0) {
+  if (threadIdx.x == 0) {
+    st_release(&c.sc->stop, 1);
     // the caller's PRNG advanced by exactly the number of draws consumed
     u64 st[4] = {init_state[0], init_state[1], init_state[2], init_state[3]};
     for (u64 k = 0; k < c.sc->rpos; ++k) xo_next(st);
     for (int k = 0; k < 4; ++k) prng[k] = st[k];
     outs[0] = c.sc->n5;
     outs[1] = c.sc->n3;
-    outs[2] = released;
+    outs[2] = bt.released;
     outs[3] = c.sc->status;
   }
 }
@@ -3169,7 +3665,8 @@ u64 resident_cells(const KParams& P, u64 ncells) {
     return 0;
   }
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, simulate_kernel, 32, P.smem_bytes) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, simulate_kernel, (int)block_threads(P.workers),
+                                                    P.smem_bytes) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -3205,14 +3702,14 @@ int launch_simulate(const KParams& P, const DevChrom& ch, const CellTask* tasks,
     tr = *trace;
     tracing = 1;
   }
-  simulate_kernel<<<(unsigned)grid, 32, P.smem_bytes, st>>>(P, ch, tasks, ncells, target_epochs, band,
+  simulate_kernel<<<(unsigned)grid, block_threads(P.workers), P.smem_bytes, st>>>(P, ch, tasks, ncells, target_epochs, band,
                                                              missed, stats, tr, tracing,
                                                              (const ulonglong2*)jump_table, work_counter,
                                                              gscratch);
   return cuda_fail(cudaGetLastError(), "simulate_kernel launch", errbuf, errlen);
 }
 
-u64 resident_batch_cells(u32 smem_bytes, u64 ntasks, u32 carveout_pct, u32 max_per_sm) {
+u64 resident_batch_cells(u32 workers, u32 smem_bytes, u64 ntasks, u32 carveout_pct, u32 max_per_sm) {
   if (cudaFuncSetAttribute(simulate_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)max_smem_per_block()) != cudaSuccess) {
     cudaGetLastError();
@@ -3223,8 +3720,8 @@ u64 resident_batch_cells(u32 smem_bytes, u64 ntasks, u32 carveout_pct, u32 max_p
                        carveout_pct ? (int)carveout_pct : -1);
   cudaGetLastError();
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, simulate_batch_kernel, 32, smem_bytes) !=
-      cudaSuccess) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, simulate_batch_kernel, (int)block_threads(workers),
+                                                    smem_bytes) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -3237,11 +3734,11 @@ u64 resident_batch_cells(u32 smem_bytes, u64 ntasks, u32 carveout_pct, u32 max_p
   return grid < ntasks ? grid : ntasks;
 }
 
-int launch_simulate_batch(const BatchPlan* plans, const BatchTask* tasks, u64 ntasks, u32 smem_bytes,
+int launch_simulate_batch(const BatchPlan* plans, const BatchTask* tasks, u64 ntasks, u32 workers, u32 smem_bytes,
                           u64 slot_bytes, mgpu_cell_stats* stats, const void* jump_table, u32* work_counter,
                           char* gscratch, u64 gscratch_bytes, u32 carveout_pct, u32 max_per_sm, void* stream,
                           char* errbuf, int errlen) {
-  u64 grid = resident_batch_cells(smem_bytes, ntasks, carveout_pct, max_per_sm);
+  u64 grid = resident_batch_cells(workers, smem_bytes, ntasks, carveout_pct, max_per_sm);
   if (grid == 0) return ntasks ? MGPU_ERR_CUDA : MGPU_OK;
   if (slot_bytes && gscratch_bytes / slot_bytes < grid) grid = gscratch_bytes / slot_bytes;
   if (grid == 0) {
@@ -3251,7 +3748,7 @@ int launch_simulate_batch(const BatchPlan* plans, const BatchTask* tasks, u64 nt
   cudaStream_t st = (cudaStream_t)stream;
   int rc = cuda_fail(cudaMemsetAsync(work_counter, 0, sizeof(u32), st), "memset", errbuf, errlen);
   if (rc) return rc;
-  simulate_batch_kernel<<<(unsigned)grid, 32, smem_bytes, st>>>(plans, tasks, ntasks, slot_bytes, stats,
+  simulate_batch_kernel<<<(unsigned)grid, block_threads(workers), smem_bytes, st>>>(plans, tasks, ntasks, slot_bytes, stats,
                                                                  (const ulonglong2*)jump_table, work_counter,
                                                                  gscratch);
   return cuda_fail(cudaGetLastError(), "simulate_batch_kernel launch", errbuf, errlen);
@@ -3266,7 +3763,7 @@ int launch_phase(const KParams& P, const DevChrom& ch, int phase, u64 n, u64* ar
                      "cudaFuncSetAttribute", errbuf, errlen);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  phase_kernel<<<1, 32, P.smem_bytes, st>>>(P, ch, phase, (u32)n, arrays, bind_mask, barrier_state, epoch,
+  phase_kernel<<<1, block_threads(P.workers), P.smem_bytes, st>>>(P, ch, phase, (u32)n, arrays, bind_mask, barrier_state, epoch,
                                             burnin_completed, partially_sorted, init_ranks, adjust,
                                             prng_state, outs, (const ulonglong2*)jump_table, gscratch);
   return cuda_fail(cudaGetLastError(), "phase_kernel launch", errbuf, errlen);
@@ -3278,22 +3775,24 @@ int launch_phase(const KParams& P, const DevChrom& ch, int phase, u64 n, u64* ar
 // the test-suite can compare them with the host's libm (glibc, the reference's) bit for bit.
 // ---------------------------------------------------------------------------------------
 
-// One block per stream (grid-stride): lane 0 draws `per` samples of one distribution from the
+// One block per stream (grid-stride): thread 0 draws `per` samples of one distribution from the
 // Xoshiro256++ state states[4 s .. 4 s + 3] through the same serial samplers the epoch loop
 // uses, writes them to out[s * per ..] and the number of raw draws taken to draws[s].
 __global__ void __launch_bounds__(32) sampler_probe_kernel(const __grid_constant__ KParams P, int kind,
                                                            const u64* states, u64 nstreams, u64 per,
                                                            double a0, double a1, double* out, u64* draws) {
   __shared__ Scalars sc;
-  __shared__ u64 ring[RING];
+  constexpr u32 PROBE_RING = 16;
+  __shared__ u64 ring[PROBE_RING];
   if (threadIdx.x != 0) return;
   for (u64 s = blockIdx.x; s < nstreams; s += gridDim.x) {
     Cell c{};
     c.sc = &sc;
     c.ring = ring;
-    sc.rpos = sc.gpos = 0;
+    c.rmask = PROBE_RING - 1;
+    sc.rpos = 0;
+    sc.gpos = 0;
     sc.status = DEV_OK;
-    sc.lanes_stale = 0;
     sc.prof = nullptr;
     for (int k = 0; k < 4; ++k) sc.canon[k] = states[4 * s + k];
     for (u64 i = 0; i < per; ++i) {
@@ -3373,3 +3872,4 @@ int launch_pack_tasks(const u64* seeds, const u64* targets, u64 n, CellTask* tas
 }
 
 }  // namespace mgpu
+

@@ -2,7 +2,7 @@
 //
 // Responsibilities: the Config derivations of the reference CLI, per-cell seeds (XXH3),
 // conversion of every floating-point random test of the epoch loop into an exact integer
-// threshold on the raw 64-bit draw, the GF(2) jump table of the per-warp PRNG, device buffer
+// threshold on the raw 64-bit draw, the GF(2) jump tables of the PRNG producers, device buffer
 // management and kernel launches.
 
 #include <cuda_runtime.h>
@@ -21,6 +21,7 @@
 
 #include "cppsort_emul.h"
 #include "mgpu_internal.h"
+#include "ziggurat_tables.h"
 
 using namespace mgpu;
 
@@ -465,7 +466,8 @@ static DevBarrier make_dev_barrier(const mgpu_barrier& b) {
 }
 
 // ===========================================================================================
-// Jump table of the per-lane PRNG: T^JUMP_DISTANCE on the 256-bit state, 4-bit chunks.
+// Constant tables of a device context: per producer count the jump T^jump_distance on the 256-bit
+// PRNG state in 4-bit chunks, then the normal ziggurat's layers in fixed point.
 // ===========================================================================================
 static void xo_linear_step(uint64_t* s) {
   const uint64_t t = s[1] << 17;
@@ -477,18 +479,17 @@ static void xo_linear_step(uint64_t* s) {
   s[3] = (s[3] << 45) | (s[3] >> 19);
 }
 
-static std::vector<uint64_t> build_jump_table() {
+static void build_jump_table(int distance, uint64_t* table) {
   std::vector<uint64_t> col(256 * 4);
   for (int b = 0; b < 256; ++b) {
     uint64_t s[4] = {0, 0, 0, 0};
     s[b / 64] = 1ull << (b % 64);
-    for (int k = 0; k < JUMP_DISTANCE; ++k) xo_linear_step(s);
+    for (int k = 0; k < distance; ++k) xo_linear_step(s);
     for (int w = 0; w < 4; ++w) col[b * 4 + w] = s[w];
   }
-  std::vector<uint64_t> table(JUMP_TABLE_ENTRIES * 4, 0);
   for (int c = 0; c < 64; ++c) {
     for (int v = 0; v < 16; ++v) {
-      uint64_t* e = &table[(c * 16 + v) * 4];
+      uint64_t* e = table + (c * 16 + v) * 4;
       for (int bit = 0; bit < 4; ++bit) {
         if (!((v >> bit) & 1)) continue;
         const int b = 4 * c + bit;
@@ -496,7 +497,27 @@ static std::vector<uint64_t> build_jump_table() {
       }
     }
   }
-  return table;
+}
+
+// Layer i of the unit normal's ziggurat: e[0] = the number of 56-bit fractions m (ascending) whose
+// double product m * 2^-56 * x_i is below x_{i+1}, so "accepted" is m < e[0]; e[1] = x_i * 2^60.  The
+// product is monotone in m and both roundings are IEEE, as on the device.
+static void build_layer(int i, uint64_t* e) {
+  const double x = mgpu_zig_normal_x[i], x1 = mgpu_zig_normal_x[i + 1];
+  uint64_t lo = 0, hi = 1ull << 56;
+  while (lo < hi) {
+    const uint64_t mid = lo + (hi - lo) / 2;
+    if ((double)mid * (1.0 / 72057594037927936.0) * x < x1) lo = mid + 1; else hi = mid;
+  }
+  e[0] = lo;
+  e[1] = (uint64_t)(x * 1152921504606846976.0);
+}
+
+static std::vector<uint64_t> build_tables() {
+  std::vector<uint64_t> t(MAX_PRODUCERS * JUMP_TABLE_ENTRIES * 4 + NORMAL_LAYERS * 2, 0);
+  for (u32 p = 1; p <= MAX_PRODUCERS; ++p) build_jump_table(jump_distance(p), &t[(p - 1) * JUMP_TABLE_ENTRIES * 4]);
+  for (u32 i = 0; i < NORMAL_LAYERS; ++i) build_layer((int)i, &t[MAX_PRODUCERS * JUMP_TABLE_ENTRIES * 4 + 2 * i]);
+  return t;
 }
 
 extern "C" void mgpu_prng_seed(uint64_t seed, uint64_t state[4]) {
@@ -601,7 +622,7 @@ extern "C" int mgpu_create(int device, const mgpu_config* cfg, mgpu_ctx** out) {
   ctx->device = device;
   ctx->cfg = *cfg;
   rc = cuda_check(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking), "cudaStreamCreate");
-  const std::vector<uint64_t> jt = build_jump_table();
+  static const std::vector<uint64_t> jt = build_tables();
   if (!rc) rc = cuda_check(cudaMalloc(&ctx->d_jump, jt.size() * 8), "cudaMalloc(jump table)");
   if (!rc) rc = cuda_check(cudaMemcpy(ctx->d_jump, jt.data(), jt.size() * 8, cudaMemcpyHostToDevice), "copy jump table");
   if (!rc) rc = cuda_check(cudaMalloc(&ctx->d_work, sizeof(u32)), "cudaMalloc(work counter)");
@@ -731,8 +752,11 @@ extern "C" int mgpu_set_chrom_config(mgpu_ctx* ctx, int chrom_id, const mgpu_con
   return MGPU_OK;
 }
 
+// Worker warps of a cell: a sweep over its LEFs takes two to four rounds of the block.
+static u32 workers_for(uint64_t nlefs) { return nlefs <= 256 ? 4 : (nlefs <= 1024 ? 8 : 16); }
+
 static int make_kparams(const mgpu_ctx* ctx, const ChromEntry& ch, uint64_t nlefs, KParams* P,
-                        uint64_t budget_override = 0) {
+                        uint64_t budget_override = 0, u32 workers = 0) {
   const mgpu_config& c = ch.own_cfg ? ch.cfg : ctx->cfg;
   std::memset(P, 0, sizeof(*P));
   if (nlefs == 0) return fail(MGPU_ERR_INVALID_ARG, "num_lefs must be positive");
@@ -810,23 +834,36 @@ static int make_kparams(const mgpu_ctx* ctx, const ChromEntry& ch, uint64_t nlef
   P->track_occ = c.track_1d_lef_position ? 1u : 0u;
   P->log_state = c.log_model_internal_state ? 1u : 0u;
   P->occ_bins = (ch.chrom.size + c.bin_size - 1) / c.bin_size;
-  // Layout: the header (scalars, PRNG ring, burn-in history, barrier bits) is always on chip;
-  // per-LEF arrays go on chip in priority order while they fit, the rest into a global slot.
+  // Layout: the scalars and the PRNG ring are always on chip; the burn-in history, the barrier bits
+  // and then the per-LEF arrays go on chip in priority order while they fit, the rest into a global
+  // slot.  A budget counts the ring as BUDGET_RING_BYTES whatever the block's own takes.
+  P->workers = workers ? workers : workers_for(nlefs);
   const u64 header = cell_header_bytes(ch.nb, P->hist_cap);
   const u64 budget = budget_override ? budget_override : ctx->smem_budget;
   const u64 limit = std::min<u64>(ctx->smem_limit, budget ? budget : ctx->smem_limit);
   if (header > limit)
     return fail(MGPU_ERR_UNSUPPORTED, "%u barriers need %llu B of shared memory (limit %llu)", ch.nb,
                 (unsigned long long)header, (unsigned long long)limit);
+  const u64 ring = ring_bytes(P->workers);
+  const u64 room = std::min<u64>(ctx->smem_limit, limit - BUDGET_RING_BYTES + ring);
   const u64 arr_bytes = ((u64)nlefs * 4 + 15) & ~15ull;
-  u64 smem_used = header, slot_used = 0;
+  u64 smem_used = CELL_HEADER_BYTES + ring, slot_used = 0;
+  const auto place = [&](u64 bytes, u32* off) {
+    const bool on_chip = smem_used + bytes <= room;
+    u64& used = on_chip ? smem_used : slot_used;
+    *off = (u32)used;
+    used += (bytes + 15) & ~15ull;
+    return on_chip ? 1u : 0u;
+  };
+  P->hist_smem = place(hist_bytes(P->hist_cap), &P->hist_off);
+  P->bst_smem = place(barrier_bits_bytes(ch.nb), &P->bst_off);
   P->arr_smem = 0;
   const int groups[][2] = {{ARR_REV, -1}, {ARR_FWD, -1}, {ARR_RR, -1}, {ARR_FR, -1}, {ARR_RM, -1},
                            {ARR_FM, -1},  {ARR_RC, -1},  {ARR_FC, -1}, {ARR_SR, ARR_SF}, {ARR_TMP, -1},
                            {ARR_BEP, -1}};
   for (const auto& g : groups) {
     const u64 bytes = g[1] < 0 ? arr_bytes : (((u64)nlefs * 8 + 15) & ~15ull);
-    const bool on_chip = smem_used + bytes <= limit;
+    const bool on_chip = smem_used + bytes <= room;
     u64& used = on_chip ? smem_used : slot_used;
     P->arr_off[g[0]] = (u32)used;
     if (g[1] >= 0) P->arr_off[g[1]] = (u32)(used + (u64)nlefs * 4);  // SF right after SR
@@ -958,6 +995,8 @@ static int status_from_stats(const mgpu_cell_stats* st, uint64_t n) {
         return fail(MGPU_ERR_INTERNAL, "cell %llu: the reference would read out of bounds", (unsigned long long)i);
       case DEV_ERR_NO_BOUND_LEF:
         return fail(MGPU_ERR_TIMEOUT, "cell %llu: no LEF could register a contact", (unsigned long long)i);
+      case DEV_ERR_RNG:
+        return fail(MGPU_ERR_TIMEOUT, "cell %llu: the random-number producers did not keep up", (unsigned long long)i);
       default:
         return fail(MGPU_ERR_INTERNAL, "cell %llu: device status %llu", (unsigned long long)i,
                     (unsigned long long)st[i].status);
@@ -1156,12 +1195,27 @@ extern "C" int mgpu_simulate_batch(mgpu_ctx* ctx, const mgpu_batch_task* tasks, 
     }
     budget = tuned->smem_budget;
   }
+  // one block size for the launch: the LEF-weighted median cell's
+  u32 workers = 0;
+  {
+    std::vector<uint64_t> nl(ntasks);
+    uint64_t total = 0, acc = 0;
+    for (uint64_t i = 0; i < ntasks; ++i) total += (nl[i] = tasks[i].num_lefs);
+    std::sort(nl.begin(), nl.end());
+    for (uint64_t v : nl) {
+      acc += v;
+      if (2 * acc >= total) {
+        workers = workers_for(v);
+        break;
+      }
+    }
+  }
   std::vector<BatchPlan> plans(keys.size());
   u32 smem_bytes = 0;
   u64 slot_bytes = 0;
   for (size_t p = 0; p < keys.size(); ++p) {
     const ChromEntry& ch = ctx->chroms[keys[p].chrom];
-    int rc = make_kparams(ctx, ch, keys[p].nlefs, &plans[p].P, budget);
+    int rc = make_kparams(ctx, ch, keys[p].nlefs, &plans[p].P, budget, workers);
     if (rc) return rc;
     plans[p].ch = DevChrom{ch.d_bars, ch.d_pos_flags, ch.nb};
     plans[p].target_epochs = keys[p].te;
@@ -1219,12 +1273,12 @@ extern "C" int mgpu_simulate_batch(mgpu_ctx* ctx, const mgpu_batch_task* tasks, 
   if (slot_bytes) {
     KParams Pslot = plans[0].P;
     Pslot.slot_bytes = slot_bytes;
-    rc = ensure_scratch(ctx, Pslot, resident_batch_cells(smem_bytes, ntasks, carveout, max_per_sm));
+    rc = ensure_scratch(ctx, Pslot, resident_batch_cells(workers, smem_bytes, ntasks, carveout, max_per_sm));
     if (rc) return rc;
   }
   char err[256] = {0};
   CK(cudaEventRecord(ctx->ev0, st));
-  rc = launch_simulate_batch((const BatchPlan*)d_plans.p, (const BatchTask*)d_tasks.p, ntasks, smem_bytes,
+  rc = launch_simulate_batch((const BatchPlan*)d_plans.p, (const BatchTask*)d_tasks.p, ntasks, workers, smem_bytes,
                              slot_bytes, (mgpu_cell_stats*)d_stats.p, ctx->d_jump, ctx->d_work, ctx->d_scratch,
                              ctx->scratch_bytes, carveout, max_per_sm, st, err, sizeof(err));
   if (rc) return fail(rc, "%s", err);

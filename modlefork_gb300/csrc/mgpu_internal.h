@@ -20,13 +20,20 @@ typedef int64_t i64;
 // Unbound unit / LEF sentinel for the 32-bit device encodings.
 constexpr u32 UNBOUND = 0xFFFFFFFFu;
 
-// PRNG ring: each of the 32 lanes of a cell's warp generates RNG_S consecutive draws of the
-// cell's single Xoshiro256++ stream per refill; RING is a power of two holding two blocks.
-constexpr int RNG_S = 16;
-constexpr int RNG_BLOCK = 32 * RNG_S;
-constexpr int RING = 2 * RNG_BLOCK;
-constexpr int JUMP_DISTANCE = 31 * RNG_S;  // lane state advance between two refills
-constexpr int JUMP_TABLE_ENTRIES = 64 * 16;  // 4-bit chunks of the 256-bit state
+// A cell's thread block: 4, 8 or 16 worker warps (the plan's choice) and one producer warp per 256
+// worker threads.  Each producer lane generates RNG_S consecutive draws of the cell's single
+// Xoshiro256++ stream per refill; the ring holds two refills.  A refill is at least four draws per
+// worker thread: a step consumes up to two per thread and window and gives them back one window later.
+constexpr u32 MAX_WORKERS = 16, MAX_PRODUCERS = 2;
+constexpr int RNG_S = 32;
+constexpr int JUMP_TABLE_ENTRIES = 64 * 16;  // 4-bit chunks of the 256-bit state, one table per producer count
+constexpr u32 NORMAL_LAYERS = 128;           // fixed-point ziggurat layers, after the jump tables
+MGPU_HD inline u32 producer_warps(u32 workers) { return workers > 8 ? 2 : 1; }
+MGPU_HD inline u32 block_threads(u32 workers) { return 32 * (workers + producer_warps(workers)); }
+constexpr int MAX_BLOCK_THREADS = 32 * (MAX_WORKERS + MAX_PRODUCERS);
+MGPU_HD inline u64 ring_bytes(u32 workers) { return (u64)producer_warps(workers) * 32 * RNG_S * 2 * 8; }
+// state advance of a producer lane between two refills: over the other lanes' draws
+MGPU_HD inline int jump_distance(u32 producers) { return (32 * (int)producers - 1) * RNG_S; }
 
 // Compact 32-bit collision word: event bits (collision_encoding.hpp:91-96) in bits 27..31,
 // index in bits 0..26.
@@ -105,6 +112,8 @@ struct KParams {
   // memory of the cell or inside its global scratch slot
   u32 arr_off[12];
   u32 arr_smem;    // bit k set: array k lives in shared memory
+  u32 workers;     // worker warps of the cell's block
+  u32 bst_off, bst_smem, hist_off, hist_smem;  // barrier bits and burn-in history, placed likewise
   u32 smem_bytes;  // dynamic shared memory of one cell
   u64 slot_bytes;  // global scratch of one resident cell (arrays that do not fit on chip)
   u32 debug_flags; // DBG_* bits: force the exact serial implementation of a step
@@ -158,14 +167,17 @@ enum : u32 {
   DEV_ERR_MOVE_RANGE = 2,    // a move does not fit the 32-bit encoding
   DEV_ERR_BAD_STATE = 3,     // the reference would read out of bounds here
   DEV_ERR_NO_BOUND_LEF = 4,  // contact sampling found no bound LEF within bounds
+  DEV_ERR_RNG = 5,           // the producer warps did not deliver draws in time
 };
 
-// Fixed part of a cell's shared memory: scalars, PRNG ring, burn-in history, barrier bits.
+// Fixed parts of a cell's shared memory after the scalars: PRNG ring, burn-in history, barrier bits.
+MGPU_HD inline u64 hist_bytes(u64 hist_cap) { return 2 * hist_cap * 8; }
+MGPU_HD inline u64 barrier_bits_bytes(u64 nbarriers) { return (((nbarriers + 31) / 32) * 4 + 15) & ~15ull; }
+// What a shared-memory budget counts besides the per-LEF arrays: a fixed 8 KiB for the ring, whatever
+// the block's own ring takes on top of that.
+constexpr u64 BUDGET_RING_BYTES = 8192;
 MGPU_HD inline u64 cell_header_bytes(u64 nbarriers, u64 hist_cap) {
-  const u64 ring = (u64)RING * 8;
-  const u64 hist = 2 * hist_cap * 8;
-  const u64 bars = (((nbarriers + 31) / 32) * 4 + 15) & ~15ull;
-  return CELL_HEADER_BYTES + ring + hist + bars;
+  return CELL_HEADER_BYTES + BUDGET_RING_BYTES + hist_bytes(hist_cap) + barrier_bits_bytes(nbarriers);
 }
 
 // Host side helpers implemented in mgpu_host.cpp, device launchers in mgpu_device.cu.
@@ -207,13 +219,13 @@ struct BatchTask {
   u32 plan;
   u32 pad;
 };
-int launch_simulate_batch(const BatchPlan* plans, const BatchTask* tasks, u64 ntasks, u32 smem_bytes,
+int launch_simulate_batch(const BatchPlan* plans, const BatchTask* tasks, u64 ntasks, u32 workers, u32 smem_bytes,
                           u64 slot_bytes, mgpu_cell_stats* stats, const void* jump_table, u32* work_counter,
                           char* gscratch, u64 gscratch_bytes, u32 carveout_pct, u32 max_per_sm, void* stream,
                           char* errbuf, int errlen);
 // Grid of a batched launch with the given per-cell shared memory (optionally capped per SM, with
 // a shared-memory carveout preference in percent, 0 = driver default).
-u64 resident_batch_cells(u32 smem_bytes, u64 ntasks, u32 carveout_pct = 0, u32 max_per_sm = 0);
+u64 resident_batch_cells(u32 workers, u32 smem_bytes, u64 ntasks, u32 carveout_pct = 0, u32 max_per_sm = 0);
 
 // Pixel table of a band (mgpu_pixels.cu): counts[i] = non-zero pixels of bin1 row i,
 // offsets[0..ncols] their exclusive scan; then the (bin1, bin2, count) pixels.
