@@ -120,6 +120,8 @@ struct Scalars {
 };
 static_assert(sizeof(Scalars) <= CELL_HEADER_BYTES, "scalars do not fit the cell header");
 
+constexpr u32 TRIAL_WORDS = 65;  // outcomes of up to 2048 draws, and a word read past them
+
 // Scratch of the block-wide steps.
 struct BlockTmp {
   u32 cnt[2][32];       // scan2
@@ -128,34 +130,117 @@ struct BlockTmp {
   u32 rem[16], rembase[16];
   u32 nrem, tie, tie2;
   u32 dev[16], okm[16], dus[16];  // sample_contacts
+  u32 trial[TRIAL_WORDS];  // secondary_dir_block
   u32 used, qend, nr, nf, released, missed, flag;
   u64 sum;
   ulonglong2 zt[128];   // normal ziggurat per layer: {draws below this are accepted, width * 2^60}
+  float2 zy[128];       // and the density at its lower and upper edge: {y_i, y_{i+1} - y_i}
 };
 
 // Pointers of one cell (lives in shared memory; identical for every thread).
 struct Cell {
   Scalars* sc;
-  BlockTmp* bt;
   u64* ring;
   u32 T;      // worker threads (0: no producers, one thread generates its own draws)
   u32 rmask;  // ring capacity - 1
   u32 lim;    // draws the producers always provide beyond the last published position
+  u32 off[NARR], bst_off;  // offsets of the arrays in dynamic shared memory (all_smem)
+  u32 all_smem;            // every array lives there
   u32 *rev, *fwd, *rr, *fr, *rm, *fm, *rc, *fc, *sr, *sf, *tmp, *bep;
   u32* bst;
   double *hcfx, *havg;
   const DevBarrier* bar;
   const uint2* bpf;  // {pos, flags}
   u32 nb;
-  u32 nl;
   const ulonglong2* jt;
   u32* band;
 };
 
+// The cell a block is working on.  Shared variables of the translation unit, so that every function
+// addresses them directly: passed by reference they become generic pointers, and each access to a
+// per-LEF array then starts with a dependent load of its pointer.
+__shared__ Cell g_c;
+__shared__ Scalars g_sc;
+__shared__ BlockTmp g_bt;
+__shared__ __align__(16) KParams g_P;
+extern __shared__ __align__(16) char dyn_smem[];  // the PRNG ring, then what the plan placed on chip
+
+// A per-LEF array of 32-bit words: an offset into dynamic shared memory when the plan placed every
+// array there (SM), which the compiler turns into shared-memory accesses with 32-bit addresses,
+// otherwise a generic pointer (shared memory or the block's global slot).
+template <bool SM>
+struct Arr;
+template <>
+struct Arr<true> {
+  u32 off;
+  template <class I>
+  __device__ __forceinline__ u32& operator[](I i) const {
+    return *reinterpret_cast<u32*>(dyn_smem + off + 4u * (u32)i);
+  }
+  __device__ __forceinline__ u64& at64(u32 i) const { return *reinterpret_cast<u64*>(dyn_smem + off + 8u * i); }
+  __device__ __forceinline__ Arr operator+(u32 k) const { return Arr{off + 4u * k}; }
+};
+template <>
+struct Arr<false> {
+  u32* p;
+  template <class I>
+  __device__ __forceinline__ u32& operator[](I i) const {
+    return p[(u32)i];
+  }
+  __device__ __forceinline__ u64& at64(u32 i) const { return reinterpret_cast<u64*>(p)[i]; }
+  __device__ __forceinline__ Arr operator+(u32 k) const { return Arr{p + k}; }
+};
+
+// What a step reads of the cell, loaded once at its start (fields it does not use cost nothing).
+template <bool SM>
+struct View {
+  u32 T, rmask, lim, nb;
+  Arr<SM> rev, fwd, rr, fr, rm, fm, rc, fc, sr, sf, tmp, bep, bst;
+  const DevBarrier* bar;
+  const uint2* bpf;
+  u32* band;
+  __device__ __forceinline__ View()
+      : T(g_c.T), rmask(g_c.rmask), lim(g_c.lim), nb(g_c.nb), bar(g_c.bar), bpf(g_c.bpf), band(g_c.band) {
+    if constexpr (SM) {
+      rev.off = g_c.off[ARR_REV];
+      fwd.off = g_c.off[ARR_FWD];
+      rr.off = g_c.off[ARR_RR];
+      fr.off = g_c.off[ARR_FR];
+      rm.off = g_c.off[ARR_RM];
+      fm.off = g_c.off[ARR_FM];
+      rc.off = g_c.off[ARR_RC];
+      fc.off = g_c.off[ARR_FC];
+      sr.off = g_c.off[ARR_SR];
+      sf.off = g_c.off[ARR_SF];
+      tmp.off = g_c.off[ARR_TMP];
+      bep.off = g_c.off[ARR_BEP];
+      bst.off = g_c.bst_off;
+    } else {
+      rev.p = g_c.rev;
+      fwd.p = g_c.fwd;
+      rr.p = g_c.rr;
+      fr.p = g_c.fr;
+      rm.p = g_c.rm;
+      fm.p = g_c.fm;
+      rc.p = g_c.rc;
+      fc.p = g_c.fc;
+      sr.p = g_c.sr;
+      sf.p = g_c.sf;
+      tmp.p = g_c.tmp;
+      bep.p = g_c.bep;
+      bst.p = g_c.bst;
+    }
+  }
+};
+
 // Position and flags of barrier i through the read-only data path (8 bytes per barrier, so the
 // sweeps over the barrier track stay in cache).
-__device__ __forceinline__ u32 bar_pos(const Cell& c, u32 i) { return __ldg(&c.bpf[i].x); }
-__device__ __forceinline__ u32 bar_flags(const Cell& c, u32 i) { return __ldg(&c.bpf[i].y); }
+__device__ __forceinline__ u32 bar_pos(const uint2* bpf, u32 i) { return __ldg(&bpf[i].x); }
+__device__ __forceinline__ u32 bar_flags(const uint2* bpf, u32 i) { return __ldg(&bpf[i].y); }
+template <class A>
+__device__ __forceinline__ bool bar_active(const A& bst, u32 i) {
+  return (bst[i >> 5] >> (i & 31)) & 1u;
+}
 
 // ---------------------------------------------------------------------------------------
 // PRNG ring
@@ -175,9 +260,9 @@ __device__ __forceinline__ u64 global_ns() {
 }
 
 // Barrier of the cell's worker warps (the producer warps do not take part).
-__device__ __forceinline__ void wsync(const Cell& c) { asm volatile("barrier.sync 1, %0;" ::"r"(c.T) : "memory"); }
+__device__ __forceinline__ void wsync(u32 T) { asm volatile("barrier.sync 1, %0;" ::"r"(T) : "memory"); }
 // The same, returning whether any worker thread passed a true predicate.
-__device__ __forceinline__ bool wsync_or(const Cell& c, bool p) {
+__device__ __forceinline__ bool wsync_or(u32 T, bool p) {
   u32 r;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
@@ -185,7 +270,7 @@ __device__ __forceinline__ bool wsync_or(const Cell& c, bool p) {
       "barrier.red.or.pred q, 1, %2, p;\n\t"
       "selp.u32 %0, 1, 0, q;\n\t}"
       : "=r"(r)
-      : "r"((u32)p), "r"(c.T)
+      : "r"((u32)p), "r"(T)
       : "memory");
   return r != 0;
 }
@@ -273,20 +358,22 @@ __device__ __noinline__ void rng_wait(Cell& c, u32 rp, u32 n) {
 
 // Every worker thread that reads draws [rp, rp + n) calls this first (n <= c.lim minus the draws
 // consumed since the last rng_publish).
-__device__ __forceinline__ void rng_ensure(Cell& c, u64 rp, u32 n) {
-  if (ld_acquire(&c.sc->gpos) - (u32)rp < n) rng_wait(c, (u32)rp, n);
+__device__ __forceinline__ void rng_ensure(u64 rp, u32 n) {
+  if (ld_acquire(&g_sc.gpos) - (u32)rp < n) rng_wait(g_c, (u32)rp, n);
 }
 
 // Thread 0, after a wsync that follows every read of the draws before rp: record the position
 // and hand the ring space back to the producers.
-__device__ __forceinline__ void rng_publish(Cell& c, u64 rp) {
+__device__ __forceinline__ void rng_publish(u64 rp) {
   if (threadIdx.x == 0) {
-    c.sc->rpos = rp;
-    st_release(&c.sc->rpub, (u32)rp);
+    g_sc.rpos = rp;
+    st_release(&g_sc.rpub, (u32)rp);
   }
 }
 
-__device__ __forceinline__ u64 ring_at(const Cell& c, u64 k) { return c.ring[(u32)k & c.rmask]; }
+__device__ __forceinline__ u64 ring_at(u32 rmask, u64 k) {
+  return *reinterpret_cast<const u64*>(dyn_smem + 8u * ((u32)k & rmask));
+}
 
 // Thread 0 only (the other workers wait at a barrier): next draw of the stream.  Without
 // producer warps (c.T == 0, the sampler probe) the thread generates it itself.
@@ -300,14 +387,14 @@ __device__ __noinline__ u64 rng_serial(Cell& c) {
       rng_wait(c, (u32)sc->rpos, 1);
     }
   }
-  const u64 v = ring_at(c, sc->rpos);
+  const u64 v = c.ring[(u32)sc->rpos & c.rmask];
   sc->rpos++;
   if (c.T) st_release(&sc->rpub, (u32)sc->rpos);
   return v;
 }
 
-__device__ __forceinline__ void prof_add(Cell& c, u32 k, u64 v) {
-  if (threadIdx.x == 0 && c.sc->prof) atomicAdd((unsigned long long*)&c.sc->prof[k], (unsigned long long)v);
+__device__ __forceinline__ void prof_add(u32 k, u64 v) {
+  if (threadIdx.x == 0 && g_sc.prof) atomicAdd((unsigned long long*)&g_sc.prof[k], (unsigned long long)v);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -321,6 +408,7 @@ __device__ u64 s_uniform_int(Cell& c, u64 a, u64 b) {
   if (range == ~0ull) return rng_serial(c) + a;
   u64 bucket = ~0ull / (range + 1);
   if (~0ull % (range + 1) == range) ++bucket;
+#pragma unroll 1
   for (u64 it = 0; it < 1000; ++it) {
     const u64 r = rng_serial(c) / bucket;
     if (r <= range) return a + r;
@@ -338,6 +426,7 @@ __device__ __forceinline__ bool s_trial(Cell& c, const Trial& t) {
 __device__ __forceinline__ double u01_of(u64 u) { return (double)u * (1.0 / 18446744073709551616.0); }
 
 __device__ double s_uniform01(Cell& c) {
+#pragma unroll 1
   for (int it = 0; it < 1000; ++it) {
     const double r = u01_of(rng_serial(c));
     if (r < 1.0) return r;
@@ -372,12 +461,11 @@ struct SerialSrc {
 };
 
 struct RingSrc {
-  const u64* ring;
   u32 mask, pos, end;
   u32 n;
   __device__ bool next(u64& u) {
     if (pos == end) return false;
-    u = ring[pos & mask];
+    u = *reinterpret_cast<const u64*>(dyn_smem + 8u * (pos & mask));
     ++pos;
     ++n;
     return true;
@@ -400,6 +488,7 @@ __device__ __forceinline__ bool below_exp(double y, double a) {
 // uniform_01<double> on one draw per attempt (values equal to 1 are rejected)
 template <class Src>
 __device__ int uniform01_t(Src& g, double& r) {
+#pragma unroll 1
   for (int it = 0; it < 1000; ++it) {
     u64 u;
     if (!g.next(u)) return SMP_DRY;
@@ -413,6 +502,7 @@ __device__ int uniform01_t(Src& g, double& r) {
 template <class Src>
 __device__ int unit_exponential_t(Src& g, double& out) {
   double shift = 0;
+#pragma unroll 1
   for (int it = 0; it < 100000; ++it) {
     u64 u;
     if (!g.next(u)) return SMP_DRY;
@@ -442,6 +532,7 @@ __device__ int unit_exponential_t(Src& g, double& out) {
 template <class Src>
 __device__ int normal_tail_t(Src& g, double& out) {
   const double tail_start = mgpu_zig_normal_x[1];
+#pragma unroll 1
   for (int it = 0; it < 100000; ++it) {
     double e1, e2;
     int r = unit_exponential_t(g, e1);
@@ -461,6 +552,7 @@ __device__ int normal_tail_t(Src& g, double& out) {
 // unit_normal_distribution: 128-layer ziggurat, sign from bit 0 of the layer byte
 template <class Src>
 __device__ int unit_normal_t(Src& g, double& out) {
+#pragma unroll 1
   for (int it = 0; it < 100000; ++it) {
     u64 u;
     if (!g.next(u)) return SMP_DRY;
@@ -522,6 +614,7 @@ __device__ __noinline__ u64 s_poisson(Cell& c, const KParams& P) {
     double p = P.pois_exp_mean;
     u64 x = 0;
     double u = s_uniform01(c);
+#pragma unroll 1
     while (u > p) {
       u = u - p;
       ++x;
@@ -535,6 +628,7 @@ __device__ __noinline__ u64 s_poisson(Cell& c, const KParams& P) {
   }
   const double smu = P.pois_smu, b = P.pois_b, a = P.pois_a, inv_alpha = P.pois_inv_alpha,
                v_r = P.pois_v_r;
+#pragma unroll 1
   for (int it = 0; it < 100000; ++it) {
     double u;
     double v = s_uniform01(c);
@@ -592,6 +686,7 @@ __device__ __noinline__ i64 s_binomial(Cell& c, const KParams& P, i64 t_, double
     double r = q_n;
     double u = s_uniform01(c);
     i64 x = 0;
+#pragma unroll 1
     while (u > r) {
       u = u - r;
       ++x;
@@ -613,6 +708,7 @@ __device__ __noinline__ i64 s_binomial(Cell& c, const KParams& P, i64 t_, double
   const double u_rv_r = 0.86 * v_r;
   i64 res = 0;
   bool done = false;
+#pragma unroll 1
   for (int it = 0; it < 100000 && !done; ++it) {
     double u;
     double v = s_uniform01(c);
@@ -702,9 +798,11 @@ __device__ __noinline__ void rank_dir_serial(Cell& c, u32 dir, u32 n, bool parti
   } else {
     pdq_sort(R, 0, n, cmp);
   }
+#pragma unroll 1
   for (u32 i = 1; i < n; ++i) {
     if (pos[R[i - 1]] == pos[R[i]]) {
       const u32 begin = i - 1;
+#pragma unroll 1
       for (; i < n; ++i) {
         if (pos[R[i - 1]] != pos[R[i]]) break;
       }
@@ -722,6 +820,7 @@ __device__ __noinline__ void adjust_dir_serial(Cell& c, const KParams& P, u32 di
   if (n == 0) return;
   const u64 start = P.start, end = P.end;
   if (dir == 0) {
+#pragma unroll 1
     for (u32 i = n - 1; i > 0; --i) {
       const u32 i1 = c.rr[i - 1], i2 = c.rr[i];
       if (c.bep[i1] != UNBOUND && c.bep[i2] != UNBOUND) {
@@ -733,6 +832,7 @@ __device__ __noinline__ void adjust_dir_serial(Cell& c, const KParams& P, u32 di
       }
     }
   } else {
+#pragma unroll 1
     for (u32 i = 1; i < n; ++i) {
       const u32 i1 = c.fr[i - 1], i2 = c.fr[i];
       if (c.bep[i1] != UNBOUND && c.bep[i2] != UNBOUND) {
@@ -746,12 +846,28 @@ __device__ __noinline__ void adjust_dir_serial(Cell& c, const KParams& P, u32 di
   }
 }
 
-// compute_lef_lef_collision_pos (simulation.cpp:514-542)
+// compute_lef_lef_collision_pos (simulation.cpp:514-542).  The reference rounds the double
+// fwd_move * (delta / rel); for moves that add up to less than 46340 bp its error is below 2^-35
+// while a value that is not exactly halfway between two integers is at least 1 / (2 rel) > 2^-17
+// away from one, so the rounded quotient of 32-bit integers is the same number.  Only an exact
+// half, whose side the doubles' rounding decides, and longer moves are evaluated in doubles (a
+// division takes some 30 instructions on a pipe that runs at 1/64 of the FP32 rate).
 __device__ __forceinline__ void lef_lef_collision_pos(u64 rev_pos, u64 fwd_pos, u64 rev_move,
                                                       u64 fwd_move, u64& p_rev, u64& p_fwd) {
-  const u64 rel = rev_move + fwd_move;
-  const double t = (double)(rev_pos - fwd_pos) / (double)rel;
-  const u64 cp = fwd_pos + (u64)round((double)fwd_move * t);
+  const u64 rel = rev_move + fwd_move, delta = rev_pos - fwd_pos;
+  u64 off = 0;
+  bool exact = true;
+  if (rel - 1 < 46339 && delta <= rel) {
+    const u32 num = 2 * (u32)fwd_move * (u32)delta + (u32)rel, den = 2 * (u32)rel;  // below 2^32
+    const u32 q = num / den;
+    exact = q * den == num;
+    off = q;
+  }
+  if (exact) {
+    const double t = (double)delta / (double)rel;
+    off = (u64)round((double)fwd_move * t);
+  }
+  const u64 cp = fwd_pos + off;
   if (cp == fwd_pos) {
     p_rev = cp + 1;
     p_fwd = cp;
@@ -761,15 +877,16 @@ __device__ __forceinline__ void lef_lef_collision_pos(u64 rev_pos, u64 fwd_pos, 
   }
 }
 
-
 // detect_units_at_chrom_boundaries (simulation_detect_collisions.cpp:30-125); lane 0.  The
 // loops stop at the first unit that is neither at nor about to reach a chromosome end.
-__device__ void detect_boundaries_serial(Cell& c, const KParams& P, u32 n, u64& n5, u64& n3) {
+template <class C>
+__device__ void detect_boundaries_serial(const C& c, const KParams& P, u32 n, u64& n5, u64& n3) {
   n5 = 0;
   n3 = 0;
   const u64 start = P.start, end = P.end;
   const u64 first_fwd_pos = pos64(c.fwd[c.fr[0]]);
   u32 last_rev = UNBOUND;
+#pragma unroll 1
   for (u32 k = n; k > 0; --k) {
     if (c.bep[c.rr[k - 1]] != UNBOUND) {
       last_rev = c.rr[k - 1];
@@ -777,10 +894,11 @@ __device__ void detect_boundaries_serial(Cell& c, const KParams& P, u32 n, u64& 
     }
   }
   if (last_rev == UNBOUND) {
-    set_status(c, DEV_ERR_BAD_STATE);
+    set_status(g_c, DEV_ERR_BAD_STATE);
     last_rev = c.rr[0];
   }
   const u64 last_rev_pos = pos64(c.rev[last_rev]);
+#pragma unroll 1
   for (u32 i = 0; i < n; ++i) {
     const u32 idx = c.rr[i];
     const u64 pos = pos64(c.rev[idx]);
@@ -796,6 +914,7 @@ __device__ void detect_boundaries_serial(Cell& c, const KParams& P, u32 n, u64& 
       break;
     }
   }
+#pragma unroll 1
   for (u32 i = n - 1; i > 0; --i) {
     const u32 idx = c.fr[i];
     const u64 pos = pos64(c.fwd[idx]);
@@ -817,7 +936,6 @@ __device__ void detect_boundaries_serial(Cell& c, const KParams& P, u32 n, u64& 
   }
 }
 
-__device__ __forceinline__ bool bar_active(const Cell& c, u32 i) { return (c.bst[i >> 5] >> (i & 31)) & 1u; }
 
 // detect_lef_bar_collisions (simulation_detect_collisions.cpp:128-252); lane 0
 __device__ __noinline__ void detect_lef_bar_serial(Cell& c, const KParams& P, u32 n, u64 n5, u64 n3) {
@@ -825,11 +943,13 @@ __device__ __noinline__ void detect_lef_bar_serial(Cell& c, const KParams& P, u3
   u32 unit_idx = c.rr[j];
   u64 unit_pos = pos64(c.rev[unit_idx]);
   bool rev_done = false;
+#pragma unroll 1
   for (u32 i = 0; i < c.nb && !rev_done; ++i) {
-    if (!bar_active(c, i)) continue;
-    const u32 dir = bar_flags(c, i) & BF_DIR_MASK;
+    if (!bar_active(c.bst, i)) continue;
+    const u32 dir = bar_flags(c.bpf, i) & BF_DIR_MASK;
     const Trial& tr = P.lef_bar[dir == MGPU_DIR_REV ? 0 : 1];
-    const u64 bpos = bar_pos(c, i);
+    const u64 bpos = bar_pos(c.bpf, i);
+#pragma unroll 1
     while (unit_pos <= bpos) {
       if (++j == n) {
         rev_done = true;
@@ -849,11 +969,13 @@ __device__ __noinline__ void detect_lef_bar_serial(Cell& c, const KParams& P, u3
   j = n - min(n3, n3 - 1);
   unit_idx = c.fr[--j];
   unit_pos = pos64(c.fwd[unit_idx]);
+#pragma unroll 1
   for (u64 i = (u64)c.nb - 1; i != ~0ull; --i) {
-    if (!bar_active(c, (u32)i)) continue;
-    const u32 dir = bar_flags(c, i) & BF_DIR_MASK;
+    if (!bar_active(c.bst, (u32)i)) continue;
+    const u32 dir = bar_flags(c.bpf, i) & BF_DIR_MASK;
     const Trial& tr = P.lef_bar[dir == MGPU_DIR_FWD ? 0 : 1];
-    const u64 bpos = bar_pos(c, i);
+    const u64 bpos = bar_pos(c.bpf, i);
+#pragma unroll 1
     while (unit_pos >= bpos) {
       if (--j == ~0ull) return;
       unit_idx = c.fr[j];
@@ -868,16 +990,18 @@ __device__ __noinline__ void detect_lef_bar_serial(Cell& c, const KParams& P, u3
   }
 }
 
-__device__ __forceinline__ u64 barrier_pos_checked(Cell& c, u32 idx) {
+template <class C>
+__device__ __forceinline__ u64 barrier_pos_checked(const C& c, u32 idx) {
   if (idx >= c.nb) {
-    set_status(c, DEV_ERR_BAD_STATE);
+    set_status(g_c, DEV_ERR_BAD_STATE);
     return 0;
   }
-  return bar_pos(c, idx);
+  return bar_pos(c.bpf, idx);
 }
 
 // The collision words of one tested primary pair (simulation_detect_collisions.cpp:344-399).
-__device__ __forceinline__ void primary_pair_update(Cell& c, u32 rev_idx, u32 fwd_idx, u64 rev_pos,
+template <class C>
+__device__ __forceinline__ void primary_pair_update(const C& c, u32 rev_idx, u32 fwd_idx, u64 rev_pos,
                                                     u64 fwd_pos, u64 rmv, u64 fmv) {
   u64 cpr, cpf;
   lef_lef_collision_pos(rev_pos, fwd_pos, rmv, fmv, cpr, cpf);
@@ -906,16 +1030,19 @@ __device__ __noinline__ void detect_primary_serial(Cell& c, const KParams& P, u3
   u64 i1 = 0, j1 = n5;
   const u64 i2 = n - min(n3, n3 - 1);
   const u64 j2 = n;
+#pragma unroll 1
   for (u64 it = 0; it < 4ull * n + 16; ++it) {
     u32 rev_idx = c.rr[j1];
     u64 rev_pos = pos64(c.rev[rev_idx]);
     u32 fwd_idx = c.fr[i1];
     u64 fwd_pos = pos64(c.fwd[fwd_idx]);
+#pragma unroll 1
     while (rev_pos <= fwd_pos) {
       if (++j1 == j2) return;
       rev_idx = c.rr[j1];
       rev_pos = pos64(c.rev[rev_idx]);
     }
+#pragma unroll 1
     while (fwd_pos < rev_pos) {
       if (++i1 == i2) return;
       fwd_idx = c.fr[i1];
@@ -934,6 +1061,7 @@ __device__ __noinline__ void detect_primary_serial(Cell& c, const KParams& P, u3
 
 // process_secondary_lef_lef_collisions (simulation_detect_collisions.cpp:404-518); lane 0
 __device__ __noinline__ void process_secondary_serial(Cell& c, const KParams& P, u32 n, u64 n5, u64 n3) {
+#pragma unroll 1
   for (u64 i = max((u64)1, n5); i < n; ++i) {
     const u32 idx1 = c.rr[i - 1];
     if (!cw_occurred(c.rc[idx1])) continue;
@@ -952,6 +1080,7 @@ __device__ __noinline__ void process_secondary_serial(Cell& c, const KParams& P,
     }
   }
   u64 i = n - min(n3, n3 - 1) - 1;
+#pragma unroll 1
   for (; i > 0 && i != ~0ull; --i) {
     const u32 idx2 = c.fr[i];
     if (!cw_occurred(c.fc[idx2])) continue;
@@ -972,7 +1101,8 @@ __device__ __noinline__ void process_secondary_serial(Cell& c, const KParams& P,
 }
 
 // One rev candidate of fix_secondary_lef_lef_collisions (simulation_detect_collisions.cpp:556-605).
-__device__ __forceinline__ void fix_rev_at(Cell& c, u64 start, u64 i) {
+template <class C>
+__device__ __forceinline__ void fix_rev_at(const C& c, u64 start, u64 i) {
   const u32 idx2 = c.rr[i];
   const u32 idx1 = c.rr[i - 1];
   const u64 pos1 = pos64(c.rev[idx1]) - c.rm[idx1];
@@ -995,7 +1125,8 @@ __device__ __forceinline__ void fix_rev_at(Cell& c, u64 start, u64 i) {
 }
 
 // One fwd candidate (simulation_detect_collisions.cpp:608-646).
-__device__ __forceinline__ void fix_fwd_at(Cell& c, u64 end, u64 i) {
+template <class C>
+__device__ __forceinline__ void fix_fwd_at(const C& c, u64 end, u64 i) {
   const u32 idx1 = c.fr[i];
   const u32 idx2 = c.fr[i + 1];
   const u64 f1 = pos64(c.fwd[idx1]);
@@ -1020,9 +1151,11 @@ __device__ __forceinline__ void fix_fwd_at(Cell& c, u64 end, u64 i) {
 // fix_secondary_lef_lef_collisions (simulation_detect_collisions.cpp:520-647); lane 0
 __device__ __noinline__ void fix_secondary_serial(Cell& c, const KParams& P, u32 n, u64 n5, u64 n3) {
   const u64 num_active_fwd = n - min(n3, n3 - 1);
+#pragma unroll 1
   for (u64 i = max((u64)1, n5); i < n; ++i) {
     if (cw_avoided_as(c.rc[c.rr[i]], EV_SECONDARY)) fix_rev_at(c, P.start, i);
   }
+#pragma unroll 1
   for (u64 i = 0; i + 1 < num_active_fwd; ++i) {
     if (cw_avoided_as(c.fc[c.fr[i]], EV_SECONDARY)) fix_fwd_at(c, P.end, i);
   }
@@ -1041,15 +1174,17 @@ __device__ __noinline__ void fix_secondary_serial(Cell& c, const KParams& P, u32
 struct Scan2 {
   u32 off0, off1, total;
 };
-__device__ __forceinline__ Scan2 scan2(Cell& c, u32 buf, bool f0, bool f1) {
+template <bool SM>
+__device__ __forceinline__ Scan2 scan2(u32 buf, bool f0, bool f1) {
+  const View<SM> c;
   const unsigned m0 = __ballot_sync(FULL, f0), m1 = __ballot_sync(FULL, f1);
   const u32 w = threadIdx.x >> 5, l = ln();
-  u32* cnt = c.bt->cnt[buf];
+  u32* cnt = g_bt.cnt[buf];
   if (l == 0) {
     cnt[w] = __popc(m0);
     cnt[16 + w] = __popc(m1);
   }
-  wsync(c);
+  wsync(c.T);
   const u32 v = (l & 15u) < (c.T >> 5) ? cnt[l] : 0u;
   const u32 before = (l & 15u) < w ? v : 0u;
   const u32 b0 = __reduce_add_sync(FULL, l < 16 ? before : 0u);
@@ -1062,33 +1197,39 @@ __device__ __forceinline__ Scan2 scan2(Cell& c, u32 buf, bool f0, bool f1) {
 }
 
 // ExtrusionBarriers::init_states (extrusion_barriers.cpp:220-231)
-__device__ __noinline__ u64 barriers_init(Cell& c, u64 rp) {
+template <bool SM>
+__device__ __noinline__ u64 barriers_init(u64 rp) {
+  const View<SM> c;
   const u32 T = c.T;
   u32 buf = 0;
+#pragma unroll 1
   for (u32 base = 0; base < c.nb; base += T) {
     const u32 i = base + threadIdx.x;
-    const bool need = i < c.nb && (bar_flags(c, i) & BF_OCC_DRAWS);
-    const Scan2 sc2 = scan2(c, buf, need, false);
-    rng_publish(c, rp);
+    const bool need = i < c.nb && (bar_flags(c.bpf, i) & BF_OCC_DRAWS);
+    const Scan2 sc2 = scan2<SM>(buf, need, false);
+    rng_publish(rp);
     buf ^= 1;
-    rng_ensure(c, rp, T);
-    const bool occ = need && ring_at(c, rp + sc2.off0) <= c.bar[i].t_occ;
+    rng_ensure(rp, T);
+    const bool occ = need && ring_at(c.rmask, rp + sc2.off0) <= c.bar[i].t_occ;
     const unsigned om = __ballot_sync(FULL, occ);
     if (ln() == 0 && i < c.nb) c.bst[i >> 5] = om;
     rp += sc2.total;
   }
-  wsync(c);
-  rng_publish(c, rp);
+  wsync(c.T);
+  rng_publish(rp);
   return rp;
 }
 
 // ExtrusionBarriers::next_state (extrusion_barriers.cpp:145-161): one draw per barrier.
-__device__ __noinline__ u64 barriers_next(Cell& c, u64 rp) {
+template <bool SM>
+__device__ __noinline__ u64 barriers_next(u64 rp) {
+  const View<SM> c;
   const u32 T = c.T, nb = c.nb;
   const uint2* __restrict__ bpf = c.bpf;
   const DevBarrier* __restrict__ bar = c.bar;
+#pragma unroll 1
   for (u32 base = 0; base < nb; base += 2 * T) {
-    rng_ensure(c, rp, 2 * T);
+    rng_ensure(rp, 2 * T);
     u32 f[2];
     u64 thr[2];
     bool st[2];
@@ -1103,14 +1244,14 @@ __device__ __noinline__ u64 barriers_next(Cell& c, u64 rp) {
 #pragma unroll
     for (u32 h = 0; h < 2; ++h) {
       const u32 k = h * T + threadIdx.x, i = base + k;
-      const bool above = ring_at(c, rp + k) >= thr[h];
+      const bool above = ring_at(c.rmask, rp + k) >= thr[h];
       const bool nst = st[h] ? !(!(f[h] & BF_ACT_NEVER) && above) : !(f[h] & BF_INA_NEVER) && above;
       const unsigned m = __ballot_sync(FULL, i < nb && nst);
       if (ln() == 0 && i < nb) c.bst[i >> 5] = m;
     }
     rp += min(2 * T, nb - base);
-    wsync(c);
-    rng_publish(c, rp);
+    wsync(c.T);
+    rng_publish(rp);
   }
   return rp;
 }
@@ -1119,47 +1260,53 @@ __device__ __noinline__ u64 barriers_next(Cell& c, u64 rp) {
 // selected LEF in index order.  Selection: mode 0 = unbound LEFs (the epoch loop), 1 =
 // nonzero entries of mask, 2 = every LEF (an empty mask in the reference).  The selected LEFs are
 // compacted first: they are a few per cent of all, and each takes a 64-bit division.
-__device__ __noinline__ u64 bind_lefs(Cell& c, const KParams& P, u64 rp, u32 n, u32 epoch, int mode,
+template <bool SM>
+__device__ __noinline__ u64 bind_lefs(u64 rp, u32 n, u32 epoch, int mode,
                                       const u64* mask) {
+  const View<SM> c;
+  const KParams& P = g_P;
   const u32 T = c.T;
-  u32* list = c.tmp;
+  const auto list = c.tmp;
   u32 nsel = 0, buf = 0;
+#pragma unroll 1
   for (u32 base = 0; base < n; base += 2 * T) {
     const u32 i0 = base + threadIdx.x, i1 = i0 + T;
     const bool f0 = i0 < n && (mode == 0 ? c.bep[i0] == UNBOUND : (mode == 1 ? mask[i0] != 0 : true));
     const bool f1 = i1 < n && (mode == 0 ? c.bep[i1] == UNBOUND : (mode == 1 ? mask[i1] != 0 : true));
-    const Scan2 s = scan2(c, buf, f0, f1);
+    const Scan2 s = scan2<SM>(buf, f0, f1);
     buf ^= 1;
     if (f0) list[nsel + s.off0] = i0;
     if (f1) list[nsel + s.off1] = i1;
     nsel += s.total;
   }
-  wsync(c);
+  wsync(c.T);
+#pragma unroll 1
   for (u32 q = 0; q < nsel; q += T) {
     const u32 cnt = min(T, nsel - q);
-    rng_ensure(c, rp, cnt);
+    rng_ensure(rp, cnt);
     const bool mine = threadIdx.x < cnt;
     u64 r = 0;
     bool ok = true;
     if (mine) {
-      r = ring_at(c, rp + threadIdx.x) / P.pos_bucket;
+      r = ring_at(c.rmask, rp + threadIdx.x) / P.pos_bucket;
       ok = r <= P.pos_range;
     }
-    if (wsync_or(c, !ok)) {
+    if (wsync_or(c.T, !ok)) {
       // a bucket rejection: the rest one by one with the exact number of draws
       if (threadIdx.x == 0) {
+#pragma unroll 1
         for (u32 j = q; j < nsel; ++j) {
-          const u64 pos = s_uniform_int(c, P.wstart, (u64)P.wend - 1);
+          const u64 pos = s_uniform_int(g_c, P.wstart, (u64)P.wend - 1);
           c.rev[list[j]] = (u32)pos;
           c.fwd[list[j]] = (u32)pos;
           c.bep[list[j]] = epoch;
         }
       }
-      wsync(c);
-      return c.sc->rpos;
+      wsync(c.T);
+      return g_sc.rpos;
     }
     rp += cnt;
-    rng_publish(c, rp);
+    rng_publish(rp);
     if (mine) {
       const u32 i = list[q + threadIdx.x], pos = (u32)(P.wstart + r);
       c.rev[i] = pos;
@@ -1167,7 +1314,7 @@ __device__ __noinline__ u64 bind_lefs(Cell& c, const KParams& P, u64 rp, u32 n, 
       c.bep[i] = epoch;
     }
   }
-  wsync(c);
+  wsync(c.T);
   return rp;
 }
 // Ranking key of a unit: position, then binding epoch ascending (rev) or descending (fwd).
@@ -1184,6 +1331,7 @@ __device__ __forceinline__ u64 rank_key(const Cell& c, u32 dir, u32 idx) {
 // indexes are shifts and masks.
 __device__ void bitonic_keyed(u32* a, u32* hi, u32* lo, u32 m) {
   u32 lg = 0;
+#pragma unroll 1
   while ((1u << lg) < m) ++lg;
   const u32 ncmp = (1u << lg) >> 1;  // comparators per stage
   auto cmpx = [&](u32 i, u32 j) {
@@ -1199,14 +1347,18 @@ __device__ void bitonic_keyed(u32* a, u32* hi, u32* lo, u32 m) {
       a[j] = x;
     }
   };
+#pragma unroll 1
   for (u32 s = 1; s <= lg; ++s) {
     // merge into sorted blocks of 2^s: mirror pairs, then strides 2^(s-2) .. 1
+#pragma unroll 1
     for (u32 t = ln(); t < ncmp; t += 32) {
       const u32 base = (t >> (s - 1)) << s, off = t & ((1u << (s - 1)) - 1u);
       cmpx(base + off, base + (1u << s) - 1u - off);
     }
     __syncwarp();
+#pragma unroll 1
     for (int q = (int)s - 2; q >= 0; --q) {
+#pragma unroll 1
       for (u32 t = ln(); t < ncmp; t += 32) {
         const u32 i = ((t >> q) << (q + 1)) | (t & ((1u << q) - 1u));
         cmpx(i, i + (1u << q));
@@ -1223,7 +1375,9 @@ __device__ __noinline__ u32 tie_fix_run(const Cell& c, u32 dir, u32* a, u32 t, u
   const u32* pos = dir ? c.fwd : c.rev;
   const u32 p = pos[a[t]];
   u32 lo = t - 1, hi = t + 1;
+#pragma unroll 1
   while (lo > 0 && pos[a[lo - 1]] == p) --lo;
+#pragma unroll 1
   while (hi < len && pos[a[hi]] == p) ++hi;
   if (dir) {
     ins_sort(a, lo, hi, KeyCmpRev{c.bep});
@@ -1272,7 +1426,7 @@ __device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
     const u32* __restrict__ Rr = R;
     const u32* __restrict__ pr = pos;
     u32* __restrict__ V = c.tmp;
-#pragma unroll 4
+#pragma unroll 1
     for (u32 r = lane; r < n; r += 32) V[r] = pr[Rr[r]];
   }
   __syncwarp();
@@ -1280,6 +1434,7 @@ __device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
   const u32 first = R[0];
   if (lane == 0) K[0] = first;
   u32 m = 0, T = V[0], E = 0, q = 0;
+#pragma unroll 1
   for (u32 base = 1; base < n; base += 32) {
     const u32 r = base + lane;
     const u32 nvalid = min(32u, n - base);
@@ -1289,6 +1444,7 @@ __device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
     const u32 vprev = __shfl_up_sync(FULL, v, 1);
     const bool pre_ok = lane == 0 || v >= vprev;
     u32 start = 0;
+#pragma unroll 1
     while (start < nvalid) {
       const bool ok = lane == start ? v >= T : pre_ok;
       const unsigned fail = __ballot_sync(FULL, !ok && lane >= start && valid);
@@ -1322,12 +1478,13 @@ __device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
   __syncwarp();
   {
     const u64 t = clock64();
-    prof_add(c, PF_RANK_PASS, t - tprof);
+    prof_add(PF_RANK_PASS, t - tprof);
     tprof = t;
   }
   const u32 ns = m + 1;
   // block size before each event, and the rotation it saw since the previous event
   u32 kacc = 0;
+#pragma unroll 1
   for (u32 b = 0; b < E; b += 32) {
     const u32 j = b + lane;
     const bool vj = j < E;
@@ -1345,6 +1502,7 @@ __device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
   __syncwarp();
   // final slot of every removed element
   const u32 qfm = kE ? q % kE : 0u;
+#pragma unroll 1
   for (u32 b = 0; b < E; b += 32) {
     const u32 j = b + lane;
     const bool vj = j < E;
@@ -1352,6 +1510,7 @@ __device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
     const u32 rd = vj ? ev_rd[j] : 0u;
     const u32 kj = vj ? (ev_q[j] >> 16) + (top != UNBOUND ? 2u : 1u) : 1u;
     u32 it = 0, ir = kj - 1;
+#pragma unroll 1
     for (u32 jj = b + 1; jj < E; ++jj) {
       const u32 w = ev_q[jj];
       const bool pop = ev_top[jj] != UNBOUND;
@@ -1381,6 +1540,7 @@ __device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
   u32* Kh = c.rm;  // position
   u32* Kl = c.fm;  // binding epoch (complemented for fwd units)
   bool full_tie = false;
+#pragma unroll 1
   for (u32 t = lane; t < kE; t += 32) {
     const u32 idx = B[t];
     const u64 k = rank_key(c, dir, idx);
@@ -1390,12 +1550,14 @@ __device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
   }
   __syncwarp();
   bitonic_keyed(Bs, Kh, Kl, kE);
+#pragma unroll 1
   for (u32 t = lane + 1; t < kE; t += 32) full_tie |= Kh[t - 1] == Kh[t] && Kl[t - 1] == Kl[t];
   const u32* Bf = Bs;
   if (__any_sync(FULL, full_tie)) {
-    prof_add(c, PF_RANK_PDQ, 1);
+    prof_add(PF_RANK_PDQ, 1);
     if (lane == 0) {
       pdq_sort(B, 0, kE, KeyCmp{pos});
+#pragma unroll 1
       for (u32 t = 1; t < kE; ++t) {
         if (pos[B[t - 1]] == pos[B[t]]) t = tie_fix_run(c, dir, B, t, kE);
       }
@@ -1405,12 +1567,13 @@ __device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
   }
   {
     const u64 t = clock64();
-    prof_add(c, PF_RANK_BLOCK, t - tprof);
+    prof_add(PF_RANK_BLOCK, t - tprof);
     tprof = t;
   }
   // tie fix of K: runs of equal positions whose epochs are out of order (each element's key is
   // read once; the previous element's comes from the adjacent lane or the previous chunk)
   u64 kprev = ns ? rank_key(c, dir, K[0]) : 0;
+#pragma unroll 1
   for (u32 base = 1; base < ns; base += 32) {
     const u32 t = base + lane;
     const u64 kt = t < ns ? rank_key(c, dir, K[t]) : ~0ull;
@@ -1421,6 +1584,7 @@ __device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
     unsigned bm = __ballot_sync(FULL, bad);
     if (bm) {
       if (lane == 0) {
+#pragma unroll 1
         while (bm) {
           const u32 t0 = base + (u32)(__ffs(bm) - 1);
           const u32 hi = tie_fix_run(c, dir, K, t0, ns);
@@ -1438,10 +1602,12 @@ __device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
   // sorted by key), so B_j lands at j + u_j and K_i at i + #{j : u_j <= i}; u is
   // non-decreasing in j, so one pass over K with a pointer into u counts the latter.
   u32* U = Bf == Bs ? B : Bs;  // the dead one of the two B buffers
+#pragma unroll 1
   for (u32 j = lane; j < kE; j += 32) {
     const u32 idx = Bf[j];
     const u64 key = rank_key(c, dir, idx);
     u32 lo = 0, hi = ns;
+#pragma unroll 1
     while (lo < hi) {
       const u32 mid = (lo + hi) >> 1;
       if (rank_key(c, dir, K[mid]) <= key) lo = mid + 1; else hi = mid;
@@ -1451,9 +1617,11 @@ __device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
   }
   __syncwarp();
   u32 jb = 0;  // B elements with u_j below the chunk
+#pragma unroll 1
   for (u32 base = 0; base < ns; base += 32) {
     const u32 i = base + lane;
     u32 cnt = jb, j = jb;
+#pragma unroll 1
     for (; j < kE; ++j) {
       const u32 uj = U[j];
       if (uj >= base + 32) break;
@@ -1463,7 +1631,7 @@ __device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
     jb = j;
   }
   __syncwarp();
-  prof_add(c, PF_RANK_MERGE, clock64() - tprof);
+  prof_add(PF_RANK_MERGE, clock64() - tprof);
   return true;
 }
 
@@ -1486,23 +1654,25 @@ __device__ __forceinline__ u64 max64(u64 a, u64 b) { return a > b ? a : b; }
 //  3 runs of 32 removed units sorted in registers;
 //  4 each removed unit's place among the removed (pairwise searches) and among the kept;
 //  5 the new order, written to rm; 6 copied to R.
-__device__ __noinline__ bool rank_dir_block(Cell& c, u32 dir, u32 n, u32 epoch) {
+template <bool SM>
+__device__ __noinline__ bool rank_dir_block(u32 dir, u32 n, u32 epoch) {
+  const View<SM> c;
   if (n < 2 || n > 0xFFFFu) return false;
   const u32 T = c.T, W = T >> 5, w = threadIdx.x >> 5, lane = ln();
-  u32* R = dir ? c.fr : c.rr;
-  const u32* pos = dir ? c.fwd : c.rev;
-  const u32* bep = c.bep;
-  u32* kh = c.rm;
-  u32* kl = c.fm;
-  u64* bk = reinterpret_cast<u64*>(c.sr);
+  const auto R = dir ? c.fr : c.rr;
+  const auto pos = dir ? c.fwd : c.rev;
+  const auto bep = c.bep;
+  const auto kh = c.rm;
+  const auto kl = c.fm;
+  const auto bk = c.sr;  // as 64-bit words
   const u32 nch = (n + 31) >> 5;
-  u32* kmask = c.sf + (n - nch);
+  const auto kmask = c.sf + (n - nch);
   const u32 maxb = n / 3;
-  u32 *bp = c.tmp, *sr0 = c.tmp + maxb, *sfin = c.tmp + 2 * maxb;
-  BlockTmp* bt = c.bt;
+  const auto bp = c.tmp, sr0 = c.tmp + maxb, sfin = c.tmp + 2 * maxb;
   const u32 ch0 = w * nch / W, ch1 = (w + 1) * nch / W;
   const u32 newlo = dir ? ~epoch : epoch;
   u64 mx = 0;
+#pragma unroll 1
   for (u32 ch = ch0; ch < ch1; ++ch) {
     const u32 r = ch * 32 + lane;
     if (r < n) {
@@ -1515,19 +1685,20 @@ __device__ __noinline__ bool rank_dir_block(Cell& c, u32 dir, u32 n, u32 epoch) 
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) mx = max64(mx, __shfl_xor_sync(FULL, mx, d));
-  if (lane == 0) bt->wmax[w] = mx;
+  if (lane == 0) g_bt.wmax[w] = mx;
   if (threadIdx.x == 0) {
-    bt->nrem = 0;
-    bt->tie = 0;
-    bt->tie2 = 0;
+    g_bt.nrem = 0;
+    g_bt.tie = 0;
+    g_bt.tie2 = 0;
   }
-  wsync(c);
-  u64 carry = lane < w ? bt->wmax[lane] : 0;
+  wsync(c.T);
+  u64 carry = lane < w ? g_bt.wmax[lane] : 0;
 #pragma unroll
   for (int d = 8; d > 0; d >>= 1) carry = max64(carry, __shfl_xor_sync(FULL, carry, d));
   carry = __shfl_sync(FULL, carry, 0);
   bool tie = false;
   u32 removed = 0;
+#pragma unroll 1
   for (u32 ch = ch0; ch < ch1; ++ch) {
     const u32 r = ch * 32 + lane;
     const bool valid = r < n;
@@ -1549,13 +1720,13 @@ __device__ __noinline__ bool rank_dir_block(Cell& c, u32 dir, u32 n, u32 epoch) 
     if (lane == 0) kmask[ch] = km;
     if (rmk) {
       u32 q = 0;
-      if (lane == 0) q = atomicAdd(&bt->nrem, (u32)__popc(rmk));
+      if (lane == 0) q = atomicAdd(&g_bt.nrem, (u32)__popc(rmk));
       q = __shfl_sync(FULL, q, 0) + __popc(rmk & lanemask_lt());
       if (rem) {
         kh[r] = (u32)(excl >> 32);
         kl[r] = (u32)excl;
         if (q < maxb) {
-          bk[q] = key;
+          bk.at64(q) = key;
           bp[q] = R[r] | (r << 16);
         }
       }
@@ -1563,20 +1734,21 @@ __device__ __noinline__ bool rank_dir_block(Cell& c, u32 dir, u32 n, u32 epoch) 
     }
     carry = max64(carry, __shfl_sync(FULL, x, 31));
   }
-  if (lane == 0) bt->rem[w] = removed;
-  if (tie) bt->tie = 1;
-  wsync(c);
-  const u32 m = bt->nrem;
-  if (m > maxb || bt->tie) return false;
+  if (lane == 0) g_bt.rem[w] = removed;
+  if (tie) g_bt.tie = 1;
+  wsync(c.T);
+  const u32 m = g_bt.nrem;
+  if (m > maxb || g_bt.tie) return false;
   // 3: runs of 32
   if (w == W - 1) {  // removed units before each warp's range
-    u32 v = lane < W ? bt->rem[lane] : 0u;
+    u32 v = lane < W ? g_bt.rem[lane] : 0u;
     const u32 ex = warp_excl_scan(v, nullptr);
-    if (lane < W) bt->rembase[lane] = ex;
+    if (lane < W) g_bt.rembase[lane] = ex;
   }
+#pragma unroll 1
   for (u32 run = w; run * 32 < m; run += W) {
     const u32 q = run * 32 + lane;
-    u64 key = q < m ? bk[q] : ~0ull;
+    u64 key = q < m ? bk.at64(q) : ~0ull;
     u32 pl = q < m ? bp[q] : 0u;
 #pragma unroll
     for (int k = 2; k <= 32; k <<= 1) {
@@ -1595,30 +1767,34 @@ __device__ __noinline__ bool rank_dir_block(Cell& c, u32 dir, u32 n, u32 epoch) 
     }
     const u64 prev = __shfl_up_sync(FULL, key, 1);
     if (q < m) {
-      bk[q] = key;
+      bk.at64(q) = key;
       bp[q] = pl;
-      if (lane > 0 && prev == key) bt->tie2 = 1;
+      if (lane > 0 && prev == key) g_bt.tie2 = 1;
     }
   }
-  wsync(c);
+  wsync(c.T);
   // 4: places
+#pragma unroll 1
   for (u32 q = threadIdx.x; q < m; q += T) {
-    const u64 key = bk[q];
+    const u64 key = bk.at64(q);
     const u32 my = q >> 5;
     u32 rank = q & 31u;
+#pragma unroll 1
     for (u32 s0 = 0; s0 < m; s0 += 32) {
       if ((s0 >> 5) == my) continue;
       const u32 len = min(32u, m - s0);
       u32 lo = 0, hi = len;
+#pragma unroll 1
       while (lo < hi) {
         const u32 mid = (lo + hi) >> 1;
-        if (bk[s0 + mid] < key) lo = mid + 1; else hi = mid;
+        if (bk.at64(s0 + mid) < key) lo = mid + 1; else hi = mid;
       }
-      if (lo < len && bk[s0 + lo] == key) bt->tie2 = 1;
+      if (lo < len && bk.at64(s0 + lo) == key) g_bt.tie2 = 1;
       rank += lo;
     }
     const u32 khi = (u32)(key >> 32), klo = (u32)key;
     u32 lo = 0, hi = n;  // first rank whose running maximum is >= key
+#pragma unroll 1
     while (lo < hi) {
       const u32 mid = (lo + hi) >> 1;
       const u32 h = kh[mid];
@@ -1626,19 +1802,21 @@ __device__ __noinline__ bool rank_dir_block(Cell& c, u32 dir, u32 n, u32 epoch) 
     }
     u32 before = m;  // removed units at ranks below lo
     if (lo < n) {
-      if (kh[lo] == khi && kl[lo] == klo) bt->tie2 = 1;
+      if (kh[lo] == khi && kl[lo] == klo) g_bt.tie2 = 1;
       const u32 ch = lo >> 5, ow = ((ch + 1) * W - 1) / nch;
-      before = bt->rembase[ow];
+      before = g_bt.rembase[ow];
+#pragma unroll 1
       for (u32 k = ow * nch / W; k < ch; ++k) before += 32 - __popc(kmask[k]);
       before += (lo & 31u) - __popc(kmask[ch] & ((1u << (lo & 31u)) - 1u));
     }
     sr0[rank] = lo;
     sfin[rank] = (bp[q] & 0xFFFFu) | ((rank + lo - before) << 16);
   }
-  wsync(c);
-  if (bt->tie2) return false;
+  wsync(c.T);
+  if (g_bt.tie2) return false;
   // 5: the new order
-  u32* O = c.rm;
+  const auto O = c.rm;
+#pragma unroll 1
   for (u32 q = threadIdx.x; q < m; q += T) {
     const u32 v = sfin[q];
     O[v >> 16] = v & 0xFFFFu;
@@ -1648,17 +1826,20 @@ __device__ __noinline__ bool rank_dir_block(Cell& c, u32 dir, u32 n, u32 epoch) 
     {
       const u32 r0 = ch0 * 32;
       u32 lo = 0, hi = m;
+#pragma unroll 1
       while (lo < hi) {
         const u32 mid = (lo + hi) >> 1;
         if (sr0[mid] < r0) lo = mid + 1; else hi = mid;
       }
       j = lo;
     }
-    u32 rb = bt->rembase[w];
+    u32 rb = g_bt.rembase[w];
+#pragma unroll 1
     for (u32 ch = ch0; ch < ch1; ++ch) {
       const u32 r = ch * 32 + lane;
       const u32 km = kmask[ch];
       u32 ins = j;
+#pragma unroll 1
       for (; j < m; ++j) {
         const u32 at = sr0[j];
         if (at >= ch * 32 + 32) break;
@@ -1668,78 +1849,68 @@ __device__ __noinline__ bool rank_dir_block(Cell& c, u32 dir, u32 n, u32 epoch) 
       rb += 32 - __popc(km);
     }
   }
-  wsync(c);
+  wsync(c.T);
+#pragma unroll 1
   for (u32 r = threadIdx.x; r < n; r += T) R[r] = O[r];
-  wsync(c);
+  wsync(c.T);
   return true;
 }
 
 // Full ties, many moved units (a young cell binds most of its units in one epoch) or a small n:
 // one warp's exact emulation; the first epoch and unsorted callers: the serial restatement.
-__device__ __noinline__ void rank_lefs(Cell& c, const KParams& P, u32 n, u32 epoch, bool partially_sorted) {
+template <bool SM>
+__device__ __noinline__ void rank_lefs(u32 n, u32 epoch, bool partially_sorted) {
+  const View<SM> c;
+  const KParams& P = g_P;
   const bool fast = partially_sorted && !(P.debug_flags & DBG_SERIAL_RANK) && n >= 2 && n <= 0xFFFFu;
+#pragma unroll 1
   for (u32 dir = 0; dir < 2; ++dir) {
     if (fast) {
-      if (rank_dir_block(c, dir, n, epoch)) continue;
+      if (rank_dir_block<SM>(dir, n, epoch)) continue;
       const u64 t0 = clock64();
-      if (threadIdx.x < 32) rank_dir_split(c, dir, n);
-      wsync(c);
-      prof_add(c, PF_RANK_SPLIT, clock64() - t0);
+      if (threadIdx.x < 32) rank_dir_split(g_c, dir, n);
+      wsync(c.T);
+      prof_add(PF_RANK_SPLIT, clock64() - t0);
     } else {
       const u64 t0 = clock64();
-      prof_add(c, PF_RANK_FALLBACK, 1);
+      prof_add(PF_RANK_FALLBACK, 1);
       if (threadIdx.x == 0) {
-        rank_dir_serial(c, dir, n, partially_sorted);
-        c.sc->sort_fallbacks++;
+        rank_dir_serial(g_c, dir, n, partially_sorted);
+        g_sc.sort_fallbacks++;
       }
-      wsync(c);
-      prof_add(c, PF_RANK_SERIAL, clock64() - t0);
+      wsync(c.T);
+      prof_add(PF_RANK_SERIAL, clock64() - t0);
     }
   }
 }
 
 // positions in rank order: sr[k] = rev[rr[k]], sf[k] = fwd[fr[k]]
-__device__ __noinline__ void gather_ranked(Cell& c, u32 n) {
-  const u32* __restrict__ rr = c.rr;
-  const u32* __restrict__ fr = c.fr;
-  const u32* __restrict__ rev = c.rev;
-  const u32* __restrict__ fwd = c.fwd;
-  u32* __restrict__ sr = c.sr;
-  u32* __restrict__ sf = c.sf;
-#pragma unroll 4
+template <bool SM>
+__device__ __noinline__ void gather_ranked(u32 n) {
+  const View<SM> c;
+  const auto rr = c.rr;
+  const auto fr = c.fr;
+  const auto rev = c.rev;
+  const auto fwd = c.fwd;
+  const auto sr = c.sr;
+  const auto sf = c.sf;
+#pragma unroll 1
   for (u32 k = threadIdx.x; k < n; k += c.T) {
     sr[k] = rev[rr[k]];
     sf[k] = fwd[fr[k]];
   }
-  wsync(c);
+  wsync(c.T);
 }
 
 // One draw of the moves' normal distribution and the move it gives: v = round(max(0, z * sd + mean)).
 // The reference evaluates this in doubles; here the ziggurat's comparison is an integer threshold on
 // the draw (zt[i].x) and the move is computed in 32.32 fixed point from the layer's width (zt[i].y =
 // x_i * 2^60) and sd * 2^36.  Both the doubles' rounding and the fixed point's are below 8 units of
-// 2^-32 for the parameters MoveSpec accepts, so the rounded move is the reference's unless the value
+// 2^-32 for the parameters MoveSpec marks as fixed, so the rounded move is the reference's unless the value
 // lies within 16 units of a half: then, for the tail layer, and where the wedge test is closer than
 // the single-precision estimate resolves, the draw is evaluated in doubles by unit_normal_t.
 // The FP64 pipe of sm_103a runs at 1/64 of the FP32 rate: with doubles alone the moves of a
 // 2,500-LEF cell kept it busy for about a third of the epoch.
-struct MoveSpec {
-  double mean, sd;
-  u64 sdq;    // sd * 2^36
-  i64 meanq;  // mean * 2^32
-  bool fixed; // fixed-point evaluation allowed
-};
-__device__ __forceinline__ MoveSpec move_spec(double mean, double sd) {
-  MoveSpec m{mean, sd, 0, 0, false};
-  // integer speeds below 2^19 with sd below 2^14: |z * sd + mean| < 2^20
-  m.fixed = mean >= 0.0 && mean < 524288.0 && sd < 16384.0 && mean == floor(mean);
-  if (m.fixed) {
-    m.sdq = (u64)(sd * 68719476736.0);
-    m.meanq = (i64)mean << 32;
-  }
-  return m;
-}
-
 __device__ __noinline__ int move_exact(RingSrc& g, const MoveSpec& ms, u32* v, bool* range) {
   double z = 0.0;
   const int st = unit_normal_t(g, z);
@@ -1749,16 +1920,17 @@ __device__ __noinline__ int move_exact(RingSrc& g, const MoveSpec& ms, u32* v, b
   return st;
 }
 
-__device__ __forceinline__ int move_sample(const ulonglong2* zt, RingSrc& g, const MoveSpec& ms, u32* v, bool* range) {
+__device__ __forceinline__ int move_sample(RingSrc& g, const MoveSpec& ms, u32* v, bool* range) {
   *range = false;
   if (ms.fixed) {
+#pragma unroll 1
     for (int it = 0; it < 64; ++it) {
       const RingSrc here = g;  // an attempt of the sampler carries nothing from the one before
       u64 u;
       if (!g.next(u)) return SMP_DRY;
       const u32 ii = (u32)u & 0xFFu, i = ii >> 1;
       const u64 m = (u & ~(1ull << 11)) >> 8;
-      const ulonglong2 e = zt[i];
+      const ulonglong2 e = g_bt.zt[i];
       const u64 t = __umul64hi(m << 8, e.y);  // x * 2^60
       bool acc = m < e.x, exact = false;
       if (!acc) {
@@ -1770,10 +1942,10 @@ __device__ __forceinline__ int move_sample(const ulonglong2* zt, RingSrc& g, con
         } else if (u2 >= ~0ull << 12) {
           exact = true;  // uniform_01 may round to 1 and be drawn again
         } else {
-          const float x = (float)t * 0x1p-60f;
+          const float x = (float)(u32)(t >> 32) * 0x1p-28f;
           const float ef = expf(-0.5f * x * x);
-          const float y0 = (float)mgpu_zig_normal_y[i], y1 = (float)mgpu_zig_normal_y[i + 1];
-          const float d = y0 + (float)u2 * 0x1p-64f * (y1 - y0) - ef;
+          const float2 y = g_bt.zy[i];
+          const float d = y.x + (float)(u32)(u2 >> 32) * 0x1p-32f * y.y - ef;
           exact = fabsf(d) <= 2e-5f * ef;
           acc = d < 0.0f;
         }
@@ -1808,119 +1980,161 @@ __device__ __forceinline__ int move_sample(const ulonglong2* zt, RingSrc& g, con
 // exponentials), so the workers evaluate a window of T candidate starts at once: thread k runs the
 // whole sampler as if a normal started at stream position rp + k.  The real starts form the chain
 // s0 = 0, s(j+1) = s(j) + len(s(j)).  Each warp tabulates, for every lane it could be entered at, the
-// number of normals starting inside it and where the chain leaves it (pointer doubling over the lanes'
-// next-start pointers); after one wsync every warp follows the few table entries before its own and
-// marks its starts.  A window serves about T normals, in stream order, to the next LEFs in index order.
-__device__ __noinline__ u64 gen_moves_dir(Cell& c, u64 rp, u32* mv, u32 n, double mean, double sd, u64 move_int) {
+// number of normals starting inside it and where the chain leaves it; after one wsync every warp
+// composes the tables of the warps before it and marks its starts.  A window serves about T normals, in stream order, to the next LEFs in index order.
+template <bool SM>
+__device__ __noinline__ u64 gen_moves_dir(u64 rp, const Arr<SM> mv, u32 n, const MoveSpec& spec) {
+  const View<SM> c;
   const u32 T = c.T, W = T >> 5, w = threadIdx.x >> 5, lane = ln();
-  if (sd == 0.0) {
-    for (u32 i = threadIdx.x; i < n; i += T) mv[i] = c.bep[i] == UNBOUND ? 0u : (u32)move_int;
-    wsync(c);
+  const MoveSpec ms = spec;
+  if (ms.constant) {
+#pragma unroll 1
+    for (u32 i = threadIdx.x; i < n; i += T) mv[i] = c.bep[i] == UNBOUND ? 0u : (u32)ms.move_int;
+    wsync(c.T);
     return rp;
   }
   // items: the bound LEFs in index order (a compacted list only when some are unbound)
   u32 nb = n;
   bool unb = false;
+#pragma unroll 1
   for (u32 i = threadIdx.x; i < n; i += T) unb |= c.bep[i] == UNBOUND;
-  const bool all = !wsync_or(c, unb);
+  const bool all = !wsync_or(c.T, unb);
   if (!all) {
     nb = 0;
     u32 buf = 0;
+#pragma unroll 1
     for (u32 base = 0; base < n; base += T) {
       const u32 i = base + threadIdx.x;
       const bool need = i < n && c.bep[i] != UNBOUND;
-      const Scan2 s = scan2(c, buf, need, false);
+      const Scan2 s = scan2<SM>(buf, need, false);
       buf ^= 1;
       if (i < n && !need) mv[i] = 0;
       if (need) c.tmp[nb + s.off0] = i;
       nb += s.total;
     }
-    wsync(c);
+    wsync(c.T);
   }
-  const MoveSpec ms = move_spec(mean, sd);
-  BlockTmp* bt = c.bt;
   const u32 DRY = 0x4000u;
   u32 t0 = 0;
+#pragma unroll 1
   while (t0 < nb) {
-    rng_ensure(c, rp, T + 64);
-    RingSrc g{c.ring, c.rmask, (u32)rp + threadIdx.x, (u32)rp + T + 64, 0};
+    rng_ensure(rp, T + 64);
+    RingSrc g{c.rmask, (u32)rp + threadIdx.x, (u32)rp + T + 64, 0};
     u32 v = 0;
     bool range = false;
-    const int st = move_sample(bt->zt, g, ms, &v, &range);
+    const int st = move_sample(g, ms, &v, &range);
     const u32 len = g.n;
-    // next-start pointers relative to the warp's first lane; DRY + lane: this sampler ran dry
-    u32 J[5], ptr = st == SMP_OK ? lane + len : DRY + lane, cnt = st == SMP_OK ? 1u : 0u;
-#pragma unroll
-    for (int b = 0; b < 5; ++b) {
-      J[b] = ptr;
-      const u32 p2 = __shfl_sync(FULL, ptr, ptr & 31u), c2 = __shfl_sync(FULL, cnt, ptr & 31u);
-      if (ptr < 32) {
-        cnt += c2;
-        ptr = p2;
+    // Per entry lane: where the chain leaves the warp (32 + the lane it enters the next one at, or
+    // DRY + the lane whose sampler ran dry) and how many normals start before that.  Almost every
+    // normal takes one draw, so the chain only bends at the few lanes of dm, taken from the last.
+    const unsigned dm = __ballot_sync(FULL, st != SMP_OK || len != 1);
+    const u32 step = st == SMP_OK ? lane + len : DRY;
+    u32 leave = 32, cnt = 32 - lane;
+#pragma unroll 1
+    for (unsigned r = dm; r;) {
+      const u32 d = 31 - __clz(r);
+      r &= ~(1u << d);
+      const u32 q = __shfl_sync(FULL, step, d);
+      const u32 l2 = __shfl_sync(FULL, leave, q & 31u), c2 = __shfl_sync(FULL, cnt, q & 31u);
+      if (lane <= d) {
+        leave = q == DRY ? DRY + d : (q < 32 ? l2 : q);
+        cnt = d - lane + (q == DRY ? 0u : (q < 32 ? c2 + 1 : 1u));
       }
     }
-    bt->tab[w][lane] = ptr | (cnt << 16);
-    wsync(c);
-    u32 e = 0, base = 0, my_e = 64, my_base = 0;
-    bool dry = false;
-    for (u32 k = 0; k < W; ++k) {
-      if (e >= 32) {
-        e -= 32;
-        continue;
+    g_bt.tab[w][lane] = leave | (cnt << 16);
+    wsync(c.T);
+    // Entry lane of every warp (lane k of each warp holds warp k's): all zero unless a normal straddles
+    // two warps, so start there and repeat until the entries agree with the warps before.
+    u32 e = 0, t = 0;
+    bool odd = false;
+#pragma unroll 1
+    for (;;) {
+      t = lane < W ? g_bt.tab[lane][e & 31u] : 32u;
+      odd = lane < W && ((t & 0xFFFFu) >= 64 || e >= 32);
+      u32 ne = __shfl_up_sync(FULL, (t & 0xFFFFu) - 32, 1);
+      if (lane == 0) ne = 0;
+      const bool same = lane >= W || ne == e;
+      e = ne;
+      if (__any_sync(FULL, odd) || __all_sync(FULL, same)) break;
+    }
+    u32 base, my_e, my_base, used;
+    if (!__any_sync(FULL, odd)) {
+      const u32 ex = warp_excl_scan(lane < W ? t >> 16 : 0u, &base);
+      my_base = __shfl_sync(FULL, ex, w);
+      my_e = __shfl_sync(FULL, e, w);
+      used = T + __shfl_sync(FULL, (t & 0xFFFFu) - 32, W - 1);
+    } else {
+      // a normal of more than 32 draws or a dry sampler: follow the entries one by one
+      u32 en = 0;
+      bool dry = false;
+      base = my_base = 0;
+      my_e = 64;
+      used = 0;
+#pragma unroll 1
+      for (u32 k = 0; k < W; ++k) {
+        if (en >= 32) {
+          en -= 32;
+          continue;
+        }
+        if (k == w) {
+          my_e = en;
+          my_base = base;
+        }
+        const u32 v2 = g_bt.tab[k][en];
+        base += v2 >> 16;
+        const u32 q = v2 & 0xFFFFu;
+        if (q & DRY) {
+          dry = true;
+          used = k * 32 + (q & 31u);  // the window ends before the sampler that ran dry
+          break;
+        }
+        en = q - 32;
       }
-      if (k == w) {
-        my_e = e;
-        my_base = base;
-      }
-      const u32 t = bt->tab[k][e];
-      base += t >> 16;
-      const u32 p = t & 0xFFFFu;
-      if (p & DRY) {
-        dry = true;
-        e = k * 32 + (p & 31u);  // the window ends before the sampler that ran dry
-        break;
-      }
-      e = p - 32;
+      if (!dry) used = T + en;
     }
     const u32 served = min(base, nb - t0);
-    u32 used = dry ? e : T + e;  // draws taken when every start of the window is served
     if (my_e < 32) {
-      u32 vis = 1u << my_e;
-#pragma unroll
-      for (int b = 0; b < 5; ++b)
-        vis |= __reduce_or_sync(FULL, ((vis >> lane) & 1u) && J[b] < 32 ? 1u << J[b] : 0u);
+      u32 vis = 0;  // lanes a normal starts at
+#pragma unroll 1
+      for (u32 q = my_e; q < 32;) {
+        const unsigned r = dm >> q << q;
+        const u32 d = r ? (u32)(__ffs(r) - 1) : 31u;
+        vis |= (0xFFFFFFFFu << q) & (0xFFFFFFFFu >> (31 - d));
+        if (!r) break;
+        q = __shfl_sync(FULL, step, d);
+      }
       const u32 ord = my_base + __popc(vis & lanemask_lt());
       if (((vis >> lane) & 1u) && st == SMP_OK && ord < served) {
-        if (range) set_status(c, DEV_ERR_MOVE_RANGE);
+        if (range) set_status(g_c, DEV_ERR_MOVE_RANGE);
         mv[all ? t0 + ord : c.tmp[t0 + ord]] = v;
-        if (ord == served - 1) bt->used = threadIdx.x + len;
+        if (ord == served - 1) g_bt.used = threadIdx.x + len;
       }
     }
-    wsync(c);
+    wsync(c.T);
     if (served == 0) {
       // the first normal needs more draws than the window holds: take it serially
       if (threadIdx.x == 0) {
-        c.sc->rpos = rp;
-        const double zz = s_unit_normal(c);
-        const double d = round(fmax(0.0, zz * sd + mean));
-        if (d > 4294967295.0) set_status(c, DEV_ERR_MOVE_RANGE);
+        g_sc.rpos = rp;
+        const double zz = s_unit_normal(g_c);
+        const double d = round(fmax(0.0, zz * ms.sd + ms.mean));
+        if (d > 4294967295.0) set_status(g_c, DEV_ERR_MOVE_RANGE);
         mv[all ? t0 : c.tmp[t0]] = (u32)(u64)d;
       }
-      wsync(c);
-      rp = c.sc->rpos;
+      wsync(c.T);
+      rp = g_sc.rpos;
       ++t0;
       continue;
     }
-    if (served < base) used = bt->used;
+    if (served < base) used = g_bt.used;
     rp += used;
-    rng_publish(c, rp);
+    rng_publish(rp);
     t0 += served;
   }
-  wsync(c);
+  wsync(c.T);
   return rp;
 }
 
-// adjust_moves_of_consecutive_extr_units (simulation.cpp:343-399), one direction.
+// adjust_moves_of_consecutive_extr_units (simulation.cpp:343-399).
 // rev: with t_k = pos_k - move_k the reference goes down the ranks and sets T_k = min(t_k, T_{k+1} - 1)
 // when the pair links (both bound, t_k > start, T_{k+1} > start), else T_k = t_k.  Every unit whose lower
 // neighbour it pushes starts a walk down the ranks that carries its target, one less per rank, until a
@@ -1928,68 +2142,133 @@ __device__ __noinline__ u64 gen_moves_dir(Cell& c, u64 rp, u32* mv, u32 n, doubl
 // smallest target that reaches it.  Pushed units are few and their walks short, so almost all threads
 // only compare two neighbours.  fwd units mirror this upwards.  A linked pair whose pushing target lies
 // beyond the chromosome end is skipped by the reference: that rejects the result (serial restatement).
-__device__ __noinline__ bool adjust_dir_block(Cell& c, const KParams& P, u32 dir, u32 n) {
-  const u32* __restrict__ R = dir ? c.fr : c.rr;
-  const u32* __restrict__ S = dir ? c.sf : c.sr;
-  const u32* __restrict__ bep = c.bep;
-  u32* M = dir ? c.fm : c.rm;
-  u32* out = c.tmp;
+// out holds the moves in rank order.
+template <class A>
+__device__ __forceinline__ bool adjust_pushes(u32 dir, const A& S, const A& out, u32 k, u32 i) {
+  // unit of rank k against the unit i it would push, on the moves before any push
+  return dir ? (u64)S[k] + out[k] >= (u64)S[i] + out[i] : (i64)S[k] - out[k] <= (i64)S[i] - out[i];
+}
+
+template <bool SM>
+__device__ __noinline__ bool adjust_walk(u32 dir, u32 n, u32 k, const Arr<SM> out) {
+  const View<SM> c;
+  const KParams& P = g_P;
+  const auto R = dir ? c.fr : c.rr;
+  const auto S = dir ? c.sf : c.sr;
+  const auto M = dir ? c.fm : c.rm;  // the moves before any push
   const i64 lim = dir ? (i64)P.end - 1 : (i64)P.start;
-#pragma unroll 4
-  for (u32 k = threadIdx.x; k < n; k += c.T) out[k] = M[R[k]];
-  wsync(c);
-  bool bad = false;
-  for (u32 k = threadIdx.x; k < n; k += c.T) {
-    // source k, pushed unit i = k - 1 (rev) or k + 1 (fwd)
-    if (dir ? k + 1 >= n : k == 0) continue;
-    const u32 src = R[k];
-    if (bep[src] == UNBOUND) continue;
-    i64 T = dir ? (i64)pos64(S[k]) + M[src] : (i64)pos64(S[k]) - M[src];
-    u32 i = dir ? k + 1 : k - 1;
-    for (;;) {
-      const u32 u = R[i];
-      if (bep[u] == UNBOUND) break;
-      const i64 p = (i64)pos64(S[i]);
-      const i64 t = dir ? p + M[u] : p - M[u];
-      if (dir ? t > lim : t <= lim) break;
-      if (dir ? T > lim : T <= lim) {
-        bad = true;
-        break;
-      }
-      if (dir ? T < t : T > t) break;
-      T += dir ? 1 : -1;
-      atomicMax(&out[i], (u32)(dir ? T - p : p - T));
-      if (dir ? i + 1 >= n : i == 0) break;
-      i += dir ? 1u : ~0u;
-    }
+  const u32 src = R[k];
+  if (c.bep[src] == UNBOUND) return true;
+  i64 T = dir ? (i64)pos64(S[k]) + M[src] : (i64)pos64(S[k]) - M[src];
+#pragma unroll 1
+  for (u32 i = dir ? k + 1 : k - 1; i < n; i += dir ? 1u : ~0u) {  // below rank 0 wraps past n
+    const u32 u = R[i];
+    if (c.bep[u] == UNBOUND) break;
+    const i64 p = (i64)pos64(S[i]);
+    const i64 t = dir ? p + M[u] : p - M[u];
+    if (dir ? t > lim : t <= lim) break;
+    if (dir ? T > lim : T <= lim) return false;
+    if (dir ? T < t : T > t) break;
+    T += dir ? 1 : -1;
+    atomicMax(&out[i], (u32)(dir ? T - p : p - T));
   }
-  if (wsync_or(c, bad)) return false;
-#pragma unroll 4
-  for (u32 k = threadIdx.x; k < n; k += c.T) M[R[k]] = out[k];
-  wsync(c);
   return true;
 }
 
-__device__ void adjust_moves(Cell& c, const KParams& P, u32 n) {
-  const bool serial = P.debug_flags & DBG_SERIAL_ADJUST;
-  for (u32 dir = 0; dir < 2; ++dir) {
-    if (serial || !adjust_dir_block(c, P, dir, n)) {
-      prof_add(c, PF_ADJUST_FALLBACK, 1);
-      if (threadIdx.x == 0) adjust_dir_serial(c, P, dir, n);
-      wsync(c);
+// The walks of all units that push a neighbour.  Returns (to every worker) false when the result is rejected.
+template <bool SM>
+__device__ __noinline__ bool adjust_pushed(u32 n, const Arr<SM> out_r, const Arr<SM> out_f) {
+  const View<SM> c;
+  const Arr<SM> S[2] = {c.sr, c.sf}, out[2] = {out_r, out_f};
+  bool bad = false;
+  // 32 items per thread and direction at a time: a bit for each unit that pushes
+#pragma unroll 1
+  for (u32 base = 0; base < n; base += 32 * c.T) {
+    u32 push[2] = {0, 0};
+#pragma unroll
+    for (u32 dir = 0; dir < 2; ++dir) {
+      u32 b = 0;
+#pragma unroll 1
+      for (u32 k = base + threadIdx.x; b < 32 && k < n; k += c.T, ++b) {
+        const bool end = dir ? k + 1 >= n : k == 0;
+        if (!end && adjust_pushes(dir, S[dir], out[dir], k, dir ? k + 1 : k - 1)) push[dir] |= 1u << b;
+      }
+    }
+    // comparisons before walks: a later group of a large cell compares moves already pushed, which only
+    // adds sources whose own, unpushed targets stop at once
+    if (wsync_or(c.T, (push[0] | push[1]) != 0)) {
+#pragma unroll
+      for (u32 dir = 0; dir < 2; ++dir) {
+#pragma unroll 1
+        for (u32 r = push[dir]; r; r &= r - 1)
+          bad |= !adjust_walk<SM>(dir, n, base + threadIdx.x + (u32)(__ffs(r) - 1) * c.T, out[dir]);
+      }
     }
   }
+  return !wsync_or(c.T, bad);
+}
+
+// Ranked positions (sr, sf), adjusted and, with clamp, clamped moves (clamp_moves,
+// simulation.cpp:325-340) in three sweeps; zeroes the collision words, one of whose arrays is its
+// scratch: callers that keep the words restore them.
+template <bool SM>
+__device__ __noinline__ void place_moves(u32 n, bool clamp) {
+  const View<SM> c;
+  const KParams& P = g_P;
+  const u32 T = c.T;
+  const auto rr = c.rr;
+  const auto fr = c.fr;
+  const auto rev = c.rev;
+  const auto fwd = c.fwd;
+  const auto rm = c.rm;
+  const auto fm = c.fm;
+  const auto out_r = c.tmp;
+  const auto out_f = c.rc;
+#pragma unroll 1
+  for (u32 k = threadIdx.x; k < n; k += T) {
+    const u32 ru = rr[k], fu = fr[k];
+    c.sr[k] = rev[ru];
+    c.sf[k] = fwd[fu];
+    out_r[k] = rm[ru];
+    out_f[k] = fm[fu];
+  }
+  wsync(c.T);
+  const bool serial = (P.debug_flags & DBG_SERIAL_ADJUST) || !adjust_pushed<SM>(n, out_r, out_f);
+  if (serial) {
+    prof_add(PF_ADJUST_FALLBACK, 1);
+    if (threadIdx.x == 0) {
+      adjust_dir_serial(g_c, P, 0, n);
+      adjust_dir_serial(g_c, P, 1, n);
+    }
+    wsync(c.T);
+  }
+  const u64 start = P.start, end = P.end;
+#pragma unroll 1
+  for (u32 k = threadIdx.x; k < n; k += T) {
+    const u32 ru = rr[k], fu = fr[k];
+    u64 mr = serial ? rm[ru] : out_r[k], mf = serial ? fm[fu] : out_f[k];
+    if (clamp && c.bep[ru] != UNBOUND) mr = min(mr, pos64(c.sr[k]) - start);
+    if (clamp && c.bep[fu] != UNBOUND) mf = min(mf, end - pos64(c.sf[k]) - 1);
+    rm[ru] = (u32)mr;
+    fm[fu] = (u32)mf;
+    c.rc[k] = 0;
+    c.fc[k] = 0;
+  }
+  wsync(c.T);
 }
 
 // clamp_moves (simulation.cpp:325-340)
-__device__ __noinline__ void clamp_moves(Cell& c, const KParams& P, u32 n) {
-  const u32* __restrict__ bep = c.bep;
-  const u32* __restrict__ rev = c.rev;
-  const u32* __restrict__ fwd = c.fwd;
-  u32* __restrict__ rm = c.rm;
-  u32* __restrict__ fm = c.fm;
+template <bool SM>
+__device__ __noinline__ void clamp_moves(u32 n) {
+  const View<SM> c;
+  const KParams& P = g_P;
+  const auto bep = c.bep;
+  const auto rev = c.rev;
+  const auto fwd = c.fwd;
+  const auto rm = c.rm;
+  const auto fm = c.fm;
   const u64 start = P.start, end = P.end;
-#pragma unroll 4
+#pragma unroll 1
   for (u32 i = threadIdx.x; i < n; i += c.T) {
     if (bep[i] == UNBOUND) continue;
     const u64 rmv = min((u64)rm[i], pos64(rev[i]) - start);
@@ -1997,29 +2276,34 @@ __device__ __noinline__ void clamp_moves(Cell& c, const KParams& P, u32 n) {
     rm[i] = (u32)rmv;
     fm[i] = (u32)fmv;
   }
-  wsync(c);
+  wsync(c.T);
 }
 
 // ranked positions sorted (non-decreasing)?  Needed by the closed forms below; the epoch loop
 // always satisfies it, caller-provided ranks may not.
-__device__ __noinline__ bool ranked_sorted(const Cell& c, u32 n) {
+template <bool SM>
+__device__ __noinline__ bool ranked_sorted(u32 n) {
+  const View<SM> c;
   bool bad = false;
+#pragma unroll 1
   for (u32 k = threadIdx.x + 1; k < n; k += c.T) bad |= c.sr[k - 1] > c.sr[k] || c.sf[k - 1] > c.sf[k];
-  return !wsync_or(c, bad);
+  return !wsync_or(c.T, bad);
 }
 
 // Bucket index over a sorted array of ranked positions (unbound units, UNBOUND, at the tail):
 // T[b] = #{k : key[k] < start + (b << shift)} for b in [0, nbk], with shift chosen so that
 // nbk + 1 <= n (about one key per bucket).  lower_bound(x) then starts from T[b(x)] and scans a
 // few keys instead of a binary search over the whole array.
+template <bool SM>
 struct BucketIndex {
-  const u32* key;
-  const u32* T;
+  Arr<SM> key, T;
   u32 n, start, shift, nbk;
+  bool table;
   // first k in [0, n) with key[k] >= x
   __device__ u32 lower_bound(u32 x) const {
-    if (!T) {  // n too small for a table
+    if (!table) {  // n too small for a table
       u32 lo = 0, hi = n;
+#pragma unroll 1
       while (lo < hi) {
         const u32 mid = (lo + hi) >> 1;
         if (key[mid] >= x) hi = mid; else lo = mid + 1;
@@ -2030,15 +2314,18 @@ struct BucketIndex {
     u32 b = (x - start) >> shift;
     if (b > nbk) b = nbk;
     u32 k = T[b];
+#pragma unroll 1
     while (k < n && key[k] < x) ++k;
     return k;
   }
 };
 
 // Collective; T needs n entries.
-__device__ __forceinline__ BucketIndex build_bucket_index(const Cell& c, const u32* key, u32 n, u32 start, u32 end,
-                                                          u32* T) {
-  BucketIndex ix{key, nullptr, n, start, 0, 0};
+template <bool SM>
+__device__ __forceinline__ BucketIndex<SM> build_bucket_index(const Arr<SM> key, u32 n, u32 start, u32 end,
+                                                               const Arr<SM> T) {
+  const View<SM> c;
+  BucketIndex<SM> ix{key, T, n, start, 0, 0, false};
   if (n < 8 || end <= start) return ix;
   const u32 range = end - start;
   // smallest shift with (range >> shift) + 2 <= n
@@ -2047,9 +2334,11 @@ __device__ __forceinline__ BucketIndex build_bucket_index(const Cell& c, const u
     const int d = __clz(n - 2) - __clz(range);
     shift = d > 0 ? (u32)d : 0u;
     if (shift && (range >> (shift - 1)) + 2 <= n) --shift;
+#pragma unroll 1
     while ((range >> shift) + 2 > n) ++shift;
   }
   const u32 nbk = range >> shift;
+#pragma unroll 1
   for (u32 k = threadIdx.x; k <= n; k += c.T) {
     u32 bmin = 0, bmax = nbk;
     if (k > 0) {
@@ -2060,10 +2349,11 @@ __device__ __forceinline__ BucketIndex build_bucket_index(const Cell& c, const u
       const u32 hi = key[k];
       if (hi != UNBOUND) bmax = min(nbk, (hi - start) >> shift);
     }
+#pragma unroll 1
     for (u32 b = bmin; b <= bmax; ++b) T[b] = k;
   }
-  wsync(c);
-  ix.T = T;
+  wsync(c.T);
+  ix.table = true;
   ix.shift = shift;
   ix.nbk = nbk;
   return ix;
@@ -2088,20 +2378,24 @@ __device__ __forceinline__ bool trial_outcome(const Trial& t, u64 u) {
 // (EV_HIT), fwd units with the complemented index.
 constexpr u32 EV_HIT = EV_COLLISION | EV_CHROM_BOUNDARY | EV_LEF_BAR;
 
-__device__ __noinline__ u64 detect_lef_bar_dir(Cell& c, const KParams& P, u64 rp, u32 dir, u32 n, u64 n5, u64 n3) {
+template <bool SM>
+__device__ __noinline__ u64 detect_lef_bar_dir(u64 rp, u32 dir, u32 n, u64 n5, u64 n3) {
+  const View<SM> c;
+  const KParams& P = g_P;
   const u32 T = c.T;
-  const u32* __restrict__ R = dir ? c.fr : c.rr;
-  const u32* __restrict__ S = dir ? c.sf : c.sr;
-  const u32* __restrict__ bep = c.bep;
-  const u32* __restrict__ M = dir ? c.fm : c.rm;
-  u32* C = dir ? c.fc : c.rc;
+  const auto R = dir ? c.fr : c.rr;
+  const auto S = dir ? c.sf : c.sr;
+  const auto bep = c.bep;
+  const auto M = dir ? c.fm : c.rm;
+  const auto C = dir ? c.fc : c.rc;
   // rev: first k >= j0 with S[k] > bpos; fwd: last k <= jtop with S[k] < bpos
   const u32 j0 = (u32)min(n5, n5 - 1);
   const u32 jtop = (u32)(n - min(n3, n3 - 1)) - 1;
-  const BucketIndex ix = build_bucket_index(c, S, n, (u32)P.start, (u32)P.end, c.tmp);
+  const BucketIndex<SM> ix = build_bucket_index<SM>(S, n, (u32)P.start, (u32)P.end, c.tmp);
   u32 buf = 0;
+#pragma unroll 1
   for (u32 base = 0; base < c.nb; base += 2 * T) {
-    rng_ensure(c, rp, 2 * T);
+    rng_ensure(rp, 2 * T);
     u32 bi[2], unit[2];
     int ti[2];
     bool cand[2], drawn[2];
@@ -2113,7 +2407,7 @@ __device__ __noinline__ u64 detect_lef_bar_dir(Cell& c, const KParams& P, u64 rp
       ti[h] = 0;
       if (o < c.nb) {
         const u32 i = dir ? c.nb - 1 - o : o;
-        if (bar_active(c, i)) {
+        if (bar_active(c.bst, i)) {
           const uint2 pf = __ldg(&c.bpf[i]);
           const u32 bdir = pf.y & BF_DIR_MASK;
           u32 k = ix.lower_bound(dir ? pf.x : pf.x + 1);
@@ -2142,41 +2436,47 @@ __device__ __noinline__ u64 detect_lef_bar_dir(Cell& c, const KParams& P, u64 rp
         }
       }
     }
-    const Scan2 s = scan2(c, buf, drawn[0], drawn[1]);
-    rng_publish(c, rp);  // the draws of the windows before
+    const Scan2 s = scan2<SM>(buf, drawn[0], drawn[1]);
+    rng_publish(rp);  // the draws of the windows before
     buf ^= 1;
 #pragma unroll
     for (u32 h = 0; h < 2; ++h) {
       if (cand[h]) {
-        const u64 u = drawn[h] ? ring_at(c, rp + (h ? s.off1 : s.off0)) : 0;
+        const u64 u = drawn[h] ? ring_at(c.rmask, rp + (h ? s.off1 : s.off0)) : 0;
         if (trial_outcome(P.lef_bar[ti[h]], u))
           atomicMax(&C[unit[h]], cw_make(dir ? CW_IDX_MASK - bi[h] : bi[h], EV_HIT));
       }
     }
     rp += s.total;
   }
-  wsync(c);
-  rng_publish(c, rp);
+  wsync(c.T);
+  rng_publish(rp);
   return rp;
 }
 
-__device__ __noinline__ u64 detect_lef_bar_block(Cell& c, const KParams& P, u64 rp, u32 n, u64 n5, u64 n3) {
-  rp = detect_lef_bar_dir(c, P, rp, 0, n, n5, n3);
-  rp = detect_lef_bar_dir(c, P, rp, 1, n, n5, n3);
+template <bool SM>
+__device__ __noinline__ u64 detect_lef_bar_block(u64 rp, u32 n, u64 n5, u64 n3) {
+  const View<SM> c;
+  rp = detect_lef_bar_dir<SM>(rp, 0, n, n5, n3);
+  rp = detect_lef_bar_dir<SM>(rp, 1, n, n5, n3);
+#pragma unroll 1
   for (u32 i = threadIdx.x; i < n; i += c.T) {
     const u32 r = c.rc[i], f = c.fc[i];
     if (cw_event(r) == EV_HIT) c.rc[i] = cw_make(cw_idx(r), EV_COLLISION | EV_LEF_BAR);
     if (cw_event(f) == EV_HIT) c.fc[i] = cw_make(CW_IDX_MASK - cw_idx(f), EV_COLLISION | EV_LEF_BAR);
   }
-  wsync(c);
+  wsync(c.T);
   return rp;
 }
 
 // No caller-provided collision word uses the sweep's own code (the epoch loop writes none).
-__device__ __noinline__ bool words_plain(const Cell& c, u32 n) {
+template <bool SM>
+__device__ __noinline__ bool words_plain(u32 n) {
+  const View<SM> c;
   bool bad = false;
+#pragma unroll 1
   for (u32 i = threadIdx.x; i < n; i += c.T) bad |= cw_event(c.rc[i]) == EV_HIT || cw_event(c.fc[i]) == EV_HIT;
-  return !wsync_or(c, bad);
+  return !wsync_or(c.T, bad);
 }
 
 // detect_primary_lef_lef_collisions (simulation_detect_collisions.cpp:255-401).
@@ -2184,15 +2484,19 @@ __device__ __noinline__ bool words_plain(const Cell& c, u32 n) {
 // exactly the rev units j >= n5 with cnt(j) > cnt(j - 1) (cnt(n5 - 1) := 0) and cnt(j) < i2,
 // each against the fwd unit of rank cnt(j) - 1.  Tested pairs are disjoint, so their
 // collision words are updated independently; trials draw in ascending j.
-__device__ __noinline__ u64 detect_primary_block(Cell& c, const KParams& P, u64 rp, u32 n, u64 n5, u64 n3) {
+template <bool SM>
+__device__ __noinline__ u64 detect_primary_block(u64 rp, u32 n, u64 n5, u64 n3) {
+  const View<SM> c;
+  const KParams& P = g_P;
   if (n5 == n || n3 == n) return rp;
   const u32 T = c.T;
   const u32 i2 = (u32)(n - min(n3, n3 - 1));
   // bucket index over the fwd ranked positions (this step can also run on its own)
-  const BucketIndex ixf = build_bucket_index(c, c.sf, n, (u32)P.start, (u32)P.end, c.tmp);
+  const BucketIndex<SM> ixf = build_bucket_index<SM>(c.sf, n, (u32)P.start, (u32)P.end, c.tmp);
   u32 buf = 0;
+#pragma unroll 1
   for (u32 base = (u32)n5; base < n; base += 2 * T) {
-    rng_ensure(c, rp, 2 * T);
+    rng_ensure(rp, 2 * T);
     u32 ru[2], fu[2], rp_[2], fp_[2], rmv[2], fmv[2];
     bool cand[2], drawn[2];
 #pragma unroll
@@ -2217,43 +2521,48 @@ __device__ __noinline__ u64 detect_primary_block(Cell& c, const KParams& P, u64 
         drawn[h] = cand[h] && trial_needs_draw(P.lef_lef);
       }
     }
-    const Scan2 s = scan2(c, buf, drawn[0], drawn[1]);
-    rng_publish(c, rp);
+    const Scan2 s = scan2<SM>(buf, drawn[0], drawn[1]);
+    rng_publish(rp);
     buf ^= 1;
 #pragma unroll
     for (u32 h = 0; h < 2; ++h) {
-      if (cand[h] && trial_outcome(P.lef_lef, drawn[h] ? ring_at(c, rp + (h ? s.off1 : s.off0)) : 0))
+      if (cand[h] && trial_outcome(P.lef_lef, drawn[h] ? ring_at(c.rmask, rp + (h ? s.off1 : s.off0)) : 0))
         primary_pair_update(c, ru[h], fu[h], pos64(rp_[h]), pos64(fp_[h]), rmv[h], fmv[h]);
     }
     rp += s.total;
   }
-  wsync(c);
-  rng_publish(c, rp);
+  wsync(c.T);
+  rng_publish(rp);
   return rp;
 }
 
 // correct_moves_for_lef_bar_collisions (simulation_correct_moves.cpp:20-51)
-__device__ __noinline__ void correct_lef_bar(Cell& c, u32 n) {
-  const u32* __restrict__ rc = c.rc;
-  const u32* __restrict__ fc = c.fc;
-  const u32* __restrict__ rev = c.rev;
-  const u32* __restrict__ fwd = c.fwd;
-  u32* __restrict__ rm = c.rm;
-  u32* __restrict__ fm = c.fm;
-#pragma unroll 4
+template <bool SM>
+__device__ __noinline__ void correct_lef_bar(u32 n) {
+  const View<SM> c;
+  const auto rc = c.rc;
+  const auto fc = c.fc;
+  const auto rev = c.rev;
+  const auto fwd = c.fwd;
+  const auto rm = c.rm;
+  const auto fm = c.fm;
+#pragma unroll 1
   for (u32 i = threadIdx.x; i < n; i += c.T) {
     const u32 r = rc[i], f = fc[i];
-    if (cw_occurred_as(r, EV_LEF_BAR)) rm[i] = (u32)(pos64(rev[i]) - bar_pos(c, cw_idx(r)) - 1);
-    if (cw_occurred_as(f, EV_LEF_BAR)) fm[i] = (u32)(bar_pos(c, cw_idx(f)) - pos64(fwd[i]) - 1);
+    if (cw_occurred_as(r, EV_LEF_BAR)) rm[i] = (u32)(pos64(rev[i]) - bar_pos(c.bpf, cw_idx(r)) - 1);
+    if (cw_occurred_as(f, EV_LEF_BAR)) fm[i] = (u32)(bar_pos(c.bpf, cw_idx(f)) - pos64(fwd[i]) - 1);
   }
-  wsync(c);
+  wsync(c.T);
 }
 
 // correct_moves_for_primary_lef_lef_collisions (simulation_correct_moves.cpp:54-122): the
 // pairs it visits are disjoint, so both passes are parallel.
-__device__ __noinline__ void correct_primary(Cell& c, u32 n) {
+template <bool SM>
+__device__ __noinline__ void correct_primary(u32 n) {
+  const View<SM> c;
   // detect_primary pairs each fwd unit with at most one rev unit, so visiting the units in
   // index order instead of rank order changes nothing
+#pragma unroll 1
   for (u32 rev_idx = threadIdx.x; rev_idx < n; rev_idx += c.T) {
     const u32 r = c.rc[rev_idx];
     if (!cw_occurred_as(r, EV_PRIMARY)) continue;
@@ -2269,7 +2578,8 @@ __device__ __noinline__ void correct_primary(Cell& c, u32 n) {
       c.rm[rev_idx] = (u32)(pos64(c.rev[rev_idx]) - (pos64(c.fwd[fwd_idx]) + c.fm[fwd_idx]) - 1);
     }
   }
-  wsync(c);
+  wsync(c.T);
+#pragma unroll 1
   for (u32 fwd_idx = threadIdx.x; fwd_idx < n; fwd_idx += c.T) {
     const u32 f = c.fc[fwd_idx];
     if (!cw_occurred_as(f, EV_PRIMARY)) continue;
@@ -2278,7 +2588,52 @@ __device__ __noinline__ void correct_primary(Cell& c, u32 n) {
       c.fm[fwd_idx] = (u32)((pos64(c.rev[rev_idx]) - c.rm[rev_idx]) - pos64(c.fwd[fwd_idx]) - 1);
     }
   }
-  wsync(c);
+  wsync(c.T);
+}
+
+// Both corrections in one sweep, as the epoch loop needs them: a pair's partner that a barrier stopped
+// takes its corrected move from the barrier's position instead of waiting for it to be written, and of a
+// primary pair the rev unit's thread writes both moves.
+template <bool SM>
+__device__ __noinline__ void correct_moves(u32 n) {
+  const View<SM> c;
+  const auto rc = c.rc;
+  const auto fc = c.fc;
+  const auto rev = c.rev;
+  const auto fwd = c.fwd;
+  const auto rm = c.rm;
+  const auto fm = c.fm;
+#pragma unroll 1
+  for (u32 i = threadIdx.x; i < n; i += c.T) {
+    const u32 r = rc[i], f = fc[i];
+    if (cw_occurred_as(r, EV_LEF_BAR)) {
+      rm[i] = (u32)(pos64(rev[i]) - bar_pos(c.bpf, cw_idx(r)) - 1);
+    } else if (cw_occurred_as(r, EV_PRIMARY)) {
+      const u32 j = cw_idx(r);
+      const u32 g = fc[j];
+      if (cw_occurred_as(g, EV_PRIMARY)) {
+        const u64 rp = pos64(rev[i]), fp = pos64(fwd[j]);
+        u64 p1, p2;
+        lef_lef_collision_pos(rp, fp, rm[i], fm[j], p1, p2);
+        rm[i] = (u32)(rp - p1);
+        fm[j] = (u32)(p2 - fp);
+      } else if (cw_occurred_as(g, EV_LEF_BAR)) {
+        const u32 mj = (u32)(bar_pos(c.bpf, cw_idx(g)) - pos64(fwd[j]) - 1);
+        rm[i] = (u32)(pos64(rev[i]) - (pos64(fwd[j]) + mj) - 1);
+      }
+    }
+    if (cw_occurred_as(f, EV_LEF_BAR)) {
+      fm[i] = (u32)(bar_pos(c.bpf, cw_idx(f)) - pos64(fwd[i]) - 1);
+    } else if (cw_occurred_as(f, EV_PRIMARY)) {
+      const u32 j = cw_idx(f);
+      const u32 g = rc[j];
+      if (cw_occurred_as(g, EV_LEF_BAR)) {
+        const u32 mj = (u32)(pos64(rev[j]) - bar_pos(c.bpf, cw_idx(g)) - 1);
+        fm[i] = (u32)((pos64(rev[j]) - mj) - pos64(fwd[i]) - 1);
+      }
+    }
+  }
+  wsync(c.T);
 }
 
 // process_secondary_lef_lef_collisions (simulation_detect_collisions.cpp:404-518).
@@ -2292,21 +2647,21 @@ __device__ __noinline__ void correct_primary(Cell& c, u32 n) {
 // chain is walked with its draws.
 enum ChainMode { CHAIN_COUNT = 0, CHAIN_RING = 1, CHAIN_SERIAL = 2 };
 
-template <int MODE>
-__device__ __forceinline__ u32 chain_walk(Cell& c, const KParams& P, u32 dir, u32 n, i64 k, u64 at) {
-  const Trial& tr = P.lef_lef;
-  const u32* R = dir ? c.fr : c.rr;
-  u32* M = dir ? c.fm : c.rm;
-  u32* C = dir ? c.fc : c.rc;
-  const u32* S = dir ? c.sf : c.sr;
+template <int MODE, class C>
+__device__ __forceinline__ u32 chain_walk(const C& c, const Trial& tr, u32 dir, u32 n, i64 k, u64 at) {
+  const auto R = dir ? c.fr : c.rr;
+  const auto M = dir ? c.fm : c.rm;
+  const auto W = dir ? c.fc : c.rc;
+  const auto S = dir ? c.sf : c.sr;
   const i64 step = dir ? -1 : 1;
   const i64 stop = dir ? -1 : (i64)n;
   u32 idx_prev = R[k - step];
   u64 tprev = dir ? pos64(S[k - step]) + M[idx_prev] : pos64(S[k - step]) - M[idx_prev];
   u32 trials = 0;
+#pragma unroll 1
   for (; k != stop; k += step) {
     const u32 idx = R[k];
-    if (cw_occurred(C[idx])) break;  // stalled on entry: the next chain starts after it
+    if (cw_occurred(W[idx])) break;  // stalled on entry: the next chain starts after it
     const u64 p = pos64(S[k]);
     const u64 m = M[idx];
     if (!(dir ? (p + m >= tprev) : (p - m <= tprev))) break;
@@ -2317,19 +2672,19 @@ __device__ __forceinline__ u32 chain_walk(Cell& c, const KParams& P, u32 dir, u3
       ok = false;
     } else {
       u64 u = 0;
-      if (MODE == CHAIN_RING) u = ring_at(c, at++);
-      if (MODE == CHAIN_SERIAL) u = rng_serial(c);
+      if (MODE == CHAIN_RING) u = ring_at(c.rmask, at++);
+      if (MODE == CHAIN_SERIAL) u = rng_serial(g_c);
       ok = MODE == CHAIN_COUNT || u <= tr.thr;
     }
     ++trials;
     if (!ok) {
-      if (MODE != CHAIN_COUNT) C[idx] = cw_make(idx_prev, EV_SECONDARY);
+      if (MODE != CHAIN_COUNT) W[idx] = cw_make(idx_prev, EV_SECONDARY);
       break;
     }
     const u64 mv = dir ? (tprev - p) : (p - tprev);
     const u64 m2 = min(mv, mv - 1);
     if (MODE != CHAIN_COUNT) {
-      C[idx] = cw_make(idx_prev, EV_COLLISION | EV_SECONDARY);
+      W[idx] = cw_make(idx_prev, EV_COLLISION | EV_SECONDARY);
       M[idx] = (u32)m2;
     }
     tprev = dir ? p + m2 : p - m2;
@@ -2338,19 +2693,22 @@ __device__ __forceinline__ u32 chain_walk(Cell& c, const KParams& P, u32 dir, u3
   return trials;
 }
 
-__device__ __noinline__ u64 secondary_dir_block(Cell& c, const KParams& P, u64 rp, u32 dir, u32 n, u64 n5, u64 n3) {
+template <bool SM>
+__device__ __noinline__ u64 secondary_dir_block(u64 rp, u32 dir, u32 n, u64 n5, u64 n3) {
+  const View<SM> c;
+  const KParams& P = g_P;
   const u32 T = c.T;
-  const u32* R = dir ? c.fr : c.rr;
-  const u32* C = dir ? c.fc : c.rc;
+  const auto R = dir ? c.fr : c.rr;
+  const auto C = dir ? c.fc : c.rc;
   // chain starts (index of the first free unit): rev: k in [max(1, n5), n) with R[k-1]
   // stalled and R[k] free, ascending; fwd: k = i - 1 for i in [1, itop] with R[i] stalled
   // and R[k] free, in descending i.  Each start pairs with its own stalled unit: at most n / 2.
-  u32* starts = c.tmp;
-  BlockTmp* bt = c.bt;
+  const auto starts = c.tmp;
   const i64 itop = (i64)(n - min(n3, n3 - 1)) - 1;
   const u32 k0 = (u32)max((u64)1, n5);
   const u32 items = dir ? (itop > 0 ? (u32)itop : 0u) : (n > k0 ? n - k0 : 0u);
   u32 nst = 0, buf = 0;
+#pragma unroll 1
   for (u32 base = 0; base < items; base += 2 * T) {
     bool st[2];
     u32 at[2];
@@ -2366,39 +2724,60 @@ __device__ __noinline__ u64 secondary_dir_block(Cell& c, const KParams& P, u64 r
         at[h] = k;
       }
     }
-    const Scan2 s = scan2(c, buf, st[0], st[1]);
+    const Scan2 s = scan2<SM>(buf, st[0], st[1]);
     buf ^= 1;
     if (st[0]) starts[nst + s.off0] = at[0];
     if (st[1]) starts[nst + s.off1] = at[1];
     nst += s.total;
   }
-  wsync(c);
+  wsync(c.T);
   if (nst == 0) return rp;
-  u32* lens = c.tmp + nst;  // trials of each chain if all succeed, then its first draw's offset
-  for (u32 q = threadIdx.x; q < nst; q += T) lens[q] = chain_walk<CHAIN_COUNT>(c, P, dir, n, starts[q], 0);
-  wsync(c);
+  const auto lens = c.tmp + nst;  // trials of each chain if all succeed, then its first draw's offset
+#pragma unroll 1
+  for (u32 q = threadIdx.x; q < nst; q += T) lens[q] = chain_walk<CHAIN_COUNT>(c, P.lef_lef, dir, n, starts[q], 0);
+  wsync(c.T);
   const bool draws = trial_needs_draw(P.lef_lef);
   const u64 thr = P.lef_lef.thr;
-  const u32 lim = c.lim;  // draws of one round at most
+  const u32 lim = min(c.lim, 32 * TRIAL_WORDS - 32);  // draws of one round at most
   u32 q0 = 0;
+#pragma unroll 1
   while (q0 < nst) {
+    // outcomes of the next lim draws as trials, one bit each
+    if (draws) {
+      rng_ensure(rp, lim);
+#pragma unroll 1
+      for (u32 k = threadIdx.x; k < lim; k += T) {
+        const unsigned m = __ballot_sync(FULL, ring_at(c.rmask, rp + k) <= thr);
+        if (ln() == 0) g_bt.trial[k >> 5] = m;
+      }
+      wsync(c.T);
+    }
     if (threadIdx.x < 32) {
       u32 off = 0, q = q0;
+#pragma unroll 1
       for (; q < nst; q += 32) {
         const u32 ci = q + ln();
         const u32 L = ci < nst && draws ? lens[ci] : 0u;
         u32 tot;
         u32 o = off + warp_excl_scan(L, &tot);
         if (off + tot > lim) break;
-        rng_ensure(c, rp, off + tot);
         u32 fixed = 0;  // lanes whose offset is settled
+#pragma unroll 1
         for (;;) {
           bool dev = false;
           u32 used = L;
           if (L >= 2 && ln() >= fixed) {
+            // trials until the first failure: 32 outcomes from bit o, more only in a very long chain
             u32 k = 0;
-            while (k + 1 < L && ring_at(c, rp + o + k) <= thr) ++k;
-            used = k + 1;
+#pragma unroll 1
+            for (;;) {
+              const u32 at = o + k;
+              const u32 bits = ~__funnelshift_r(g_bt.trial[at >> 5], g_bt.trial[(at >> 5) + 1], at & 31u);
+              const u32 f = bits ? (u32)(__ffs(bits) - 1) : 32u;
+              k += f;
+              if (f < 32 || k >= L) break;
+            }
+            used = min(L, k + 1);
             dev = used < L;
           }
           const unsigned dm = __ballot_sync(FULL, dev);
@@ -2413,156 +2792,176 @@ __device__ __noinline__ u64 secondary_dir_block(Cell& c, const KParams& P, u64 r
         off += tot;
       }
       if (ln() == 0) {
-        bt->qend = min(q, nst);
-        bt->used = off;
+        g_bt.qend = min(q, nst);
+        g_bt.used = off;
       }
     }
-    wsync(c);
-    const u32 q1 = bt->qend, used = bt->used;
+    wsync(c.T);
+    const u32 q1 = g_bt.qend, used = g_bt.used;
     if (q1 == q0) {
       // 32 chains that might outrun the ring: walk them one by one
-      prof_add(c, PF_CHAIN_SERIAL, 1);
+      prof_add(PF_CHAIN_SERIAL, 1);
       const u32 qe = min(q0 + 32, nst);
       if (threadIdx.x == 0) {
-        for (u32 q = q0; q < qe; ++q) chain_walk<CHAIN_SERIAL>(c, P, dir, n, starts[q], 0);
+#pragma unroll 1
+        for (u32 q = q0; q < qe; ++q) chain_walk<CHAIN_SERIAL>(c, P.lef_lef, dir, n, starts[q], 0);
       }
-      wsync(c);
-      rp = c.sc->rpos;
+      wsync(c.T);
+      rp = g_sc.rpos;
       q0 = qe;
       continue;
     }
-    rng_ensure(c, rp, used);
+#pragma unroll 1
     for (u32 q = q0 + threadIdx.x; q < q1; q += T)
-      chain_walk<CHAIN_RING>(c, P, dir, n, starts[q], rp + lens[q]);
+      chain_walk<CHAIN_RING>(c, P.lef_lef, dir, n, starts[q], rp + lens[q]);
     rp += used;
     q0 = q1;
-    wsync(c);
-    rng_publish(c, rp);
+    wsync(c.T);
+    rng_publish(rp);
   }
-  wsync(c);
+  wsync(c.T);
   return rp;
 }
 
 // fix_secondary_lef_lef_collisions: candidates (units marked avoided) are never
 // adjacent in rank order (the unit before a rev candidate, after a fwd candidate, is stalled),
 // so each is an independent swap of two neighbours.
-__device__ __noinline__ bool fix_secondary_block(Cell& c, const KParams& P, u32 n, u64 n5, u64 n3) {
+template <bool SM>
+__device__ __noinline__ bool fix_secondary_block(u32 n, u64 n5, u64 n3) {
+  const View<SM> c;
+  const KParams& P = g_P;
   const u32 T = c.T;
   const u32 k0 = (u32)max((u64)1, n5);
   const u32 naf = (u32)(n - min(n3, n3 - 1));
-  BlockTmp* bt = c.bt;
-  if (threadIdx.x == 0) bt->nr = bt->nf = 0;
-  wsync(c);
+  if (threadIdx.x == 0) g_bt.nr = g_bt.nf = 0;
+  wsync(c.T);
   // candidate ranks: rev [k0, n), fwd [0, naf - 1); rev list from the front of tmp, fwd list from its end
-  u32* list = c.tmp;
+  const auto list = c.tmp;
   bool adj = false;
+#pragma unroll 1
   for (u32 k = k0 + threadIdx.x; k < n; k += T) {
     if (!cw_avoided_as(c.rc[c.rr[k]], EV_SECONDARY)) continue;
     if (k > k0 && cw_avoided_as(c.rc[c.rr[k - 1]], EV_SECONDARY)) adj = true;
-    const u32 s = atomicAdd(&bt->nr, 1u);
+    const u32 s = atomicAdd(&g_bt.nr, 1u);
     if (s < n) list[s] = k;
   }
-  wsync(c);
-  const u32 nr = bt->nr;
+  wsync(c.T);
+  const u32 nr = g_bt.nr;
+#pragma unroll 1
   for (u32 k = threadIdx.x; k + 1 < naf; k += T) {
     if (!cw_avoided_as(c.fc[c.fr[k]], EV_SECONDARY)) continue;
     if (k > 0 && cw_avoided_as(c.fc[c.fr[k - 1]], EV_SECONDARY)) adj = true;
-    const u32 s = atomicAdd(&bt->nf, 1u);
+    const u32 s = atomicAdd(&g_bt.nf, 1u);
     if (nr + s < n) list[nr + s] = k;
   }
-  if (wsync_or(c, adj)) return false;
-  const u32 nf = bt->nf;
+  if (wsync_or(c.T, adj)) return false;
+  const u32 nf = g_bt.nf;
   if (nr + nf > n) return false;
+#pragma unroll 1
   for (u32 t = threadIdx.x; t < nr; t += T) fix_rev_at(c, P.start, list[t]);
-  wsync(c);
+  wsync(c.T);
+#pragma unroll 1
   for (u32 t = threadIdx.x; t < nf; t += T) fix_fwd_at(c, P.end, list[nr + t]);
-  wsync(c);
+  wsync(c.T);
   return true;
 }
 
 // process_collisions (simulation.cpp:925-955) in the reference's order.
 // sorted_ranks: the ranked positions are known to be sorted (the epoch loop ranks them itself);
 // otherwise (caller state) they are checked and unsorted ones take the serial restatement.
-__device__ __noinline__ u64 process_collisions(Cell& c, const KParams& P, u64 rp, u32 n, bool fix,
+template <bool SM>
+__device__ __noinline__ u64 process_collisions(u64 rp, u32 n, bool fix,
                                                bool sorted_ranks = false) {
-  Scalars* sc = c.sc;
+  const View<SM> c;
+  const KParams& P = g_P;
   u64 t0 = clock64();
-  const bool serial = (P.debug_flags & DBG_SERIAL_COLLISIONS) || !(sorted_ranks || (ranked_sorted(c, n) && words_plain(c, n)));
+  const bool serial = (P.debug_flags & DBG_SERIAL_COLLISIONS) || !(sorted_ranks || (ranked_sorted<SM>(n) && words_plain<SM>(n)));
   if (threadIdx.x == 0) {
     u64 n5, n3;
     detect_boundaries_serial(c, P, n, n5, n3);
-    sc->n5 = n5;
-    sc->n3 = n3;
+    g_sc.n5 = n5;
+    g_sc.n3 = n3;
   }
-  wsync(c);
+  wsync(c.T);
   u64 t1 = clock64();
-  prof_add(c, PF_BOUNDARIES, t1 - t0);
-  const u64 n5 = sc->n5, n3 = sc->n3;
+  prof_add(PF_BOUNDARIES, t1 - t0);
+  const u64 n5 = g_sc.n5, n3 = g_sc.n3;
   if (serial) {
     if (threadIdx.x == 0) {
-      detect_lef_bar_serial(c, P, n, n5, n3);
-      detect_primary_serial(c, P, n, n5, n3);
+      detect_lef_bar_serial(g_c, P, n, n5, n3);
+      detect_primary_serial(g_c, P, n, n5, n3);
     }
-    wsync(c);
-    rp = sc->rpos;
+    wsync(c.T);
+    rp = g_sc.rpos;
   } else {
-    rp = detect_lef_bar_block(c, P, rp, n, n5, n3);
+    rp = detect_lef_bar_block<SM>(rp, n, n5, n3);
     t0 = clock64();
-    prof_add(c, PF_LEF_BAR, t0 - t1);
+    prof_add(PF_LEF_BAR, t0 - t1);
     t1 = t0;
-    rp = detect_primary_block(c, P, rp, n, n5, n3);
+    rp = detect_primary_block<SM>(rp, n, n5, n3);
   }
   t0 = clock64();
-  prof_add(c, PF_PRIMARY, t0 - t1);
-  correct_lef_bar(c, n);
-  correct_primary(c, n);
+  prof_add(PF_PRIMARY, t0 - t1);
+  if (sorted_ranks) {
+    correct_moves<SM>(n);
+  } else {
+    correct_lef_bar<SM>(n);
+    correct_primary<SM>(n);
+  }
   t1 = clock64();
-  prof_add(c, PF_CORRECT, t1 - t0);
+  prof_add(PF_CORRECT, t1 - t0);
   if (serial) {
-    if (threadIdx.x == 0) process_secondary_serial(c, P, n, n5, n3);
-    wsync(c);
-    rp = sc->rpos;
+    if (threadIdx.x == 0) process_secondary_serial(g_c, P, n, n5, n3);
+    wsync(c.T);
+    rp = g_sc.rpos;
   } else {
     // chains read ranked positions; secondary moves only change moves and words
-    rp = secondary_dir_block(c, P, rp, 0, n, n5, n3);
-    rp = secondary_dir_block(c, P, rp, 1, n, n5, n3);
+    rp = secondary_dir_block<SM>(rp, 0, n, n5, n3);
+    rp = secondary_dir_block<SM>(rp, 1, n, n5, n3);
   }
   t0 = clock64();
-  prof_add(c, PF_SECONDARY, t0 - t1);
+  prof_add(PF_SECONDARY, t0 - t1);
   if (fix) {
-    if (serial || !fix_secondary_block(c, P, n, n5, n3)) {
-      prof_add(c, PF_FIX_FALLBACK, 1);
-      if (threadIdx.x == 0) fix_secondary_serial(c, P, n, n5, n3);
-      wsync(c);
+    if (serial || !fix_secondary_block<SM>(n, n5, n3)) {
+      prof_add(PF_FIX_FALLBACK, 1);
+      if (threadIdx.x == 0) fix_secondary_serial(g_c, P, n, n5, n3);
+      wsync(c.T);
     }
   }
-  prof_add(c, PF_FIX, clock64() - t0);
+  prof_add(PF_FIX, clock64() - t0);
   return rp;
 }
 
 // extrude (simulation.cpp:489-512)
-__device__ __noinline__ void extrude(Cell& c, u32 n) {
-  const u32* __restrict__ bep = c.bep;
-  const u32* __restrict__ rm = c.rm;
-  const u32* __restrict__ fm = c.fm;
-  u32* __restrict__ rev = c.rev;
-  u32* __restrict__ fwd = c.fwd;
-#pragma unroll 4
+template <bool SM>
+__device__ __noinline__ void extrude(u32 n) {
+  const View<SM> c;
+  const auto bep = c.bep;
+  const auto rm = c.rm;
+  const auto fm = c.fm;
+  const auto rev = c.rev;
+  const auto fwd = c.fwd;
+#pragma unroll 1
   for (u32 i = threadIdx.x; i < n; i += c.T) {
     if (bep[i] == UNBOUND) continue;
     rev[i] -= rm[i];
     fwd[i] += fm[i];
   }
-  wsync(c);
+  wsync(c.T);
 }
 
-// release_lefs (simulation.cpp:544-592): one draw per bound LEF with p > 0.  bt->released counts
-// the released units (reset by the caller that wants it).
-__device__ __noinline__ u64 release_lefs(Cell& c, const KParams& P, u64 rp, u32 n, bool completed) {
+// release_lefs (simulation.cpp:544-592): one draw per bound LEF with p > 0; with move, after extrude
+// (simulation.cpp:489-512) of the units that stay.  bt->released counts the released units (reset by
+// the caller that wants it).
+template <bool SM>
+__device__ __noinline__ u64 release_lefs(u64 rp, u32 n, bool completed, bool move = false) {
+  const View<SM> c;
+  const KParams& P = g_P;
   const u32 T = c.T;
   u32 buf = 0;
+#pragma unroll 1
   for (u32 base = 0; base < n; base += 2 * T) {
-    rng_ensure(c, rp, 2 * T);
+    rng_ensure(rp, 2 * T);
     u64 thr[2];
     bool need[2];
 #pragma unroll
@@ -2573,89 +2972,125 @@ __device__ __noinline__ u64 release_lefs(Cell& c, const KParams& P, u64 rp, u32 
       if (i < n && c.bep[i] != UNBOUND) {
         const u32 r = c.rc[i], f = c.fc[i];
         u32 nh = 0;
-        if (cw_occurred_as(r, EV_LEF_BAR) && (bar_flags(c, cw_idx(r)) & BF_DIR_MASK) == MGPU_DIR_REV) ++nh;
-        if (cw_occurred_as(f, EV_LEF_BAR) && (bar_flags(c, cw_idx(f)) & BF_DIR_MASK) == MGPU_DIR_FWD) ++nh;
+        if (cw_occurred_as(r, EV_LEF_BAR) && (bar_flags(c.bpf, cw_idx(r)) & BF_DIR_MASK) == MGPU_DIR_REV) ++nh;
+        if (cw_occurred_as(f, EV_LEF_BAR) && (bar_flags(c.bpf, cw_idx(f)) & BF_DIR_MASK) == MGPU_DIR_FWD) ++nh;
         const Trial& tr = P.release[completed ? 1 : 0][nh];
         need[h] = tr.draws;
         thr[h] = tr.thr;
       }
     }
-    const Scan2 s = scan2(c, buf, need[0], need[1]);
-    rng_publish(c, rp);
+    const Scan2 s = scan2<SM>(buf, need[0], need[1]);
+    rng_publish(rp);
     buf ^= 1;
 #pragma unroll
     for (u32 h = 0; h < 2; ++h) {
       const u32 i = base + h * T + threadIdx.x;
-      const bool rel = need[h] && ring_at(c, rp + (h ? s.off1 : s.off0)) <= thr[h];
+      const bool rel = need[h] && ring_at(c.rmask, rp + (h ? s.off1 : s.off0)) <= thr[h];
       if (rel) {
         c.rev[i] = UNBOUND;
         c.fwd[i] = UNBOUND;
         c.bep[i] = UNBOUND;
+      } else if (move && i < n && c.bep[i] != UNBOUND) {
+        c.rev[i] -= c.rm[i];
+        c.fwd[i] += c.fm[i];
       }
       const unsigned m = __ballot_sync(FULL, rel);
-      if (m && ln() == 0) atomicAdd(&c.bt->released, (u32)__popc(m));
+      if (m && ln() == 0) atomicAdd(&g_bt.released, (u32)__popc(m));
     }
     rp += s.total;
   }
-  wsync(c);
-  rng_publish(c, rp);
+  wsync(c.T);
+  rng_publish(rp);
   return rp;
 }
 
-// Sum of n non-negative doubles with the rounding of the loop s = s + t[i], by one warp.
-// While s stays inside one binade, adding t rounds to a multiple of that binade's unit in the last
-// place: s + ulp * rint(t / ulp), unless t / ulp lies exactly halfway between two integers (then the
-// parity of s decides).  So a group of terms adds as integers; terms that would carry s out of the
-// binade, and exact halves, are added one at a time in double precision.
-__device__ __noinline__ double ordered_sum(const double* t, u32 n) {
+// Sum of n non-negative doubles with the rounding of the loop s = s + t[i], by one warp, in integers.
+// While s stays inside one binade, adding t adds t rounded to a multiple of that binade's unit in the
+// last place, unless t lies exactly halfway between two multiples (then the parity of s decides).
+// So a group of terms adds as integers; a term that carries s out of the binade, or is an exact
+// half, is added in double precision, and the group goes on after it.  (A loop of double additions
+// waits about 60 cycles for each.)
+__device__ __forceinline__ u64 ulp_multiple(double t, u32 e, bool* stop) {
+  const u64 b = (u64)__double_as_longlong(t);
+  const u32 te = (u32)(b >> 52);
+  if (b == 0) return 0;
+  if (te == 0 || te > e) {  // denormal, or above s
+    *stop = true;
+    return 0;
+  }
+  const u32 sh = e - te;
+  const u64 m = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+  if (sh == 0) return m;
+  if (sh > 53) return 0;  // below half a unit
+  const u64 half = 1ull << (sh - 1), rem = m & (2 * half - 1);
+  if (rem == half) *stop = true;
+  return (m >> sh) + (rem > half ? 1 : 0);
+}
+
+template <bool SM>
+__device__ __noinline__ double ordered_sum(u32 n) {
+  const View<SM> c;
+  const auto t = c.sr;
   const u32 lane = ln();
+  const u64 MANT = 0xFFFFFFFFFFFFFull, TOP = 1ull << 53;
   double s = 0.0;
   u32 i = 0;
-  // s grows through most of its binades in the first terms
-  const u32 head = min(n, 32u);
-  {
-    const double mine = lane < head ? t[lane] : 0.0;
-    for (u32 k = 0; k < head; ++k) s = s + __shfl_sync(FULL, mine, k);
-    i = head;
-  }
+#pragma unroll 1
   while (i < n) {
-    const u64 sb = (u64)__double_as_longlong(s);
-    const u32 e = (u32)(sb >> 52) & 0x7FFu;
+    u64 sb = (u64)__double_as_longlong(s);
+    u32 e = (u32)(sb >> 52);
+    // four terms per lane while none of them needs care
     const u32 cnt = min(n - i, 128u);
-    bool done = false;
-    if (e > 60 && e < 1900) {
-      // t / ulp by an exact scaling with 2^(1075 - e)
-      const double scale = __longlong_as_double((i64)(2098 - e) << 52);
-      i64 part = 0;
-      bool stop = false;
+    {
+      bool stop = e == 0;
+      u64 part = 0;
 #pragma unroll
       for (u32 h = 0; h < 4; ++h) {
         const u32 k = 32 * h + lane;
-        const double q = k < cnt ? t[i + k] * scale : 0.0;
-        stop |= !(q < 9007199254740992.0);
-        const double r = rint(q);
-        stop |= fabs(q - r) == 0.5;
-        part += stop ? 0 : (i64)r;
+        if (k < cnt) part += ulp_multiple(__longlong_as_double((i64)t.at64(i + k)), e, &stop);
       }
       if (!__any_sync(FULL, stop)) {
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(FULL, part, d);
-        const u64 mant = (sb & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-        if (mant + (u64)part < (1ull << 53)) {
-          s = __longlong_as_double((i64)((sb & ~0xFFFFFFFFFFFFFull) | ((mant + (u64)part) & 0xFFFFFFFFFFFFFull)));
-          done = true;
+        // part < 2^55: three partial sums of at most 21 bits per lane
+        const u64 total = (u64)__reduce_add_sync(FULL, (u32)part & 0x1FFFFFu) +
+                          ((u64)__reduce_add_sync(FULL, (u32)(part >> 21) & 0x1FFFFFu) << 21) +
+                          ((u64)__reduce_add_sync(FULL, (u32)(part >> 42)) << 42);
+        const u64 mant = (sb & MANT) | (1ull << 52);
+        if (mant + total < TOP) {
+          s = __longlong_as_double((i64)((sb & ~MANT) | ((mant + total) & MANT)));
+          i += cnt;
+          continue;
         }
       }
     }
-    if (!done) {
-#pragma unroll
-      for (u32 h = 0; h < 4; ++h) {
-        const u32 k0 = 32 * h;
-        if (k0 < cnt) {
-          const double mine = k0 + lane < cnt ? t[i + k0 + lane] : 0.0;
-          const u32 m = min(32u, cnt - k0);
-          for (u32 k = 0; k < m; ++k) s = s + __shfl_sync(FULL, mine, k);
+#pragma unroll 1
+    for (u32 k0 = 0; k0 < cnt; k0 += 32) {
+      const u32 m = min(32u, cnt - k0);
+      const double mine = lane < m ? __longlong_as_double((i64)t.at64(i + k0 + lane)) : 0.0;
+      u32 from = 0;  // terms [from, m) of the 32 are still to be added
+#pragma unroll 1
+      while (from < m) {
+        sb = (u64)__double_as_longlong(s);
+        e = (u32)(sb >> 52);
+        bool stop = false;
+        u64 r = 0;
+        if (lane >= from && lane < m) {
+          r = ulp_multiple(mine, e, &stop);
+          stop |= e == 0;
         }
+        u64 x = r;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const u64 y = __shfl_up_sync(FULL, x, d);
+          if ((int)lane >= d) x += y;
+        }
+        const u64 mant = (sb & MANT) | (1ull << 52);
+        const unsigned bad = __ballot_sync(FULL, stop || (lane >= from && mant + x >= TOP));
+        const u32 f = bad ? (u32)(__ffs(bad) - 1) : 31u;
+        const u64 upto = __shfl_sync(FULL, bad ? x - r : x, f);
+        if (e != 0) s = __longlong_as_double((i64)((sb & ~MANT) | ((mant + upto) & MANT)));
+        if (!bad) break;
+        s = s + __shfl_sync(FULL, mine, f);
+        from = f + 1;
       }
     }
     i += cnt;
@@ -2667,67 +3102,71 @@ __device__ __noinline__ double ordered_sum(const double* t, u32 n) {
 // integers below 2^32, so the reference's double sum is exact and the mean is computed from an
 // integer sum; the sum of squared deviations keeps the reference's left-to-right rounding
 // (ordered_sum).
-__device__ __noinline__ bool burnin_stats(Cell& c, const KParams& P, u32 n) {
-  Scalars* sc = c.sc;
-  BlockTmp* bt = c.bt;
+template <bool SM>
+__device__ __noinline__ bool burnin_stats(u32 n) {
+  const View<SM> c;
+  const KParams& P = g_P;
   const u32 cap = P.hist_cap;
   if (n == 0) {
     if (threadIdx.x == 0) {
-      sc->hist_size = 0;
-      sc->hist_head = 0;
+      g_sc.hist_size = 0;
+      g_sc.hist_head = 0;
     }
-    wsync(c);
+    wsync(c.T);
     return false;
   }
-  if (threadIdx.x == 0) bt->sum = 0;
-  wsync(c);
+  if (threadIdx.x == 0) g_bt.sum = 0;
+  wsync(c.T);
   u64 part = 0;
-#pragma unroll 4
+#pragma unroll 1
   for (u32 i = threadIdx.x; i < n; i += c.T) part += pos64(c.fwd[i]) - pos64(c.rev[i]);
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) part += __shfl_xor_sync(FULL, part, d);
-  if (ln() == 0) atomicAdd((unsigned long long*)&bt->sum, (unsigned long long)part);
-  wsync(c);
-  const double mean = (double)bt->sum / (double)n;
-  double* terms = reinterpret_cast<double*>(c.sr);  // sr and sf are adjacent: n doubles
+  if (ln() == 0) atomicAdd((unsigned long long*)&g_bt.sum, (unsigned long long)part);
+  wsync(c.T);
+  const double mean = (double)g_bt.sum / (double)n;
+#pragma unroll 1
   for (u32 i = threadIdx.x; i < n; i += c.T) {
     const double d = (double)(pos64(c.fwd[i]) - pos64(c.rev[i])) - mean;
-    terms[i] = d * d;
+    c.sr.at64(i) = (u64)__double_as_longlong(d * d);  // sr and sf are adjacent: n doubles
   }
-  wsync(c);
+  wsync(c.T);
   if (threadIdx.x < 32) {
-    const double ssd = ordered_sum(terms, n);
+    const double ssd = ordered_sum<SM>(n);
     if (ln() == 0) {
       const double sd = sqrt(ssd / (double)n);
-      if (sc->hist_size == cap) {
-        sc->hist_head = (sc->hist_head + 1) % cap;
-        sc->hist_size--;
+      if (g_sc.hist_size == cap) {
+        g_sc.hist_head = (g_sc.hist_head + 1) % cap;
+        g_sc.hist_size--;
       }
-      const u32 slot = (sc->hist_head + sc->hist_size) % cap;
-      c.havg[slot] = mean;
-      c.hcfx[slot] = sd / mean;
-      sc->hist_size++;
+      const u32 slot = (g_sc.hist_head + g_sc.hist_size) % cap;
+      g_c.havg[slot] = mean;
+      g_c.hcfx[slot] = sd / mean;
+      g_sc.hist_size++;
     }
     __syncwarp();
     bool done = false;
-    if (sc->hist_size == cap) {
+    if (g_sc.hist_size == cap) {
       // evaluate_burnin's smoothed-dip ratio: window pairs (i1, i2) = (k + 1, k + 1 + w) for
       // k < cap - w - 1, one window per lane, each window summed in the reference's order
       const u32 w = P.smooth_w;
-      const u32 head = sc->hist_head;
+      const u32 head = g_sc.hist_head;
       auto ratio = [&](const double* d) {
         u32 nd = 0;
+#pragma unroll 1
         for (u32 i1 = 1 + ln(); i1 + w < cap; i1 += 32) {
           const u32 i2 = i1 + w;
           double a1 = 0.0, a2 = 0.0;
           u32 k = head + i1 - 1;
           if (k >= cap) k -= cap;
+#pragma unroll 1
           for (u32 t = 0; t < w; ++t) {
             a1 = a1 + d[k];
             if (++k == cap) k = 0;
           }
           k = head + i1;
           if (k >= cap) k -= cap;
+#pragma unroll 1
           for (u32 t = 0; t < w; ++t) {
             a2 = a2 + d[k];
             if (++k == cap) k = 0;
@@ -2739,49 +3178,53 @@ __device__ __noinline__ bool burnin_stats(Cell& c, const KParams& P, u32 n) {
         for (int o = 16; o > 0; o >>= 1) nd += __shfl_xor_sync(FULL, nd, o);
         return (double)nd / (double)((u64)cap - w - nd);
       };
-      const double r1 = ratio(c.hcfx);
+      const double r1 = ratio(g_c.hcfx);
       if (r1 >= 0.95 && r1 <= 1.05) {
-        const double r2 = ratio(c.havg);
+        const double r2 = ratio(g_c.havg);
         done = r2 >= 0.95 && r2 <= 1.05;
       }
     }
-    if (ln() == 0) bt->flag = done ? 1 : 0;
+    if (ln() == 0) g_bt.flag = done ? 1 : 0;
   }
-  wsync(c);
-  return bt->flag != 0;
+  wsync(c.T);
+  return g_bt.flag != 0;
 }
 
 // run_burnin (simulation.cpp:1027-1054)
-__device__ __noinline__ u64 run_burnin(Cell& c, const KParams& P, u64 rp) {
-  Scalars* sc = c.sc;
+template <bool SM>
+__device__ __noinline__ u64 run_burnin(u64 rp) {
+  const View<SM> c;
+  const KParams& P = g_P;
+#pragma unroll 1
   for (u64 it = 0; it < MGPU_ITER_LIMIT; ++it) {
-    const bool active = sc->num_active == P.nlefs;
-    wsync(c);  // thread 0 changes num_active below
+    const bool active = g_sc.num_active == P.nlefs;
+    wsync(c.T);  // thread 0 changes num_active below
     bool done = false;
-    if (active) done = burnin_stats(c, P, P.nlefs);
+    if (active) done = burnin_stats<SM>(P.nlefs);
     if (threadIdx.x == 0) {
-      ++sc->num_burnin_epochs;
+      ++g_sc.num_burnin_epochs;
       if (!active) {
-        const u64 k = s_poisson(c, P);
-        sc->num_active = min(sc->num_active + k, (u64)P.nlefs);
+        const u64 k = s_poisson(g_c, P);
+        g_sc.num_active = min(g_sc.num_active + k, (u64)P.nlefs);
       } else {
-        done = done && (sc->epoch > P.min_burnin);
-        if (!done && sc->epoch >= P.max_burnin) done = true;
-        sc->burnin_completed = done ? 1 : 0;
+        done = done && (g_sc.epoch > P.min_burnin);
+        if (!done && g_sc.epoch >= P.max_burnin) done = true;
+        g_sc.burnin_completed = done ? 1 : 0;
       }
     }
-    wsync(c);
-    rp = sc->rpos;
-    if (sc->num_active != 0) return rp;
+    wsync(c.T);
+    rp = g_sc.rpos;
+    if (g_sc.num_active != 0) return rp;
   }
-  if (threadIdx.x == 0) set_status(c, DEV_ERR_ITER_LIMIT);
-  wsync(c);
+  if (threadIdx.x == 0) set_status(g_c, DEV_ERR_ITER_LIMIT);
+  wsync(c.T);
   return rp;
 }
 
 // ContactMatrixDense::increment (contact_matrix_dense_safe_impl.hpp:52-87); returns whether
 // the contact fell outside the band (missed update).
-__device__ __forceinline__ bool band_increment(Cell& c, const KParams& P, u64 row, u64 col) {
+template <class C>
+__device__ __forceinline__ bool band_increment(const C& c, const KParams& P, u64 row, u64 col) {
   u64 i, j;
   if (row > col) {
     i = row - col;
@@ -2798,14 +3241,17 @@ __device__ __forceinline__ bool band_increment(Cell& c, const KParams& P, u64 ro
 // One contact attempt read from draws at `at` (register_contacts.cpp:129-198).  Returns the
 // draws it takes; *ok tells whether it registers a contact; *regular is false when the attempt
 // hit a bucket rejection (exact handling needs the serial path).
-__device__ __forceinline__ u32 contact_attempt(const Cell& c, const KParams& P, u64 at, bool tad,
+template <bool SM>
+__device__ __forceinline__ u32 contact_attempt(u64 at, bool tad,
                                                u64 na, u64 lbucket, bool* ok, bool* regular,
                                                u64* row, u64* col) {
+  const View<SM> c;
+  const KParams& P = g_P;
   *ok = false;
   *regular = true;
   const u64 start = (u64)P.wstart + 1, end = (u64)P.wend - 1;
   u32 used = 0;
-  const u64 li = ring_at(c, at + used++) / lbucket;
+  const u64 li = ring_at(c.rmask, at + used++) / lbucket;
   if (li > na - 1) {
     *regular = false;
     return used;
@@ -2815,13 +3261,13 @@ __device__ __forceinline__ u32 contact_attempt(const Cell& c, const KParams& P, 
   if (!(rp > start && rp < end && fp > start && fp < end)) return used;
   double n1 = 0.0, n2 = 0.0;
   if (P.noisify) {
-    const double u1 = canonical_of(ring_at(c, at + used++));
+    const double u1 = canonical_of(ring_at(c.rmask, at + used++));
     n1 = (P.gev_xi == 0.0) ? (P.gev_mu - P.gev_sigma) * log(-log(u1))
                            : P.gev_mu + (P.gev_sigma * (1.0 - pow(-log(u1), P.gev_xi))) / P.gev_xi;
   }
   const double a = (double)rp - n1;
   if (P.noisify) {
-    const double u2 = canonical_of(ring_at(c, at + used++));
+    const double u2 = canonical_of(ring_at(c.rmask, at + used++));
     n2 = (P.gev_xi == 0.0) ? (P.gev_mu - P.gev_sigma) * log(-log(u2))
                            : P.gev_mu + (P.gev_sigma * (1.0 - pow(-log(u2), P.gev_xi))) / P.gev_xi;
   }
@@ -2841,12 +3287,12 @@ __device__ __forceinline__ u32 contact_attempt(const Cell& c, const KParams& P, 
   if (range != 0) {
     u64 bucket = ~0ull / (range + 1);
     if (~0ull % (range + 1) == range) ++bucket;
-    const u64 r1 = ring_at(c, at + used++) / bucket;
+    const u64 r1 = ring_at(c.rmask, at + used++) / bucket;
     if (r1 > range) {
       *regular = false;
       return used;
     }
-    const u64 r2 = ring_at(c, at + used++) / bucket;
+    const u64 r2 = ring_at(c.rmask, at + used++) / bucket;
     if (r2 > range) {
       *regular = false;
       return used;
@@ -2902,12 +3348,13 @@ __device__ __noinline__ void contact_attempt_serial(Cell& c, const KParams& P, b
 // 2 for the noise, 2 more for a TAD contact).  The workers commit up to the first attempt that
 // took a different number (a LEF or position outside the bounds, a zero-width TAD range) and
 // resume after it; an attempt that hit a uniform_int bucket rejection is redone serially.
-__device__ __noinline__ u64 sample_contacts(Cell& c, const KParams& P, u64 rp, u64 target) {
-  Scalars* sc = c.sc;
-  BlockTmp* bt = c.bt;
+template <bool SM>
+__device__ __noinline__ u64 sample_contacts(u64 rp, u64 target) {
+  const View<SM> c;
+  const KParams& P = g_P;
   const u32 T = c.T, W = T >> 5, w = threadIdx.x >> 5, lane = ln();
   u64 num = P.spe;
-  if (P.density_positive) num = min(num, target - sc->num_contacts);
+  if (P.density_positive) num = min(num, target - g_sc.num_contacts);
   if (num == 0) return rp;
   if (threadIdx.x == 0) {
     u64 n_loop;
@@ -2916,15 +3363,15 @@ __device__ __noinline__ u64 sample_contacts(Cell& c, const KParams& P, u64 rp, u
     } else if (P.ratio_mode == 1) {
       n_loop = 0;
     } else {
-      n_loop = (u64)s_binomial(c, P, (i64)num, P.p_loop);
+      n_loop = (u64)s_binomial(g_c, P, (i64)num, P.p_loop);
     }
-    sc->bc0 = n_loop;
-    bt->missed = 0;
+    g_sc.bc0 = n_loop;
+    g_bt.missed = 0;
   }
-  wsync(c);
-  rp = sc->rpos;
-  const u64 n_loop = sc->bc0;
-  const u64 na = sc->num_active;
+  wsync(c.T);
+  rp = g_sc.rpos;
+  const u64 n_loop = g_sc.bc0;
+  const u64 na = g_sc.num_active;
   u64 lbucket;
   {
     const u64 range = na - 1;
@@ -2934,54 +3381,56 @@ __device__ __noinline__ u64 sample_contacts(Cell& c, const KParams& P, u64 rp, u
   u64 budget = 1000 * num + 1000000;  // attempts before giving up (see DEV_ERR_NO_BOUND_LEF)
   u32 missed = 0;
   const int passes = P.track_occ ? 3 : 2;  // loop, TAD, then the 1D occupancy
+#pragma unroll 1
   for (int pass = 0; pass < passes; ++pass) {
     const bool tad = pass == 1, occ = pass == 2;
     u64 todo = occ ? num : (tad ? num - n_loop : n_loop);
     const u32 nominal = 1 + (P.noisify ? 2 : 0) + (tad ? 2 : 0);
     const u32 most = min(T, c.lim / nominal);
+#pragma unroll 1
     while (todo != 0) {
       if (budget < T) {
         if (threadIdx.x == 0) {
-          rng_publish(c, rp);
-          set_status(c, DEV_ERR_NO_BOUND_LEF);
+          rng_publish(rp);
+          set_status(g_c, DEV_ERR_NO_BOUND_LEF);
         }
-        wsync(c);
+        wsync(c.T);
         return rp;
       }
       // a few attempts more than contacts are wanted, in whole warps
       const u32 active = (u32)min((u64)most, (u64)((todo + todo / 16 + 32) & ~31ull));
       budget -= active;
-      rng_ensure(c, rp, active * nominal);
+      rng_ensure(rp, active * nominal);
       bool ok = false, regular = true;
       u64 row = 0, col = 0;
       u32 used = nominal;
       if (threadIdx.x < active)
-        used = contact_attempt(c, P, rp + (u64)threadIdx.x * nominal, tad, na, lbucket, &ok, &regular, &row, &col);
+        used = contact_attempt<SM>(rp + (u64)threadIdx.x * nominal, tad, na, lbucket, &ok, &regular, &row, &col);
       const bool deviates = !regular || used != nominal;
       const unsigned dm = __ballot_sync(FULL, deviates), om = __ballot_sync(FULL, ok);
       const u32 fl = dm ? (u32)(__ffs(dm) - 1) : 0u;
       const u32 fu = __shfl_sync(FULL, used | (regular ? 0x80000000u : 0u), fl);
       if (lane == 0) {
-        bt->dev[w] = dm;
-        bt->okm[w] = om;
-        bt->dus[w] = fu;
+        g_bt.dev[w] = dm;
+        g_bt.okm[w] = om;
+        g_bt.dus[w] = fu;
       }
-      wsync(c);
+      wsync(c.T);
       // first deviating attempt f, its draws, and the commit limit: attempts [0, lim) are exact
-      const u32 myd = lane < W ? bt->dev[lane] : 0u;
+      const u32 myd = lane < W ? g_bt.dev[lane] : 0u;
       const unsigned dw = __ballot_sync(FULL, myd != 0);
       u32 f = active, f_used = nominal;
       bool f_regular = false;
       if (dw) {
         const u32 fw = (u32)(__ffs(dw) - 1);
         f = fw * 32 + (u32)(__ffs(__shfl_sync(FULL, myd, fw)) - 1);
-        const u32 v = bt->dus[fw];
+        const u32 v = g_bt.dus[fw];
         f_used = v & 0x7FFFFFFFu;
         f_regular = (v & 0x80000000u) != 0;
       }
       u32 lim = f_regular ? f + 1 : f;
       // contacts among them; the todo-th success ends the pass
-      u32 okw = lane < W ? bt->okm[lane] : 0u;
+      u32 okw = lane < W ? g_bt.okm[lane] : 0u;
       if (lim <= lane * 32) okw = 0;
       else if (lim < lane * 32 + 32) okw &= (1u << (lim - lane * 32)) - 1u;
       u32 total;
@@ -2992,6 +3441,7 @@ __device__ __noinline__ u64 sample_contacts(Cell& c, const KParams& P, u64 rp, u
         const u32 hw = (u32)(__ffs(hit) - 1);
         unsigned mm = __shfl_sync(FULL, okw, hw);
         const u32 skip = want - 1 - __shfl_sync(FULL, ex, hw);
+#pragma unroll 1
         for (u32 t = 0; t < skip; ++t) mm &= mm - 1;
         lim = hw * 32 + (u32)__ffs(mm);
         total = want;
@@ -3005,33 +3455,33 @@ __device__ __noinline__ u64 sample_contacts(Cell& c, const KParams& P, u64 rp, u
       }
       if (lim) rp += (u64)(lim - 1) * nominal + (lim - 1 == f ? f_used : nominal);
       todo -= total;
-      wsync(c);  // the draws are read and bt may be written again
-      rng_publish(c, rp);
+      wsync(c.T);  // the draws are read and bt may be written again
+      rng_publish(rp);
       if (todo != 0 && lim == f && f < active) {
         // attempt f could not be evaluated from the ring: run it serially
-        prof_add(c, PF_CONTACT_SERIAL, 1);
+        prof_add(PF_CONTACT_SERIAL, 1);
         if (threadIdx.x == 0) {
           bool sok, smiss;
-          contact_attempt_serial(c, P, tad, na, &sok, &smiss, occ);
-          sc->bc1 = sok ? 1 : 0;
-          if (smiss) sc->missed++;
+          contact_attempt_serial(g_c, P, tad, na, &sok, &smiss, occ);
+          g_sc.bc1 = sok ? 1 : 0;
+          if (smiss) g_sc.missed++;
         }
-        wsync(c);
-        rp = sc->rpos;
-        if (sc->bc1) todo -= 1;
-        wsync(c);
+        wsync(c.T);
+        rp = g_sc.rpos;
+        if (g_sc.bc1) todo -= 1;
+        wsync(c.T);
       }
     }
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) missed += __shfl_xor_sync(FULL, missed, d);
-  if (lane == 0 && missed) atomicAdd(&bt->missed, missed);
-  wsync(c);
+  if (lane == 0 && missed) atomicAdd(&g_bt.missed, missed);
+  wsync(c.T);
   if (threadIdx.x == 0) {
-    sc->missed += bt->missed;
-    sc->num_contacts += num;
+    g_sc.missed += g_bt.missed;
+    g_sc.num_contacts += num;
   }
-  wsync(c);
+  wsync(c.T);
   return rp;
 }
 
@@ -3052,8 +3502,10 @@ __device__ __noinline__ void sample_contacts_serial(Cell& c, const KParams& P, u
   }
   u64 budget = 1000 * num + 1000000;
   const int passes = P.track_occ ? 3 : 2;  // loop, TAD, then the 1D occupancy
+#pragma unroll 1
   for (int pass = 0; pass < passes; ++pass) {
     u64 todo = pass == 0 ? n_loop : (pass == 1 ? num - n_loop : num);
+#pragma unroll 1
     while (todo != 0) {
       if (--budget == 0 || sc->status != DEV_OK) {
         set_status(c, DEV_ERR_NO_BOUND_LEF);
@@ -3081,16 +3533,21 @@ __device__ __forceinline__ u64 mix64(u64 z) {
 }
 
 // mgpu_state_digest of the cell's state, and the full arrays when requested.
-__device__ __noinline__ void trace_record(Cell& c, const KParams& P, const DevTrace& T, u64 rec) {
+template <bool SM>
+__device__ __noinline__ void trace_record(const DevTrace& T, u64 rec) {
+  const View<SM> c;
+  const KParams& P = g_P;
   const u32 nl = P.nlefs;
   const bool full = rec < T.max_records;
   u64 part = 0;
-  if (threadIdx.x == 0) c.bt->sum = 0;
-  wsync(c);
+  if (threadIdx.x == 0) g_bt.sum = 0;
+  wsync(c.T);
+#pragma unroll 1
   for (u32 i = threadIdx.x; i < nl; i += c.T) {
     const u64 v[9] = {pos64(c.rev[i]), pos64(c.fwd[i]), pos64(c.bep[i]), c.rr[i], c.fr[i],
                       c.rm[i], c.fm[i], cw_to_ref(c.rc[i]), cw_to_ref(c.fc[i])};
     u64 h = mix64((u64)i * 0x9E3779B97F4A7C15ull + 0x632BE59BD9B4E019ull);
+#pragma unroll 1
     for (int k = 0; k < 9; ++k) h = mix64(h ^ v[k]);
     part += h;
     if (full) {
@@ -3108,61 +3565,77 @@ __device__ __noinline__ void trace_record(Cell& c, const KParams& P, const DevTr
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(FULL, part, off);
-  if (ln() == 0) atomicAdd((unsigned long long*)&c.bt->sum, (unsigned long long)part);
-  wsync(c);
+  if (ln() == 0) atomicAdd((unsigned long long*)&g_bt.sum, (unsigned long long)part);
+  wsync(c.T);
   if (threadIdx.x == 0) {
-    const Scalars* sc = c.sc;
-    mgpu_trace_header h;
-    h.epoch = sc->epoch;
-    h.num_active_lefs = sc->num_active;
-    h.burnin_completed = sc->burnin_completed;
-    h.num_burnin_epochs = sc->num_burnin_epochs;
-    h.num_contacts = sc->num_contacts;
-    h.rng_draws = sc->rpos;
-    h.n5prime = sc->n5;
-    h.n3prime = sc->n3;
-    h.digest = c.bt->sum;
+      mgpu_trace_header h;
+    h.epoch = g_sc.epoch;
+    h.num_active_lefs = g_sc.num_active;
+    h.burnin_completed = g_sc.burnin_completed;
+    h.num_burnin_epochs = g_sc.num_burnin_epochs;
+    h.num_contacts = g_sc.num_contacts;
+    h.rng_draws = g_sc.rpos;
+    h.n5prime = g_sc.n5;
+    h.n3prime = g_sc.n3;
+    h.digest = g_bt.sum;
     if (T.all_headers && rec < T.max_epochs) T.all_headers[rec] = h;
     if (full && T.headers) T.headers[rec] = h;
   }
-  wsync(c);
+  wsync(c.T);
 }
 
-// Lay out one cell: the header in shared memory, then each per-LEF array either in shared
-// memory or in the block's global scratch slot, as planned by the host.  Thread 0; the caller's
-// barrier follows.
-__device__ void carve(Cell& c, BlockTmp* bt, char* smem, char* gslot, const KParams& P, u32 nl, const DevChrom& ch,
-                      const ulonglong2* jt, u32* band) {
+// Lay out one cell: each per-LEF array, the barrier bits and the burn-in history either in dynamic
+// shared memory behind the ring or in the block's global scratch slot, as the plan in g_P places them.
+// Thread 0; the caller's barrier follows.
+__device__ void carve(char* gslot, const DevChrom& ch, const ulonglong2* jt, u32* band) {
   if (threadIdx.x != 0) return;
+  Cell& c = g_c;
+  const KParams& P = g_P;
   const u32 workers = P.workers, pw = producer_warps(workers);
-  c.sc = reinterpret_cast<Scalars*>(smem);
-  c.bt = bt;
+  c.sc = &g_sc;
   c.T = workers * 32;
   c.lim = pw * 32 * RNG_S;
   c.rmask = 2 * c.lim - 1;
-  c.ring = reinterpret_cast<u64*>(smem + CELL_HEADER_BYTES);
-  c.hcfx = reinterpret_cast<double*>((P.hist_smem ? smem : gslot) + P.hist_off);
+  c.ring = reinterpret_cast<u64*>(dyn_smem);
+  c.hcfx = reinterpret_cast<double*>((P.hist_smem ? dyn_smem : gslot) + P.hist_off);
   c.havg = c.hcfx + P.hist_cap;
-  c.bst = reinterpret_cast<u32*>((P.bst_smem ? smem : gslot) + P.bst_off);
+  c.bst = reinterpret_cast<u32*>((P.bst_smem ? dyn_smem : gslot) + P.bst_off);
+  c.bst_off = P.bst_off;
   u32** arr[NARR] = {&c.rev, &c.fwd, &c.rr, &c.fr, &c.rm, &c.fm, &c.rc, &c.fc, &c.sr, &c.sf, &c.tmp, &c.bep};
   for (u32 k = 0; k < NARR; ++k) {
-    char* base = ((P.arr_smem >> k) & 1u) ? smem : gslot;
+    char* base = ((P.arr_smem >> k) & 1u) ? dyn_smem : gslot;
     *arr[k] = reinterpret_cast<u32*>(base + P.arr_off[k]);
+    c.off[k] = P.arr_off[k];
   }
+  c.all_smem = P.arr_smem == (1u << NARR) - 1 && P.bst_smem;
   c.bar = ch.barriers;
   c.bpf = ch.pos_flags;
   c.nb = ch.nbarriers;
-  c.nl = nl;
   c.jt = jt + (u64)(pw - 1) * 2 * JUMP_TABLE_ENTRIES;
   c.band = band;
 }
 
-// The normal ziggurat's fixed-point layers (after the two jump tables) into the block's scratch.
-__device__ __forceinline__ void load_layers(BlockTmp* bt, const ulonglong2* jt) {
-  for (u32 i = threadIdx.x; i < 128; i += blockDim.x) bt->zt[i] = jt[4 * JUMP_TABLE_ENTRIES + i];
+// Launch parameters into shared memory (the caller's barrier follows).
+__device__ __forceinline__ void load_plan(const KParams& P) {
+  const u32* src = reinterpret_cast<const u32*>(&P);
+  u32* dst = reinterpret_cast<u32*>(&g_P);
+  for (u32 w = threadIdx.x; w < sizeof(KParams) / 4; w += blockDim.x) dst[w] = src[w];
 }
 
-__device__ __noinline__ void cell_reset(Cell& c, u32 nl, u64 seed, u64* prof) {
+// The normal ziggurat's fixed-point layers (after the two jump tables) into the block's scratch.
+__device__ __forceinline__ void load_layers(const ulonglong2* jt) {
+#pragma unroll 1
+  for (u32 i = threadIdx.x; i < 128; i += blockDim.x) {
+    g_bt.zt[i] = jt[4 * JUMP_TABLE_ENTRIES + i];
+    const double y0 = mgpu_zig_normal_y[i], y1 = mgpu_zig_normal_y[i + 1];
+    g_bt.zy[i] = make_float2((float)y0, (float)(y1 - y0));
+  }
+}
+
+__device__ __noinline__ void cell_reset(u64 seed) {
+  Cell& c = g_c;
+  const u32 nl = g_P.nlefs;
+#pragma unroll 1
   for (u32 i = threadIdx.x; i < nl; i += blockDim.x) {
     c.rev[i] = UNBOUND;
     c.fwd[i] = UNBOUND;
@@ -3174,10 +3647,12 @@ __device__ __noinline__ void cell_reset(Cell& c, u32 nl, u64 seed, u64* prof) {
     c.rc[i] = 0;
     c.fc[i] = 0;
   }
+#pragma unroll 1
   for (u32 w = threadIdx.x; w < (c.nb + 31) / 32; w += blockDim.x) c.bst[w] = 0;
   if (threadIdx.x == 0) {
-    Scalars* sc = c.sc;
+    Scalars* sc = &g_sc;
     u64 st = seed;  // SplitMix64 seeding (random.hpp:26-30)
+#pragma unroll 1
     for (int k = 0; k < 4; ++k) {
       u64 z = (st += 0x9e3779b97f4a7c15ull);
       z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
@@ -3201,18 +3676,21 @@ __device__ __noinline__ void cell_reset(Cell& c, u32 nl, u64 seed, u64* prof) {
     sc->hist_size = 0;
     sc->hist_head = 0;
     sc->bc0 = sc->bc1 = sc->bc2 = 0;
-    sc->prof = prof;
+    sc->prof = g_P.prof;
   }
 }
 
 // Simulation::dump_stats (simulation.cpp:1166-1224): the epoch's model-state record, taken after
 // extrude and before release_lefs; the loop-size mean is exact (an integer sum below 2^53).
 // Warp 0; the caller's barrier follows.
-__device__ __noinline__ void log_model_state(Cell& c, const KParams& P, u32 n, u64 cell) {
-  Scalars* sc = c.sc;
-  if (!P.records || sc->nrec >= P.rec_max || threadIdx.x >= 32) return;
+template <bool SM>
+__device__ __noinline__ void log_model_state(u32 n, u64 cell) {
+  const View<SM> c;
+  const KParams& P = g_P;
+  if (!P.records || g_sc.nrec >= P.rec_max || threadIdx.x >= 32) return;
   u32 st_rev = 0, st_fwd = 0, st_both = 0, lb = 0, pri = 0, sec = 0;
   u64 loop = 0;
+#pragma unroll 1
   for (u32 i = threadIdx.x; i < n; i += 32) {
     const u32 r = c.rc[i], f = c.fc[i];
     const bool sr = cw_occurred(r), sf = cw_occurred(f);
@@ -3225,6 +3703,7 @@ __device__ __noinline__ void log_model_state(Cell& c, const KParams& P, u32 n, u
     loop += pos64(c.fwd[i]) - pos64(c.rev[i]);
   }
   u32 occ = 0;
+#pragma unroll 1
   for (u32 w = threadIdx.x; w < (c.nb + 31) / 32; w += 32) occ += __popc(c.bst[w]);
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {
@@ -3238,10 +3717,10 @@ __device__ __noinline__ void log_model_state(Cell& c, const KParams& P, u32 n, u
     occ += __shfl_xor_sync(FULL, occ, d);
   }
   if (ln() == 0) {
-    mgpu_epoch_record* r = P.records + cell * P.rec_max + sc->nrec;
-    r->epoch = sc->epoch;
+    mgpu_epoch_record* r = P.records + cell * P.rec_max + g_sc.nrec;
+    r->epoch = g_sc.epoch;
     r->cell = cell;
-    r->burnin = sc->burnin_completed ? 0 : 1;
+    r->burnin = g_sc.burnin_completed ? 0 : 1;
     r->barriers_occupied = occ;
     r->nbarriers = c.nb;
     r->num_lefs = n;
@@ -3252,123 +3731,123 @@ __device__ __noinline__ void log_model_state(Cell& c, const KParams& P, u32 n, u
     r->lef_lef_primary = pri;
     r->lef_lef_secondary = sec;
     r->avg_loop_size = n ? (double)loop / (double)n : 0.0;
-    sc->nrec++;
+    g_sc.nrec++;
   }
   __syncwarp();
 }
 
 // The epoch loop of one cell (simulation.cpp:1056-1152), run by the worker threads.
-__device__ __noinline__ void run_cell(Cell& c, const KParams& P, u64 target, u64 target_epochs, const DevTrace* trace,
+template <bool SM>
+__device__ __noinline__ void run_cell(u64 target, u64 target_epochs, const DevTrace* trace,
                                       mgpu_cell_stats* stats, u64 cell) {
-  Scalars* sc = c.sc;
+  const View<SM> c;
+  const KParams& P = g_P;
   const u32 nl = P.nlefs;
-  u64 rp = barriers_init(c, 0);
+  u64 rp = barriers_init<SM>(0);
   if (P.skip_burnin && threadIdx.x == 0) {
-    sc->num_active = nl;
-    sc->burnin_completed = 1;
+    g_sc.num_active = nl;
+    g_sc.burnin_completed = 1;
   }
-  wsync(c);
+  wsync(c.T);
+#pragma unroll 1
   for (u64 guard = 0; guard < MGPU_ITER_LIMIT; ++guard) {
-    const bool go = P.contact_mode ? (sc->num_contacts < target)
-                                   : (sc->epoch - sc->num_burnin_epochs < target_epochs);
+    const bool go = P.contact_mode ? (g_sc.num_contacts < target)
+                                   : (g_sc.epoch - g_sc.num_burnin_epochs < target_epochs);
     if (!go) break;
     const u64 te0 = clock64();
-    if (!sc->burnin_completed) rp = run_burnin(c, P, rp);
+    if (!g_sc.burnin_completed) rp = run_burnin<SM>(rp);
     u64 ta = clock64();
-    prof_add(c, PF_BURNIN, ta - te0);
-    const u32 n = (u32)sc->num_active;
-    const u32 epoch = (u32)sc->epoch;
-    const bool completed = sc->burnin_completed != 0;
-    if (threadIdx.x == 0) sc->lef_epochs += n;
-    rp = bind_lefs(c, P, rp, n, epoch, 0, nullptr);
+    prof_add(PF_BURNIN, ta - te0);
+    const u32 n = (u32)g_sc.num_active;
+    const u32 epoch = (u32)g_sc.epoch;
+    const bool completed = g_sc.burnin_completed != 0;
+    if (threadIdx.x == 0) g_sc.lef_epochs += n;
+    rp = bind_lefs<SM>(rp, n, epoch, 0, nullptr);
     u64 tb = clock64();
-    prof_add(c, PF_BIND, tb - ta);
-    rank_lefs(c, P, n, epoch, epoch != 0);
+    prof_add(PF_BIND, tb - ta);
+    rank_lefs<SM>(n, epoch, epoch != 0);
     ta = clock64();
-    prof_add(c, PF_RANK, ta - tb);
+    prof_add(PF_RANK, ta - tb);
     if (completed) {
       if (P.debug_flags & DBG_SERIAL_CONTACTS) {
-        if (threadIdx.x == 0) sample_contacts_serial(c, P, target);
-        wsync(c);
-        rp = sc->rpos;
+        if (threadIdx.x == 0) sample_contacts_serial(g_c, P, target);
+        wsync(c.T);
+        rp = g_sc.rpos;
       } else {
-        rp = sample_contacts(c, P, rp, target);
+        rp = sample_contacts<SM>(rp, target);
       }
       tb = clock64();
-      prof_add(c, PF_CONTACTS, tb - ta);
+      prof_add(PF_CONTACTS, tb - ta);
       ta = tb;
-      if (target != 0 && sc->num_contacts >= target) {
-        prof_add(c, PF_TOTAL, clock64() - te0);
+      if (target != 0 && g_sc.num_contacts >= target) {
+        prof_add(PF_TOTAL, clock64() - te0);
         break;
       }
-      if (sc->status != DEV_OK) break;
-      wsync(c);  // no worker writes a status before all have read it
+      if (g_sc.status != DEV_OK) break;
+      wsync(c.T);  // no worker writes a status before all have read it
     }
-    rp = gen_moves_dir(c, rp, c.rm, n, P.rev_speed[completed], P.rev_std, P.rev_move_int[completed]);
-    rp = gen_moves_dir(c, rp, c.fm, n, P.fwd_speed[completed], P.fwd_std, P.fwd_move_int[completed]);
+    rp = gen_moves_dir<SM>(rp, c.rm, n, P.rev_move[completed]);
+    rp = gen_moves_dir<SM>(rp, c.fm, n, P.fwd_move[completed]);
     tb = clock64();
-    prof_add(c, PF_MOVES, tb - ta);
-    gather_ranked(c, n);
-    adjust_moves(c, P, n);
-    clamp_moves(c, P, n);
+    prof_add(PF_MOVES, tb - ta);
+    place_moves<SM>(n, true);
     ta = clock64();
-    prof_add(c, PF_ADJUST, ta - tb);
-    for (u32 i = threadIdx.x; i < n; i += c.T) {
-      c.rc[i] = 0;
-      c.fc[i] = 0;
-    }
-    rp = barriers_next(c, rp);
-    wsync(c);
+    prof_add(PF_ADJUST, ta - tb);
+    rp = barriers_next<SM>(rp);
     tb = clock64();
-    prof_add(c, PF_BARRIERS, tb - ta);
-    rp = process_collisions(c, P, rp, n, true, true);
+    prof_add(PF_BARRIERS, tb - ta);
+    rp = process_collisions<SM>(rp, n, true, true);
     ta = clock64();
-    extrude(c, n);
-    if (P.log_state) {
-      log_model_state(c, P, n, cell);
-      wsync(c);
+    if (P.log_state) {  // the record is taken between the two
+      extrude<SM>(n);
+      log_model_state<SM>(n, cell);
+      wsync(c.T);
     }
-    rp = release_lefs(c, P, rp, n, completed);
+    rp = release_lefs<SM>(rp, n, completed, !P.log_state);
     tb = clock64();
-    prof_add(c, PF_EXTRUDE_RELEASE, tb - ta);
-    if (trace) trace_record(c, P, *trace, sc->epoch);
-    const bool failed = sc->status != DEV_OK;
-    wsync(c);
-    if (threadIdx.x == 0) sc->epoch++;
-    wsync(c);
-    prof_add(c, PF_TRACE, clock64() - tb);
-    prof_add(c, PF_TOTAL, clock64() - te0);
-    prof_add(c, PF_EPOCHS, 1);
+    prof_add(PF_EXTRUDE_RELEASE, tb - ta);
+    if (trace) trace_record<SM>(*trace, g_sc.epoch);
+    const bool failed = g_sc.status != DEV_OK;
+    wsync(c.T);
+    if (threadIdx.x == 0) g_sc.epoch++;
+    wsync(c.T);
+    prof_add(PF_TRACE, clock64() - tb);
+    prof_add(PF_TOTAL, clock64() - te0);
+    prof_add(PF_EPOCHS, 1);
     if (failed) break;
   }
   if (threadIdx.x == 0) {
-    if (P.rec_count) P.rec_count[cell] = sc->nrec;
-    if (trace && trace->num_recorded) *trace->num_recorded = sc->epoch;
+    if (P.rec_count) P.rec_count[cell] = g_sc.nrec;
+    if (trace && trace->num_recorded) *trace->num_recorded = g_sc.epoch;
     if (stats) {
-      stats->epochs = sc->epoch;
-      stats->burnin_epochs = sc->num_burnin_epochs;
-      stats->contacts = sc->num_contacts;
-      stats->missed_updates = sc->missed;
-      stats->lef_epochs = sc->lef_epochs;
+      stats->epochs = g_sc.epoch;
+      stats->burnin_epochs = g_sc.num_burnin_epochs;
+      stats->contacts = g_sc.num_contacts;
+      stats->missed_updates = g_sc.missed;
+      stats->lef_epochs = g_sc.lef_epochs;
       stats->rng_draws = rp;
-      stats->sort_fallbacks = sc->sort_fallbacks;
-      stats->status = sc->status;
+      stats->sort_fallbacks = g_sc.sort_fallbacks;
+      stats->status = g_sc.status;
     }
   }
 }
 
 // One cell on the whole block: reset, then the workers run the epoch loop while the producers
 // generate its draws.
-__device__ __forceinline__ void block_cell(Cell& c, const KParams& P, const CellTask& task, u64 target_epochs,
-                                           const DevTrace* trace, mgpu_cell_stats* stats, u64 cell) {
-  cell_reset(c, P.nlefs, task.seed, P.prof);
+__device__ __forceinline__ void block_cell(const CellTask& task, u64 target_epochs, const DevTrace* trace,
+                                           mgpu_cell_stats* stats, u64 cell) {
+  cell_reset(task.seed);
   __syncthreads();
-  if (threadIdx.x < c.T) {
-    run_cell(c, P, task.target_contacts, target_epochs, trace, stats, cell);
-    wsync(c);
-    if (threadIdx.x == 0) st_release(&c.sc->stop, 1);
+  if (threadIdx.x < g_c.T) {
+    if (g_c.all_smem) {
+      run_cell<true>(task.target_contacts, target_epochs, trace, stats, cell);
+    } else {
+      run_cell<false>(task.target_contacts, target_epochs, trace, stats, cell);
+    }
+    wsync(g_c.T);
+    if (threadIdx.x == 0) st_release(&g_sc.stop, 1);
   } else {
-    rng_produce(c);
+    rng_produce(g_c);
   }
   __syncthreads();
 }
@@ -3389,17 +3868,16 @@ __global__ void __launch_bounds__(MAX_BLOCK_THREADS) simulate_kernel(const __gri
                                                                      const __grid_constant__ DevTrace trace,
                                                                      u32 tracing, const ulonglong2* jt, u32* work,
                                                                      char* gscratch) {
-  extern __shared__ __align__(16) char smem[];
-  __shared__ Cell c;
-  __shared__ BlockTmp bt;
   __shared__ u32 slot;
-  load_layers(&bt, jt);
-  carve(c, &bt, smem, gscratch + (u64)blockIdx.x * P.slot_bytes, P, P.nlefs, ch, jt, band);
+  load_layers(jt);
+  load_plan(P);
+  __syncthreads();
+  carve(gscratch + (u64)blockIdx.x * P.slot_bytes, ch, jt, band);
   for (;;) {
     const u32 cell = next_cell(work, &slot);
     if (cell >= ncells) break;
-    block_cell(c, P, tasks[cell], target_epochs, tracing ? &trace : nullptr, stats ? stats + cell : nullptr, cell);
-    if (threadIdx.x == 0 && missed) atomicAdd((unsigned long long*)missed, (unsigned long long)c.sc->missed);
+    block_cell(tasks[cell], target_epochs, tracing ? &trace : nullptr, stats ? stats + cell : nullptr, cell);
+    if (threadIdx.x == 0 && missed) atomicAdd((unsigned long long*)missed, (unsigned long long)g_sc.missed);
   }
 }
 
@@ -3411,13 +3889,8 @@ __global__ void __launch_bounds__(MAX_BLOCK_THREADS) simulate_batch_kernel(const
                                                                            u64 slot_bytes, mgpu_cell_stats* stats,
                                                                            const ulonglong2* jt, u32* work,
                                                                            char* gscratch) {
-  extern __shared__ __align__(16) char smem[];
-  __shared__ Cell c;
-  __shared__ BlockTmp bt;
-  __shared__ __align__(16) KParams Psh;
   __shared__ u32 slot;
-  char* gslot = gscratch + (u64)blockIdx.x * slot_bytes;
-  load_layers(&bt, jt);
+  load_layers(jt);
   u32 cur = 0xFFFFFFFFu;
   for (;;) {
     const u32 cell = next_cell(work, &slot);
@@ -3425,18 +3898,118 @@ __global__ void __launch_bounds__(MAX_BLOCK_THREADS) simulate_batch_kernel(const
     const BatchTask t = tasks[cell];
     const BatchPlan& pl = plans[t.plan];
     if (t.plan != cur) {
-      const u32* src = reinterpret_cast<const u32*>(&pl.P);
-      u32* dst = reinterpret_cast<u32*>(&Psh);
-      for (u32 w = threadIdx.x; w < sizeof(KParams) / 4; w += blockDim.x) dst[w] = src[w];
+      load_plan(pl.P);
       __syncthreads();
-      carve(c, &bt, smem, gslot, Psh, Psh.nlefs, pl.ch, jt, pl.band);
+      carve(gscratch + (u64)blockIdx.x * slot_bytes, pl.ch, jt, pl.band);
       __syncthreads();
       cur = t.plan;
     }
     const CellTask ct{t.seed, t.target_contacts};
-    block_cell(c, Psh, ct, pl.target_epochs, nullptr, stats ? stats + cell : nullptr, cell);
-    if (threadIdx.x == 0 && pl.missed) atomicAdd(pl.missed, (unsigned long long)c.sc->missed);
+    block_cell(ct, pl.target_epochs, nullptr, stats ? stats + cell : nullptr, cell);
+    if (threadIdx.x == 0 && pl.missed) atomicAdd(pl.missed, (unsigned long long)g_sc.missed);
   }
+}
+
+// One step of the epoch loop on the state in g_c (mgpu_run_phase).
+template <bool SM>
+__device__ __noinline__ void run_phase(int phase, u32 n, const u64* bind_mask, u64 epoch, bool completed,
+                                       u32 partially_sorted, u32 init_ranks, u32 adjust) {
+  const View<SM> c;
+  const KParams& P = g_P;
+  const bool fast = !(P.debug_flags & DBG_SERIAL_COLLISIONS);
+  u64 rp = 0;
+  switch (phase) {
+    case MGPU_PHASE_BIND:
+      rp = bind_lefs<SM>(rp, n, (u32)epoch, bind_mask ? 1 : 2, bind_mask);
+      rank_lefs<SM>(n, (u32)epoch, epoch != 0);
+      break;
+    case MGPU_PHASE_RANK:
+      if (init_ranks) {
+#pragma unroll 1
+        for (u32 i = threadIdx.x; i < n; i += c.T) {
+          c.rr[i] = i;
+          c.fr[i] = i;
+        }
+        wsync(c.T);
+      }
+      rank_lefs<SM>(n, (u32)epoch, partially_sorted != 0);
+      break;
+    case MGPU_PHASE_ADJUST_AND_CLAMP:
+      place_moves<SM>(n, true);
+      break;
+    case MGPU_PHASE_GENERATE_MOVES:
+      rp = gen_moves_dir<SM>(rp, c.rm, n, P.rev_move[completed]);
+      rp = gen_moves_dir<SM>(rp, c.fm, n, P.fwd_move[completed]);
+      if (adjust) place_moves<SM>(n, true);
+      else clamp_moves<SM>(n);
+      break;
+    case MGPU_PHASE_PROCESS_COLLISIONS:
+      gather_ranked<SM>(n);
+      rp = process_collisions<SM>(rp, n, false);
+      break;
+    case MGPU_PHASE_FIX_SECONDARY:
+      if (threadIdx.x == 0) fix_secondary_serial(g_c, P, n, 0, 0);
+      break;
+    case MGPU_PHASE_DETECT_LEF_BAR:
+      gather_ranked<SM>(n);
+      if (ranked_sorted<SM>(n) && words_plain<SM>(n) && fast) {
+        rp = detect_lef_bar_block<SM>(rp, n, 0, 0);
+      } else if (threadIdx.x == 0) {
+        detect_lef_bar_serial(g_c, P, n, 0, 0);
+      }
+      break;
+    case MGPU_PHASE_LEF_LEF:
+      gather_ranked<SM>(n);
+      if (ranked_sorted<SM>(n) && fast) {
+        rp = detect_primary_block<SM>(rp, n, 0, 0);
+        correct_primary<SM>(n);
+        rp = secondary_dir_block<SM>(rp, 0, n, 0, 0);
+        rp = secondary_dir_block<SM>(rp, 1, n, 0, 0);
+      } else {
+        if (threadIdx.x == 0) detect_primary_serial(g_c, P, n, 0, 0);
+        wsync(c.T);
+        correct_primary<SM>(n);
+        if (threadIdx.x == 0) process_secondary_serial(g_c, P, n, 0, 0);
+      }
+      break;
+    case MGPU_PHASE_DETECT_PRIMARY:
+      gather_ranked<SM>(n);
+      if (ranked_sorted<SM>(n) && fast) {
+        rp = detect_primary_block<SM>(rp, n, 0, 0);
+      } else if (threadIdx.x == 0) {
+        detect_primary_serial(g_c, P, n, 0, 0);
+      }
+      break;
+    case MGPU_PHASE_DETECT_BOUNDARIES:
+      if (threadIdx.x == 0) {
+        u64 n5, n3;
+        detect_boundaries_serial(c, P, n, n5, n3);
+        g_sc.n5 = n5;
+        g_sc.n3 = n3;
+      }
+      break;
+    case MGPU_PHASE_CORRECT_LEF_BAR:
+      correct_lef_bar<SM>(n);
+      break;
+    case MGPU_PHASE_CORRECT_PRIMARY:
+      correct_primary<SM>(n);
+      break;
+    case MGPU_PHASE_EXTRUDE:
+      extrude<SM>(n);
+      break;
+    case MGPU_PHASE_RELEASE:
+      rp = release_lefs<SM>(rp, n, completed);
+      break;
+    case MGPU_PHASE_BARRIER_NEXT:
+      rp = barriers_next<SM>(rp);
+      break;
+    case MGPU_PHASE_BARRIER_INIT:
+      rp = barriers_init<SM>(rp);
+      break;
+    default:
+      break;
+  }
+  wsync(c.T);
 }
 
 // One step of the epoch loop on caller state (mgpu_run_phase).
@@ -3446,14 +4019,16 @@ __global__ void __launch_bounds__(MAX_BLOCK_THREADS) phase_kernel(const __grid_c
                                                    u32 burnin_completed, u32 partially_sorted,
                                                    u32 init_ranks, u32 adjust, u64* prng,
                                                    u64* outs, const ulonglong2* jt, char* gslot) {
-  extern __shared__ __align__(16) char smem[];
-  __shared__ Cell c;
-  __shared__ BlockTmp bt;
-  load_layers(&bt, jt);
-  carve(c, &bt, smem, gslot, P, n, ch, jt, nullptr);
+  load_layers(jt);
+  load_plan(P);
   __syncthreads();
+  carve(gslot, ch, jt, nullptr);
+  __syncthreads();
+  Cell& c = g_c;
   u64* A[9];
+#pragma unroll 1
   for (int k = 0; k < 9; ++k) A[k] = arrays + (u64)k * n;
+#pragma unroll 1
   for (u32 i = threadIdx.x; i < n; i += blockDim.x) {
     c.rev[i] = A[0][i] == ~0ull ? UNBOUND : (u32)A[0][i];
     c.fwd[i] = A[1][i] == ~0ull ? UNBOUND : (u32)A[1][i];
@@ -3465,8 +4040,10 @@ __global__ void __launch_bounds__(MAX_BLOCK_THREADS) phase_kernel(const __grid_c
     c.rc[i] = cw_from_ref(A[7][i]);
     c.fc[i] = cw_from_ref(A[8][i]);
   }
+#pragma unroll 1
   for (u32 w = threadIdx.x; w < (c.nb + 31) / 32; w += blockDim.x) {
     u32 bits = 0;
+#pragma unroll 1
     for (u32 b = 0; b < 32; ++b) {
       const u32 i = w * 32 + b;
       if (i < c.nb && barrier_state && barrier_state[i]) bits |= 1u << b;
@@ -3474,9 +4051,11 @@ __global__ void __launch_bounds__(MAX_BLOCK_THREADS) phase_kernel(const __grid_c
     c.bst[w] = bits;
   }
   u64 init_state[4];
+#pragma unroll 1
   for (int k = 0; k < 4; ++k) init_state[k] = prng[k];
   if (threadIdx.x == 0) {
-    Scalars* sc = c.sc;
+    Scalars* sc = &g_sc;
+#pragma unroll 1
     for (int k = 0; k < 4; ++k) sc->canon[k] = prng[k];
     sc->rpos = 0;
     sc->gpos = sc->rpub = 0;
@@ -3488,114 +4067,23 @@ __global__ void __launch_bounds__(MAX_BLOCK_THREADS) phase_kernel(const __grid_c
     sc->sort_fallbacks = 0;
     sc->n5 = sc->n3 = 0;
     sc->prof = nullptr;
-    bt.released = 0;
+    g_bt.released = 0;
   }
   __syncthreads();
   if (threadIdx.x >= c.T) {
-    rng_produce(c);
+    rng_produce(g_c);
     return;
   }
   const bool completed = burnin_completed != 0;
-  const bool fast = !(P.debug_flags & DBG_SERIAL_COLLISIONS);
-  u64 rp = 0;
-  switch (phase) {
-    case MGPU_PHASE_BIND:
-      rp = bind_lefs(c, P, rp, n, (u32)epoch, bind_mask ? 1 : 2, bind_mask);
-      rank_lefs(c, P, n, (u32)epoch, epoch != 0);
-      break;
-    case MGPU_PHASE_RANK:
-      if (init_ranks) {
-        for (u32 i = threadIdx.x; i < n; i += c.T) {
-          c.rr[i] = i;
-          c.fr[i] = i;
-        }
-        wsync(c);
-      }
-      rank_lefs(c, P, n, (u32)epoch, partially_sorted != 0);
-      break;
-    case MGPU_PHASE_ADJUST_AND_CLAMP:
-      gather_ranked(c, n);
-      adjust_moves(c, P, n);
-      clamp_moves(c, P, n);
-      break;
-    case MGPU_PHASE_GENERATE_MOVES:
-      rp = gen_moves_dir(c, rp, c.rm, n, P.rev_speed[completed], P.rev_std, P.rev_move_int[completed]);
-      rp = gen_moves_dir(c, rp, c.fm, n, P.fwd_speed[completed], P.fwd_std, P.fwd_move_int[completed]);
-      if (adjust) {
-        gather_ranked(c, n);
-        adjust_moves(c, P, n);
-      }
-      clamp_moves(c, P, n);
-      break;
-    case MGPU_PHASE_PROCESS_COLLISIONS:
-      gather_ranked(c, n);
-      rp = process_collisions(c, P, rp, n, false);
-      break;
-    case MGPU_PHASE_FIX_SECONDARY:
-      if (threadIdx.x == 0) fix_secondary_serial(c, P, n, 0, 0);
-      break;
-    case MGPU_PHASE_DETECT_LEF_BAR:
-      gather_ranked(c, n);
-      if (ranked_sorted(c, n) && words_plain(c, n) && fast) {
-        rp = detect_lef_bar_block(c, P, rp, n, 0, 0);
-      } else if (threadIdx.x == 0) {
-        detect_lef_bar_serial(c, P, n, 0, 0);
-      }
-      break;
-    case MGPU_PHASE_LEF_LEF:
-      gather_ranked(c, n);
-      if (ranked_sorted(c, n) && fast) {
-        rp = detect_primary_block(c, P, rp, n, 0, 0);
-        correct_primary(c, n);
-        rp = secondary_dir_block(c, P, rp, 0, n, 0, 0);
-        rp = secondary_dir_block(c, P, rp, 1, n, 0, 0);
-      } else {
-        if (threadIdx.x == 0) detect_primary_serial(c, P, n, 0, 0);
-        wsync(c);
-        correct_primary(c, n);
-        if (threadIdx.x == 0) process_secondary_serial(c, P, n, 0, 0);
-      }
-      break;
-    case MGPU_PHASE_DETECT_PRIMARY:
-      gather_ranked(c, n);
-      if (ranked_sorted(c, n) && fast) {
-        rp = detect_primary_block(c, P, rp, n, 0, 0);
-      } else if (threadIdx.x == 0) {
-        detect_primary_serial(c, P, n, 0, 0);
-      }
-      break;
-    case MGPU_PHASE_DETECT_BOUNDARIES:
-      if (threadIdx.x == 0) {
-        u64 n5, n3;
-        detect_boundaries_serial(c, P, n, n5, n3);
-        c.sc->n5 = n5;
-        c.sc->n3 = n3;
-      }
-      break;
-    case MGPU_PHASE_CORRECT_LEF_BAR:
-      correct_lef_bar(c, n);
-      break;
-    case MGPU_PHASE_CORRECT_PRIMARY:
-      correct_primary(c, n);
-      break;
-    case MGPU_PHASE_EXTRUDE:
-      extrude(c, n);
-      break;
-    case MGPU_PHASE_RELEASE:
-      rp = release_lefs(c, P, rp, n, completed);
-      break;
-    case MGPU_PHASE_BARRIER_NEXT:
-      rp = barriers_next(c, rp);
-      break;
-    case MGPU_PHASE_BARRIER_INIT:
-      rp = barriers_init(c, rp);
-      break;
-    default:
-      break;
+  if (g_c.all_smem) {
+    run_phase<true>(phase, n, bind_mask, epoch, completed, partially_sorted, init_ranks, adjust);
+  } else {
+    run_phase<false>(phase, n, bind_mask, epoch, completed, partially_sorted, init_ranks, adjust);
   }
-  wsync(c);
-  // rank_lefs uses the move arrays as scratch: the caller's moves stay as they were
+  // rank_lefs uses the move arrays as scratch, place_moves the collision words: the caller's stay as they were
   const bool moves_kept = phase == MGPU_PHASE_BIND || phase == MGPU_PHASE_RANK;
+  const bool words_kept = phase == MGPU_PHASE_ADJUST_AND_CLAMP || phase == MGPU_PHASE_GENERATE_MOVES;
+#pragma unroll 1
   for (u32 i = threadIdx.x; i < n; i += c.T) {
     A[0][i] = pos64(c.rev[i]);
     A[1][i] = pos64(c.fwd[i]);
@@ -3606,21 +4094,26 @@ __global__ void __launch_bounds__(MAX_BLOCK_THREADS) phase_kernel(const __grid_c
       A[5][i] = c.rm[i];
       A[6][i] = c.fm[i];
     }
-    A[7][i] = cw_to_ref(c.rc[i]);
-    A[8][i] = cw_to_ref(c.fc[i]);
+    if (!words_kept) {
+      A[7][i] = cw_to_ref(c.rc[i]);
+      A[8][i] = cw_to_ref(c.fc[i]);
+    }
   }
+#pragma unroll 1
   for (u32 i = threadIdx.x; i < c.nb; i += c.T) {
-    if (barrier_state) barrier_state[i] = bar_active(c, i) ? 1 : 0;
+    if (barrier_state) barrier_state[i] = bar_active(c.bst, i) ? 1 : 0;
   }
   if (threadIdx.x == 0) {
     st_release(&c.sc->stop, 1);
     // the caller's PRNG advanced by exactly the number of draws consumed
     u64 st[4] = {init_state[0], init_state[1], init_state[2], init_state[3]};
+#pragma unroll 1
     for (u64 k = 0; k < c.sc->rpos; ++k) xo_next(st);
+#pragma unroll 1
     for (int k = 0; k < 4; ++k) prng[k] = st[k];
     outs[0] = c.sc->n5;
     outs[1] = c.sc->n3;
-    outs[2] = bt.released;
+    outs[2] = g_bt.released;
     outs[3] = c.sc->status;
   }
 }

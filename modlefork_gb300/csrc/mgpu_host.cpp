@@ -752,6 +752,18 @@ extern "C" int mgpu_set_chrom_config(mgpu_ctx* ctx, int chrom_id, const mgpu_con
   return MGPU_OK;
 }
 
+// Fixed-point constants of a move distribution: integer speeds below 2^19 with sd below 2^14, so
+// that |z * sd + mean| < 2^20 and the errors stay below a few units of 2^-32.
+static MoveSpec move_spec(double mean, double sd) {
+  MoveSpec m{mean, sd, 0, 0, (uint64_t)std::round(mean), sd == 0.0 ? 1u : 0u, 0u};
+  if (mean >= 0.0 && mean < 524288.0 && sd < 16384.0 && mean == std::floor(mean)) {
+    m.fixed = 1;
+    m.sdq = (uint64_t)(sd * 68719476736.0);
+    m.meanq = (int64_t)mean << 32;
+  }
+  return m;
+}
+
 // Worker warps of a cell: a sweep over its LEFs takes two to four rounds of the block.
 static u32 workers_for(uint64_t nlefs) { return nlefs <= 256 ? 4 : (nlefs <= 1024 ? 8 : 16); }
 
@@ -778,16 +790,10 @@ static int make_kparams(const mgpu_ctx* ctx, const ChromEntry& ch, uint64_t nlef
   P->skip_burnin = c.skip_burnin ? 1 : 0;
   P->min_burnin = c.min_burnin_epochs;
   P->max_burnin = c.max_burnin_epochs;
-  P->rev_speed[0] = (double)c.rev_extrusion_speed_burnin;
-  P->rev_speed[1] = (double)c.rev_extrusion_speed;
-  P->fwd_speed[0] = (double)c.fwd_extrusion_speed_burnin;
-  P->fwd_speed[1] = (double)c.fwd_extrusion_speed;
-  P->rev_std = c.rev_extrusion_speed_std;
-  P->fwd_std = c.fwd_extrusion_speed_std;
-  for (int k = 0; k < 2; ++k) {
-    P->rev_move_int[k] = (uint64_t)std::round(P->rev_speed[k]);
-    P->fwd_move_int[k] = (uint64_t)std::round(P->fwd_speed[k]);
-  }
+  P->rev_move[0] = move_spec((double)c.rev_extrusion_speed_burnin, c.rev_extrusion_speed_std);
+  P->rev_move[1] = move_spec((double)c.rev_extrusion_speed, c.rev_extrusion_speed_std);
+  P->fwd_move[0] = move_spec((double)c.fwd_extrusion_speed_burnin, c.fwd_extrusion_speed_std);
+  P->fwd_move[1] = move_spec((double)c.fwd_extrusion_speed, c.fwd_extrusion_speed_std);
   const double aff[3] = {1.0, 1.0 / c.soft_stall_lef_stability_multiplier,
                          1.0 / c.hard_stall_lef_stability_multiplier};
   for (int nh = 0; nh < 3; ++nh) {
@@ -834,7 +840,7 @@ static int make_kparams(const mgpu_ctx* ctx, const ChromEntry& ch, uint64_t nlef
   P->track_occ = c.track_1d_lef_position ? 1u : 0u;
   P->log_state = c.log_model_internal_state ? 1u : 0u;
   P->occ_bins = (ch.chrom.size + c.bin_size - 1) / c.bin_size;
-  // Layout: the scalars and the PRNG ring are always on chip; the burn-in history, the barrier bits
+  // Layout: the PRNG ring is always on chip (the scalars are static shared memory); the burn-in history, the barrier bits
   // and then the per-LEF arrays go on chip in priority order while they fit, the rest into a global
   // slot.  A budget counts the ring as BUDGET_RING_BYTES whatever the block's own takes.
   P->workers = workers ? workers : workers_for(nlefs);
@@ -845,9 +851,9 @@ static int make_kparams(const mgpu_ctx* ctx, const ChromEntry& ch, uint64_t nlef
     return fail(MGPU_ERR_UNSUPPORTED, "%u barriers need %llu B of shared memory (limit %llu)", ch.nb,
                 (unsigned long long)header, (unsigned long long)limit);
   const u64 ring = ring_bytes(P->workers);
-  const u64 room = std::min<u64>(ctx->smem_limit, limit - BUDGET_RING_BYTES + ring);
+  const u64 room = std::min<u64>(ctx->smem_limit, limit - CELL_HEADER_BYTES - BUDGET_RING_BYTES + ring);
   const u64 arr_bytes = ((u64)nlefs * 4 + 15) & ~15ull;
-  u64 smem_used = CELL_HEADER_BYTES + ring, slot_used = 0;
+  u64 smem_used = ring, slot_used = 0;
   const auto place = [&](u64 bytes, u32* off) {
     const bool on_chip = smem_used + bytes <= room;
     u64& used = on_chip ? smem_used : slot_used;

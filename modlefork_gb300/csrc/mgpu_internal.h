@@ -77,6 +77,16 @@ struct Trial {
   u32 always; // 1: the reference short-circuits to true without drawing
 };
 
+// Distribution of a direction's moves: round(max(0, normal(mean, sd))), or a constant.
+struct MoveSpec {
+  double mean, sd;
+  u64 sdq;       // sd * 2^36
+  i64 meanq;     // mean * 2^32
+  u64 move_int;  // the constant move (sd == 0)
+  u32 constant;
+  u32 fixed;     // the fixed-point evaluation is exact enough (move_sample)
+};
+
 struct KParams {
   u32 start, end;    // chromosome range [start, end): move clamps, boundary collisions
   u32 wstart, wend;  // simulated window: binding, contacts and the band (= start, end for a chromosome)
@@ -85,10 +95,8 @@ struct KParams {
   u32 hist_cap, smooth_w;
   u32 skip_burnin;
   u64 min_burnin, max_burnin;
-  // moves: [0] = burn-in speeds, [1] = after burn-in
-  double rev_speed[2], fwd_speed[2];
-  double rev_std, fwd_std;
-  u64 rev_move_int[2], fwd_move_int[2];
+  // moves: [0] = during burn-in, [1] = after it
+  MoveSpec rev_move[2], fwd_move[2];
   // release_lefs: [burnin_completed][number of hard LEF-BAR collisions 0..2]
   Trial release[2][3];
   Trial lef_lef;      // run_lef_lef_collision_trial
