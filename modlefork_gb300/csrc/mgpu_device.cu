@@ -117,9 +117,11 @@ struct Scalars {
   u64 bc0, bc1, bc2;  // broadcast slots for lane 0 results
   u64 nrec;           // model-state records written for this cell
   u64* prof;          // profile counters of the launch (device memory) or null
+  u64 mark;           // clock of the last profile mark
 };
 static_assert(sizeof(Scalars) <= CELL_HEADER_BYTES, "scalars do not fit the cell header");
 
+constexpr u32 MAX_TIES = 64;     // full ties among the units of one ranking that still form the sequence
 constexpr u32 TRIAL_WORDS = 65;  // outcomes of up to 2048 draws, and a word read past them
 
 // Scratch of the block-wide steps.
@@ -128,10 +130,11 @@ struct BlockTmp {
   u32 tab[16][32];      // gen_moves_dir: per warp and entry lane, leaving position | normals << 16
   u64 wmax[16];         // rank_dir_block
   u32 rem[16], rembase[16];
-  u32 nrem, tie, tie2;
+  u32 nrem, ntie, tie2;
+  u32 tierank[MAX_TIES];
   u32 dev[16], okm[16], dus[16];  // sample_contacts
   u32 trial[TRIAL_WORDS];  // secondary_dir_block
-  u32 used, qend, nr, nf, released, missed, flag;
+  u32 used, qend, nr, nf, released, missed, flag, total;
   u64 sum;
   ulonglong2 zt[128];   // normal ziggurat per layer: {draws below this are accepted, width * 2^60}
   float2 zy[128];       // and the density at its lower and upper edge: {y_i, y_{i+1} - y_i}
@@ -393,7 +396,19 @@ __device__ __noinline__ u64 rng_serial(Cell& c) {
   return v;
 }
 
-__device__ __forceinline__ void prof_add(u32 k, u64 v) {
+// Profile mark (all workers call it): adds the cycles since the previous mark to step k.  Out of line,
+// as everything the epoch loop does in many places: with several cells on an SM, each in another step,
+// the loop's code competes for the instruction caches.
+__device__ __noinline__ void prof_mark(u32 k) {
+  if (threadIdx.x != 0 || !g_sc.prof) return;
+  const u64 t = clock64();
+  if (k < PF_COUNT) {
+    atomicAdd((unsigned long long*)&g_sc.prof[k], (unsigned long long)(t - g_sc.mark));
+    atomicAdd((unsigned long long*)&g_sc.prof[PF_TOTAL], (unsigned long long)(t - g_sc.mark));
+  }
+  g_sc.mark = t;
+}
+__device__ __noinline__ void prof_add(u32 k, u64 v) {
   if (threadIdx.x == 0 && g_sc.prof) atomicAdd((unsigned long long*)&g_sc.prof[k], (unsigned long long)v);
 }
 
@@ -402,7 +417,7 @@ __device__ __forceinline__ void prof_add(u32 k, u64 v) {
 // line-by-line restatement; thresholds replace bernoulli / canonical comparisons.
 // ---------------------------------------------------------------------------------------
 
-__device__ u64 s_uniform_int(Cell& c, u64 a, u64 b) {
+__device__ __noinline__ u64 s_uniform_int(Cell& c, u64 a, u64 b) {
   const u64 range = b - a;
   if (range == 0) return a;
   if (range == ~0ull) return rng_serial(c) + a;
@@ -425,7 +440,7 @@ __device__ __forceinline__ bool s_trial(Cell& c, const Trial& t) {
 
 __device__ __forceinline__ double u01_of(u64 u) { return (double)u * (1.0 / 18446744073709551616.0); }
 
-__device__ double s_uniform01(Cell& c) {
+__device__ __noinline__ double s_uniform01(Cell& c) {
 #pragma unroll 1
   for (int it = 0; it < 1000; ++it) {
     const double r = u01_of(rng_serial(c));
@@ -1196,6 +1211,32 @@ __device__ __forceinline__ Scan2 scan2(u32 buf, bool f0, bool f1) {
   return r;
 }
 
+// floor(a / b), and the bucket width of a uniform_int over [0, range]: a 64-bit division is about 70
+// instructions, so the steps share one copy.
+__device__ __noinline__ u64 div64(u64 a, u64 b) { return a / b; }
+__device__ __forceinline__ u64 bucket_of(u64 range) {
+  const u64 q = div64(~0ull, range + 1);
+  return ~0ull - q * (range + 1) == range ? q + 1 : q;
+}
+
+// The same for one flag per thread.
+struct Scan1 {
+  u32 off, total;
+};
+template <bool SM>
+__device__ __forceinline__ Scan1 scan1(u32 T, u32 buf, bool f) {
+  const unsigned m = __ballot_sync(FULL, f);
+  const u32 w = threadIdx.x >> 5, l = ln();
+  u32* cnt = g_bt.cnt[buf];
+  if (l == 0) cnt[w] = __popc(m);
+  wsync(T);
+  const u32 v = l < (T >> 5) ? cnt[l] : 0u;
+  Scan1 r;
+  r.total = __reduce_add_sync(FULL, v);
+  r.off = __reduce_add_sync(FULL, l < w ? v : 0u) + __popc(m & lanemask_lt());
+  return r;
+}
+
 // ExtrusionBarriers::init_states (extrusion_barriers.cpp:220-231)
 template <bool SM>
 __device__ __noinline__ u64 barriers_init(u64 rp) {
@@ -1288,7 +1329,7 @@ __device__ __noinline__ u64 bind_lefs(u64 rp, u32 n, u32 epoch, int mode,
     u64 r = 0;
     bool ok = true;
     if (mine) {
-      r = ring_at(c.rmask, rp + threadIdx.x) / P.pos_bucket;
+      r = div64(ring_at(c.rmask, rp + threadIdx.x), P.pos_bucket);
       ok = r <= P.pos_range;
     }
     if (wsync_or(c.T, !ok)) {
@@ -1637,6 +1678,91 @@ __device__ __noinline__ bool rank_dir_split(Cell& c, u32 dir, u32 n) {
 
 __device__ __forceinline__ u64 max64(u64 a, u64 b) { return a > b ? a : b; }
 
+// Whether the kept unit of rank r and the one of rank r - 1, which it ties with in position and epoch,
+// surely stay in this order in the reference.  Its split_sort keeps a stack: an element below the top
+// leaves together with the top, the others are pushed; what stays keeps its order, even in a tie.  So
+// the pair's order is certain when neither can have left:
+//  * later pops reach rank r only if they outnumber the pushes after it.  Every pop needs a removed unit
+//    (one below its predecessors, or one bound this epoch that the next unit pops), so with the k-th
+//    removed unit after r at rank q_k, q_k - r >= 2 k + 2 for all k keeps a push in front of each pop;
+//  * the units themselves pop something only if a removed unit before them is still on the stack, and each
+//    of those is popped by one unit after it: (r - 1) - p_j >= 2 j + 2 for the j-th one before;
+//  * except that the bottom of the stack is never popped: rank 0 has to be a kept unit.
+template <class A>
+__device__ __noinline__ bool tie_keeps_order(const A& kmask, u32 nch, u32 r) {
+  const u32 a = r - 1;
+  if (r == 0 || !(kmask[0] & 1u) || !((kmask[a >> 5] >> (a & 31)) & 1u)) return false;
+  u32 k = 0;
+#pragma unroll 1
+  for (u32 ch = r >> 5; ch < nch; ++ch) {
+    u32 gone = ~kmask[ch];
+    if (ch == r >> 5) gone &= (r & 31) == 31 ? 0u : ~0u << ((r & 31) + 1);
+#pragma unroll 1
+    for (; gone; gone &= gone - 1) {
+      const u32 q = ch * 32 + (u32)(__ffs(gone) - 1);
+      if (q - r < 2 * ++k + 2) return false;
+    }
+  }
+  k = 0;
+#pragma unroll 1
+  for (u32 ch = a >> 5; ch != ~0u; --ch) {
+    u32 gone = ~kmask[ch];
+    if (ch == a >> 5) gone &= (1u << (a & 31)) - 1u;
+#pragma unroll 1
+    for (; gone; gone &= ~(1u << (31 - __clz(gone)))) {
+      const u32 q = ch * 32 + 31 - __clz(gone);
+      if (a - q < 2 * ++k + 2) return false;
+    }
+  }
+  return true;
+}
+
+// Which ranks stay on the stack of the reference's split_sort, one warp: a bit mask, from the positions in
+// rank order.  The pass runs 32 elements at a time as in rank_dir_split; the stack holds ranks.
+template <bool SM>
+__device__ __noinline__ void split_mask(u32 n, const Arr<SM> pos, const Arr<SM> stack, const Arr<SM> kmask) {
+  const u32 lane = ln();
+#pragma unroll 1
+  for (u32 ch = lane; ch < (n + 31) >> 5; ch += 32) kmask[ch] = n - ch * 32 >= 32 ? FULL : (1u << (n & 31)) - 1u;
+  if (lane == 0) stack[0] = 0;
+  u32 m = 0, T = pos[0];
+#pragma unroll 1
+  for (u32 base = 1; base < n; base += 32) {
+    const u32 r = base + lane, nvalid = min(32u, n - base);
+    const bool valid = lane < nvalid;
+    const u32 v = valid ? pos[r] : 0;
+    const u32 vprev = __shfl_up_sync(FULL, v, 1);
+    const bool pre_ok = lane == 0 || v >= vprev;
+    u32 start = 0;
+#pragma unroll 1
+    while (start < nvalid) {
+      const bool ok = lane == start ? v >= T : pre_ok;
+      const unsigned fail = __ballot_sync(FULL, !ok && lane >= start && valid);
+      const u32 f = fail ? (u32)(__ffs(fail) - 1) : nvalid;
+      if (lane >= start && lane < f) stack[m + 1 + lane - start] = r;
+      if (f > start) {
+        m += f - start;
+        T = __shfl_sync(FULL, v, f - 1);
+      }
+      if (f == nvalid) break;
+      __syncwarp();
+      const u32 rd = base + f, top = stack[m];
+      if (m > 0) {
+        --m;
+        T = pos[stack[m]];
+      }
+      if (lane == 0) {
+        kmask[rd >> 5] &= ~(1u << (rd & 31));
+        if (m > 0 || stack[0] != top) kmask[top >> 5] &= ~(1u << (top & 31));
+      }
+      start = f + 1;
+    }
+  }
+  __syncwarp();
+}
+
+enum : u32 { RANK_DONE = 0, RANK_TIE = 1, RANK_MANY = 2 };  // rank_dir_block's outcome
+
 // rank_lefs for one direction with the previous order reused, by all workers.
 //
 // Unless two units share position and binding epoch (a full tie), the reference's order (split_sort,
@@ -1644,8 +1770,11 @@ __device__ __forceinline__ u64 max64(u64 a, u64 b) { return a > b ? a : b; }
 // split into those that still form a non-decreasing sequence and the few that do not: the units bound
 // this epoch and every other one below the running maximum of the rest.  The few are sorted by key
 // (runs of 32 in registers, then each finds its place in the other runs by binary search) and merged
-// back by rank.  Returns false with R untouched when a full tie turns up or when too many units moved:
-// the caller then takes rank_dir_split, the exact restatement.
+// back by rank.  R stays untouched when a full tie turns up whose order is not certain
+// (tie_keeps_order, RANK_TIE) or when too many units moved (RANK_MANY); n is 2 to 65535.  With exact, the kept units are those the
+// reference's own pass keeps (split_mask): then ties among them and with a removed unit have the
+// order the stable merge gives them, and only a tie between two removed units is left to
+// rank_dir_split.
 //
 // Phases, each ended by a wsync; warp w owns a contiguous range of the ranks:
 //  1 keys in rank order to rm / fm, and their maximum per warp;
@@ -1655,9 +1784,8 @@ __device__ __forceinline__ u64 max64(u64 a, u64 b) { return a > b ? a : b; }
 //  4 each removed unit's place among the removed (pairwise searches) and among the kept;
 //  5 the new order, written to rm; 6 copied to R.
 template <bool SM>
-__device__ __noinline__ bool rank_dir_block(u32 dir, u32 n, u32 epoch) {
+__device__ __noinline__ u32 rank_dir_block(u32 dir, u32 n, u32 epoch, bool exact) {
   const View<SM> c;
-  if (n < 2 || n > 0xFFFFu) return false;
   const u32 T = c.T, W = T >> 5, w = threadIdx.x >> 5, lane = ln();
   const auto R = dir ? c.fr : c.rr;
   const auto pos = dir ? c.fwd : c.rev;
@@ -1671,7 +1799,7 @@ __device__ __noinline__ bool rank_dir_block(u32 dir, u32 n, u32 epoch) {
   const auto bp = c.tmp, sr0 = c.tmp + maxb, sfin = c.tmp + 2 * maxb;
   const u32 ch0 = w * nch / W, ch1 = (w + 1) * nch / W;
   const u32 newlo = dir ? ~epoch : epoch;
-  u64 mx = 0;
+  u32 mh = 0, ml = 0;  // this lane's largest key
 #pragma unroll 1
   for (u32 ch = ch0; ch < ch1; ++ch) {
     const u32 r = ch * 32 + lane;
@@ -1680,41 +1808,84 @@ __device__ __noinline__ bool rank_dir_block(u32 dir, u32 n, u32 epoch) {
       const u32 p = pos[idx], e = bep[idx], lo = dir ? ~e : e;
       kh[r] = p;
       kl[r] = lo;
-      if (lo != newlo) mx = max64(mx, ((u64)p << 32) | lo);
+      if (lo != newlo && (p > mh || (p == mh && lo > ml))) {
+        mh = p;
+        ml = lo;
+      }
     }
   }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) mx = max64(mx, __shfl_xor_sync(FULL, mx, d));
+  const u32 wh = __reduce_max_sync(FULL, mh);
+  const u64 mx = ((u64)wh << 32) | __reduce_max_sync(FULL, mh == wh ? ml : 0u);
   if (lane == 0) g_bt.wmax[w] = mx;
   if (threadIdx.x == 0) {
     g_bt.nrem = 0;
-    g_bt.tie = 0;
+    g_bt.ntie = 0;
     g_bt.tie2 = 0;
   }
   wsync(c.T);
+  if (exact) {
+    if (w == 0) split_mask<SM>(n, kh, c.sr, kmask);
+    wsync(c.T);
+    // maxima of the kept units
+    u64 kmx = 0;
+#pragma unroll 1
+    for (u32 ch = ch0; ch < ch1; ++ch) {
+      const u32 r = ch * 32 + lane;
+      if ((kmask[ch] >> lane) & 1u) kmx = max64(kmx, ((u64)kh[r] << 32) | kl[r]);
+    }
+#pragma unroll 1
+    for (int d = 16; d > 0; d >>= 1) kmx = max64(kmx, __shfl_xor_sync(FULL, kmx, d));
+    if (lane == 0) g_bt.wmax[w] = kmx;
+    wsync(c.T);
+  }
   u64 carry = lane < w ? g_bt.wmax[lane] : 0;
-#pragma unroll
+#pragma unroll 1
   for (int d = 8; d > 0; d >>= 1) carry = max64(carry, __shfl_xor_sync(FULL, carry, d));
   carry = __shfl_sync(FULL, carry, 0);
-  bool tie = false;
   u32 removed = 0;
 #pragma unroll 1
   for (u32 ch = ch0; ch < ch1; ++ch) {
     const u32 r = ch * 32 + lane;
     const bool valid = r < n;
     const u32 hi = valid ? kh[r] : 0u, lo = valid ? kl[r] : 0u;
-    const u64 key = ((u64)hi << 32) | lo;
-    const bool old = valid && lo != newlo;
-    u64 x = old ? key : 0;
-#pragma unroll
+    const bool old = exact ? (kmask[ch] >> lane) & 1u : valid && lo != newlo;
+    // running maximum of the old units before this one: by position alone unless positions repeat
+    u32 x = old ? hi : 0;
+#pragma unroll 1
     for (int d = 1; d < 32; d <<= 1) {
-      const u64 y = __shfl_up_sync(FULL, x, d);
-      if ((int)lane >= d) x = max64(x, y);
+      const u32 y = __shfl_up_sync(FULL, x, d);
+      if ((int)lane >= d) x = max(x, y);
     }
-    u64 excl = __shfl_up_sync(FULL, x, 1);
-    excl = lane == 0 ? carry : max64(excl, carry);
-    const bool keep = old && key >= excl;
-    tie |= keep && key == excl;
+    const u32 px = __shfl_up_sync(FULL, x, 1);
+    const u32 eh = max(lane == 0 ? 0u : px, (u32)(carry >> 32));
+    bool keep = old && hi > eh;
+    u64 excl;
+    const u64 key = ((u64)hi << 32) | lo;
+    if (!exact && !__any_sync(FULL, old && hi == eh)) {
+      // the maximum's epoch is that of the last unit kept before
+      const unsigned kb = __ballot_sync(FULL, keep), before = kb & lanemask_lt();
+      const u32 el = __shfl_sync(FULL, lo, before ? 31 - __clz(before) : 0);
+      excl = ((u64)eh << 32) | (before ? el : (u32)carry);
+      const u32 top = __shfl_sync(FULL, lo, kb ? 31 - __clz(kb) : 0);
+      const u32 th = __shfl_sync(FULL, hi, kb ? 31 - __clz(kb) : 0);
+      if (kb) carry = ((u64)th << 32) | top;
+    } else {
+      u64 z = old ? key : 0;
+#pragma unroll 1
+      for (int d = 1; d < 32; d <<= 1) {
+        const u64 y = __shfl_up_sync(FULL, z, d);
+        if ((int)lane >= d) z = max64(z, y);
+      }
+      excl = __shfl_up_sync(FULL, z, 1);
+      excl = lane == 0 ? carry : max64(excl, carry);
+      keep = old && key >= excl;
+      if (exact && keep != old) g_bt.tie2 = 1;  // equal positions out of epoch order
+      if (!exact && keep && key == excl) {
+        const u32 q = atomicAdd(&g_bt.ntie, 1u);
+        if (q < MAX_TIES) g_bt.tierank[q] = r;
+      }
+      carry = max64(carry, __shfl_sync(FULL, z, 31));
+    }
     const bool rem = valid && !keep;
     const unsigned km = __ballot_sync(FULL, keep), rmk = __ballot_sync(FULL, rem);
     if (lane == 0) kmask[ch] = km;
@@ -1732,13 +1903,14 @@ __device__ __noinline__ bool rank_dir_block(u32 dir, u32 n, u32 epoch) {
       }
       removed += __popc(rmk);
     }
-    carry = max64(carry, __shfl_sync(FULL, x, 31));
   }
   if (lane == 0) g_bt.rem[w] = removed;
-  if (tie) g_bt.tie = 1;
   wsync(c.T);
   const u32 m = g_bt.nrem;
-  if (m > maxb || g_bt.tie) return false;
+  const u32 nt = g_bt.ntie;
+  if (m > maxb) return RANK_MANY;
+  if (nt > MAX_TIES) return RANK_TIE;
+  if (threadIdx.x < nt && !tie_keeps_order(kmask, nch, g_bt.tierank[threadIdx.x])) g_bt.tie2 = 1;
   // 3: runs of 32
   if (w == W - 1) {  // removed units before each warp's range
     u32 v = lane < W ? g_bt.rem[lane] : 0u;
@@ -1750,9 +1922,9 @@ __device__ __noinline__ bool rank_dir_block(u32 dir, u32 n, u32 epoch) {
     const u32 q = run * 32 + lane;
     u64 key = q < m ? bk.at64(q) : ~0ull;
     u32 pl = q < m ? bp[q] : 0u;
-#pragma unroll
+#pragma unroll 1
     for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
+#pragma unroll 1
       for (int j = k >> 1; j > 0; j >>= 1) {
         const u64 ok = __shfl_xor_sync(FULL, key, j);
         const u32 op = __shfl_xor_sync(FULL, pl, j);
@@ -1798,11 +1970,11 @@ __device__ __noinline__ bool rank_dir_block(u32 dir, u32 n, u32 epoch) {
     while (lo < hi) {
       const u32 mid = (lo + hi) >> 1;
       const u32 h = kh[mid];
-      if (h < khi || (h == khi && kl[mid] < klo)) lo = mid + 1; else hi = mid;
+      if (h < khi || (h == khi && kl[mid] < klo + ((exact && klo != ~0u) ? 1u : 0u))) lo = mid + 1; else hi = mid;
     }
     u32 before = m;  // removed units at ranks below lo
     if (lo < n) {
-      if (kh[lo] == khi && kl[lo] == klo) g_bt.tie2 = 1;
+      if (kh[lo] == khi && kl[lo] == klo) g_bt.tie2 = 1;  // exact: passed above
       const u32 ch = lo >> 5, ow = ((ch + 1) * W - 1) / nch;
       before = g_bt.rembase[ow];
 #pragma unroll 1
@@ -1813,7 +1985,7 @@ __device__ __noinline__ bool rank_dir_block(u32 dir, u32 n, u32 epoch) {
     sfin[rank] = (bp[q] & 0xFFFFu) | ((rank + lo - before) << 16);
   }
   wsync(c.T);
-  if (g_bt.tie2) return false;
+  if (g_bt.tie2) return RANK_TIE;
   // 5: the new order
   const auto O = c.rm;
 #pragma unroll 1
@@ -1853,33 +2025,102 @@ __device__ __noinline__ bool rank_dir_block(u32 dir, u32 n, u32 epoch) {
 #pragma unroll 1
   for (u32 r = threadIdx.x; r < n; r += T) R[r] = O[r];
   wsync(c.T);
+  return RANK_DONE;
+}
+
+// Sort of all units of one direction by key, by all workers: a bitonic network of ascending comparators
+// (see bitonic_keyed) on keys in rm / fm and indices in tmp.  Returns false, R untouched, on a full tie.
+template <bool SM>
+__device__ __noinline__ bool rank_dir_all(u32 dir, u32 n) {
+  const View<SM> c;
+  const u32 T = c.T;
+  const auto R = dir ? c.fr : c.rr;
+  const auto pos = dir ? c.fwd : c.rev;
+  const auto hi = c.rm, lo = c.fm, ix = c.tmp;
+#pragma unroll 1
+  for (u32 r = threadIdx.x; r < n; r += T) {
+    const u32 u = R[r], e = c.bep[u];
+    ix[r] = u;
+    hi[r] = pos[u];
+    lo[r] = dir ? ~e : e;
+  }
+  wsync(T);
+  u32 lg = 0;
+#pragma unroll 1
+  while ((1u << lg) < n) ++lg;
+  const u32 ncmp = (1u << lg) >> 1;
+#pragma unroll 1
+  for (u32 s = 1; s <= lg; ++s) {
+#pragma unroll 1
+    for (int q = (int)s - 1; q >= 0; --q) {
+#pragma unroll 1
+      for (u32 t = threadIdx.x; t < ncmp; t += T) {
+        u32 i, j;
+        if (q == (int)s - 1) {  // mirror pairs
+          const u32 base = (t >> q) << s, off = t & ((1u << q) - 1u);
+          i = base + off;
+          j = base + (1u << s) - 1u - off;
+        } else {
+          i = ((t >> q) << (q + 1)) | (t & ((1u << q) - 1u));
+          j = i + (1u << q);
+        }
+        if (j >= n) continue;
+        const u32 hi_i = hi[i], hi_j = hi[j], lo_i = lo[i], lo_j = lo[j];
+        if (hi_i > hi_j || (hi_i == hi_j && lo_i > lo_j)) {
+          hi[i] = hi_j;
+          hi[j] = hi_i;
+          lo[i] = lo_j;
+          lo[j] = lo_i;
+          const u32 x = ix[i];
+          ix[i] = ix[j];
+          ix[j] = x;
+        }
+      }
+      wsync(T);
+    }
+  }
+  bool tie = false;
+#pragma unroll 1
+  for (u32 r = threadIdx.x + 1; r < n; r += T) tie |= hi[r - 1] == hi[r] && lo[r - 1] == lo[r];
+  if (wsync_or(T, tie)) return false;
+#pragma unroll 1
+  for (u32 r = threadIdx.x; r < n; r += T) R[r] = ix[r];
+  wsync(T);
   return true;
 }
 
-// Full ties, many moved units (a young cell binds most of its units in one epoch) or a small n:
-// one warp's exact emulation; the first epoch and unsorted callers: the serial restatement.
+// The incremental merge; after a full tie the merge on the reference's own kept units; a sort of all
+// units when many moved (a young cell binds most of its units in one epoch) and for the first epoch;
+// and where ties are left to pdq_sort's element moves, one warp's exact emulation or, without a previous
+// order, the serial restatement.  sort_fallbacks counts the directions without a reusable order.
 template <bool SM>
 __device__ __noinline__ void rank_lefs(u32 n, u32 epoch, bool partially_sorted) {
   const View<SM> c;
   const KParams& P = g_P;
-  const bool fast = partially_sorted && !(P.debug_flags & DBG_SERIAL_RANK) && n >= 2 && n <= 0xFFFFu;
+  const bool serial = P.debug_flags & DBG_SERIAL_RANK;
+  const bool fast = partially_sorted && !serial && n >= 2 && n <= 0xFFFFu;
 #pragma unroll 1
   for (u32 dir = 0; dir < 2; ++dir) {
     if (fast) {
-      if (rank_dir_block<SM>(dir, n, epoch)) continue;
-      const u64 t0 = clock64();
+      u32 got = rank_dir_block<SM>(dir, n, epoch, false);
+      if (got == RANK_DONE) continue;
+      wsync(c.T);  // the scratch is written again
+      if (got == RANK_TIE) {
+        got = rank_dir_block<SM>(dir, n, epoch, true);
+        if (got == RANK_DONE) continue;
+        wsync(c.T);
+      }
+      if (got == RANK_MANY && rank_dir_all<SM>(dir, n)) continue;
+      prof_add(PF_RANK_SPLIT, 1);
       if (threadIdx.x < 32) rank_dir_split(g_c, dir, n);
       wsync(c.T);
-      prof_add(PF_RANK_SPLIT, clock64() - t0);
     } else {
-      const u64 t0 = clock64();
       prof_add(PF_RANK_FALLBACK, 1);
-      if (threadIdx.x == 0) {
-        rank_dir_serial(g_c, dir, n, partially_sorted);
-        g_sc.sort_fallbacks++;
+      if (threadIdx.x == 0) g_sc.sort_fallbacks++;
+      if (serial || !rank_dir_all<SM>(dir, n)) {
+        if (threadIdx.x == 0) rank_dir_serial(g_c, dir, n, partially_sorted);
+        wsync(c.T);
       }
-      wsync(c.T);
-      prof_add(PF_RANK_SERIAL, clock64() - t0);
     }
   }
 }
@@ -1985,7 +2226,7 @@ __device__ __forceinline__ int move_sample(RingSrc& g, const MoveSpec& ms, u32* 
 template <bool SM>
 __device__ __noinline__ u64 gen_moves_dir(u64 rp, const Arr<SM> mv, u32 n, const MoveSpec& spec) {
   const View<SM> c;
-  const u32 T = c.T, W = T >> 5, w = threadIdx.x >> 5, lane = ln();
+  const u32 T = c.T, w = threadIdx.x >> 5, lane = ln();
   const MoveSpec ms = spec;
   if (ms.constant) {
 #pragma unroll 1
@@ -2018,17 +2259,23 @@ __device__ __noinline__ u64 gen_moves_dir(u64 rp, const Arr<SM> mv, u32 n, const
   u32 t0 = 0;
 #pragma unroll 1
   while (t0 < nb) {
-    rng_ensure(rp, T + 64);
-    RingSrc g{c.rmask, (u32)rp + threadIdx.x, (u32)rp + T + 64, 0};
-    u32 v = 0;
+    // warps of the window: those that serve the remaining normals, and one for longer ones
+    const u32 W = min(T >> 5, (nb - t0 + 31) / 32 + 1), span = 32 * W;
+    u32 v = 0, len = 1;
     bool range = false;
-    const int st = move_sample(g, ms, &v, &range);
-    const u32 len = g.n;
+    int st = SMP_OK;
+    unsigned dm = 0;
+    u32 step = 0;
+    if (w < W) {
+    rng_ensure(rp, span + 64);
+    RingSrc g{c.rmask, (u32)rp + threadIdx.x, (u32)rp + span + 64, 0};
+    st = move_sample(g, ms, &v, &range);
+    len = g.n;
     // Per entry lane: where the chain leaves the warp (32 + the lane it enters the next one at, or
     // DRY + the lane whose sampler ran dry) and how many normals start before that.  Almost every
     // normal takes one draw, so the chain only bends at the few lanes of dm, taken from the last.
-    const unsigned dm = __ballot_sync(FULL, st != SMP_OK || len != 1);
-    const u32 step = st == SMP_OK ? lane + len : DRY;
+    dm = __ballot_sync(FULL, st != SMP_OK || len != 1);
+    step = st == SMP_OK ? lane + len : DRY;
     u32 leave = 32, cnt = 32 - lane;
 #pragma unroll 1
     for (unsigned r = dm; r;) {
@@ -2042,6 +2289,7 @@ __device__ __noinline__ u64 gen_moves_dir(u64 rp, const Arr<SM> mv, u32 n, const
       }
     }
     g_bt.tab[w][lane] = leave | (cnt << 16);
+    }
     wsync(c.T);
     // Entry lane of every warp (lane k of each warp holds warp k's): all zero unless a normal straddles
     // two warps, so start there and repeat until the entries agree with the warps before.
@@ -2061,8 +2309,8 @@ __device__ __noinline__ u64 gen_moves_dir(u64 rp, const Arr<SM> mv, u32 n, const
     if (!__any_sync(FULL, odd)) {
       const u32 ex = warp_excl_scan(lane < W ? t >> 16 : 0u, &base);
       my_base = __shfl_sync(FULL, ex, w);
-      my_e = __shfl_sync(FULL, e, w);
-      used = T + __shfl_sync(FULL, (t & 0xFFFFu) - 32, W - 1);
+      my_e = w < W ? __shfl_sync(FULL, e, w) : 64u;
+      used = span + __shfl_sync(FULL, (t & 0xFFFFu) - 32, W - 1);
     } else {
       // a normal of more than 32 draws or a dry sampler: follow the entries one by one
       u32 en = 0;
@@ -2090,7 +2338,7 @@ __device__ __noinline__ u64 gen_moves_dir(u64 rp, const Arr<SM> mv, u32 n, const
         }
         en = q - 32;
       }
-      if (!dry) used = T + en;
+      if (!dry) used = span + en;
     }
     const u32 served = min(base, nb - t0);
     if (my_e < 32) {
@@ -2299,26 +2547,26 @@ struct BucketIndex {
   Arr<SM> key, T;
   u32 n, start, shift, nbk;
   bool table;
-  // first k in [0, n) with key[k] >= x
-  __device__ u32 lower_bound(u32 x) const {
-    if (!table) {  // n too small for a table
-      u32 lo = 0, hi = n;
-#pragma unroll 1
-      while (lo < hi) {
-        const u32 mid = (lo + hi) >> 1;
-        if (key[mid] >= x) hi = mid; else lo = mid + 1;
-      }
-      return lo;
-    }
-    if (x <= start) return 0;
-    u32 b = (x - start) >> shift;
-    if (b > nbk) b = nbk;
-    u32 k = T[b];
-#pragma unroll 1
-    while (k < n && key[k] < x) ++k;
-    return k;
-  }
 };
+
+// first k in [0, n) with key[k] >= x
+template <bool SM>
+__device__ __noinline__ u32 lower_bound(const BucketIndex<SM> ix, u32 x) {
+  if (!ix.table) {  // n too small for a table
+    u32 lo = 0, hi = ix.n;
+#pragma unroll 1
+    while (lo < hi) {
+      const u32 mid = (lo + hi) >> 1;
+      if (ix.key[mid] >= x) hi = mid; else lo = mid + 1;
+    }
+    return lo;
+  }
+  if (x <= ix.start) return 0;
+  u32 k = ix.T[min((x - ix.start) >> ix.shift, ix.nbk)];
+#pragma unroll 1
+  while (k < ix.n && ix.key[k] < x) ++k;
+  return k;
+}
 
 // Collective; T needs n entries.
 template <bool SM>
@@ -2379,7 +2627,7 @@ __device__ __forceinline__ bool trial_outcome(const Trial& t, u64 u) {
 constexpr u32 EV_HIT = EV_COLLISION | EV_CHROM_BOUNDARY | EV_LEF_BAR;
 
 template <bool SM>
-__device__ __noinline__ u64 detect_lef_bar_dir(u64 rp, u32 dir, u32 n, u64 n5, u64 n3) {
+__device__ __noinline__ u64 detect_lef_bar_dir(u64 rp, u32 dir, u32 n, u32 n5, u32 n3) {
   const View<SM> c;
   const KParams& P = g_P;
   const u32 T = c.T;
@@ -2389,64 +2637,50 @@ __device__ __noinline__ u64 detect_lef_bar_dir(u64 rp, u32 dir, u32 n, u64 n5, u
   const auto M = dir ? c.fm : c.rm;
   const auto C = dir ? c.fc : c.rc;
   // rev: first k >= j0 with S[k] > bpos; fwd: last k <= jtop with S[k] < bpos
-  const u32 j0 = (u32)min(n5, n5 - 1);
-  const u32 jtop = (u32)(n - min(n3, n3 - 1)) - 1;
+  const u32 j0 = min(n5, n5 - 1);
+  const u32 jtop = (n - min(n3, n3 - 1)) - 1;
   const BucketIndex<SM> ix = build_bucket_index<SM>(S, n, (u32)P.start, (u32)P.end, c.tmp);
   u32 buf = 0;
 #pragma unroll 1
-  for (u32 base = 0; base < c.nb; base += 2 * T) {
-    rng_ensure(rp, 2 * T);
-    u32 bi[2], unit[2];
-    int ti[2];
-    bool cand[2], drawn[2];
-#pragma unroll
-    for (u32 h = 0; h < 2; ++h) {
-      const u32 o = base + h * T + threadIdx.x;
-      cand[h] = drawn[h] = false;
-      bi[h] = unit[h] = 0;
-      ti[h] = 0;
-      if (o < c.nb) {
-        const u32 i = dir ? c.nb - 1 - o : o;
-        if (bar_active(c.bst, i)) {
-          const uint2 pf = __ldg(&c.bpf[i]);
-          const u32 bdir = pf.y & BF_DIR_MASK;
-          u32 k = ix.lower_bound(dir ? pf.x : pf.x + 1);
-          bool ok;
-          if (dir == 0) {
-            k = max(j0, k);
-            ok = k < n;
-          } else {
-            k = min(jtop + 1, k);
-            ok = k > 0;
-            --k;
-          }
-          if (ok) {
-            const u32 u = R[k], kpos = S[k];
-            if (bep[u] != UNBOUND) {
-              const u64 delta = dir ? (u64)pf.x - kpos : (u64)kpos - pf.x;
-              if (delta > 0 && delta <= M[u]) {
-                cand[h] = true;
-                bi[h] = i;
-                unit[h] = u;
-                ti[h] = dir ? (bdir == MGPU_DIR_FWD ? 0 : 1) : (bdir == MGPU_DIR_REV ? 0 : 1);
-                drawn[h] = trial_needs_draw(P.lef_bar[ti[h]]);
-              }
+  for (u32 base = 0; base < c.nb; base += T) {
+    rng_ensure(rp, T);
+    const u32 o = base + threadIdx.x;
+    bool cand = false, drawn = false;
+    u32 bi = 0, unit = 0, ti = 0;
+    if (o < c.nb) {
+      const u32 i = dir ? c.nb - 1 - o : o;
+      if (bar_active(c.bst, i)) {
+        const uint2 pf = __ldg(&c.bpf[i]);
+        u32 k = lower_bound<SM>(ix, dir ? pf.x : pf.x + 1);
+        bool ok;
+        if (dir == 0) {
+          k = max(j0, k);
+          ok = k < n;
+        } else {
+          k = min(jtop + 1, k);
+          ok = k > 0;
+          --k;
+        }
+        if (ok) {
+          const u32 u = R[k], kpos = S[k];
+          if (bep[u] != UNBOUND) {
+            const u64 delta = dir ? (u64)pf.x - kpos : (u64)kpos - pf.x;
+            if (delta > 0 && delta <= M[u]) {
+              cand = true;
+              bi = i;
+              unit = u;
+              ti = (pf.y & BF_DIR_MASK) == (dir ? MGPU_DIR_FWD : MGPU_DIR_REV) ? 0u : 1u;
+              drawn = trial_needs_draw(P.lef_bar[ti]);
             }
           }
         }
       }
     }
-    const Scan2 s = scan2<SM>(buf, drawn[0], drawn[1]);
+    const Scan1 s = scan1<SM>(T, buf, drawn);
     rng_publish(rp);  // the draws of the windows before
     buf ^= 1;
-#pragma unroll
-    for (u32 h = 0; h < 2; ++h) {
-      if (cand[h]) {
-        const u64 u = drawn[h] ? ring_at(c.rmask, rp + (h ? s.off1 : s.off0)) : 0;
-        if (trial_outcome(P.lef_bar[ti[h]], u))
-          atomicMax(&C[unit[h]], cw_make(dir ? CW_IDX_MASK - bi[h] : bi[h], EV_HIT));
-      }
-    }
+    if (cand && trial_outcome(P.lef_bar[ti], drawn ? ring_at(c.rmask, rp + s.off) : 0))
+      atomicMax(&C[unit], cw_make(dir ? CW_IDX_MASK - bi : bi, EV_HIT));
     rp += s.total;
   }
   wsync(c.T);
@@ -2455,7 +2689,7 @@ __device__ __noinline__ u64 detect_lef_bar_dir(u64 rp, u32 dir, u32 n, u64 n5, u
 }
 
 template <bool SM>
-__device__ __noinline__ u64 detect_lef_bar_block(u64 rp, u32 n, u64 n5, u64 n3) {
+__device__ __noinline__ u64 detect_lef_bar_block(u64 rp, u32 n, u32 n5, u32 n3) {
   const View<SM> c;
   rp = detect_lef_bar_dir<SM>(rp, 0, n, n5, n3);
   rp = detect_lef_bar_dir<SM>(rp, 1, n, n5, n3);
@@ -2485,51 +2719,43 @@ __device__ __noinline__ bool words_plain(u32 n) {
 // each against the fwd unit of rank cnt(j) - 1.  Tested pairs are disjoint, so their
 // collision words are updated independently; trials draw in ascending j.
 template <bool SM>
-__device__ __noinline__ u64 detect_primary_block(u64 rp, u32 n, u64 n5, u64 n3) {
+__device__ __noinline__ u64 detect_primary_block(u64 rp, u32 n, u32 n5, u32 n3) {
   const View<SM> c;
   const KParams& P = g_P;
   if (n5 == n || n3 == n) return rp;
   const u32 T = c.T;
-  const u32 i2 = (u32)(n - min(n3, n3 - 1));
+  const u32 i2 = (n - min(n3, n3 - 1));
   // bucket index over the fwd ranked positions (this step can also run on its own)
   const BucketIndex<SM> ixf = build_bucket_index<SM>(c.sf, n, (u32)P.start, (u32)P.end, c.tmp);
   u32 buf = 0;
 #pragma unroll 1
-  for (u32 base = (u32)n5; base < n; base += 2 * T) {
-    rng_ensure(rp, 2 * T);
-    u32 ru[2], fu[2], rp_[2], fp_[2], rmv[2], fmv[2];
-    bool cand[2], drawn[2];
-#pragma unroll
-    for (u32 h = 0; h < 2; ++h) {
-      const u32 j = base + h * T + threadIdx.x;
-      const bool valid = j < n;
-      u32 cnt = 0;
-      if (valid) cnt = min(i2, ixf.lower_bound(c.sr[j]));  // first i < i2 with sf[i] >= rev position
-      u32 prev = __shfl_up_sync(FULL, cnt, 1);
-      if (ln() == 0 && valid) prev = j == (u32)n5 ? 0u : min(i2, ixf.lower_bound(c.sr[j - 1]));
-      cand[h] = drawn[h] = false;
-      ru[h] = fu[h] = rp_[h] = fp_[h] = rmv[h] = fmv[h] = 0;
-      if (valid && cnt > prev && cnt < i2) {
-        ru[h] = c.rr[j];
-        fu[h] = c.fr[cnt - 1];
-        rp_[h] = c.sr[j];
-        fp_[h] = c.sf[cnt - 1];
-        rmv[h] = c.rm[ru[h]];
-        fmv[h] = c.fm[fu[h]];
-        const u64 delta = pos64(rp_[h]) - pos64(fp_[h]);
-        cand[h] = delta > 0 && delta < (u64)rmv[h] + fmv[h];
-        drawn[h] = cand[h] && trial_needs_draw(P.lef_lef);
-      }
+  for (u32 base = n5; base < n; base += T) {
+    rng_ensure(rp, T);
+    const u32 j = base + threadIdx.x;
+    const bool valid = j < n;
+    const u32 pr = valid ? c.sr[j] : 0u;
+    u32 cnt = 0;
+    if (valid) cnt = min(i2, lower_bound<SM>(ixf, pr));  // first i < i2 with sf[i] >= rev position
+    u32 prev = __shfl_up_sync(FULL, cnt, 1);
+    if (ln() == 0 && valid) prev = j == n5 ? 0u : min(i2, lower_bound<SM>(ixf, c.sr[j - 1]));
+    bool cand = false, drawn = false;
+    u32 ru = 0, fu = 0, pf = 0, rmv = 0, fmv = 0;
+    if (valid && cnt > prev && cnt < i2) {
+      ru = c.rr[j];
+      fu = c.fr[cnt - 1];
+      pf = c.sf[cnt - 1];
+      rmv = c.rm[ru];
+      fmv = c.fm[fu];
+      const u64 delta = pos64(pr) - pos64(pf);
+      cand = delta > 0 && delta < (u64)rmv + fmv;
+      drawn = cand && trial_needs_draw(P.lef_lef);
     }
-    const Scan2 s = scan2<SM>(buf, drawn[0], drawn[1]);
+    const Scan1 sc = scan1<SM>(T, buf, drawn);
     rng_publish(rp);
     buf ^= 1;
-#pragma unroll
-    for (u32 h = 0; h < 2; ++h) {
-      if (cand[h] && trial_outcome(P.lef_lef, drawn[h] ? ring_at(c.rmask, rp + (h ? s.off1 : s.off0)) : 0))
-        primary_pair_update(c, ru[h], fu[h], pos64(rp_[h]), pos64(fp_[h]), rmv[h], fmv[h]);
-    }
-    rp += s.total;
+    if (cand && trial_outcome(P.lef_lef, drawn ? ring_at(c.rmask, rp + sc.off) : 0))
+      primary_pair_update(c, ru, fu, pos64(pr), pos64(pf), rmv, fmv);
+    rp += sc.total;
   }
   wsync(c.T);
   rng_publish(rp);
@@ -2694,7 +2920,14 @@ __device__ __forceinline__ u32 chain_walk(const C& c, const Trial& tr, u32 dir, 
 }
 
 template <bool SM>
-__device__ __noinline__ u64 secondary_dir_block(u64 rp, u32 dir, u32 n, u64 n5, u64 n3) {
+__device__ __noinline__ void chains_serial(u32 dir, u32 n, const Arr<SM> starts, u32 q0, u32 q1) {
+  const View<SM> c;
+#pragma unroll 1
+  for (u32 q = q0; q < q1; ++q) chain_walk<CHAIN_SERIAL>(c, g_P.lef_lef, dir, n, starts[q], 0);
+}
+
+template <bool SM>
+__device__ __noinline__ u64 secondary_dir_block(u64 rp, u32 dir, u32 n, u32 n5, u32 n3) {
   const View<SM> c;
   const KParams& P = g_P;
   const u32 T = c.T;
@@ -2705,8 +2938,9 @@ __device__ __noinline__ u64 secondary_dir_block(u64 rp, u32 dir, u32 n, u64 n5, 
   // and R[k] free, in descending i.  Each start pairs with its own stalled unit: at most n / 2.
   const auto starts = c.tmp;
   const i64 itop = (i64)(n - min(n3, n3 - 1)) - 1;
-  const u32 k0 = (u32)max((u64)1, n5);
+  const u32 k0 = max(1u, n5);
   const u32 items = dir ? (itop > 0 ? (u32)itop : 0u) : (n > k0 ? n - k0 : 0u);
+  if (threadIdx.x == 0) g_bt.total = 0;
   u32 nst = 0, buf = 0;
 #pragma unroll 1
   for (u32 base = 0; base < items; base += 2 * T) {
@@ -2734,11 +2968,16 @@ __device__ __noinline__ u64 secondary_dir_block(u64 rp, u32 dir, u32 n, u64 n5, 
   if (nst == 0) return rp;
   const auto lens = c.tmp + nst;  // trials of each chain if all succeed, then its first draw's offset
 #pragma unroll 1
-  for (u32 q = threadIdx.x; q < nst; q += T) lens[q] = chain_walk<CHAIN_COUNT>(c, P.lef_lef, dir, n, starts[q], 0);
+  for (u32 q = threadIdx.x; q < nst; q += T) {
+    const u32 L = chain_walk<CHAIN_COUNT>(c, P.lef_lef, dir, n, starts[q], 0);
+    lens[q] = L;
+    atomicAdd(&g_bt.total, L);
+  }
   wsync(c.T);
   const bool draws = trial_needs_draw(P.lef_lef);
   const u64 thr = P.lef_lef.thr;
-  const u32 lim = min(c.lim, 32 * TRIAL_WORDS - 32);  // draws of one round at most
+  // draws of one round at most
+  const u32 lim = min(min(c.lim, 32 * TRIAL_WORDS - 32), (g_bt.total + 31) & ~31u);
   u32 q0 = 0;
 #pragma unroll 1
   while (q0 < nst) {
@@ -2746,7 +2985,7 @@ __device__ __noinline__ u64 secondary_dir_block(u64 rp, u32 dir, u32 n, u64 n5, 
     if (draws) {
       rng_ensure(rp, lim);
 #pragma unroll 1
-      for (u32 k = threadIdx.x; k < lim; k += T) {
+      for (u32 k = threadIdx.x; k < lim; k += T) {  // whole warps: lim is a multiple of 32
         const unsigned m = __ballot_sync(FULL, ring_at(c.rmask, rp + k) <= thr);
         if (ln() == 0) g_bt.trial[k >> 5] = m;
       }
@@ -2802,10 +3041,7 @@ __device__ __noinline__ u64 secondary_dir_block(u64 rp, u32 dir, u32 n, u64 n5, 
       // 32 chains that might outrun the ring: walk them one by one
       prof_add(PF_CHAIN_SERIAL, 1);
       const u32 qe = min(q0 + 32, nst);
-      if (threadIdx.x == 0) {
-#pragma unroll 1
-        for (u32 q = q0; q < qe; ++q) chain_walk<CHAIN_SERIAL>(c, P.lef_lef, dir, n, starts[q], 0);
-      }
+      if (threadIdx.x == 0) chains_serial<SM>(dir, n, starts, q0, qe);
       wsync(c.T);
       rp = g_sc.rpos;
       q0 = qe;
@@ -2827,12 +3063,12 @@ __device__ __noinline__ u64 secondary_dir_block(u64 rp, u32 dir, u32 n, u64 n5, 
 // adjacent in rank order (the unit before a rev candidate, after a fwd candidate, is stalled),
 // so each is an independent swap of two neighbours.
 template <bool SM>
-__device__ __noinline__ bool fix_secondary_block(u32 n, u64 n5, u64 n3) {
+__device__ __noinline__ bool fix_secondary_block(u32 n, u32 n5, u32 n3) {
   const View<SM> c;
   const KParams& P = g_P;
   const u32 T = c.T;
-  const u32 k0 = (u32)max((u64)1, n5);
-  const u32 naf = (u32)(n - min(n3, n3 - 1));
+  const u32 k0 = max(1u, n5);
+  const u32 naf = (n - min(n3, n3 - 1));
   if (threadIdx.x == 0) g_bt.nr = g_bt.nf = 0;
   wsync(c.T);
   // candidate ranks: rev [k0, n), fwd [0, naf - 1); rev list from the front of tmp, fwd list from its end
@@ -2874,7 +3110,6 @@ __device__ __noinline__ u64 process_collisions(u64 rp, u32 n, bool fix,
                                                bool sorted_ranks = false) {
   const View<SM> c;
   const KParams& P = g_P;
-  u64 t0 = clock64();
   const bool serial = (P.debug_flags & DBG_SERIAL_COLLISIONS) || !(sorted_ranks || (ranked_sorted<SM>(n) && words_plain<SM>(n)));
   if (threadIdx.x == 0) {
     u64 n5, n3;
@@ -2883,9 +3118,8 @@ __device__ __noinline__ u64 process_collisions(u64 rp, u32 n, bool fix,
     g_sc.n3 = n3;
   }
   wsync(c.T);
-  u64 t1 = clock64();
-  prof_add(PF_BOUNDARIES, t1 - t0);
-  const u64 n5 = g_sc.n5, n3 = g_sc.n3;
+  prof_mark(PF_BOUNDARIES);
+  const u32 n5 = (u32)g_sc.n5, n3 = (u32)g_sc.n3;
   if (serial) {
     if (threadIdx.x == 0) {
       detect_lef_bar_serial(g_c, P, n, n5, n3);
@@ -2895,21 +3129,17 @@ __device__ __noinline__ u64 process_collisions(u64 rp, u32 n, bool fix,
     rp = g_sc.rpos;
   } else {
     rp = detect_lef_bar_block<SM>(rp, n, n5, n3);
-    t0 = clock64();
-    prof_add(PF_LEF_BAR, t0 - t1);
-    t1 = t0;
+    prof_mark(PF_LEF_BAR);
     rp = detect_primary_block<SM>(rp, n, n5, n3);
   }
-  t0 = clock64();
-  prof_add(PF_PRIMARY, t0 - t1);
+  prof_mark(PF_PRIMARY);
   if (sorted_ranks) {
     correct_moves<SM>(n);
   } else {
     correct_lef_bar<SM>(n);
     correct_primary<SM>(n);
   }
-  t1 = clock64();
-  prof_add(PF_CORRECT, t1 - t0);
+  prof_mark(PF_CORRECT);
   if (serial) {
     if (threadIdx.x == 0) process_secondary_serial(g_c, P, n, n5, n3);
     wsync(c.T);
@@ -2919,8 +3149,7 @@ __device__ __noinline__ u64 process_collisions(u64 rp, u32 n, bool fix,
     rp = secondary_dir_block<SM>(rp, 0, n, n5, n3);
     rp = secondary_dir_block<SM>(rp, 1, n, n5, n3);
   }
-  t0 = clock64();
-  prof_add(PF_SECONDARY, t0 - t1);
+  prof_mark(PF_SECONDARY);
   if (fix) {
     if (serial || !fix_secondary_block<SM>(n, n5, n3)) {
       prof_add(PF_FIX_FALLBACK, 1);
@@ -2928,7 +3157,7 @@ __device__ __noinline__ u64 process_collisions(u64 rp, u32 n, bool fix,
       wsync(c.T);
     }
   }
-  prof_add(PF_FIX, clock64() - t0);
+  prof_mark(PF_FIX);
   return rp;
 }
 
@@ -2960,43 +3189,35 @@ __device__ __noinline__ u64 release_lefs(u64 rp, u32 n, bool completed, bool mov
   const u32 T = c.T;
   u32 buf = 0;
 #pragma unroll 1
-  for (u32 base = 0; base < n; base += 2 * T) {
-    rng_ensure(rp, 2 * T);
-    u64 thr[2];
-    bool need[2];
-#pragma unroll
-    for (u32 h = 0; h < 2; ++h) {
-      const u32 i = base + h * T + threadIdx.x;
-      need[h] = false;
-      thr[h] = 0;
-      if (i < n && c.bep[i] != UNBOUND) {
-        const u32 r = c.rc[i], f = c.fc[i];
-        u32 nh = 0;
-        if (cw_occurred_as(r, EV_LEF_BAR) && (bar_flags(c.bpf, cw_idx(r)) & BF_DIR_MASK) == MGPU_DIR_REV) ++nh;
-        if (cw_occurred_as(f, EV_LEF_BAR) && (bar_flags(c.bpf, cw_idx(f)) & BF_DIR_MASK) == MGPU_DIR_FWD) ++nh;
-        const Trial& tr = P.release[completed ? 1 : 0][nh];
-        need[h] = tr.draws;
-        thr[h] = tr.thr;
-      }
+  for (u32 base = 0; base < n; base += T) {
+    rng_ensure(rp, T);
+    const u32 i = base + threadIdx.x;
+    const bool bound = i < n && c.bep[i] != UNBOUND;
+    u64 thr = 0;
+    bool need = false;
+    if (bound) {
+      const u32 r = c.rc[i], f = c.fc[i];
+      u32 nh = 0;
+      if (cw_occurred_as(r, EV_LEF_BAR) && (bar_flags(c.bpf, cw_idx(r)) & BF_DIR_MASK) == MGPU_DIR_REV) ++nh;
+      if (cw_occurred_as(f, EV_LEF_BAR) && (bar_flags(c.bpf, cw_idx(f)) & BF_DIR_MASK) == MGPU_DIR_FWD) ++nh;
+      const Trial& tr = P.release[completed ? 1 : 0][nh];
+      need = tr.draws;
+      thr = tr.thr;
     }
-    const Scan2 s = scan2<SM>(buf, need[0], need[1]);
+    const Scan1 s = scan1<SM>(T, buf, need);
     rng_publish(rp);
     buf ^= 1;
-#pragma unroll
-    for (u32 h = 0; h < 2; ++h) {
-      const u32 i = base + h * T + threadIdx.x;
-      const bool rel = need[h] && ring_at(c.rmask, rp + (h ? s.off1 : s.off0)) <= thr[h];
-      if (rel) {
-        c.rev[i] = UNBOUND;
-        c.fwd[i] = UNBOUND;
-        c.bep[i] = UNBOUND;
-      } else if (move && i < n && c.bep[i] != UNBOUND) {
-        c.rev[i] -= c.rm[i];
-        c.fwd[i] += c.fm[i];
-      }
-      const unsigned m = __ballot_sync(FULL, rel);
-      if (m && ln() == 0) atomicAdd(&g_bt.released, (u32)__popc(m));
+    const bool rel = need && ring_at(c.rmask, rp + s.off) <= thr;
+    if (rel) {
+      c.rev[i] = UNBOUND;
+      c.fwd[i] = UNBOUND;
+      c.bep[i] = UNBOUND;
+    } else if (move && bound) {
+      c.rev[i] -= c.rm[i];
+      c.fwd[i] += c.fm[i];
     }
+    const unsigned m = __ballot_sync(FULL, rel);
+    if (m && ln() == 0) atomicAdd(&g_bt.released, (u32)__popc(m));
     rp += s.total;
   }
   wsync(c.T);
@@ -3238,6 +3459,14 @@ __device__ __forceinline__ bool band_increment(const C& c, const KParams& P, u64
   return false;
 }
 
+// genextreme noise of one draw (register_contacts.cpp:48-64)
+__device__ __noinline__ double gev_noise(u64 u) {
+  const KParams& P = g_P;
+  const double l = -log(canonical_of(u));
+  if (P.gev_xi == 0.0) return (P.gev_mu - P.gev_sigma) * log(l);
+  return P.gev_mu + (P.gev_sigma * (1.0 - pow(l, P.gev_xi))) / P.gev_xi;
+}
+
 // One contact attempt read from draws at `at` (register_contacts.cpp:129-198).  Returns the
 // draws it takes; *ok tells whether it registers a contact; *regular is false when the attempt
 // hit a bucket rejection (exact handling needs the serial path).
@@ -3251,7 +3480,7 @@ __device__ __forceinline__ u32 contact_attempt(u64 at, bool tad,
   *regular = true;
   const u64 start = (u64)P.wstart + 1, end = (u64)P.wend - 1;
   u32 used = 0;
-  const u64 li = ring_at(c.rmask, at + used++) / lbucket;
+  const u64 li = div64(ring_at(c.rmask, at + used++), lbucket);
   if (li > na - 1) {
     *regular = false;
     return used;
@@ -3261,23 +3490,20 @@ __device__ __forceinline__ u32 contact_attempt(u64 at, bool tad,
   if (!(rp > start && rp < end && fp > start && fp < end)) return used;
   double n1 = 0.0, n2 = 0.0;
   if (P.noisify) {
-    const double u1 = canonical_of(ring_at(c.rmask, at + used++));
-    n1 = (P.gev_xi == 0.0) ? (P.gev_mu - P.gev_sigma) * log(-log(u1))
-                           : P.gev_mu + (P.gev_sigma * (1.0 - pow(-log(u1), P.gev_xi))) / P.gev_xi;
+    n1 = gev_noise(ring_at(c.rmask, at + used++));
   }
   const double a = (double)rp - n1;
   if (P.noisify) {
-    const double u2 = canonical_of(ring_at(c.rmask, at + used++));
-    n2 = (P.gev_xi == 0.0) ? (P.gev_mu - P.gev_sigma) * log(-log(u2))
-                           : P.gev_mu + (P.gev_sigma * (1.0 - pow(-log(u2), P.gev_xi))) / P.gev_xi;
+    n2 = gev_noise(ring_at(c.rmask, at + used++));
   }
   const double b = (double)fp + n2;
   const double p1 = fmin(a, b), p2 = fmax(a, b);
   const double ds = (double)start, de = (double)end;
   if (!(p1 >= ds && p2 >= ds && p1 < de && p2 < de)) return used;
+  // positions are below 2^32
   if (!tad) {
-    *row = ((u64)p1 - start) / P.bin;
-    *col = ((u64)p2 - start) / P.bin;
+    *row = ((u32)(u64)p1 - (u32)start) / P.bin;
+    *col = ((u32)(u64)p2 - (u32)start) / P.bin;
     *ok = true;
     return used;
   }
@@ -3285,14 +3511,13 @@ __device__ __forceinline__ u32 contact_attempt(u64 at, bool tad,
   const u64 range = q2 - q1;
   u64 p11 = q1, p22 = q1;
   if (range != 0) {
-    u64 bucket = ~0ull / (range + 1);
-    if (~0ull % (range + 1) == range) ++bucket;
-    const u64 r1 = ring_at(c.rmask, at + used++) / bucket;
+    const u64 bucket = bucket_of(range);
+    const u64 r1 = div64(ring_at(c.rmask, at + used++), bucket);
     if (r1 > range) {
       *regular = false;
       return used;
     }
-    const u64 r2 = ring_at(c.rmask, at + used++) / bucket;
+    const u64 r2 = div64(ring_at(c.rmask, at + used++), bucket);
     if (r2 > range) {
       *regular = false;
       return used;
@@ -3300,8 +3525,8 @@ __device__ __forceinline__ u32 contact_attempt(u64 at, bool tad,
     p11 = q1 + r1;
     p22 = q1 + r2;
   }
-  *row = (p11 - start) / P.bin;
-  *col = (p22 - start) / P.bin;
+  *row = ((u32)p11 - (u32)start) / P.bin;
+  *col = ((u32)p22 - (u32)start) / P.bin;
   *ok = true;
   return used;
 }
@@ -3372,12 +3597,7 @@ __device__ __noinline__ u64 sample_contacts(u64 rp, u64 target) {
   rp = g_sc.rpos;
   const u64 n_loop = g_sc.bc0;
   const u64 na = g_sc.num_active;
-  u64 lbucket;
-  {
-    const u64 range = na - 1;
-    lbucket = ~0ull / (range + 1);
-    if (~0ull % (range + 1) == range) ++lbucket;
-  }
+  const u64 lbucket = bucket_of(na - 1);
   u64 budget = 1000 * num + 1000000;  // attempts before giving up (see DEV_ERR_NO_BOUND_LEF)
   u32 missed = 0;
   const int passes = P.track_occ ? 3 : 2;  // loop, TAD, then the 1D occupancy
@@ -3754,20 +3974,17 @@ __device__ __noinline__ void run_cell(u64 target, u64 target_epochs, const DevTr
     const bool go = P.contact_mode ? (g_sc.num_contacts < target)
                                    : (g_sc.epoch - g_sc.num_burnin_epochs < target_epochs);
     if (!go) break;
-    const u64 te0 = clock64();
+    prof_mark(PF_COUNT);
     if (!g_sc.burnin_completed) rp = run_burnin<SM>(rp);
-    u64 ta = clock64();
-    prof_add(PF_BURNIN, ta - te0);
+    prof_mark(PF_BURNIN);
     const u32 n = (u32)g_sc.num_active;
     const u32 epoch = (u32)g_sc.epoch;
     const bool completed = g_sc.burnin_completed != 0;
     if (threadIdx.x == 0) g_sc.lef_epochs += n;
     rp = bind_lefs<SM>(rp, n, epoch, 0, nullptr);
-    u64 tb = clock64();
-    prof_add(PF_BIND, tb - ta);
+    prof_mark(PF_BIND);
     rank_lefs<SM>(n, epoch, epoch != 0);
-    ta = clock64();
-    prof_add(PF_RANK, ta - tb);
+    prof_mark(PF_RANK);
     if (completed) {
       if (P.debug_flags & DBG_SERIAL_CONTACTS) {
         if (threadIdx.x == 0) sample_contacts_serial(g_c, P, target);
@@ -3776,11 +3993,8 @@ __device__ __noinline__ void run_cell(u64 target, u64 target_epochs, const DevTr
       } else {
         rp = sample_contacts<SM>(rp, target);
       }
-      tb = clock64();
-      prof_add(PF_CONTACTS, tb - ta);
-      ta = tb;
+        prof_mark(PF_CONTACTS);
       if (target != 0 && g_sc.num_contacts >= target) {
-        prof_add(PF_TOTAL, clock64() - te0);
         break;
       }
       if (g_sc.status != DEV_OK) break;
@@ -3788,31 +4002,25 @@ __device__ __noinline__ void run_cell(u64 target, u64 target_epochs, const DevTr
     }
     rp = gen_moves_dir<SM>(rp, c.rm, n, P.rev_move[completed]);
     rp = gen_moves_dir<SM>(rp, c.fm, n, P.fwd_move[completed]);
-    tb = clock64();
-    prof_add(PF_MOVES, tb - ta);
+    prof_mark(PF_MOVES);
     place_moves<SM>(n, true);
-    ta = clock64();
-    prof_add(PF_ADJUST, ta - tb);
+    prof_mark(PF_ADJUST);
     rp = barriers_next<SM>(rp);
-    tb = clock64();
-    prof_add(PF_BARRIERS, tb - ta);
+    prof_mark(PF_BARRIERS);
     rp = process_collisions<SM>(rp, n, true, true);
-    ta = clock64();
     if (P.log_state) {  // the record is taken between the two
       extrude<SM>(n);
       log_model_state<SM>(n, cell);
       wsync(c.T);
     }
     rp = release_lefs<SM>(rp, n, completed, !P.log_state);
-    tb = clock64();
-    prof_add(PF_EXTRUDE_RELEASE, tb - ta);
+    prof_mark(PF_EXTRUDE_RELEASE);
     if (trace) trace_record<SM>(*trace, g_sc.epoch);
     const bool failed = g_sc.status != DEV_OK;
     wsync(c.T);
     if (threadIdx.x == 0) g_sc.epoch++;
     wsync(c.T);
-    prof_add(PF_TRACE, clock64() - tb);
-    prof_add(PF_TOTAL, clock64() - te0);
+    prof_mark(PF_TRACE);
     prof_add(PF_EPOCHS, 1);
     if (failed) break;
   }

@@ -38,3 +38,12 @@ def test_barrier_counts(nbarriers):
     cfg = genome.genome_config(num_cells=4, skip_burnin=1, seed=nbarriers)
     chrom, bars = small_genome(cfg, 10_000_000, nbarriers, seed=nbarriers, occupancy="beta")
     compare_cell(cfg, chrom, bars, nl=260, target=1500)
+
+
+@pytest.mark.parametrize("nl", [700, 2500])
+def test_ties_at_the_chromosome_ends(nl):
+    """Units bound in the first epoch pile up at the ends with equal positions and epochs: the ranking's
+    order of full ties is the reference's."""
+    cfg = genome.genome_config(num_cells=4, skip_burnin=1, seed=nl, avg_lef_processivity=4_000_000)
+    chrom, bars = small_genome(cfg, nl * 8000, 20, seed=nl, occupancy="beta")
+    compare_cell(cfg, chrom, bars, nl=nl, target=60 * (nl // 6))
