@@ -137,6 +137,7 @@ struct BlockTmp {
   u32 used, qend, nr, nf, released, missed, flag, total;
   u64 sum;
   ulonglong2 zt[128];   // normal ziggurat per layer: {draws below this are accepted, width * 2^60}
+  ulonglong2 ln[128];   // logarithm by table: {1 / c * 2^64, ln c * 2^63} for the 128 parts c of [1, 2)
   float2 zy[128];       // and the density at its lower and upper edge: {y_i, y_{i+1} - y_i}
 };
 
@@ -3467,6 +3468,46 @@ __device__ __noinline__ double gev_noise(u64 u) {
   return P.gev_mu + (P.gev_sigma * (1.0 - pow(l, P.gev_xi))) / P.gev_xi;
 }
 
+// The same in fixed point, 2^-25 bp: n = base + scale * L * (e^y - 1) / y with L = ln(-ln u) and
+// y = xi * L.  The positions that follow from it are only needed as whole base pairs, so the caller
+// takes gev_noise when the fixed-point value is too close to one to tell.  CUDA's double log and pow
+// take some 250 instructions on the FP64 pipe (1/64 of the FP32 rate); this takes about 110 integer
+// ones.  Logarithms: x = c (1 + r) with |r| < 2^-8 from a table of 128 parts, and the series of
+// ln(1 + r) to r^5; absolute error below 2^-44.  Error of n: |scale| * 2^-44 / -ln u, and the caller's
+// margin is 2^-13 for |scale| < 2^15 and -ln u >= 2^-15.  Returns false outside that range.
+__device__ __forceinline__ i64 ln_mantissa(u64 m) {  // m = x * 2^63, x in [1, 2): ln x * 2^63
+  const ulonglong2 e = g_bt.ln[(m >> 56) & 127u];
+  const i64 r = (i64)(__umul64hi(m, e.x) - (1ull << 63));
+  const i32 r39 = (i32)(r >> 24), r32 = r39 >> 7;
+  const i32 a = (1 << 30) - __mulhi(r32, 858993459);  // 1/4 - r/5
+  const i32 b = 1431655765 - __mulhi(r32, a);         // 1/3 - r (..)
+  const u32 q = (u32)((1 << 30) - (__mulhi(r32, b) >> 1));  // (1/2 - r (..)) * 2^31
+  const u32 r2 = (u32)((u64)((i64)r39 * r39) >> 32);  // r^2 * 2^46
+  return (i64)e.y + r - (i64)(((u64)r2 * q) >> 14);
+}
+
+__device__ __noinline__ bool gev_fixed(u64 u, i64* n) {
+  const KParams& P = g_P;
+  const u64 LN2_57 = 0x162E42FEFA39EF3ull;  // ln 2 * 2^57
+  const u32 lz = u ? (u32)__clzll((i64)u) : 63u;
+  const i64 e = (i64)((u64)(1 + lz) * LN2_57) - (ln_mantissa(u << lz) >> 6);
+  if (u == 0 || e < (1ll << 42)) return false;
+  const u32 lz2 = (u32)__clzll(e);
+  const i64 L = (6 - (i64)lz2) * (i64)LN2_57 + (ln_mantissa((u64)e << lz2) >> 6);
+  const bool neg = L < 0;
+  const u64 aL = (u64)(neg ? -L : L);
+  const u64 t = __umul64hi(aL, P.gev_scale);  // |scale L| * 2^25
+  const u64 y = __umul64hi(aL, P.gev_xiq);    // |y| * 2^57
+  const i64 half = (i64)(__umul64hi(t << 20, y) >> 14);  // |scale L| |y| / 2
+  const bool yneg = neg != (P.gev_xi < 0.0f);
+  const float yf = (float)(u32)(y >> 26) * 0x1p-31f, ys = yneg ? -yf : yf;
+  const float tf = (float)(u32)(t >> 12) * 0x1p-13f;
+  const float more = tf * (yf * yf * (1.0f / 6.0f + ys * (1.0f / 24.0f + ys * (1.0f / 120.0f))));
+  const i64 mag = (i64)t + (yneg ? -half : half) + (i64)(i32)(more * 0x1p25f);
+  *n = P.gev_base + (neg != (P.gev_scale_neg != 0) ? -mag : mag);
+  return true;
+}
+
 // One contact attempt read from draws at `at` (register_contacts.cpp:129-198).  Returns the
 // draws it takes; *ok tells whether it registers a contact; *regular is false when the attempt
 // hit a bucket rejection (exact handling needs the serial path).
@@ -3488,22 +3529,31 @@ __device__ __forceinline__ u32 contact_attempt(u64 at, bool tad,
   if (c.bep[li] == UNBOUND) return used;
   const u64 rp = pos64(c.rev[li]), fp = pos64(c.fwd[li]);
   if (!(rp > start && rp < end && fp > start && fp < end)) return used;
-  double n1 = 0.0, n2 = 0.0;
+  // whole base pairs of the two noised positions
+  i64 ia = (i64)rp, ib = (i64)fp;
   if (P.noisify) {
-    n1 = gev_noise(ring_at(c.rmask, at + used++));
+    const u64 u1 = ring_at(c.rmask, at + used), u2 = ring_at(c.rmask, at + used + 1);
+    used += 2;
+    i64 n1, n2;
+    bool exact = !P.gev_fixed || !gev_fixed(u1, &n1) || !gev_fixed(u2, &n2);
+    if (!exact) {
+      const i64 a = ((i64)rp << 25) - n1, d = ((i64)fp << 25) + n2;
+      const u32 near = 1u << 12, one = 1u << 25;  // fractions within 2^-13 of a whole number
+      exact = (((u32)a + near) & (one - 1)) <= 2 * near || (((u32)d + near) & (one - 1)) <= 2 * near;
+      ia = a >> 25;
+      ib = d >> 25;
+    }
+    if (exact) {
+      // positions outside [0, 2^32) fail the bounds below in any case
+      ia = (i64)floor(fmin(fmax((double)rp - gev_noise(u1), -1.0), 4294967296.0));
+      ib = (i64)floor(fmin(fmax((double)fp + gev_noise(u2), -1.0), 4294967296.0));
+    }
   }
-  const double a = (double)rp - n1;
-  if (P.noisify) {
-    n2 = gev_noise(ring_at(c.rmask, at + used++));
-  }
-  const double b = (double)fp + n2;
-  const double p1 = fmin(a, b), p2 = fmax(a, b);
-  const double ds = (double)start, de = (double)end;
-  if (!(p1 >= ds && p2 >= ds && p1 < de && p2 < de)) return used;
-  // positions are below 2^32
+  const i64 p1 = min(ia, ib), p2 = max(ia, ib);
+  if (!(p1 >= (i64)start && p2 < (i64)end)) return used;
   if (!tad) {
-    *row = ((u32)(u64)p1 - (u32)start) / P.bin;
-    *col = ((u32)(u64)p2 - (u32)start) / P.bin;
+    *row = ((u32)p1 - (u32)start) / P.bin;
+    *col = ((u32)p2 - (u32)start) / P.bin;
     *ok = true;
     return used;
   }
@@ -3847,6 +3897,7 @@ __device__ __forceinline__ void load_layers(const ulonglong2* jt) {
 #pragma unroll 1
   for (u32 i = threadIdx.x; i < 128; i += blockDim.x) {
     g_bt.zt[i] = jt[4 * JUMP_TABLE_ENTRIES + i];
+    g_bt.ln[i] = jt[4 * JUMP_TABLE_ENTRIES + NORMAL_LAYERS + i];
     const double y0 = mgpu_zig_normal_y[i], y1 = mgpu_zig_normal_y[i + 1];
     g_bt.zy[i] = make_float2((float)y0, (float)(y1 - y0));
   }

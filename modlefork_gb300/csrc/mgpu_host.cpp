@@ -514,9 +514,17 @@ static void build_layer(int i, uint64_t* e) {
 }
 
 static std::vector<uint64_t> build_tables() {
-  std::vector<uint64_t> t(MAX_PRODUCERS * JUMP_TABLE_ENTRIES * 4 + NORMAL_LAYERS * 2, 0);
+  std::vector<uint64_t> t(MAX_PRODUCERS * JUMP_TABLE_ENTRIES * 4 + (NORMAL_LAYERS + LOG_PARTS) * 2, 0);
   for (u32 p = 1; p <= MAX_PRODUCERS; ++p) build_jump_table(jump_distance(p), &t[(p - 1) * JUMP_TABLE_ENTRIES * 4]);
   for (u32 i = 0; i < NORMAL_LAYERS; ++i) build_layer((int)i, &t[MAX_PRODUCERS * JUMP_TABLE_ENTRIES * 4 + 2 * i]);
+  for (u32 i = 0; i < LOG_PARTS; ++i) {
+    // 1 / c as a 32-bit fraction, so that 1 + r = x / c is formed exactly enough by one product, and
+    // the logarithm of that very fraction's reciprocal
+    const uint64_t inv = (uint64_t)std::llround(4294967296.0 / (1.0 + (i + 0.5) / LOG_PARTS));
+    uint64_t* e = &t[MAX_PRODUCERS * JUMP_TABLE_ENTRIES * 4 + 2 * (NORMAL_LAYERS + i)];
+    e[0] = inv << 32;
+    e[1] = (uint64_t)(-logl((long double)inv / 4294967296.0L) * 9223372036854775808.0L);
+  }
   return t;
 }
 
@@ -765,7 +773,7 @@ static MoveSpec move_spec(double mean, double sd) {
 }
 
 // Worker warps of a cell: a sweep over its LEFs takes two to four rounds of the block.
-static u32 workers_for(uint64_t nlefs) { return nlefs <= 256 ? 4 : (nlefs <= 1024 ? 8 : 16); }
+static u32 workers_for(uint64_t nlefs) { return nlefs <= 256 ? 8 : 16; }
 
 static int make_kparams(const mgpu_ctx* ctx, const ChromEntry& ch, uint64_t nlefs, KParams* P,
                         uint64_t budget_override = 0, u32 workers = 0) {
@@ -827,6 +835,18 @@ static int make_kparams(const mgpu_ctx* ctx, const ChromEntry& ch, uint64_t nlef
   P->gev_mu = c.genextreme_mu;
   P->gev_sigma = c.genextreme_sigma;
   P->gev_xi = c.genextreme_xi;
+  // fixed-point noise for the parameters its error bound covers (xi == 0 has a formula of its own)
+  {
+    const double scale = c.genextreme_xi == 0.0 ? c.genextreme_mu - c.genextreme_sigma : -c.genextreme_sigma;
+    const double base = c.genextreme_xi == 0.0 ? 0.0 : c.genextreme_mu;
+    P->gev_fixed = std::fabs(scale) < 32768.0 && std::fabs(base) < 1e9 && std::fabs(c.genextreme_xi) <= 0.0014;
+    if (P->gev_fixed) {
+      P->gev_base = (int64_t)std::llround(base * 33554432.0);
+      P->gev_scale = (uint64_t)(std::fabs(scale) * 4294967296.0);
+      P->gev_scale_neg = scale < 0.0;
+      P->gev_xiq = (uint64_t)(std::fabs(c.genextreme_xi) * 18446744073709551616.0);
+    }
+  }
   {
     const double p = (0.5 < P->p_loop) ? (1 - P->p_loop) : P->p_loop;
     P->bin_q_n = std::pow((1 - p), (double)(int64_t)P->spe);

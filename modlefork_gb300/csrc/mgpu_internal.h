@@ -16,6 +16,7 @@ namespace mgpu {
 typedef uint32_t u32;
 typedef uint64_t u64;
 typedef int64_t i64;
+typedef int32_t i32;
 
 // Unbound unit / LEF sentinel for the 32-bit device encodings.
 constexpr u32 UNBOUND = 0xFFFFFFFFu;
@@ -28,6 +29,7 @@ constexpr u32 MAX_WORKERS = 16, MAX_PRODUCERS = 2;
 constexpr int RNG_S = 32;
 constexpr int JUMP_TABLE_ENTRIES = 64 * 16;  // 4-bit chunks of the 256-bit state, one table per producer count
 constexpr u32 NORMAL_LAYERS = 128;           // fixed-point ziggurat layers, after the jump tables
+constexpr u32 LOG_PARTS = 128;               // logarithm table, after the layers
 MGPU_HD inline u32 producer_warps(u32 workers) { return workers > 8 ? 2 : 1; }
 MGPU_HD inline u32 block_threads(u32 workers) { return 32 * (workers + producer_warps(workers)); }
 constexpr int MAX_BLOCK_THREADS = 32 * (MAX_WORKERS + MAX_PRODUCERS);
@@ -111,6 +113,10 @@ struct KParams {
   u32 noisify;
   double p_loop;         // 1 / (ratio + 1)
   double gev_mu, gev_sigma, gev_xi;
+  // the noise in fixed point (gev_fixed): base * 2^25, |scale| * 2^32, |xi| * 2^64
+  i64 gev_base;
+  u64 gev_scale, gev_xiq;
+  u32 gev_scale_neg, gev_fixed;
   // binomial(spe, p_loop) constants computed on the host
   double bin_q_n;
   // binding positions: uniform_int[start, end - 1]
