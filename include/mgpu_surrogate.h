@@ -127,6 +127,11 @@ int msur_adam(float* p, const float* g, float* m, float* v, uint64_t n, float lr
               float wd, int step, float gscale, void* p_bf16, void* stream);
 /* wt[c][t][n] = w[n][taps - 1 - t][c]: the weights of the data gradient. */
 int msur_weight_transpose(const void* w, int N, int taps, int C, void* wt, void* stream);
+/* msur_weight_transpose of `count` convolutions (at most MSUR_MAX_TRANSPOSES) in one launch; the arrays are
+ * host memory.  Channel counts must be multiples of 8 and buffers 16-byte aligned. */
+#define MSUR_MAX_TRANSPOSES 64
+int msur_weight_transpose_list(int count, const void* const* w, const int* N, const int* taps, const int* C,
+                               void* const* wt, void* stream);
 /* Network input: x[b, l, 0:4] = track[b][0:4][l] (occupancy, + motifs, - motifs, LEF density),
  * x[b, l, 4:8] = params[b][0:4], the other C - 8 channels zero. */
 int msur_assemble_input(const float* track, const float* params, int B, int L, int C, void* x, void* stream);

@@ -566,6 +566,12 @@ __global__ void __launch_bounds__(THREADS, 1) conv_fwd_persistent_kernel(const _
 // Weight gradient: dW[n][t][c] += sum_{b,l} dZ[b, l, n] X[b, l + t - pad, c], split over the
 // (b, 64-position block) range; M = output channels (128 per tile), N = input channels (BN per
 // tile), one TMEM accumulator of BN columns per tap; both operands M/N-major.
+//
+// The splits' partial sums meet in dw.  A thread holds one output channel's row of the accumulators;
+// adding it word by word (32 rows per warp and instruction) took longer than the products: 113 of
+// 133 us for 16 x 999 positions, 256 to 256 channels.  So the rows go to the operand stages, free by
+// then (a row is padded by 16 bytes: conflict-free 16-byte stores), and each thread adds its row with
+// one bulk reduction per tap (cp.reduce.async.bulk, up to 512 contiguous bytes).
 // ---------------------------------------------------------------------------------------
 struct WgradArgs {
   CUtensorMap tm_dz;  // [B][L][Cout]: dims {Cout, L, B}, box {64, 64, 1}
@@ -574,9 +580,22 @@ struct WgradArgs {
   int lblocks;        // 64-position blocks per sequence
   int total;          // B * lblocks
   int per_split;      // blocks per split
+  int bulk;           // dw is 16-byte aligned: bulk reductions
   float* dw;          // [Cout][taps][Cin], accumulated into
   unsigned* err;
 };
+
+// Shared memory of a weight-gradient kernel before its barriers: the operand stages, later the
+// padded accumulator rows.
+template <int BN, int NT>
+__host__ __device__ constexpr int wgrad_row_bytes() {
+  return NT * BN * 4 + 16;
+}
+template <int BN, int NT, int STAGES>
+__host__ __device__ constexpr int wgrad_region() {
+  const int stages = STAGES * (2 * 8192 + NT * (BN / 64) * 8192), rows = BM * wgrad_row_bytes<BN, NT>();
+  return stages > rows ? stages : (rows + 1023) / 1024 * 1024;
+}
 
 template <int BN, int NT, int STAGES>
 __global__ void __launch_bounds__(THREADS, 1) wgrad_kernel(const __grid_constant__ WgradArgs a) {
@@ -588,7 +607,7 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_kernel(const __grid_constant
   static_assert(NT * BN <= 512, "accumulators exceed tensor memory");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + wgrad_region<BN, NT, STAGES>());
   uint64_t* empty = full + STAGES;
   uint64_t* done = empty + STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
@@ -675,10 +694,29 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_kernel(const __grid_constant
           umma::tmem_ld32(tmem + (static_cast<uint32_t>(32 * q) << 16) + t * BN + c * 32, v);
           const int cc = c0 + c * 32;
           if (n >= a.Cout || cc >= a.Cin) continue;
+          if (a.bulk) {
+            float4* row = reinterpret_cast<float4*>(smem + (32 * q + lane) * wgrad_row_bytes<BN, NT>() +
+                                                    (t * BN + c * 32) * 4);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) row[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+            continue;
+          }
           float* dst = a.dw + (static_cast<size_t>(n) * a.taps + t) * a.Cin + cc;
           const int nv = min(32, a.Cin - cc);
           for (int j = 0; j < nv; ++j) atomicAdd(dst + j, v[j]);
         }
+      }
+      if (a.bulk) {
+        if (n < a.Cout) {
+          umma::fence_async_smem();  // this thread's row, read by its own reductions
+          const uint8_t* row = smem + (32 * q + lane) * wgrad_row_bytes<BN, NT>();
+          for (int t = 0; t < NT; ++t)
+            umma::bulk_reduce_add_f32(a.dw + (static_cast<size_t>(n) * a.taps + t) * a.Cin + c0, row + t * BN * 4,
+                                      4 * min(BN, a.Cin - c0));
+          umma::bulk_commit();
+          umma::bulk_wait_all();
+        }
+        __syncwarp();
       }
     }
   }
@@ -864,6 +902,66 @@ __global__ void bias_grad_kernel(const bf16* dz, size_t rows, int C, int stride,
   }
 }
 
+// A running sum as a pair of floats (see map_sums_pair_kernel).
+struct PairSum {
+  float h = 0.0f, l = 0.0f;
+  __device__ __forceinline__ void add(float x) {
+    const float t = __fadd_rn(h, x), z = __fsub_rn(t, h);
+    l = __fadd_rn(l, __fadd_rn(__fsub_rn(h, __fsub_rn(t, z)), __fsub_rn(x, z)));
+    h = t;
+  }
+  // a * b + rest, rest far smaller
+  __device__ __forceinline__ void add_product(float a, float b, float rest) {
+    const float p = __fmul_rn(a, b);
+    const float e = __fmaf_rn(a, b, -p);
+    add(p);
+    l = __fadd_rn(l, __fadd_rn(e, rest));
+  }
+  __device__ __forceinline__ double value() const { return static_cast<double>(h) + static_cast<double>(l); }
+};
+__device__ __forceinline__ void exact_difference(float a, float b, float& h, float& l) {
+  h = __fsub_rn(a, b);
+  const float z = __fsub_rn(h, a);
+  l = __fsub_rn(__fsub_rn(a, __fsub_rn(h, z)), __fadd_rn(b, z));
+}
+
+// The same eight channels (16 bytes) per thread: a block covers 64 channels and 32 rows at a time.  Reads at
+// the memory's rate (the scalar form above took 1.0 of a batch-16 gradient's 4.9 ms of kernel time).
+__global__ void __launch_bounds__(256) bias_grad_v8_kernel(const bf16* __restrict__ dz, size_t rows, int C,
+                                                           int stride, float* db) {
+  const int g = threadIdx.x & 7, y = threadIdx.x >> 3;
+  const int c = blockIdx.x * 64 + g * 8;
+  float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  if (c < C) {
+    const size_t step = static_cast<size_t>(gridDim.y) * 32;
+    size_t r = static_cast<size_t>(blockIdx.y) * 32 + y;
+    for (; r + 3 * step < rows; r += 4 * step) {
+      float t[4][8];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) ld8(dz + (r + k * step) * stride + c, t[k]);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] += t[k][e];
+    }
+    for (; r < rows; r += step) {
+      float t[8];
+      ld8(dz + r * stride + c, t);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) s[e] += t[e];
+    }
+  }
+  __shared__ float red[32][65];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) red[y][g * 8 + e] = s[e];
+  __syncthreads();
+  if (threadIdx.x < 64 && static_cast<int>(blockIdx.x * 64 + threadIdx.x) < C) {
+    float sum = 0.0f;
+    for (int k = 0; k < 32; ++k) sum += red[k][threadIdx.x];
+    atomicAdd(db + blockIdx.x * 64 + threadIdx.x, sum);
+  }
+}
+
 // Mean-squared error over n_valid channels of each row: loss += sum (p - t)^2 (FP64 per block),
 // dp[r, c] = scale * (p - t) for c < n_valid and 0 for the padded channels up to dstride.
 __global__ void mse_kernel(const float* pred, int pstride, const float* target, int tstride, size_t rows, int n_valid,
@@ -892,6 +990,65 @@ __global__ void mse_kernel(const float* pred, int pstride, const float* target, 
   }
 }
 
+// Four channels per thread (counts and strides multiples of 4, aligned buffers), the squares summed in pairs of
+// floats (PairSum) per 64 values and then in FP64.  I: 32-bit indexes where they reach.
+template <typename I>
+__global__ void __launch_bounds__(256) mse_v4_kernel(const float* __restrict__ pred, int pstride,
+                                                     const float* __restrict__ target, int tstride, size_t rows,
+                                                     int n_valid, bf16* dp, int dstride, float scale, double* loss) {
+  const I q = dstride / 4;  // groups of four channels per row
+  const I n = static_cast<I>(rows) * q, step = static_cast<I>(gridDim.x) * blockDim.x;
+  double acc = 0.0;
+  I i = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x;
+  while (i < n) {
+    PairSum t;
+    uint32_t mx = 0;
+    const I first = i;
+    for (int k = 0; k < 16 && i < n; ++k, i += step) {
+      const I row = i / q;
+      const int c = static_cast<int>(i - row * q) * 4;
+      const size_t r = row;
+      float d[4] = {0, 0, 0, 0};
+      if (c < n_valid) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(pred + r * pstride + c));
+        const float4 b = __ldg(reinterpret_cast<const float4*>(target + r * tstride + c));
+        d[0] = a.x - b.x, d[1] = a.y - b.y, d[2] = a.z - b.z, d[3] = a.w - b.w;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          mx = max(mx, __float_as_uint(fabsf(d[e])));
+          t.add_product(d[e], d[e], 0.0f);
+        }
+      }
+      if (dp)
+        *reinterpret_cast<uint2*>(dp + r * dstride + c) =
+            make_uint2(pack_bf16x2(scale * d[0], scale * d[1]), pack_bf16x2(scale * d[2], scale * d[3]));
+    }
+    if (mx < 0x58800000u && (mx >= 0x30800000u || mx == 0)) {
+      acc += t.value();
+    } else {  // out of the pairs' range (see map_sums_pair_kernel): FP64
+      I j = first;
+      for (int k = 0; k < 16 && j < n; ++k, j += step) {
+        const I row = j / q;
+        const int c = static_cast<int>(j - row * q) * 4;
+        const size_t r = row;
+        for (int e = 0; e < 4 && c < n_valid; ++e) {
+          const float x = pred[r * pstride + c + e] - target[r * tstride + c + e];
+          acc += static_cast<double>(x) * x;
+        }
+      }
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  __shared__ double red[8];
+  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int w = 0; w < 8; ++w) s += red[w];
+    atomicAdd(loss, s);
+  }
+}
+
 // Adam with decoupled weight decay on FP32 masters; also writes the BF16 copy the MMAs read.
 __global__ void adam_kernel(float* p, const float* g, float* m, float* v, size_t n, float lr, float b1, float b2,
                             float eps, float wd, float bc1, float bc2, float gscale, bf16* p_bf16) {
@@ -908,6 +1065,33 @@ __global__ void adam_kernel(float* p, const float* g, float* m, float* v, size_t
   }
 }
 
+// Four parameters per thread and access (n a multiple of 4, 16-byte aligned buffers).
+__global__ void __launch_bounds__(256) adam_v4_kernel(float4* p, const float4* g, float4* m, float4* v, size_t n4,
+                                                      float lr, float b1, float b2, float eps, float wd, float bc1,
+                                                      float bc2, float gscale, uint2* p_bf16) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
+    float4 p4 = p[i], m4 = m[i], v4 = v[i];
+    const float4 g4 = g[i];
+    const float* ge = &g4.x;
+    float *pe = &p4.x, *me = &m4.x, *ve = &v4.x;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float gi = ge[k] * gscale;
+      const float mi = b1 * me[k] + (1.0f - b1) * gi;
+      const float vi = b2 * ve[k] + (1.0f - b2) * gi * gi;
+      me[k] = mi;
+      ve[k] = vi;
+      float pi = pe[k] * (1.0f - lr * wd);
+      pi -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+      pe[k] = pi;
+    }
+    m[i] = m4;
+    v[i] = v4;
+    p[i] = p4;
+    if (p_bf16) p_bf16[i] = make_uint2(pack_bf16x2(p4.x, p4.y), pack_bf16x2(p4.z, p4.w));
+  }
+}
+
 // wt[c][t'][n] = w[n][taps - 1 - t'][c]: the data gradient's weights (transposed, taps reversed)
 __global__ void weight_transpose_kernel(const bf16* w, int N, int taps, int C, bf16* wt) {
   const size_t n = static_cast<size_t>(N) * taps * C;
@@ -917,6 +1101,51 @@ __global__ void weight_transpose_kernel(const bf16* w, int N, int taps, int C, b
     const int t = ct % taps;
     const int c = ct / taps;
     wt[i] = w[(static_cast<size_t>(o) * taps + (taps - 1 - t)) * C + c];
+  }
+}
+
+// The same for a list of convolutions in one launch (the data gradients' weights of a whole network after an
+// optimiser step): 64 x 64 (output channel, input channel) blocks of one tap through shared memory, so that
+// both sides move 128-byte rows.  Channel counts must be multiples of 8 and buffers 16-byte aligned.
+struct TransposeList {
+  int count;
+  int first[MSUR_MAX_TRANSPOSES + 1];  // first block of each convolution
+  const bf16* w[MSUR_MAX_TRANSPOSES];
+  bf16* wt[MSUR_MAX_TRANSPOSES];
+  int N[MSUR_MAX_TRANSPOSES], taps[MSUR_MAX_TRANSPOSES], C[MSUR_MAX_TRANSPOSES];
+};
+__global__ void __launch_bounds__(256) weight_transpose_list_kernel(const __grid_constant__ TransposeList a) {
+  int k = 0;
+  while (k + 1 < a.count && static_cast<int>(blockIdx.x) >= a.first[k + 1]) ++k;
+  const int N = a.N[k], T = a.taps[k], C = a.C[k];
+  const int nn = (N + 63) / 64, nc = (C + 63) / 64;
+  int blk = blockIdx.x - a.first[k];
+  const int c0 = (blk % nc) * 64;
+  blk /= nc;
+  const int n0 = (blk % nn) * 64, t = blk / nn;
+  __shared__ bf16 tile[64][66];
+  const int g = threadIdx.x & 7, y = threadIdx.x >> 3;  // 8 channels of one row, 32 rows at a time
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int n = n0 + y + 32 * h, c = c0 + 8 * g;
+    if (n < N && c < C) {
+      const uint4 u = *reinterpret_cast<const uint4*>(a.w[k] + (static_cast<size_t>(n) * T + (T - 1 - t)) * C + c);
+      const bf16* e = reinterpret_cast<const bf16*>(&u);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) tile[8 * g + q][y + 32 * h] = e[q];
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int c = c0 + y + 32 * h, n = n0 + 8 * g;
+    if (c < C && n < N) {
+      uint4 u;
+      bf16* e = reinterpret_cast<bf16*>(&u);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) e[q] = tile[y + 32 * h][8 * g + q];
+      *reinterpret_cast<uint4*>(a.wt[k] + (static_cast<size_t>(c) * T + t) * N + n) = u;
+    }
   }
 }
 
@@ -932,6 +1161,25 @@ __global__ void assemble_input_kernel(const float* track, const float* params, i
     if (c < 4) v = track[(static_cast<size_t>(b) * 4 + c) * L + l];
     else if (c < 8) v = params[b * 4 + (c - 4)];
     x[i] = __float2bfloat16(v);
+  }
+}
+
+// Eight channels (16 bytes) per thread: only the first group of a row reads anything.  I: 32-bit indexes where
+// they reach (a 64-bit division per 16 bytes costs more than the store).
+template <typename I>
+__global__ void __launch_bounds__(256) assemble_input_v8_kernel(const float* track, const float* params, int B, int L,
+                                                                int C, uint4* x) {
+  const I C8 = C / 8, n = static_cast<I>(B) * L * C8;
+  for (I i = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; i < n; i += static_cast<I>(gridDim.x) * blockDim.x) {
+    const I bl = i / C8;
+    uint4 u = make_uint4(0, 0, 0, 0);
+    if (i - bl * C8 == 0) {
+      const I b = bl / L, l = bl - b * L;
+      const float* t = track + static_cast<size_t>(b) * 4 * L + l;
+      const float4 q = make_float4(params[b * 4], params[b * 4 + 1], params[b * 4 + 2], params[b * 4 + 3]);
+      u = make_uint4(pack_bf16x2(t[0], t[L]), pack_bf16x2(t[2 * L], t[3 * L]), pack_bf16x2(q.x, q.y), pack_bf16x2(q.z, q.w));
+    }
+    x[i] = u;
   }
 }
 
@@ -955,23 +1203,104 @@ __global__ void band_target_kernel(const uint32_t* band, size_t ncols, int nrows
 // out[m] = {sum p', sum r', sum p'^2, sum r'^2, sum p' r', sum (p - r)^2} with p' = p - mean_p,
 // r' = r - mean_r when means (2 per map) are given, the raw values otherwise: the two passes of
 // the reference's Pearson (mean, then covariances of the deviations).
-__global__ void map_sums_kernel(const float* pred, size_t pstride_map, const float* ref, size_t rstride_map,
-                                size_t n, const double* means, double* out) {
+//
+// FP64's accuracy at the FP32 pipes' rate (FP64 runs at 1/64 of it on sm_103a: 11 FP64 operations per
+// element took 1.7 ms for 32 maps of 2.4 M values, of which the memory needs 0.1).  Each thread sums chunks of 64
+// elements in pairs of floats: differences, products and sums with their exact rounding errors (Knuth's
+// two-sum, two-product by FMA), and adds each chunk's pair to FP64 totals.  The means are split into a float
+// m and a remainder d: the deviations from m are exact pairs, and d enters the FP64 totals,
+// sum (a - d)^2 = sum a^2 - 2 d sum a + n d^2.  A pair carries 2^-47 per operation and the chunks' errors
+// average out over the map; measured against 64-bit sums the scores are as close as before (a few 1e-16).
+// A chunk with values outside [2^-30, 2^50) in size throughout, infinities or NaN is summed in FP64.
+constexpr int SUM_VECS = 16;  // float4 per thread and chunk
+template <bool VEC>
+__global__ void __launch_bounds__(256) map_sums_pair_kernel(const float* pred, size_t pstride_map, const float* ref,
+                                                            size_t rstride_map, size_t n, const double* means,
+                                                            double* out) {
   const int m = blockIdx.y;
-  const float* p = pred + m * pstride_map;
-  const float* r = ref + m * rstride_map;
+  const float* __restrict__ p = pred + m * pstride_map;
+  const float* __restrict__ r = ref + m * rstride_map;
   const double mp = means ? means[2 * m] : 0.0, mr = means ? means[2 * m + 1] : 0.0;
+  const float fp = static_cast<float>(mp), fr = static_cast<float>(mr);
+  const double dp = mp - fp, dr = mr - fr;
   double s[6] = {0, 0, 0, 0, 0, 0};
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const double a = p[i] - mp, b = r[i] - mr;
-    s[0] += a;
-    s[1] += b;
-    s[2] += a * a;
-    s[3] += b * b;
-    s[4] += a * b;
-    s[5] += (static_cast<double>(p[i]) - r[i]) * (static_cast<double>(p[i]) - r[i]);
+  double cnt = 0.0;
+  const size_t span = static_cast<size_t>(SUM_VECS) * 256 * 4;  // elements of a block's step
+  const uint32_t LO = 0x30800000u, HI = 0x58800000u;           // 2^-30, 2^50
+  const bool means_ok = __float_as_uint(fabsf(fp)) < HI && __float_as_uint(fabsf(fr)) < HI;
+  for (size_t base = blockIdx.x * span; base < n; base += gridDim.x * span) {
+    PairSum t[6];
+    uint32_t mxp = 0, mxr = 0;
+    int k = 0;
+#pragma unroll 2
+    for (int v = 0; v < SUM_VECS; ++v) {
+      const size_t i = base + (static_cast<size_t>(v) * 256 + threadIdx.x) * 4;
+      if (i >= n) break;
+      float a[4], b[4];
+      int valid = 4;
+      if constexpr (VEC) {
+        const float4 pa = __ldg(reinterpret_cast<const float4*>(p + i)), rb = __ldg(reinterpret_cast<const float4*>(r + i));
+        a[0] = pa.x, a[1] = pa.y, a[2] = pa.z, a[3] = pa.w;
+        b[0] = rb.x, b[1] = rb.y, b[2] = rb.z, b[3] = rb.w;
+      } else {
+        valid = static_cast<int>(n - i < 4 ? n - i : 4);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          a[e] = e < valid ? p[i + e] : fp;  // no deviation
+          b[e] = e < valid ? r[i + e] : fr;
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        mxp = max(mxp, __float_as_uint(fabsf(a[e])));
+        mxr = max(mxr, __float_as_uint(fabsf(b[e])));
+        float ah, al, bh, bl, h, l;
+        exact_difference(a[e], fp, ah, al);
+        exact_difference(b[e], fr, bh, bl);
+        exact_difference(a[e], b[e], h, l);
+        if (!VEC && e >= valid) h = l = 0.0f;
+        t[0].add(ah);
+        t[0].l += al;
+        t[1].add(bh);
+        t[1].l += bl;
+        t[2].add_product(ah, ah, 2.0f * ah * al);
+        t[3].add_product(bh, bh, 2.0f * bh * bl);
+        t[4].add_product(ah, bh, ah * bl + al * bh);
+        t[5].add_product(h, h, 2.0f * h * l);
+      }
+      k += valid;
+    }
+    const bool plain = means_ok && mxp < HI && mxr < HI && (mxp >= LO || (mxp == 0 && fp == 0.0f)) &&
+                       (mxr >= LO || (mxr == 0 && fr == 0.0f));
+    if (plain || k == 0) {
+      const double sa = t[0].value(), sb = t[1].value(), c = k;
+      s[0] += sa;
+      s[1] += sb;
+      s[2] += t[2].value() - 2.0 * dp * sa + c * dp * dp;
+      s[3] += t[3].value() - 2.0 * dr * sb + c * dr * dr;
+      s[4] += t[4].value() - dr * sa - dp * sb + c * dp * dr;
+      s[5] += t[5].value();
+      cnt += c;
+    } else {
+      for (int v = 0; v < SUM_VECS; ++v) {
+        for (int e = 0; e < 4; ++e) {
+          const size_t i = base + (static_cast<size_t>(v) * 256 + threadIdx.x) * 4 + e;
+          if (i >= n) break;
+          const double a = p[i] - mp, b = r[i] - mr, d = static_cast<double>(p[i]) - r[i];
+          s[0] += a + dp;  // the totals of s[0] and s[1] are relative to fp and fr
+          s[1] += b + dr;
+          s[2] += a * a;
+          s[3] += b * b;
+          s[4] += a * b;
+          s[5] += d * d;
+          cnt += 1.0;
+        }
+      }
+    }
   }
-  __shared__ double red[6][32];
+  s[0] -= cnt * dp;
+  s[1] -= cnt * dr;
+  __shared__ double red[6][8];
   for (int k = 0; k < 6; ++k) {
     double x = s[k];
     for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
@@ -980,7 +1309,7 @@ __global__ void map_sums_kernel(const float* pred, size_t pstride_map, const flo
   __syncthreads();
   if (threadIdx.x < 6) {
     double x = 0;
-    for (int w = 0; w < (int)(blockDim.x / 32); ++w) x += red[threadIdx.x][w];
+    for (int w = 0; w < 8; ++w) x += red[threadIdx.x][w];
     atomicAdd(out + 6 * m + threadIdx.x, x);
   }
 }
@@ -1158,7 +1487,7 @@ int dispatch_conv(const ConvArgs& a, int ntn, bool persistent, bool staged, int 
 
 template <int BN, int NT, int STAGES>
 int launch_wgrad(const WgradArgs& a, int splits, cudaStream_t st) {
-  constexpr int smem = STAGES * (2 * 8192 + NT * (BN / 64) * 8192) + 1024 + 256;
+  constexpr int smem = wgrad_region<BN, NT, STAGES>() + 1024 + 256;
   auto kern = wgrad_kernel<BN, NT, STAGES>;
   int rc = cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attribute");
   if (rc) return rc;
@@ -1356,14 +1685,16 @@ int msur_conv_wgrad(const void* x, const void* dz, int B, int L, int Cin, int Co
   a.lblocks = (L + 63) / 64;
   a.total = B * a.lblocks;
   if (splits <= 0) {
-    // enough CTAs for the machine: about two waves of 152 SMs over the (n, c) tiles
-    const int tiles = ((Cin + 127) / 128) * ((Cout + BM - 1) / BM);
-    splits = (2 * 152 + tiles - 1) / tiles;
+    // one CTA per SM and one wave: a second wave would add every accumulator to dw a second time
+    const int bn = taps == 3 && Cin <= 64 ? 64 : 128;
+    const int tiles = ((Cin + bn - 1) / bn) * ((Cout + BM - 1) / BM);
+    splits = std::max(1, 152 / tiles);
   }
   if (splits > a.total) splits = a.total;
   a.per_split = (a.total + splits - 1) / splits;
   splits = (a.total + a.per_split - 1) / a.per_split;
   a.dw = dw;
+  a.bulk = aligned16(dw) ? 1 : 0;
   a.err = err;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (taps == 3) {
@@ -1431,6 +1762,15 @@ int msur_upcat_bwd(const void* dcat, const void* z, int B, int Lh, int C1, int C
 
 int msur_bias_grad(const void* dz, uint64_t rows, int C, int stride, float* db, void* stream) {
   if (!dz || !db || C <= 0 || stride < C) return fail(MSUR_ERR_INVALID_ARG, "msur_bias_grad: bad argument");
+  if (C % 8 == 0 && stride % 8 == 0 && aligned16(dz)) {
+    // four blocks per SM, but at least four rows per thread
+    const unsigned gx = (C + 63) / 64;
+    const uint64_t most = (rows + 127) / 128;
+    const unsigned gy = static_cast<unsigned>(std::min<uint64_t>(std::max(1u, 4 * 152 / gx), most ? most : 1));
+    bias_grad_v8_kernel<<<dim3(gx, gy), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const bf16*>(dz),
+                                                                                     rows, C, stride, db);
+    return cuda_ok(cudaGetLastError(), "bias_grad_v8_kernel launch");
+  }
   dim3 block(32, 8);
   const uint64_t gy = (rows + 8 * 64 - 1) / (8 * 64);
   dim3 grid((C + 31) / 32, static_cast<unsigned>(gy < 512 ? (gy ? gy : 1) : 512));
@@ -1444,6 +1784,19 @@ int msur_mse(const float* pred, int pstride, const float* target, int tstride, u
   if (!pred || !target || !loss || n_valid <= 0 || pstride < n_valid || tstride < n_valid || dstride < n_valid)
     return fail(MSUR_ERR_INVALID_ARG, "msur_mse: bad argument");
   const size_t n = rows * static_cast<size_t>(dstride);
+  if (n_valid % 4 == 0 && pstride % 4 == 0 && tstride % 4 == 0 && dstride % 4 == 0 && aligned16(pred) &&
+      aligned16(target) && (!dp || (reinterpret_cast<uintptr_t>(dp) & 7u) == 0)) {
+    const unsigned blocks = std::min(grid_for(n / 4), 152u * 8u);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (n / 4 < (1ull << 31)) {
+      mse_v4_kernel<unsigned><<<blocks, 256, 0, st>>>(pred, pstride, target, tstride, rows, n_valid,
+                                                      static_cast<bf16*>(dp), dstride, scale, loss);
+    } else {
+      mse_v4_kernel<size_t><<<blocks, 256, 0, st>>>(pred, pstride, target, tstride, rows, n_valid,
+                                                    static_cast<bf16*>(dp), dstride, scale, loss);
+    }
+    return cuda_ok(cudaGetLastError(), "mse_v4_kernel launch");
+  }
   mse_kernel<<<grid_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(pred, pstride, target, tstride, rows, n_valid,
                                                                          static_cast<bf16*>(dp), dstride, scale, loss);
   return cuda_ok(cudaGetLastError(), "mse_kernel launch");
@@ -1454,6 +1807,13 @@ int msur_adam(float* p, const float* g, float* m, float* v, uint64_t n, float lr
   if (!p || !g || !m || !v || step <= 0) return fail(MSUR_ERR_INVALID_ARG, "msur_adam: bad argument");
   const float bc1 = 1.0f - std::pow(b1, static_cast<float>(step));
   const float bc2 = 1.0f - std::pow(b2, static_cast<float>(step));
+  if (n % 4 == 0 && aligned16(p) && aligned16(g) && aligned16(m) && aligned16(v) &&
+      (!p_bf16 || (reinterpret_cast<uintptr_t>(p_bf16) & 7u) == 0)) {
+    adam_v4_kernel<<<grid_for(n / 4), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        reinterpret_cast<float4*>(p), reinterpret_cast<const float4*>(g), reinterpret_cast<float4*>(m),
+        reinterpret_cast<float4*>(v), n / 4, lr, b1, b2, eps, wd, bc1, bc2, gscale, static_cast<uint2*>(p_bf16));
+    return cuda_ok(cudaGetLastError(), "adam_v4_kernel launch");
+  }
   adam_kernel<<<grid_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(p, g, m, v, n, lr, b1, b2, eps, wd, bc1,
                                                                           bc2, gscale, static_cast<bf16*>(p_bf16));
   return cuda_ok(cudaGetLastError(), "adam_kernel launch");
@@ -1467,9 +1827,45 @@ int msur_weight_transpose(const void* w, int N, int taps, int C, void* wt, void*
   return cuda_ok(cudaGetLastError(), "weight_transpose_kernel launch");
 }
 
+int msur_weight_transpose_list(int count, const void* const* w, const int* N, const int* taps, const int* C,
+                               void* const* wt, void* stream) {
+  if (count <= 0 || count > MSUR_MAX_TRANSPOSES || !w || !N || !taps || !C || !wt)
+    return fail(MSUR_ERR_INVALID_ARG, "msur_weight_transpose_list: bad argument");
+  TransposeList a;
+  std::memset(&a, 0, sizeof(a));
+  a.count = count;
+  int blocks = 0;
+  for (int k = 0; k < count; ++k) {
+    if (!w[k] || !wt[k] || N[k] <= 0 || taps[k] <= 0 || C[k] <= 0)
+      return fail(MSUR_ERR_INVALID_ARG, "msur_weight_transpose_list: bad entry %d", k);
+    if ((N[k] % 8) || (C[k] % 8) || !aligned16(w[k]) || !aligned16(wt[k]))
+      return fail(MSUR_ERR_INVALID_ARG, "msur_weight_transpose_list: entry %d: channels must be multiples of 8, "
+                                        "buffers 16-byte aligned", k);
+    a.first[k] = blocks;
+    a.w[k] = static_cast<const bf16*>(w[k]);
+    a.wt[k] = static_cast<bf16*>(wt[k]);
+    a.N[k] = N[k];
+    a.taps[k] = taps[k];
+    a.C[k] = C[k];
+    blocks += ((N[k] + 63) / 64) * ((C[k] + 63) / 64) * taps[k];
+  }
+  a.first[count] = blocks;
+  weight_transpose_list_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  return cuda_ok(cudaGetLastError(), "weight_transpose_list_kernel launch");
+}
+
 int msur_assemble_input(const float* track, const float* params, int B, int L, int C, void* x, void* stream) {
   if (!track || !params || !x || C < 8 || (C % 8)) return fail(MSUR_ERR_INVALID_ARG, "msur_assemble_input: bad argument");
   const size_t n = static_cast<size_t>(B) * L * C;
+  if (aligned16(x)) {
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (n / 8 < (1ull << 31)) {
+      assemble_input_v8_kernel<unsigned><<<grid_for(n / 8), 256, 0, st>>>(track, params, B, L, C, static_cast<uint4*>(x));
+    } else {
+      assemble_input_v8_kernel<size_t><<<grid_for(n / 8), 256, 0, st>>>(track, params, B, L, C, static_cast<uint4*>(x));
+    }
+    return cuda_ok(cudaGetLastError(), "assemble_input_v8_kernel launch");
+  }
   assemble_input_kernel<<<grid_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(track, params, B, L, C,
                                                                                    static_cast<bf16*>(x));
   return cuda_ok(cudaGetLastError(), "assemble_input_kernel launch");
@@ -1484,10 +1880,16 @@ int msur_band_target(const uint32_t* band, uint64_t ncols, int nrows, float* out
 int msur_map_sums(const float* pred, uint64_t pstride_map, const float* ref, uint64_t rstride_map, uint64_t n,
                   int nmaps, const double* means, double* out, void* stream) {
   if (!pred || !ref || !out || nmaps <= 0 || nmaps > 65535) return fail(MSUR_ERR_INVALID_ARG, "msur_map_sums: bad argument");
-  dim3 grid(static_cast<unsigned>(std::min<uint64_t>((n + 255) / 256, 64)), nmaps);
-  map_sums_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(pred, pstride_map, ref, rstride_map, n,
-                                                                        means, out);
-  return cuda_ok(cudaGetLastError(), "map_sums_kernel launch");
+  // blocks of 16384 elements, about eight per SM over all maps
+  const uint64_t steps = (n + 16383) / 16384, most = std::max(1, 8 * 152 / nmaps);
+  const dim3 grid(static_cast<unsigned>(std::min(steps, most)), nmaps);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (n % 4 == 0 && pstride_map % 4 == 0 && rstride_map % 4 == 0 && aligned16(pred) && aligned16(ref)) {
+    map_sums_pair_kernel<true><<<grid, 256, 0, st>>>(pred, pstride_map, ref, rstride_map, n, means, out);
+  } else {
+    map_sums_pair_kernel<false><<<grid, 256, 0, st>>>(pred, pstride_map, ref, rstride_map, n, means, out);
+  }
+  return cuda_ok(cudaGetLastError(), "map_sums_pair_kernel launch");
 }
 
 int msur_compact_rows(const float* in, int stride, uint64_t rows, int n_valid, float* out, void* stream) {

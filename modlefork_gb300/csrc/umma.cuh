@@ -119,6 +119,13 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void*
                : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// Add `bytes` (a multiple of 16, both addresses 16-byte aligned) of FP32 values in shared memory to global
+// memory; joins this thread's current bulk group.
+__device__ __forceinline__ void bulk_reduce_add_f32(float* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst),
+               "r"(smem_u32(src)), "r"(bytes)
+               : "memory");
+}
 // Wait until at most N of this thread's bulk groups still read their shared-memory source.
 template <int N>
 __device__ __forceinline__ void bulk_wait_read() {

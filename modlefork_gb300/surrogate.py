@@ -114,6 +114,7 @@ class UNet:
             self.gw[s.name] = self.g[wo:wo + s.wsize].view(shape)
             self.gb[s.name] = self.g[bo:bo + s.cout]
             self.wt[s.name] = torch.empty(s.cin, s.taps, s.cout, dtype=torch.bfloat16, **kw)
+        self._transposes = ops.TransposeList((self.wb[s.name], self.wt[s.name]) for s in specs)
         self.step_count = 0
         self._ws = {}
         self._init(seed, head_bias)
@@ -137,8 +138,7 @@ class UNet:
         self._refresh_transposes()
 
     def _refresh_transposes(self):
-        for name in self.specs:
-            ops.weight_transpose(self.wb[name], self.wt[name])
+        self._transposes.run()
 
     def params_dict(self):
         """name -> (w [Cout, taps, Cin], b [Cout]) as numpy float32 copies."""

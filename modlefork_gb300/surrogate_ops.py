@@ -14,6 +14,7 @@ import torch
 
 LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "_lib", "libmgpu_surrogate.so")
 ACT_NONE, ACT_SILU = 0, 1
+MAX_TRANSPOSES = 64  # MSUR_MAX_TRANSPOSES
 _lib = None
 
 
@@ -42,6 +43,8 @@ def load(path=LIB_PATH):
         "msur_mse": (i32, [vp, i32, vp, i32, u64, i32, vp, i32, f32, vp, vp]),
         "msur_adam": (i32, [vp, vp, vp, vp, u64, f32, f32, f32, f32, f32, i32, f32, vp, vp]),
         "msur_weight_transpose": (i32, [vp, i32, i32, i32, vp, vp]),
+        "msur_weight_transpose_list": (i32, [i32, C.POINTER(vp), C.POINTER(i32), C.POINTER(i32), C.POINTER(i32),
+                                             C.POINTER(vp), vp]),
         "msur_assemble_input": (i32, [vp, vp, i32, i32, i32, vp, vp]),
         "msur_band_target": (i32, [vp, u64, i32, vp, vp]),
         "msur_map_sums": (i32, [vp, u64, vp, u64, u64, i32, vp, vp, vp]),
@@ -172,6 +175,25 @@ def adam(p, g, m, v, step, lr, b1=0.9, b2=0.999, eps=1e-8, wd=0.0, gscale=1.0, p
 def weight_transpose(w, wt):
     N, taps, Cw = w.shape
     _check(load().msur_weight_transpose(_p(w), N, taps, Cw, _p(wt), _stream()), "msur_weight_transpose")
+
+
+class TransposeList:
+    """The weight transposes of several convolutions, [(w, wt), ...], as one launch (run); the tensors are
+    kept alive and must not be reallocated."""
+
+    def __init__(self, pairs):
+        self.pairs = list(pairs)
+        self.calls = []
+        for k in range(0, len(self.pairs), MAX_TRANSPOSES):
+            part = self.pairs[k:k + MAX_TRANSPOSES]
+            n = len(part)
+            dims = [(C.c_int * n)(*(w.shape[d] for w, _ in part)) for d in range(3)]
+            self.calls.append((n, (C.c_void_p * n)(*(w.data_ptr() for w, _ in part)), *dims,
+                               (C.c_void_p * n)(*(t.data_ptr() for _, t in part))))
+
+    def run(self):
+        for call in self.calls:
+            _check(load().msur_weight_transpose_list(*call, _stream()), "msur_weight_transpose_list")
 
 
 def assemble_input(track, params, x):
