@@ -145,8 +145,42 @@ int msur_band_target(const uint32_t* band, uint64_t ncols, int nrows, float* out
  * pass of the reference's two-pass Pearson, src/stats/correlation_impl.hpp:66-87). */
 int msur_map_sums(const float* pred, uint64_t pstride_map, const float* ref, uint64_t rstride_map, uint64_t n,
                   int nmaps, const double* means, double* out, void* stream);
+/* The same for a selection of the sums (bit k: sum k; the others of out stay as they are): what a map's
+ * scores need of the raw values (p, r, r^2, (p - r)^2) and of the deviations (all but (p - r)^2). */
+#define MSUR_SUMS_RAW 0x2Bu
+#define MSUR_SUMS_CENTRED 0x1Fu
+#define MSUR_SUMS_ALL 0x3Fu
+int msur_map_sums_of(unsigned which, const float* pred, uint64_t pstride_map, const float* ref, uint64_t rstride_map,
+                     uint64_t n, int nmaps, const double* means, double* out, void* stream);
 /* out[r][c] = in[r * stride + c] for c < n_valid (drop the padded channels of the head). */
 int msur_compact_rows(const float* in, int stride, uint64_t rows, int n_valid, float* out, void* stream);
+
+/* A list of the operations above in one call, enqueued in order: a network's pass without a foreign-function
+ * call per layer.  p, i, f and rows hold the operation's arguments in the order of its function:
+ *   CONV      p: x w bias out_pre out_post out_f32 gate out_skip out_dup out_pool;
+ *             i: B L Cin Cout taps act out_stride n_valid skip_stride dup_stride pool_stride;
+ *             form and stages: the kernel form and depth, -1 for the width's current settings
+ *   WGRAD     p: x dz dw; i: B L Cin Cout taps splits
+ *   BIAS_GRAD p: dz db; i: C stride; rows
+ *   POOL2     p: x y; i: B Lout C
+ *   SKIP_GRAD p: dpool dcat z dz; i: Lp cat_stride cat_off B L C
+ *   UPCAT     p: x skip out; i: B L C1 C2
+ *   UPCAT_BWD p: dcat z dz; i: B Lh C1 C
+ *   MSE       p: pred target dp loss; i: pstride tstride n_valid dstride; rows; f: scale
+ *   ZERO      p: buffer; rows: bytes
+ * Stops at the first operation that fails and returns its status. */
+enum {
+  MSUR_OP_CONV = 0, MSUR_OP_WGRAD, MSUR_OP_BIAS_GRAD, MSUR_OP_POOL2, MSUR_OP_SKIP_GRAD, MSUR_OP_UPCAT,
+  MSUR_OP_UPCAT_BWD, MSUR_OP_MSE, MSUR_OP_ZERO
+};
+typedef struct msur_op {
+  int kind, form, stages;
+  float f;
+  int i[12];
+  uint64_t rows;
+  void* p[10];
+} msur_op;
+int msur_run(const msur_op* ops, int n, void* stream);
 
 #ifdef __cplusplus
 }

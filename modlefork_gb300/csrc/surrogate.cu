@@ -25,6 +25,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdint>
@@ -1212,15 +1213,16 @@ __global__ void band_target_kernel(const uint32_t* band, size_t ncols, int nrows
 // sum (a - d)^2 = sum a^2 - 2 d sum a + n d^2.  A pair carries 2^-47 per operation and the chunks' errors
 // average out over the map; measured against 64-bit sums the scores are as close as before (a few 1e-16).
 // A chunk with values outside [2^-30, 2^50) in size throughout, infinities or NaN is summed in FP64.
+// WHICH: the sums wanted (bit k: sum k); MEANS: deviations from the means, raw values otherwise.
 constexpr int SUM_VECS = 16;  // float4 per thread and chunk
-template <bool VEC>
+template <bool VEC, bool MEANS, unsigned WHICH>
 __global__ void __launch_bounds__(256) map_sums_pair_kernel(const float* pred, size_t pstride_map, const float* ref,
                                                             size_t rstride_map, size_t n, const double* means,
                                                             double* out) {
   const int m = blockIdx.y;
   const float* __restrict__ p = pred + m * pstride_map;
   const float* __restrict__ r = ref + m * rstride_map;
-  const double mp = means ? means[2 * m] : 0.0, mr = means ? means[2 * m + 1] : 0.0;
+  const double mp = MEANS ? means[2 * m] : 0.0, mr = MEANS ? means[2 * m + 1] : 0.0;
   const float fp = static_cast<float>(mp), fr = static_cast<float>(mr);
   const double dp = mp - fp, dr = mr - fr;
   double s[6] = {0, 0, 0, 0, 0, 0};
@@ -1255,18 +1257,28 @@ __global__ void __launch_bounds__(256) map_sums_pair_kernel(const float* pred, s
         mxp = max(mxp, __float_as_uint(fabsf(a[e])));
         mxr = max(mxr, __float_as_uint(fabsf(b[e])));
         float ah, al, bh, bl, h, l;
-        exact_difference(a[e], fp, ah, al);
-        exact_difference(b[e], fr, bh, bl);
-        exact_difference(a[e], b[e], h, l);
-        if (!VEC && e >= valid) h = l = 0.0f;
-        t[0].add(ah);
-        t[0].l += al;
-        t[1].add(bh);
-        t[1].l += bl;
-        t[2].add_product(ah, ah, 2.0f * ah * al);
-        t[3].add_product(bh, bh, 2.0f * bh * bl);
-        t[4].add_product(ah, bh, ah * bl + al * bh);
-        t[5].add_product(h, h, 2.0f * h * l);
+        if constexpr (MEANS) {
+          exact_difference(a[e], fp, ah, al);
+          exact_difference(b[e], fr, bh, bl);
+        } else {
+          ah = a[e], al = 0.0f, bh = b[e], bl = 0.0f;
+        }
+        if constexpr (WHICH & 1) {
+          t[0].add(ah);
+          t[0].l += al;
+        }
+        if constexpr (WHICH & 2) {
+          t[1].add(bh);
+          t[1].l += bl;
+        }
+        if constexpr (WHICH & 4) t[2].add_product(ah, ah, MEANS ? 2.0f * ah * al : 0.0f);
+        if constexpr (WHICH & 8) t[3].add_product(bh, bh, MEANS ? 2.0f * bh * bl : 0.0f);
+        if constexpr (WHICH & 16) t[4].add_product(ah, bh, MEANS ? ah * bl + al * bh : 0.0f);
+        if constexpr (WHICH & 32) {
+          exact_difference(a[e], b[e], h, l);
+          if (!VEC && e >= valid) h = l = 0.0f;
+          t[5].add_product(h, h, 2.0f * h * l);
+        }
       }
       k += valid;
     }
@@ -1307,7 +1319,7 @@ __global__ void __launch_bounds__(256) map_sums_pair_kernel(const float* pred, s
     if (threadIdx.x % 32 == 0) red[k][threadIdx.x / 32] = x;
   }
   __syncthreads();
-  if (threadIdx.x < 6) {
+  if (threadIdx.x < 6 && ((WHICH >> threadIdx.x) & 1u)) {
     double x = 0;
     for (int w = 0; w < 8; ++w) x += red[threadIdx.x][w];
     atomicAdd(out + 6 * m + threadIdx.x, x);
@@ -1438,11 +1450,37 @@ constexpr int conv_smem() {
   return STAGES * (BM * BK * 2 + BN * BK * 2) + 1024 + (STAGED ? 1024 + STAGE_OUT_BYTES : 256);
 }
 
+// Once per kernel and device: the shared-memory permission and the CTAs that fit an SM (asking the runtime
+// on every launch took longer than the launch).
+struct KernelLimits {
+  std::atomic<int> per_sm[64] = {};
+  int get(const void* kern, int smem, int* out) {
+    int dev = 0;
+    int rc = cuda_ok(cudaGetDevice(&dev), "cudaGetDevice");
+    if (rc) return rc;
+    if (dev < 0 || dev >= 64) return fail(MSUR_ERR_UNSUPPORTED, "device %d out of range", dev);
+    int n = per_sm[dev].load(std::memory_order_acquire);
+    if (n == 0) {
+      rc = cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attribute");
+      if (!rc) rc = cuda_ok(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, THREADS, smem), "occupancy");
+      int sms = 0;
+      if (!rc) rc = cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
+      if (rc) return rc;
+      n = (sms << 8) | std::max(1, n);
+      per_sm[dev].store(n, std::memory_order_release);
+    }
+    *out = n;
+    return MSUR_OK;
+  }
+};
+
 template <int BN, int STAGES, bool STAGED>
 int launch_conv(const ConvArgs& a, int ntiles_n, cudaStream_t st) {
   constexpr int smem = conv_smem<BN, STAGES, STAGED>();
   auto kern = conv_fwd_kernel<BN, STAGES, STAGED>;
-  int rc = cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attribute");
+  static KernelLimits limits;
+  int lim = 0;
+  const int rc = limits.get(reinterpret_cast<const void*>(kern), smem, &lim);
   if (rc) return rc;
   dim3 grid(ntiles_n, (a.L + BM - 1) / BM, a.B);
   kern<<<grid, THREADS, smem, st>>>(a);
@@ -1454,13 +1492,12 @@ int launch_conv_persistent(const ConvArgs& a, int ntn, cudaStream_t st) {
   constexpr int smem = conv_smem<BN, STAGES, STAGED>();
   constexpr int tcols = static_cast<int>(tmem_cols<2 * BN>());
   auto kern = conv_fwd_persistent_kernel<BN, STAGES, STAGED>;
-  int rc = cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attribute");
+  static KernelLimits limits;
+  int lim = 0;
+  const int rc = limits.get(reinterpret_cast<const void*>(kern), smem, &lim);
   if (rc) return rc;
-  int dev = 0, sms = 0, per_sm = 0;
-  rc = cuda_ok(cudaGetDevice(&dev), "cudaGetDevice");
-  if (!rc) rc = cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
-  if (!rc) rc = cuda_ok(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, THREADS, smem), "occupancy");
-  if (rc) return rc;
+  const int sms = lim >> 8;
+  int per_sm = lim & 255;
   per_sm = std::max(1, std::min(per_sm, 512 / tcols));  // each resident CTA holds its accumulators in TMEM
   const int ntl = (a.L + BM - 1) / BM;
   const int ntiles = ntn * ntl * a.B;
@@ -1489,7 +1526,9 @@ template <int BN, int NT, int STAGES>
 int launch_wgrad(const WgradArgs& a, int splits, cudaStream_t st) {
   constexpr int smem = wgrad_region<BN, NT, STAGES>() + 1024 + 256;
   auto kern = wgrad_kernel<BN, NT, STAGES>;
-  int rc = cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attribute");
+  static KernelLimits limits;
+  int lim = 0;
+  const int rc = limits.get(reinterpret_cast<const void*>(kern), smem, &lim);
   if (rc) return rc;
   dim3 grid((a.Cin + BN - 1) / BN, (a.Cout + BM - 1) / BM, splits);
   kern<<<grid, THREADS, smem, st>>>(a);
@@ -1522,7 +1561,8 @@ int msur_take_error(unsigned* code) {
 static int conv_forward_impl(const void* x, int B, int L, int Cin, const void* w, int Cout, int taps,
                              const float* bias, int act, void* out_pre, void* out_post, float* out_f32,
                              int out_stride, int n_valid, const void* gate, void* out_skip, int skip_stride,
-                             void* out_dup, int dup_stride, void* out_pool, int pool_stride, void* stream) {
+                             void* out_dup, int dup_stride, void* out_pool, int pool_stride, int form, int stages,
+                             void* stream) {
   if (!x || !w || B <= 0 || L <= 0 || Cin <= 0 || Cout <= 0 || taps <= 0 || n_valid <= 0 || n_valid > Cout)
     return fail(MSUR_ERR_INVALID_ARG, "msur_conv_forward: bad shape or null pointer");
   if (Cin % BK) return fail(MSUR_ERR_INVALID_ARG, "msur_conv_forward: Cin (%d) must be a multiple of 64", Cin);
@@ -1544,7 +1584,14 @@ static int conv_forward_impl(const void* x, int B, int L, int Cin, const void* w
   unsigned* err = nullptr;
   int rc = setup(&err);
   if (rc) return rc;
-  const int BN = Cout <= 64 ? 64 : (Cout % 256 == 0 ? 256 : 128);
+  const int slot = conv_slot(Cout <= 64 ? 64 : (Cout % 256 == 0 ? 256 : 128));
+  if (form < 0) form = g_conv_form[slot];
+  if (stages < 0) stages = g_conv_stages[slot];
+  // A tile is one CTA's chain of K steps, and a step's time is its operands' transfer, so while the tiles
+  // leave SMs idle a narrower one halves the chain's time on twice the SMs (the products and their order
+  // are the same).  One map: the deep levels have 2 to 16 tiles at 256 columns, 8 to 64 at 64.
+  int BN = slot == 2 ? 256 : (slot == 1 ? 128 : 64);
+  while (BN > 64 && static_cast<long long>((Cout + BN - 1) / BN) * ((L + BM - 1) / BM) * B < 152) BN /= 2;
   ConvArgs a;
   std::memset(&a, 0, sizeof(a));
   const uint64_t dims_a[3] = {static_cast<uint64_t>(Cin), static_cast<uint64_t>(L), static_cast<uint64_t>(B)};
@@ -1571,12 +1618,9 @@ static int conv_forward_impl(const void* x, int B, int L, int Cin, const void* w
   a.err = err;
   const int ntn = (Cout + BN - 1) / BN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int slot = BN == 256 ? 2 : (BN == 128 ? 1 : 0);
-  const int stages = g_conv_stages[slot];
   // kernel form: bit 0 the persistent kernel, bit 1 the staged epilogue (outputs through shared
   // memory and TMA), which needs no gate: the data gradient's gate is read row by row, so that
   // epilogue stays per thread
-  const int form = g_conv_form[slot];
   const bool persistent = (form & 1) != 0;
   const bool staged = (form & 2) != 0 && !gate;
   if ((out_skip || out_dup || out_pool) && !staged)
@@ -1609,7 +1653,7 @@ int msur_conv_forward(const void* x, int B, int L, int Cin, const void* w, int C
                       int act, void* out_pre, void* out_post, float* out_f32, int out_stride, int n_valid,
                       const void* gate, void* stream) {
   return conv_forward_impl(x, B, L, Cin, w, Cout, taps, bias, act, out_pre, out_post, out_f32, out_stride, n_valid,
-                           gate, nullptr, 0, nullptr, 0, nullptr, 0, stream);
+                           gate, nullptr, 0, nullptr, 0, nullptr, 0, -1, -1, stream);
 }
 
 int msur_conv_forward_fused(const void* x, int B, int L, int Cin, const void* w, int Cout, int taps,
@@ -1617,7 +1661,7 @@ int msur_conv_forward_fused(const void* x, int B, int L, int Cin, const void* w,
                             int skip_stride, void* out_dup, int dup_stride, void* out_pool, int pool_stride,
                             int n_valid, void* stream) {
   return conv_forward_impl(x, B, L, Cin, w, Cout, taps, bias, act, nullptr, out_post, nullptr, out_stride, n_valid,
-                           nullptr, out_skip, skip_stride, out_dup, dup_stride, out_pool, pool_stride, stream);
+                           nullptr, out_skip, skip_stride, out_dup, dup_stride, out_pool, pool_stride, -1, -1, stream);
 }
 
 int msur_conv_set_stages(int bn, int stages) {
@@ -1827,6 +1871,52 @@ int msur_weight_transpose(const void* w, int N, int taps, int C, void* wt, void*
   return cuda_ok(cudaGetLastError(), "weight_transpose_kernel launch");
 }
 
+int msur_run(const msur_op* ops, int n, void* stream) {
+  if (n < 0 || (n && !ops)) return fail(MSUR_ERR_INVALID_ARG, "msur_run: bad argument");
+  for (int k = 0; k < n; ++k) {
+    const msur_op& o = ops[k];
+    const int* i = o.i;
+    void* const* p = o.p;
+    int rc = MSUR_OK;
+    switch (o.kind) {
+      case MSUR_OP_CONV:
+        rc = conv_forward_impl(p[0], i[0], i[1], i[2], p[1], i[3], i[4], static_cast<const float*>(p[2]), i[5], p[3],
+                               p[4], static_cast<float*>(p[5]), i[6], i[7], p[6], p[7], i[8], p[8], i[9], p[9], i[10],
+                               o.form, o.stages, stream);
+        break;
+      case MSUR_OP_WGRAD:
+        rc = msur_conv_wgrad(p[0], p[1], i[0], i[1], i[2], i[3], i[4], static_cast<float*>(p[2]), i[5], stream);
+        break;
+      case MSUR_OP_BIAS_GRAD:
+        rc = msur_bias_grad(p[0], o.rows, i[0], i[1], static_cast<float*>(p[1]), stream);
+        break;
+      case MSUR_OP_POOL2:
+        rc = msur_pool2(p[0], i[0], i[1], i[2], p[1], stream);
+        break;
+      case MSUR_OP_SKIP_GRAD:
+        rc = msur_skip_grad(p[0], i[0], p[1], i[1], i[2], p[2], i[3], i[4], i[5], p[3], stream);
+        break;
+      case MSUR_OP_UPCAT:
+        rc = msur_upcat(p[0], p[1], i[0], i[1], i[2], i[3], p[2], stream);
+        break;
+      case MSUR_OP_UPCAT_BWD:
+        rc = msur_upcat_bwd(p[0], p[1], i[0], i[1], i[2], i[3], p[2], stream);
+        break;
+      case MSUR_OP_MSE:
+        rc = msur_mse(static_cast<const float*>(p[0]), i[0], static_cast<const float*>(p[1]), i[1], o.rows, i[2], p[2],
+                      i[3], o.f, static_cast<double*>(p[3]), stream);
+        break;
+      case MSUR_OP_ZERO:
+        rc = cuda_ok(cudaMemsetAsync(p[0], 0, o.rows, static_cast<cudaStream_t>(stream)), "cudaMemsetAsync");
+        break;
+      default:
+        rc = fail(MSUR_ERR_INVALID_ARG, "msur_run: operation %d has an unknown kind %d", k, o.kind);
+    }
+    if (rc) return rc;
+  }
+  return MSUR_OK;
+}
+
 int msur_weight_transpose_list(int count, const void* const* w, const int* N, const int* taps, const int* C,
                                void* const* wt, void* stream) {
   if (count <= 0 || count > MSUR_MAX_TRANSPOSES || !w || !N || !taps || !C || !wt)
@@ -1877,19 +1967,40 @@ int msur_band_target(const uint32_t* band, uint64_t ncols, int nrows, float* out
   return cuda_ok(cudaGetLastError(), "band_target_kernel launch");
 }
 
-int msur_map_sums(const float* pred, uint64_t pstride_map, const float* ref, uint64_t rstride_map, uint64_t n,
-                  int nmaps, const double* means, double* out, void* stream) {
+}  // extern "C"
+
+namespace {
+template <unsigned WHICH>
+void launch_map_sums(const float* pred, uint64_t ps, const float* ref, uint64_t rs, uint64_t n, dim3 grid,
+                     const double* means, double* out, bool vec, cudaStream_t st) {
+  if (vec && means) map_sums_pair_kernel<true, true, WHICH><<<grid, 256, 0, st>>>(pred, ps, ref, rs, n, means, out);
+  else if (vec) map_sums_pair_kernel<true, false, WHICH><<<grid, 256, 0, st>>>(pred, ps, ref, rs, n, means, out);
+  else if (means) map_sums_pair_kernel<false, true, WHICH><<<grid, 256, 0, st>>>(pred, ps, ref, rs, n, means, out);
+  else map_sums_pair_kernel<false, false, WHICH><<<grid, 256, 0, st>>>(pred, ps, ref, rs, n, means, out);
+}
+}  // namespace
+
+extern "C" {
+
+int msur_map_sums_of(unsigned which, const float* pred, uint64_t pstride_map, const float* ref, uint64_t rstride_map,
+                     uint64_t n, int nmaps, const double* means, double* out, void* stream) {
   if (!pred || !ref || !out || nmaps <= 0 || nmaps > 65535) return fail(MSUR_ERR_INVALID_ARG, "msur_map_sums: bad argument");
   // blocks of 16384 elements, about eight per SM over all maps
   const uint64_t steps = (n + 16383) / 16384, most = std::max(1, 8 * 152 / nmaps);
   const dim3 grid(static_cast<unsigned>(std::min(steps, most)), nmaps);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (n % 4 == 0 && pstride_map % 4 == 0 && rstride_map % 4 == 0 && aligned16(pred) && aligned16(ref)) {
-    map_sums_pair_kernel<true><<<grid, 256, 0, st>>>(pred, pstride_map, ref, rstride_map, n, means, out);
-  } else {
-    map_sums_pair_kernel<false><<<grid, 256, 0, st>>>(pred, pstride_map, ref, rstride_map, n, means, out);
-  }
+  const bool vec = n % 4 == 0 && pstride_map % 4 == 0 && rstride_map % 4 == 0 && aligned16(pred) && aligned16(ref);
+  if (which == MSUR_SUMS_RAW) launch_map_sums<MSUR_SUMS_RAW>(pred, pstride_map, ref, rstride_map, n, grid, means, out, vec, st);
+  else if (which == MSUR_SUMS_CENTRED)
+    launch_map_sums<MSUR_SUMS_CENTRED>(pred, pstride_map, ref, rstride_map, n, grid, means, out, vec, st);
+  else if (which == MSUR_SUMS_ALL) launch_map_sums<MSUR_SUMS_ALL>(pred, pstride_map, ref, rstride_map, n, grid, means, out, vec, st);
+  else return fail(MSUR_ERR_INVALID_ARG, "msur_map_sums_of: unknown selection %u", which);
   return cuda_ok(cudaGetLastError(), "map_sums_pair_kernel launch");
+}
+
+int msur_map_sums(const float* pred, uint64_t pstride_map, const float* ref, uint64_t rstride_map, uint64_t n,
+                  int nmaps, const double* means, double* out, void* stream) {
+  return msur_map_sums_of(MSUR_SUMS_ALL, pred, pstride_map, ref, rstride_map, n, nmaps, means, out, stream);
 }
 
 int msur_compact_rows(const float* in, int stride, uint64_t rows, int n_valid, float* out, void* stream) {

@@ -210,24 +210,11 @@ class UNet:
         bn = tile_width(self.specs[name].cout)
         return ops.conv_get_form(bn), ops.conv_get_stages(bn)
 
-    def _set_layer(self, name):
-        cfg = LAYER_CFG.get(name)
-        if cfg is not None:
-            bn = tile_width(self.specs[name].cout)
-            ops.conv_set_form(bn, cfg[0])
-            ops.conv_set_stages(bn, cfg[1])
-
-    def _conv(self, name, x, pre=None, post=None, f32=None, **kw):
+    def _conv_op(self, name, x, **kw):
         s = self.specs[name]
-        self._set_layer(name)
-        ops.conv_forward(x, self.wb[name], bias=self.b32[name], act=ops.ACT_SILU if s.act else ops.ACT_NONE,
-                         out_pre=pre, out_post=post, out_f32=f32, **kw)
-
-    def _conv_fused(self, name, x, post=None, skip=None, dup=None, pool=None):
-        s = self.specs[name]
-        self._set_layer(name)
-        ops.conv_forward_fused(x, self.wb[name], bias=self.b32[name], act=ops.ACT_SILU if s.act else ops.ACT_NONE,
-                               out_post=post, skip=skip, dup=dup, pool=pool)
+        form, stages = LAYER_CFG.get(name, (-1, -1))
+        return ops.conv_op(x, self.wb[name], bias=self.b32[name], act=ops.ACT_SILU if s.act else ops.ACT_NONE,
+                           form=form, stages=stages, **kw)
 
     def fusable(self):
         """Whether inference can fill the decoder's concatenation buffers from the convolutions
@@ -246,77 +233,102 @@ class UNet:
         the other half, so no separate pooling or upsample-and-concatenate step runs; the results
         are the same either way."""
         B = x.shape[0]
+        assert tuple(x.shape[1:]) == (self.length, IN_CH) and x.dtype == torch.bfloat16
         ws = self._workspace(B, train)
-        get = (lambda k: ws.get(k)) if train else (lambda k: None)
-        fused = fuse and not train and self.fusable()
-        h = x
+        fused = bool(fuse and not train and self.fusable())
+        # the pass as a list of operations on the workspace; only its input and output differ by call
+        key = (fused, tuple(LAYER_CFG.items()))
+        if ws.get("forward_key") != key:
+            ws["forward_ops"], ws["forward_key"] = self._forward_ops(B, ws, train, fused), key
+        oplist = ws["forward_ops"]
+        dst = ws["out"] if out is None else out
+        oplist[0].p[0] = x.data_ptr()
+        oplist[len(oplist) - 1].p[5] = dst.data_ptr()
         ws["h_in0"] = x
+        ops.run(oplist)
+        return dst
+
+    def _forward_ops(self, B, ws, train, fused):
+        get = (lambda k: ws.get(k)) if train else (lambda k: None)
+        lst = []
+        h = ws["x"]  # a stand-in of the input's shape
         for i in range(self.depth):
-            self._conv(f"enc{i}a", h, pre=get(f"za{i}"), post=ws[f"ya{i}"])
+            lens = self.length >> i
+            lst.append(self._conv_op(f"enc{i}a", h, pre=get(f"za{i}"), post=ws[f"ya{i}"]))
             if fused:
                 cat = ws[f"cat{i}"]
-                self._conv_fused(f"enc{i}b", ws[f"ya{i}"], skip=cat[:, :, cat.shape[-1] - self.widths[i]:],
-                                 pool=ws[f"p{i}"])
+                lst.append(self._conv_op(f"enc{i}b", ws[f"ya{i}"], skip=cat[:, :, cat.shape[-1] - self.widths[i]:],
+                                         pool=ws[f"p{i}"]))
             else:
-                self._conv(f"enc{i}b", ws[f"ya{i}"], pre=get(f"zb{i}"), post=ws[f"yb{i}"])
-                ops.pool2(ws[f"yb{i}"], ws[f"p{i}"])
+                lst.append(self._conv_op(f"enc{i}b", ws[f"ya{i}"], pre=get(f"zb{i}"), post=ws[f"yb{i}"]))
+                lst.append(ops.op(ops.OP_POOL2, (ws[f"yb{i}"], ws[f"p{i}"]), (B, lens // 2, self.widths[i])))
             h = ws[f"p{i}"]
-        self._conv("mid_a", h, pre=get("zma"), post=ws["yma"])
+        lst.append(self._conv_op("mid_a", h, pre=get("zma"), post=ws["yma"]))
         if fused:
-            self._conv_fused("mid_b", ws["yma"], dup=ws[f"cat{self.depth - 1}"][:, :, :self.mid])
+            lst.append(self._conv_op("mid_b", ws["yma"], dup=ws[f"cat{self.depth - 1}"][:, :, :self.mid]))
         else:
-            self._conv("mid_b", ws["yma"], pre=get("zmb"), post=ws["ymb"])
+            lst.append(self._conv_op("mid_b", ws["yma"], pre=get("zmb"), post=ws["ymb"]))
             h = ws["ymb"]
         for i in reversed(range(self.depth)):
             if not fused:
-                ops.upcat(h, ws[f"yb{i}"], ws[f"cat{i}"])
-            self._conv(f"dec{i}a", ws[f"cat{i}"], pre=get(f"zda{i}"), post=ws[f"yda{i}"])
+                lst.append(ops.op(ops.OP_UPCAT, (h, ws[f"yb{i}"], ws[f"cat{i}"]),
+                                  (B, self.length >> i, h.shape[-1], self.widths[i])))
+            lst.append(self._conv_op(f"dec{i}a", ws[f"cat{i}"], pre=get(f"zda{i}"), post=ws[f"yda{i}"]))
             if fused and i > 0:
-                self._conv_fused(f"dec{i}b", ws[f"yda{i}"], dup=ws[f"cat{i - 1}"][:, :, :self.widths[i]])
+                lst.append(self._conv_op(f"dec{i}b", ws[f"yda{i}"], dup=ws[f"cat{i - 1}"][:, :, :self.widths[i]]))
             else:
-                self._conv(f"dec{i}b", ws[f"yda{i}"], pre=get(f"zdb{i}"), post=ws[f"ydb{i}"])
+                lst.append(self._conv_op(f"dec{i}b", ws[f"yda{i}"], pre=get(f"zdb{i}"), post=ws[f"ydb{i}"]))
                 h = ws[f"ydb{i}"]
-        dst = ws["out"] if out is None else out
-        self._conv("head", h, f32=dst, n_valid=NROWS, out_stride=NROWS)
-        return dst
+        lst.append(self._conv_op("head", h, f32=ws["out"]))
+        return (ops.Op * len(lst))(*lst)
 
     # ---- backward ------------------------------------------------------------------------
-    def _grads(self, name, x, dz):
+    def _grad_ops(self, name, x, dz):
         """Weight and bias gradients of convolution `name` with input x and output gradient dz."""
-        ops.conv_wgrad(x, dz, self.gw[name])
-        ops.bias_grad(dz, self.gb[name])
+        B, L, cin = x.shape
+        s = self.specs[name]
+        return [ops.op(ops.OP_WGRAD, (x, dz, self.gw[name]), (B, L, cin, s.cout, s.taps, 0)),
+                ops.op(ops.OP_BIAS_GRAD, (dz, self.gb[name]), (s.cout, dz.shape[-1]), rows=B * L)]
 
-    def _dgrad(self, name, dz, out, gate=None):
-        ops.conv_forward(dz, self.wt[name], out_post=out, gate=gate)
+    def _dgrad_op(self, name, dz, out, gate=None):
+        return ops.conv_op(dz, self.wt[name], post=out, gate=gate)
+
+    def _backward_ops(self, B, ws):
+        D = self.depth
+        lst = self._grad_ops("head", ws["ydb0"], ws["dout"])
+        lst.append(self._dgrad_op("head", ws["dout"], ws["ddb0"], gate=ws["zdb0"]))
+        for i in range(D):
+            lst += self._grad_ops(f"dec{i}b", ws[f"yda{i}"], ws[f"ddb{i}"])
+            lst.append(self._dgrad_op(f"dec{i}b", ws[f"ddb{i}"], ws[f"dda{i}"], gate=ws[f"zda{i}"]))
+            lst += self._grad_ops(f"dec{i}a", ws[f"cat{i}"], ws[f"dda{i}"])
+            lst.append(self._dgrad_op(f"dec{i}a", ws[f"dda{i}"], ws[f"dcat{i}"]))
+            z, dz = (ws[f"zdb{i + 1}"], ws[f"ddb{i + 1}"]) if i + 1 < D else (ws["zmb"], ws["dmb"])
+            lst.append(ops.op(ops.OP_UPCAT_BWD, (ws[f"dcat{i}"], z, dz),
+                              (B, z.shape[1], z.shape[2], ws[f"dcat{i}"].shape[-1])))
+        lst += self._grad_ops("mid_b", ws["yma"], ws["dmb"])
+        lst.append(self._dgrad_op("mid_b", ws["dmb"], ws["dma"], gate=ws["zma"]))
+        lst += self._grad_ops("mid_a", ws[f"p{D - 1}"], ws["dma"])
+        lst.append(self._dgrad_op("mid_a", ws["dma"], ws[f"dp{D - 1}"]))
+        for i in reversed(range(D)):
+            ch = self.mid if i == D - 1 else self.widths[i + 1]
+            z = ws[f"zb{i}"]
+            lst.append(ops.op(ops.OP_SKIP_GRAD, (ws[f"dp{i}"], ws[f"dcat{i}"], z, ws[f"dzb{i}"]),
+                              (ws[f"dp{i}"].shape[1], ws[f"dcat{i}"].shape[-1], ch, B, z.shape[1], z.shape[2])))
+            lst += self._grad_ops(f"enc{i}b", ws[f"ya{i}"], ws[f"dzb{i}"])
+            lst.append(self._dgrad_op(f"enc{i}b", ws[f"dzb{i}"], ws[f"dza{i}"], gate=ws[f"za{i}"]))
+            lst += self._grad_ops(f"enc{i}a", ws["x"] if i == 0 else ws[f"p{i - 1}"], ws[f"dza{i}"])
+            if i > 0:
+                lst.append(self._dgrad_op(f"enc{i}a", ws[f"dza{i}"], ws[f"dp{i - 1}"]))
+        return (ops.Op * len(lst))(*lst)
 
     def backward(self, B):
         """Gradients of the last training forward pass into self.g (after ws['dout'] is set)."""
         ws = self._ws[(B, True)]
-        D = self.depth
-        self._grads("head", ws["ydb0"], ws["dout"])
-        self._dgrad("head", ws["dout"], ws["ddb0"], gate=ws["zdb0"])
-        for i in range(D):
-            self._grads(f"dec{i}b", ws[f"yda{i}"], ws[f"ddb{i}"])
-            self._dgrad(f"dec{i}b", ws[f"ddb{i}"], ws[f"dda{i}"], gate=ws[f"zda{i}"])
-            self._grads(f"dec{i}a", ws[f"cat{i}"], ws[f"dda{i}"])
-            self._dgrad(f"dec{i}a", ws[f"dda{i}"], ws[f"dcat{i}"])
-            if i + 1 < D:
-                ops.upcat_bwd(ws[f"dcat{i}"], ws[f"zdb{i + 1}"], ws[f"ddb{i + 1}"])
-            else:
-                ops.upcat_bwd(ws[f"dcat{i}"], ws["zmb"], ws["dmb"])
-        self._grads("mid_b", ws["yma"], ws["dmb"])
-        self._dgrad("mid_b", ws["dmb"], ws["dma"], gate=ws["zma"])
-        self._grads("mid_a", ws[f"p{D - 1}"], ws["dma"])
-        self._dgrad("mid_a", ws["dma"], ws[f"dp{D - 1}"])
-        for i in reversed(range(D)):
-            ch = self.mid if i == D - 1 else self.widths[i + 1]
-            ops.skip_grad(ws[f"zb{i}"], ws[f"dzb{i}"], dpool=ws[f"dp{i}"], dcat=ws[f"dcat{i}"], cat_off=ch)
-            self._grads(f"enc{i}b", ws[f"ya{i}"], ws[f"dzb{i}"])
-            self._dgrad(f"enc{i}b", ws[f"dzb{i}"], ws[f"dza{i}"], gate=ws[f"za{i}"])
-            x_in = ws["h_in0"] if i == 0 else ws[f"p{i - 1}"]
-            self._grads(f"enc{i}a", x_in, ws[f"dza{i}"])
-            if i > 0:
-                self._dgrad(f"enc{i}a", ws[f"dza{i}"], ws[f"dp{i - 1}"])
+        if "backward_ops" not in ws:
+            ws["backward_ops"] = self._backward_ops(B, ws)
+        oplist = ws["backward_ops"]
+        oplist[len(oplist) - 2].p[0] = ws["h_in0"].data_ptr()  # enc0a's weight gradient reads the input
+        ops.run(oplist)
 
     def loss_and_grad(self, x, target):
         """Forward, MSE loss against target [B, L, 600] and gradients in self.g (scaled by

@@ -22,6 +22,16 @@ class SurrogateKernelError(RuntimeError):
     pass
 
 
+class Op(C.Structure):
+    """msur_op: one operation of a list (run)."""
+
+    _fields_ = [("kind", C.c_int), ("form", C.c_int), ("stages", C.c_int), ("f", C.c_float), ("i", C.c_int * 12),
+                ("rows", C.c_uint64), ("p", C.c_void_p * 10)]
+
+
+(OP_CONV, OP_WGRAD, OP_BIAS_GRAD, OP_POOL2, OP_SKIP_GRAD, OP_UPCAT, OP_UPCAT_BWD, OP_MSE, OP_ZERO) = range(9)
+
+
 def load(path=LIB_PATH):
     global _lib
     if _lib is not None:
@@ -43,11 +53,13 @@ def load(path=LIB_PATH):
         "msur_mse": (i32, [vp, i32, vp, i32, u64, i32, vp, i32, f32, vp, vp]),
         "msur_adam": (i32, [vp, vp, vp, vp, u64, f32, f32, f32, f32, f32, i32, f32, vp, vp]),
         "msur_weight_transpose": (i32, [vp, i32, i32, i32, vp, vp]),
+        "msur_run": (i32, [C.POINTER(Op), i32, vp]),
         "msur_weight_transpose_list": (i32, [i32, C.POINTER(vp), C.POINTER(i32), C.POINTER(i32), C.POINTER(i32),
                                              C.POINTER(vp), vp]),
         "msur_assemble_input": (i32, [vp, vp, i32, i32, i32, vp, vp]),
         "msur_band_target": (i32, [vp, u64, i32, vp, vp]),
         "msur_map_sums": (i32, [vp, u64, vp, u64, u64, i32, vp, vp, vp]),
+        "msur_map_sums_of": (i32, [C.c_uint, vp, u64, vp, u64, u64, i32, vp, vp, vp]),
         "msur_compact_rows": (i32, [vp, i32, u64, i32, vp, vp]),
         "msur_conv_set_stages": (i32, [i32, i32]),
         "msur_conv_get_stages": (i32, [i32]),
@@ -177,6 +189,37 @@ def weight_transpose(w, wt):
     _check(load().msur_weight_transpose(_p(w), N, taps, Cw, _p(wt), _stream()), "msur_weight_transpose")
 
 
+def op(kind, tensors, ints, rows=0, f=0.0, form=-1, stages=-1):
+    """One Op: tensors (or None) and integers in msur_op's order.  Holds addresses only: the caller keeps the
+    tensors alive for as long as the operation is run."""
+    o = Op(kind, form, stages, f)
+    o.rows = rows
+    for k, t in enumerate(tensors):
+        o.p[k] = _p(t)
+    for k, v in enumerate(ints):
+        o.i[k] = v
+    return o
+
+
+def conv_op(x, w, bias=None, act=ACT_NONE, pre=None, post=None, f32=None, gate=None, skip=None, dup=None, pool=None,
+            form=-1, stages=-1):
+    """conv_forward / conv_forward_fused as an Op (outputs dense, the copies row-strided views)."""
+    B, L, Cin = x.shape
+    Cout, taps, Cin_w = w.shape
+    assert Cin_w == Cin and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
+    outs = [t for t in (pre, post, f32) if t is not None]
+    stride = outs[0].shape[-1] if outs else Cout
+    row = lambda t: t.stride(1) if t is not None else 0  # noqa: E731
+    return op(OP_CONV, (x, w, bias, pre, post, f32, gate, skip, dup, pool),
+              (B, L, Cin, Cout, taps, act, stride, min(Cout, stride), row(skip), row(dup), row(pool)),
+              form=form, stages=stages)
+
+
+def run(oplist):
+    """Enqueue a list of operations (a ctypes array of Op) on the current stream."""
+    _check(load().msur_run(oplist, len(oplist), _stream()), "msur_run")
+
+
 class TransposeList:
     """The weight transposes of several convolutions, [(w, wt), ...], as one launch (run); the tensors are
     kept alive and must not be reallocated."""
@@ -205,11 +248,14 @@ def band_target(band, ncols, nrows, out):
     _check(load().msur_band_target(_p(band), ncols, nrows, _p(out), _stream()), "msur_band_target")
 
 
-def map_sums(pred, ref, n, nmaps, out, pstride=None, rstride=None, means=None):
+SUMS_RAW, SUMS_CENTRED, SUMS_ALL = 0x2B, 0x1F, 0x3F  # MSUR_SUMS_*
+
+
+def map_sums(pred, ref, n, nmaps, out, pstride=None, rstride=None, means=None, which=SUMS_ALL):
     pstride = pstride if pstride is not None else n
     rstride = rstride if rstride is not None else n
-    _check(load().msur_map_sums(_p(pred), pstride, _p(ref), rstride, n, nmaps, _p(means), _p(out), _stream()),
-           "msur_map_sums")
+    _check(load().msur_map_sums_of(which, _p(pred), pstride, _p(ref), rstride, n, nmaps, _p(means), _p(out),
+                                   _stream()), "msur_map_sums")
 
 
 def map_scores(pred, ref, n, nmaps, pstride=None, rstride=None):
@@ -218,14 +264,14 @@ def map_scores(pred, ref, n, nmaps, pstride=None, rstride=None):
     ||p - r|| / ||r||, both in FP64 on the device.  Returns two numpy arrays of nmaps values."""
     dev = pred.device
     s1 = torch.zeros(nmaps, 6, dtype=torch.float64, device=dev)
-    map_sums(pred, ref, n, nmaps, s1, pstride, rstride)
+    map_sums(pred, ref, n, nmaps, s1, pstride, rstride, which=SUMS_RAW)
     means = (s1[:, :2] / n).contiguous()
     s2 = torch.zeros(nmaps, 6, dtype=torch.float64, device=dev)
-    map_sums(pred, ref, n, nmaps, s2, pstride, rstride, means=means)
+    map_sums(pred, ref, n, nmaps, s2, pstride, rstride, means=means, which=SUMS_CENTRED)
     s2 = s2.cpu().numpy()
     raw = s1.cpu().numpy()
     r = np.clip(s2[:, 4] / np.sqrt(s2[:, 2] * s2[:, 3]), -1.0, 1.0)
-    rel_l2 = np.sqrt(s2[:, 5] / raw[:, 3])
+    rel_l2 = np.sqrt(raw[:, 5] / raw[:, 3])
     return r, rel_l2
 
 
