@@ -345,6 +345,8 @@ __global__ void __launch_bounds__(THREADS, 1) conv_fwd_kernel(const __grid_const
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
+  umma::pdl_wait();
+  umma::pdl_trigger();
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
@@ -464,6 +466,8 @@ __global__ void __launch_bounds__(THREADS, 1) conv_fwd_persistent_kernel(const _
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
+  umma::pdl_wait();
+  umma::pdl_trigger();
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
@@ -633,6 +637,8 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_kernel(const __grid_constant
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
+  umma::pdl_wait();
+  umma::pdl_trigger();
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
@@ -814,6 +820,8 @@ __device__ __forceinline__ void st8(bf16* p, const float (&f)[8]) {
 }
 
 __global__ void pool2_v8_kernel(const bf16* x, int B, int Lout, int C, bf16* y) {
+  umma::pdl_wait();
+  umma::pdl_trigger();
   const int C8 = C / 8;
   const size_t n = static_cast<size_t>(B) * Lout * C8;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -831,6 +839,8 @@ __global__ void pool2_v8_kernel(const bf16* x, int B, int Lout, int C, bf16* y) 
 
 __global__ void skip_grad_v8_kernel(const bf16* dpool, int Lp, const bf16* dcat, int cat_stride, int cat_off,
                                     const bf16* z, int B, int L, int C, bf16* dz) {
+  umma::pdl_wait();
+  umma::pdl_trigger();
   const int C8 = C / 8;
   const size_t n = static_cast<size_t>(B) * L * C8;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -857,6 +867,8 @@ __global__ void skip_grad_v8_kernel(const bf16* dpool, int Lp, const bf16* dcat,
 }
 
 __global__ void upcat_v8_kernel(const bf16* x, const bf16* skip, int B, int L, int C1, int C2, bf16* out) {
+  umma::pdl_wait();
+  umma::pdl_trigger();
   const int C = C1 + C2, C8 = C / 8;
   const size_t n = static_cast<size_t>(B) * L * C8;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -870,6 +882,8 @@ __global__ void upcat_v8_kernel(const bf16* x, const bf16* skip, int B, int L, i
 }
 
 __global__ void upcat_bwd_v8_kernel(const bf16* dcat, const bf16* z, int B, int Lh, int C1, int C, bf16* dz) {
+  umma::pdl_wait();
+  umma::pdl_trigger();
   const int C8 = C1 / 8;
   const size_t n = static_cast<size_t>(B) * Lh * C8;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
@@ -930,6 +944,8 @@ __device__ __forceinline__ void exact_difference(float a, float b, float& h, flo
 // the memory's rate (the scalar form above took 1.0 of a batch-16 gradient's 4.9 ms of kernel time).
 __global__ void __launch_bounds__(256) bias_grad_v8_kernel(const bf16* __restrict__ dz, size_t rows, int C,
                                                            int stride, float* db) {
+  umma::pdl_wait();
+  umma::pdl_trigger();
   const int g = threadIdx.x & 7, y = threadIdx.x >> 3;
   const int c = blockIdx.x * 64 + g * 8;
   float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -997,6 +1013,8 @@ template <typename I>
 __global__ void __launch_bounds__(256) mse_v4_kernel(const float* __restrict__ pred, int pstride,
                                                      const float* __restrict__ target, int tstride, size_t rows,
                                                      int n_valid, bf16* dp, int dstride, float scale, double* loss) {
+  umma::pdl_wait();
+  umma::pdl_trigger();
   const I q = dstride / 4;  // groups of four channels per row
   const I n = static_cast<I>(rows) * q, step = static_cast<I>(gridDim.x) * blockDim.x;
   double acc = 0.0;
@@ -1170,6 +1188,8 @@ __global__ void assemble_input_kernel(const float* track, const float* params, i
 template <typename I>
 __global__ void __launch_bounds__(256) assemble_input_v8_kernel(const float* track, const float* params, int B, int L,
                                                                 int C, uint4* x) {
+  umma::pdl_wait();
+  umma::pdl_trigger();
   const I C8 = C / 8, n = static_cast<I>(B) * L * C8;
   for (I i = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x; i < n; i += static_cast<I>(gridDim.x) * blockDim.x) {
     const I bl = i / C8;
@@ -1450,6 +1470,24 @@ constexpr int conv_smem() {
   return STAGES * (BM * BK * 2 + BN * BK * 2) + 1024 + (STAGED ? 1024 + STAGE_OUT_BYTES : 256);
 }
 
+// Launch as a programmatic dependent of the stream's previous kernel: set-up and launch latency overlap
+// its tail (the 23 convolutions of one map: 277 to 227 us; gradients of 16 maps:
+// 1.66 to 1.47 ms; a single convolution called again and again: 35.6 to 34.1 us).  Only kernels that begin with pdl_wait.
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, int threads, int smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // Once per kernel and device: the shared-memory permission and the CTAs that fit an SM (asking the runtime
 // on every launch took longer than the launch).
 struct KernelLimits {
@@ -1483,8 +1521,8 @@ int launch_conv(const ConvArgs& a, int ntiles_n, cudaStream_t st) {
   const int rc = limits.get(reinterpret_cast<const void*>(kern), smem, &lim);
   if (rc) return rc;
   dim3 grid(ntiles_n, (a.L + BM - 1) / BM, a.B);
-  kern<<<grid, THREADS, smem, st>>>(a);
-  return cuda_ok(cudaGetLastError(), "conv_fwd_kernel launch");
+  return cuda_ok(launch_pdl(kern, grid, THREADS, smem, st, a),
+                 "conv_fwd_kernel launch");
 }
 
 template <int BN, int STAGES, bool STAGED>
@@ -1502,8 +1540,8 @@ int launch_conv_persistent(const ConvArgs& a, int ntn, cudaStream_t st) {
   const int ntl = (a.L + BM - 1) / BM;
   const int ntiles = ntn * ntl * a.B;
   const int grid = std::min(ntiles, sms * per_sm);
-  kern<<<grid, THREADS, smem, st>>>(a, ntn, ntl, ntiles);
-  return cuda_ok(cudaGetLastError(), "conv_fwd_persistent_kernel launch");
+  return cuda_ok(launch_pdl(kern, dim3(grid), THREADS, smem, st, a, ntn, ntl, ntiles),
+                 "conv_fwd_persistent_kernel launch");
 }
 
 template <int BN, int STAGES>
@@ -1531,8 +1569,8 @@ int launch_wgrad(const WgradArgs& a, int splits, cudaStream_t st) {
   const int rc = limits.get(reinterpret_cast<const void*>(kern), smem, &lim);
   if (rc) return rc;
   dim3 grid((a.Cin + BN - 1) / BN, (a.Cout + BM - 1) / BM, splits);
-  kern<<<grid, THREADS, smem, st>>>(a);
-  return cuda_ok(cudaGetLastError(), "wgrad_kernel launch");
+  return cuda_ok(launch_pdl(kern, grid, THREADS, smem, st, a),
+                 "wgrad_kernel launch");
 }
 
 unsigned grid_for(size_t n, unsigned block = 256) {
@@ -1752,9 +1790,10 @@ int msur_pool2(const void* x, int B, int Lout, int C, void* y, void* stream) {
   if (!x || !y || B <= 0 || Lout <= 0 || C <= 0) return fail(MSUR_ERR_INVALID_ARG, "msur_pool2: bad argument");
   const size_t n = static_cast<size_t>(B) * Lout * C;
   if (C % 8 == 0 && aligned16(x) && aligned16(y)) {
-    pool2_v8_kernel<<<grid_for(n / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const bf16*>(x), B,
-                                                                                   Lout, C, static_cast<bf16*>(y));
-    return cuda_ok(cudaGetLastError(), "pool2_v8_kernel launch");
+    return cuda_ok(launch_pdl(pool2_v8_kernel, dim3(grid_for(n / 8)), 256, 0,
+                              static_cast<cudaStream_t>(stream), static_cast<const bf16*>(x), B, Lout, C,
+                              static_cast<bf16*>(y)),
+                   "pool2_v8_kernel launch");
   }
   pool2_kernel<<<grid_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const bf16*>(x), B, Lout, C,
                                                                            static_cast<bf16*>(y));
@@ -1767,10 +1806,11 @@ int msur_skip_grad(const void* dpool, int Lp, const void* dcat, int cat_stride, 
   const size_t n = static_cast<size_t>(B) * L * C;
   if (C % 8 == 0 && cat_stride % 8 == 0 && cat_off % 8 == 0 && aligned16(z) && aligned16(dz) &&
       (!dpool || aligned16(dpool)) && (!dcat || aligned16(dcat))) {
-    skip_grad_v8_kernel<<<grid_for(n / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const bf16*>(dpool), Lp, static_cast<const bf16*>(dcat), cat_stride, cat_off,
-        static_cast<const bf16*>(z), B, L, C, static_cast<bf16*>(dz));
-    return cuda_ok(cudaGetLastError(), "skip_grad_v8_kernel launch");
+    return cuda_ok(launch_pdl(skip_grad_v8_kernel, dim3(grid_for(n / 8)), 256, 0,
+                              static_cast<cudaStream_t>(stream), static_cast<const bf16*>(dpool), Lp,
+                              static_cast<const bf16*>(dcat), cat_stride, cat_off,
+                              static_cast<const bf16*>(z), B, L, C, static_cast<bf16*>(dz)),
+                   "skip_grad_v8_kernel launch");
   }
   skip_grad_kernel<<<grid_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const bf16*>(dpool), Lp, static_cast<const bf16*>(dcat), cat_stride, cat_off,
@@ -1782,9 +1822,10 @@ int msur_upcat(const void* x, const void* skip, int B, int L, int C1, int C2, vo
   if (!x || !skip || !out || B <= 0 || L <= 0 || (L % 2)) return fail(MSUR_ERR_INVALID_ARG, "msur_upcat: bad argument");
   const size_t n = static_cast<size_t>(B) * L * (C1 + C2);
   if (C1 % 8 == 0 && C2 % 8 == 0 && aligned16(x) && aligned16(skip) && aligned16(out)) {
-    upcat_v8_kernel<<<grid_for(n / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const bf16*>(x), static_cast<const bf16*>(skip), B, L, C1, C2, static_cast<bf16*>(out));
-    return cuda_ok(cudaGetLastError(), "upcat_v8_kernel launch");
+    return cuda_ok(launch_pdl(upcat_v8_kernel, dim3(grid_for(n / 8)), 256, 0,
+                              static_cast<cudaStream_t>(stream), static_cast<const bf16*>(x),
+                              static_cast<const bf16*>(skip), B, L, C1, C2, static_cast<bf16*>(out)),
+                   "upcat_v8_kernel launch");
   }
   upcat_kernel<<<grid_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const bf16*>(x), static_cast<const bf16*>(skip), B, L, C1, C2, static_cast<bf16*>(out));
@@ -1795,9 +1836,10 @@ int msur_upcat_bwd(const void* dcat, const void* z, int B, int Lh, int C1, int C
   if (!dcat || !z || !dz || B <= 0 || Lh <= 0 || C1 > C) return fail(MSUR_ERR_INVALID_ARG, "msur_upcat_bwd: bad argument");
   const size_t n = static_cast<size_t>(B) * Lh * C1;
   if (C1 % 8 == 0 && C % 8 == 0 && aligned16(dcat) && aligned16(z) && aligned16(dz)) {
-    upcat_bwd_v8_kernel<<<grid_for(n / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const bf16*>(dcat), static_cast<const bf16*>(z), B, Lh, C1, C, static_cast<bf16*>(dz));
-    return cuda_ok(cudaGetLastError(), "upcat_bwd_v8_kernel launch");
+    return cuda_ok(launch_pdl(upcat_bwd_v8_kernel, dim3(grid_for(n / 8)), 256, 0,
+                              static_cast<cudaStream_t>(stream), static_cast<const bf16*>(dcat),
+                              static_cast<const bf16*>(z), B, Lh, C1, C, static_cast<bf16*>(dz)),
+                   "upcat_bwd_v8_kernel launch");
   }
   upcat_bwd_kernel<<<grid_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const bf16*>(dcat), static_cast<const bf16*>(z), B, Lh, C1, C, static_cast<bf16*>(dz));
@@ -1811,9 +1853,9 @@ int msur_bias_grad(const void* dz, uint64_t rows, int C, int stride, float* db, 
     const unsigned gx = (C + 63) / 64;
     const uint64_t most = (rows + 127) / 128;
     const unsigned gy = static_cast<unsigned>(std::min<uint64_t>(std::max(1u, 4 * 152 / gx), most ? most : 1));
-    bias_grad_v8_kernel<<<dim3(gx, gy), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const bf16*>(dz),
-                                                                                     rows, C, stride, db);
-    return cuda_ok(cudaGetLastError(), "bias_grad_v8_kernel launch");
+    return cuda_ok(launch_pdl(bias_grad_v8_kernel, dim3(gx, gy), 256, 0, static_cast<cudaStream_t>(stream),
+                              static_cast<const bf16*>(dz), rows, C, stride, db),
+                   "bias_grad_v8_kernel launch");
   }
   dim3 block(32, 8);
   const uint64_t gy = (rows + 8 * 64 - 1) / (8 * 64);
@@ -1833,13 +1875,14 @@ int msur_mse(const float* pred, int pstride, const float* target, int tstride, u
     const unsigned blocks = std::min(grid_for(n / 4), 152u * 8u);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (n / 4 < (1ull << 31)) {
-      mse_v4_kernel<unsigned><<<blocks, 256, 0, st>>>(pred, pstride, target, tstride, rows, n_valid,
-                                                      static_cast<bf16*>(dp), dstride, scale, loss);
+      return cuda_ok(launch_pdl(mse_v4_kernel<unsigned>, dim3(blocks), 256, 0, st, pred, pstride, target,
+                                tstride, rows, n_valid, static_cast<bf16*>(dp), dstride, scale, loss),
+                     "mse_v4_kernel launch");
     } else {
-      mse_v4_kernel<size_t><<<blocks, 256, 0, st>>>(pred, pstride, target, tstride, rows, n_valid,
-                                                    static_cast<bf16*>(dp), dstride, scale, loss);
+      return cuda_ok(launch_pdl(mse_v4_kernel<size_t>, dim3(blocks), 256, 0, st, pred, pstride, target,
+                                tstride, rows, n_valid, static_cast<bf16*>(dp), dstride, scale, loss),
+                     "mse_v4_kernel launch");
     }
-    return cuda_ok(cudaGetLastError(), "mse_v4_kernel launch");
   }
   mse_kernel<<<grid_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(pred, pstride, target, tstride, rows, n_valid,
                                                                          static_cast<bf16*>(dp), dstride, scale, loss);
@@ -1950,11 +1993,14 @@ int msur_assemble_input(const float* track, const float* params, int B, int L, i
   if (aligned16(x)) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (n / 8 < (1ull << 31)) {
-      assemble_input_v8_kernel<unsigned><<<grid_for(n / 8), 256, 0, st>>>(track, params, B, L, C, static_cast<uint4*>(x));
+      return cuda_ok(launch_pdl(assemble_input_v8_kernel<unsigned>, dim3(grid_for(n / 8)), 256, 0, st,
+                                track, params, B, L, C, static_cast<uint4*>(x)),
+                     "assemble_input_v8_kernel launch");
     } else {
-      assemble_input_v8_kernel<size_t><<<grid_for(n / 8), 256, 0, st>>>(track, params, B, L, C, static_cast<uint4*>(x));
+      return cuda_ok(launch_pdl(assemble_input_v8_kernel<size_t>, dim3(grid_for(n / 8)), 256, 0, st, track,
+                                params, B, L, C, static_cast<uint4*>(x)),
+                     "assemble_input_v8_kernel launch");
     }
-    return cuda_ok(cudaGetLastError(), "assemble_input_v8_kernel launch");
   }
   assemble_input_kernel<<<grid_for(n), 256, 0, static_cast<cudaStream_t>(stream)>>>(track, params, B, L, C,
                                                                                    static_cast<bf16*>(x));

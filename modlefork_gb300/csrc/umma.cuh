@@ -89,6 +89,13 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
       : "memory");
 }
 
+// ---- programmatic dependent launch ----------------------------------------------------------
+// A kernel launched as a dependent may start while its predecessor in the stream still runs:
+// pdl_wait returns once the predecessor has completed and its writes are visible, so it comes before the
+// first access to global memory; pdl_trigger lets the next kernel start its own set-up.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- tensor memory ----------------------------------------------------------------------
 // One full warp: allocate ncols (a power of two >= 32) TMEM columns; the address lands in *slot.
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
