@@ -156,7 +156,7 @@ int msur_map_sums_of(unsigned which, const float* pred, uint64_t pstride_map, co
 int msur_compact_rows(const float* in, int stride, uint64_t rows, int n_valid, float* out, void* stream);
 
 /* A list of the operations above in one call, enqueued in order: a network's pass without a foreign-function
- * call per layer.  p, i, f and rows hold the operation's arguments in the order of its function:
+ * call per layer.  p, i and rows hold the operation's arguments in the order of its function:
  *   CONV      p: x w bias out_pre out_post out_f32 gate out_skip out_dup out_pool;
  *             i: B L Cin Cout taps act out_stride n_valid skip_stride dup_stride pool_stride;
  *             form and stages: the kernel form and depth, -1 for the width's current settings
@@ -166,16 +166,13 @@ int msur_compact_rows(const float* in, int stride, uint64_t rows, int n_valid, f
  *   SKIP_GRAD p: dpool dcat z dz; i: Lp cat_stride cat_off B L C
  *   UPCAT     p: x skip out; i: B L C1 C2
  *   UPCAT_BWD p: dcat z dz; i: B Lh C1 C
- *   MSE       p: pred target dp loss; i: pstride tstride n_valid dstride; rows; f: scale
- *   ZERO      p: buffer; rows: bytes
  * Stops at the first operation that fails and returns its status. */
 enum {
   MSUR_OP_CONV = 0, MSUR_OP_WGRAD, MSUR_OP_BIAS_GRAD, MSUR_OP_POOL2, MSUR_OP_SKIP_GRAD, MSUR_OP_UPCAT,
-  MSUR_OP_UPCAT_BWD, MSUR_OP_MSE, MSUR_OP_ZERO
+  MSUR_OP_UPCAT_BWD
 };
 typedef struct msur_op {
   int kind, form, stages;
-  float f;
   int i[12];
   uint64_t rows;
   void* p[10];

@@ -32,6 +32,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "../../include/mgpu_surrogate.h"
 #include "umma.cuh"
@@ -49,11 +50,19 @@ enum : unsigned { ERR_PRODUCER = 1u, ERR_MMA = 2u, ERR_EPILOGUE = 4u };
 __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
   return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
 }
-// SiLU and its derivative with the fast reciprocal-based division (within 2 ulp; the result is
-// 0 when 1 + exp(-z) overflows, the limit of both): the epilogues evaluate one per output element.
-__device__ __forceinline__ float silu(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
+// The logistic function as two hardware approximations (relative error about 2^-22), SiLU and its
+// derivative: the epilogues evaluate one per output element.  Flushing subnormals loses nothing here: added to 1
+// a subnormal exponential vanishes, and the reciprocal of a sum above 2^126 is 0, the limit (as in
+// __fdividef, whose results these are bit for bit at a third of the instructions of __fdividef(z, 1 + __expf(-z))).
+__device__ __forceinline__ float logistic(float z) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.44269504088896340736f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+  return r;
+}
+__device__ __forceinline__ float silu(float z) { return z * logistic(z); }
 __device__ __forceinline__ float dsilu(float z) {
-  const float s = __fdividef(1.0f, 1.0f + __expf(-z));
+  const float s = logistic(z);
   return s * (1.0f + z * (1.0f - s));
 }
 
@@ -171,15 +180,18 @@ __device__ __forceinline__ void conv_epilogue_chunk(const ConvArgs& a, float (&v
   }
 }
 
-// One 32-row x 128-byte box goes through this warp's staging buffer (two 4 KB buffers used in
+// One 32-row x 128-byte box goes through this warp's staging buffer (one or two 4 KB buffers used in
 // turn; nb counts the warp's stores).  stage_begin waits until the buffer's previous store has
 // read it; the lanes then write their rows with the 128-byte swizzle (16-byte unit k of row r at
 // unit k ^ (r % 8), which also keeps the eight lanes of each vector store on distinct banks);
 // stage_end makes the writes visible to the bulk-copy proxy and lane 0 issues the TMA store.
-__device__ __forceinline__ uint8_t* stage_begin(uint8_t* stg, int nb) {
-  if (nb >= 2 && (threadIdx.x & 31) == 0) umma::bulk_wait_read<1>();
+__device__ __forceinline__ uint8_t* stage_begin(uint8_t* stg, int nb, int bufs) {
+  if (nb >= bufs && umma::elect()) {
+    if (bufs == 2) umma::bulk_wait_read<1>();
+    else umma::bulk_wait_read<0>();
+  }
   __syncwarp();
-  return stg + (nb & 1) * 4096;
+  return stg + (bufs == 2 ? (nb & 1) * 4096 : 0);
 }
 __device__ __forceinline__ void stage_put(uint8_t* buf, int k, uint4 w) {
   const int lane = threadIdx.x & 31;
@@ -188,7 +200,7 @@ __device__ __forceinline__ void stage_put(uint8_t* buf, int k, uint4 w) {
 __device__ __forceinline__ void stage_end(const CUtensorMap* map, uint8_t* buf, int& nb, int x, int y, int z) {
   umma::fence_async_smem();
   __syncwarp();
-  if ((threadIdx.x & 31) == 0) {
+  if (umma::elect()) {
     umma::tma_store_3d(map, buf, x, y, z);
     umma::bulk_commit();
   }
@@ -200,116 +212,145 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&p);
 }
 
-// Staged epilogue of one tile row block (32 rows y .. y+31 of sequence z, columns n0 .. n0+BN):
-// per 64-column unit, bias, then the FP32 (two boxes), pre-activation and post-activation (one
-// box each) outputs through shared memory and TMA.  Rows >= L and columns >= n_valid are dropped
-// by the stores.  Collective over the warp; the caller waits for the stores (bulk_wait_all)
-// before the block exits.
-template <int BN>
-__device__ void conv_epilogue_staged(const ConvArgs& a, uint32_t tmem_row, uint8_t* stg, int& nb, int n0, int y,
-                                     int z) {
-#pragma unroll 1
-  for (int u = 0; u < BN / 64; ++u) {
-    float v[64];
-    umma::tmem_ld32(tmem_row + u * 64, *reinterpret_cast<float(*)[32]>(v));
-    umma::tmem_ld32(tmem_row + u * 64 + 32, *reinterpret_cast<float(*)[32]>(v + 32));
-    const int col0 = n0 + u * 64;
-    if (y >= a.L || col0 >= a.n_valid) continue;
-    if (a.bias) {
-      const int nv = min(64, a.n_valid - col0);
-      if (nv == 64 && (reinterpret_cast<uintptr_t>(a.bias) & 15u) == 0) {
-        const float4* b4 = reinterpret_cast<const float4*>(a.bias + col0);
+// 32 columns (col0 ..) of this thread's row as the epilogue's value: accumulator, bias, gated SiLU derivative.
+__device__ __forceinline__ void conv_value32(const ConvArgs& a, uint32_t tmem_cols32, const bf16* gate, int col0,
+                                             float (&v)[32]) {
+  umma::tmem_ld32(tmem_cols32, v);
+  const int nv = a.n_valid - col0;
+  if (a.bias) {
+    if (nv >= 32 && (reinterpret_cast<uintptr_t>(a.bias) & 15u) == 0) {
+      const float4* b4 = reinterpret_cast<const float4*>(a.bias + col0);
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          const float4 bb = __ldg(b4 + k);
-          v[4 * k] += bb.x;
-          v[4 * k + 1] += bb.y;
-          v[4 * k + 2] += bb.z;
-          v[4 * k + 3] += bb.w;
+      for (int k = 0; k < 8; ++k) {
+        const float4 bb = __ldg(b4 + k);
+        v[4 * k] += bb.x;
+        v[4 * k + 1] += bb.y;
+        v[4 * k + 2] += bb.z;
+        v[4 * k + 3] += bb.w;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] += (j < nv) ? __ldg(a.bias + col0 + j) : 0.0f;
+    }
+  }
+  if (gate) {
+    if (nv >= 32) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint4 u = __ldg(reinterpret_cast<const uint4*>(gate) + k);
+        const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          const __nv_bfloat162 g2 = *reinterpret_cast<const __nv_bfloat162*>(&w4[h]);
+          v[8 * k + 2 * h] *= dsilu(__low2float(g2));
+          v[8 * k + 2 * h + 1] *= dsilu(__high2float(g2));
         }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 64; ++j) v[j] += (j < nv) ? __ldg(a.bias + col0 + j) : 0.0f;
       }
-    }
-    if (a.out_f32) {
+    } else {
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        if (col0 + 32 * h >= a.n_valid) break;
-        uint8_t* buf = stage_begin(stg, nb);
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          stage_put(buf, k,
-                    make_uint4(__float_as_uint(v[32 * h + 4 * k]), __float_as_uint(v[32 * h + 4 * k + 1]),
-                               __float_as_uint(v[32 * h + 4 * k + 2]), __float_as_uint(v[32 * h + 4 * k + 3])));
-        stage_end(&a.tm_f32, buf, nb, col0 + 32 * h, y, z);
-      }
+      for (int j = 0; j < 32; ++j)
+        if (j < nv) v[j] *= dsilu(__bfloat162float(gate[j]));
     }
-    if (a.out_pre) {
-      uint8_t* buf = stage_begin(stg, nb);
+  }
+}
+
+// Staged epilogue of one unit: 32 rows (y .. y+31 of sequence z) x 64 columns from col0: the FP32 (two boxes),
+// pre-activation and post-activation (one box each) outputs through shared memory and TMA.  Rows >= L and
+// columns >= n_valid are dropped by the stores.  Collective over the warp; the caller waits for the
+// stores (staged_drain) before the block exits.
+//
+// One pass over the accumulator per output, 32 columns at a time: a warp comes through here once per tile, so what
+// it runs has to be short loops.  As straight code over 64 columns and all outputs at once the fetches bound
+// it: 8100 cycles for 128 columns, of which 5300 with every memory operation and all arithmetic left out.
+__device__ __forceinline__ void conv_epilogue_unit(const ConvArgs& a, uint32_t tmem_unit, uint8_t* stg, int bufs,
+                                                   int& nb, int col0, int y, int z) {
+  if (y >= a.L || col0 >= a.n_valid) return;
+  const int lane = threadIdx.x & 31;
+  // rows past the end read the last row's gate; their values are dropped
+  const bf16* gate = a.gate ? a.gate + (static_cast<size_t>(z) * a.L + min(y + lane, a.L - 1)) * a.out_stride + col0
+                            : nullptr;
+  if (a.out_f32) {
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+      if (col0 + 32 * h >= a.n_valid) break;
+      float v[32];
+      conv_value32(a, tmem_unit + 32 * h, gate ? gate + 32 * h : nullptr, col0 + 32 * h, v);
+      uint8_t* buf = stage_begin(stg, nb, bufs);
 #pragma unroll
       for (int k = 0; k < 8; ++k)
-        stage_put(buf, k,
+        stage_put(buf, k, make_uint4(__float_as_uint(v[4 * k]), __float_as_uint(v[4 * k + 1]),
+                                     __float_as_uint(v[4 * k + 2]), __float_as_uint(v[4 * k + 3])));
+      stage_end(&a.tm_f32, buf, nb, col0 + 32 * h, y, z);
+    }
+  }
+  const bool post = a.out_post || a.has_skip || a.has_dup || a.has_pool;
+#pragma unroll 1
+  for (int out = a.out_pre ? 0 : 1; out < (post ? 2 : 1); ++out) {
+    uint8_t* buf = stage_begin(stg, nb, bufs);
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+      float v[32];
+      conv_value32(a, tmem_unit + 32 * h, gate ? gate + 32 * h : nullptr, col0 + 32 * h, v);
+      if (out == 1 && a.act == MSUR_ACT_SILU) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = silu(v[j]);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        stage_put(buf, 4 * h + k,
                   make_uint4(pack_bf16x2(v[8 * k], v[8 * k + 1]), pack_bf16x2(v[8 * k + 2], v[8 * k + 3]),
                              pack_bf16x2(v[8 * k + 4], v[8 * k + 5]), pack_bf16x2(v[8 * k + 6], v[8 * k + 7])));
-      stage_end(&a.tm_pre, buf, nb, col0, y, z);
     }
-    if (a.out_post || a.has_skip || a.has_dup || a.has_pool) {
-      if (a.act == MSUR_ACT_SILU) {
-#pragma unroll
-        for (int j = 0; j < 64; ++j) v[j] = silu(v[j]);
-      }
-      uint32_t pk[32];  // this row's 64 BF16 values in pairs
-#pragma unroll
-      for (int j = 0; j < 32; ++j) pk[j] = pack_bf16x2(v[2 * j], v[2 * j + 1]);
-      if (a.out_post || a.has_skip || a.has_dup) {
-        uint8_t* buf = stage_begin(stg, nb);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) stage_put(buf, k, make_uint4(pk[4 * k], pk[4 * k + 1], pk[4 * k + 2], pk[4 * k + 3]));
-        // one staged box, stored to every destination of the post-activation value
-        umma::fence_async_smem();
-        __syncwarp();
-        if ((threadIdx.x & 31) == 0) {
-          if (a.out_post) umma::tma_store_3d(&a.tm_post, buf, col0, y, z);
-          if (a.has_skip) umma::tma_store_3d(&a.tm_skip, buf, col0, y, z);
-          if (a.has_dup) {
-            umma::tma_store_3d(&a.tm_dup0, buf, col0, y, z);
-            umma::tma_store_3d(&a.tm_dup1, buf, col0, y, z);
-          }
-          umma::bulk_commit();
+    // one staged box, stored to every destination of its value
+    umma::fence_async_smem();
+    __syncwarp();
+    if (umma::elect()) {
+      if (out == 0) {
+        umma::tma_store_3d(&a.tm_pre, buf, col0, y, z);
+      } else {
+        if (a.out_post) umma::tma_store_3d(&a.tm_post, buf, col0, y, z);
+        if (a.has_skip) umma::tma_store_3d(&a.tm_skip, buf, col0, y, z);
+        if (a.has_dup) {
+          umma::tma_store_3d(&a.tm_dup0, buf, col0, y, z);
+          umma::tma_store_3d(&a.tm_dup1, buf, col0, y, z);
         }
-        ++nb;
       }
-      if (a.has_pool) {
-        // row pairs (2m, 2m + 1) sit on lanes (2m, 2m + 1): the even lane averages them and
-        // writes pooled row m of a 16-row box (y is a multiple of 32)
-        const int lane = threadIdx.x & 31;
-        uint8_t* buf = stage_begin(stg, nb);
+      umma::bulk_commit();
+    }
+    ++nb;
+    if (out == 1 && a.has_pool) {
+      // rows 2m and 2m + 1 of the staged box are averaged into row m of a 16-row box (y is a multiple of 32):
+      // 16 rows x 8 units of 16 bytes, four to a lane
+      uint4 w[4];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          uint32_t q[4];
+      for (int i = 0; i < 4; ++i) {
+        const int m = (lane >> 3) + 4 * i, k = lane & 7;
+        const uint4 p0 = *reinterpret_cast<const uint4*>(buf + 2 * m * 128 + ((k ^ ((2 * m) & 7)) << 4));
+        const uint4 p1 = *reinterpret_cast<const uint4*>(buf + (2 * m + 1) * 128 + ((k ^ ((2 * m + 1) & 7)) << 4));
+        const uint32_t x0[4] = {p0.x, p0.y, p0.z, p0.w}, x1[4] = {p1.x, p1.y, p1.z, p1.w};
+        uint32_t q[4];
 #pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            const uint32_t mine = pk[4 * k + h];
-            const uint32_t next = __shfl_down_sync(0xFFFFFFFFu, mine, 1);
-            const float2 fa = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&mine));
-            const float2 fb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&next));
-            q[h] = pack_bf16x2(0.5f * (fa.x + fb.x), 0.5f * (fa.y + fb.y));
-          }
-          if ((lane & 1) == 0) {
-            const int r = lane >> 1;
-            *reinterpret_cast<uint4*>(buf + r * 128 + ((k ^ (r & 7)) << 4)) = make_uint4(q[0], q[1], q[2], q[3]);
-          }
+        for (int h = 0; h < 4; ++h) {
+          const float2 fa = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x0[h]));
+          const float2 fb = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x1[h]));
+          q[h] = pack_bf16x2(0.5f * (fa.x + fb.x), 0.5f * (fa.y + fb.y));
         }
-        stage_end(&a.tm_pool, buf, nb, col0, y >> 1, z);
+        w[i] = make_uint4(q[0], q[1], q[2], q[3]);
       }
+      uint8_t* pbuf = stage_begin(stg, nb, bufs);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int m = (lane >> 3) + 4 * i, k = lane & 7;
+        *reinterpret_cast<uint4*>(pbuf + m * 128 + ((k ^ (m & 7)) << 4)) = w[i];
+      }
+      stage_end(&a.tm_pool, pbuf, nb, col0, y >> 1, z);
     }
   }
 }
 
 // Every TMA store of this warp has completed (before the block and its shared memory exit).
 __device__ __forceinline__ void staged_drain() {
-  if ((threadIdx.x & 31) == 0) umma::bulk_wait_all();
+  if (umma::elect()) umma::bulk_wait_all();
   __syncwarp();
 }
 
@@ -397,8 +438,10 @@ __global__ void __launch_bounds__(THREADS, 1) conv_fwd_kernel(const __grid_const
     if constexpr (STAGED) {
       if (ok) {
         int nb = 0;
-        conv_epilogue_staged<BN>(a, tmem + (static_cast<uint32_t>(32 * q) << 16),
-                                 smem + STAGES * STAGE_BYTES + 1024 + q * 8192, nb, n0, l0 + 32 * q, b);
+#pragma unroll 1
+        for (int u = 0; u < BN / 64; ++u)
+          conv_epilogue_unit(a, tmem + (static_cast<uint32_t>(32 * q) << 16) + u * 64,
+                             smem + STAGES * STAGE_BYTES + 1024 + q * 8192, 2, nb, n0 + u * 64, l0 + 32 * q, b);
         staged_drain();
       }
     } else if (ok) {
@@ -422,40 +465,180 @@ __global__ void __launch_bounds__(THREADS, 1) conv_fwd_kernel(const __grid_const
 
 // ---------------------------------------------------------------------------------------
 // The same convolution as a persistent kernel: each CTA walks tiles t = blockIdx.x,
-// blockIdx.x + gridDim.x, ... (N tile fastest, then position tile, then sequence) with a
-// double-buffered TMEM accumulator, so the epilogue of one tile overlaps the MMAs of the next
-// and a CTA's set-up (barriers, TMEM allocation, tensor-map prefetch) is paid once.
-// Barriers: full / empty per smem stage (TMA <-> MMA), tfull / tempty per accumulator
-// (MMA <-> the 128 epilogue threads), done (the MMA issuer's last commit).
+// blockIdx.x + gridDim.x, ... (N tile fastest, then position tile, then sequence) with two to eight
+// TMEM accumulators, so the epilogue of one tile overlaps the MMAs of the next and a CTA's
+// set-up (barriers, TMEM allocation, tensor-map prefetch) is paid once.
+//
+// What bounds it: with few input channels memory and the epilogue (two transcendental operations per element),
+// with many the operands' way from L2 to shared memory (about 70 bytes per clock and SM), between them the
+// MMA warp's own steps.  So
+//  - up to four groups of four epilogue warps take the 64-column units of the tiles in turn;
+//  - a tile's activations are loaded once for all taps (ConvPlan::aslots): the chunk of 64 input channels is
+//    kept as 128 + taps - 1 rows, and tap t's operand starts t rows into it;
+//  - weights whose K steps all fit stay for the CTA's life (ConvPlan::wres).
+// The order of the products (tap, then channel) is that of the plain form, so are the results.
+// 256 maps, with four epilogue warps, both operands by stage and single-thread loops / now: 192 to 64 channels
+// at 4000 positions 174 / 87 us, 128 to 128 at 2000 82 / 48, 384 to 128 at 2000 171 / 117, 896 to 384 at
+// 500 271 / 173 (with tiles of 192 columns instead of 128), 1024 to 512 at 250 129 / 117.
+//
+// Warps: 0 weights (and activations per K step without slots), 1 MMA and TMEM, 2 activation
+// slots, from 4 on the epilogue (warp w reads TMEM lanes 32 (w % 4) .. +31).
+// Barriers: full / empty per stage and afull / aempty per slot (TMA <-> MMA), tfull / tempty per
+// accumulator (MMA <-> epilogue warps), done (the MMA issuer's last commit).
 // ---------------------------------------------------------------------------------------
-template <int BN, int STAGES, bool STAGED>
-__global__ void __launch_bounds__(THREADS, 1) conv_fwd_persistent_kernel(const __grid_constant__ ConvArgs a, int ntn,
-                                                                         int ntl, int ntiles) {
-  constexpr int A_BYTES = BM * BK * 2;
-  constexpr int B_BYTES = BN * BK * 2;
-  constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  constexpr uint32_t TCOLS = tmem_cols<2 * BN>();
+constexpr int PTHREADS = 640;  // at most: four warps and up to four groups of four epilogue warps
+constexpr int SLOT_BYTES = (BM + 8) * BK * 2;  // a chunk of up to 8 more rows than the tile, 1 KB aligned
+constexpr int MAX_STAGES = 16, MAX_SLOTS = 12;
+
+struct ConvPlan {
+  int ntn, ntl, ntiles;
+  int stages;  // operand stages
+  int aslots;  // activation slots (0: activations travel with the weights, stage by stage)
+  int wres;    // stages == K steps: every CTA keeps one N tile and loads its weights once
+  int groups;  // groups of four epilogue warps
+  int bufs;    // 4 KB staging buffers per epilogue warp (0: epilogue without staging)
+};
+
+// Shared-memory addresses of the persistent kernel's barriers (arrays of 8 bytes) and buffers.
+struct ConvSmem {
+  uint32_t full, empty, afull, aempty, tfull, tempty, done, ring, slots;
+};
+
+// The MMA warp's loop.  What it issues runs behind it, so a step of the loop must not take longer than its
+// products (64 to 512 cycles per K step): addresses are stepped, the next stage's barrier is tested before the
+// step's products go out, and the first and last tap, which acquire and release slots, have loops of their own.
+template <int BN, int ACCS, bool ASLOTS, bool WRES>
+__device__ __forceinline__ void conv_mma_loop(const ConvArgs& a, const ConvPlan& p, const ConvSmem& m, uint32_t tmem,
+                                              int kc) {
+  constexpr uint32_t idesc = umma::idesc_bf16_f32(BM, BN, false, false);
+  constexpr uint32_t W_BYTES = BN * BK * 2, STAGE = W_BYTES + (ASLOTS ? 0 : BM * BK * 2);
+  const uint32_t full_end = m.full + 8 * p.stages;
+  const int taps = a.taps;
+  int acc = 0, base = 0;              // accumulator, slot of the tile's first chunk
+  uint32_t tph = 1, ph = 0, aph = 0;  // parities of the phases waited for
+  uint32_t fb = m.full, sb = m.ring;  // the stage's barrier and operands
+  uint32_t d = tmem, accumulate = 0;
+  bool first = true;
+  bool ready = !WRES && umma::mbar_test(fb, 0);
+  auto tap_loop = [&](auto acquire, auto release, int tap) {
+    uint32_t sa = m.slots + base * SLOT_BYTES + tap * (BK * 2), sl = 8 * base;
+    if (WRES && !first && !decltype(acquire)::value) {  // nothing to wait for
+      if (umma::elect()) {
+        uint32_t a_lo = umma::sdesc_sw128_lo(sa), b_lo = umma::sdesc_sw128_lo(sb);
+        for (int c = 0; c < kc; ++c) {
+          umma::mma_bf16_k64(d, a_lo, b_lo, idesc, 1);
+          if (decltype(release)::value) umma::mma_commit(m.aempty + sl + 8 * c);
+          a_lo += SLOT_BYTES / 16;
+          b_lo += W_BYTES / 16;
+        }
+      }
+      sb += kc * W_BYTES;
+      if (decltype(release)::value) fb = m.full, sb = m.ring;
+      return true;
+    }
+    for (int c = 0; c < kc; ++c) {
+      if (ASLOTS && decltype(acquire)::value)
+        if (!umma::mbar_wait_warp(m.afull + sl, aph, a.err, ERR_MMA)) return false;
+      if (WRES ? first : !__all_sync(0xFFFFFFFFu, ready))
+        if (!umma::mbar_wait_warp(fb, ph, a.err, ERR_MMA)) return false;
+      const uint32_t eb = fb + (m.empty - m.full);
+      const uint32_t b_lo = umma::sdesc_sw128_lo(sb), a_lo = umma::sdesc_sw128_lo(ASLOTS ? sa : sb + W_BYTES);
+      fb += 8;
+      sb += STAGE;
+      if (fb == full_end) fb = m.full, sb = m.ring, ph ^= 1;
+      if (!WRES) ready = umma::mbar_test(fb, ph);
+      if (umma::elect()) {
+        umma::mma_bf16_k64(d, a_lo, b_lo, idesc, accumulate);
+        if (!WRES) umma::mma_commit(eb);
+        if (ASLOTS && decltype(release)::value) umma::mma_commit(m.aempty + sl);
+      }
+      accumulate = 1;
+      sa += SLOT_BYTES;
+      sl += 8;
+    }
+    if (WRES && decltype(release)::value) fb = m.full, sb = m.ring;
+    return true;
+  };
+  const std::true_type yes;
+  const std::false_type no;
+  for (int t = blockIdx.x; t < p.ntiles; t += gridDim.x) {
+    if (!umma::mbar_wait_warp(m.tempty + 8 * acc, tph, a.err, ERR_MMA)) break;
+    umma::fence_after_sync();
+    d = tmem + acc * BN;
+    accumulate = 0;
+    bool ok = true;
+    if (!ASLOTS) {
+      for (int tap = 0; tap < taps && ok; ++tap) ok = tap_loop(no, no, tap);
+    } else if (taps == 1) {
+      ok = tap_loop(yes, yes, 0);
+    } else {
+      ok = tap_loop(yes, no, 0);
+      for (int tap = 1; tap < taps - 1 && ok; ++tap) ok = tap_loop(no, no, tap);
+      if (ok) ok = tap_loop(no, yes, taps - 1);
+    }
+    if (!ok) break;
+    if (umma::elect()) umma::mma_commit(m.tfull + 8 * acc);
+    if (++acc == ACCS) acc = 0, tph ^= 1;
+    if (ASLOTS && (base += kc) == p.aslots) base = 0, aph ^= 1;
+    first = false;
+  }
+  // every MMA this warp issued has completed before TMEM is released
+  if (umma::elect()) umma::mma_commit(m.done);
+  umma::mbar_wait_warp(m.done, 0, a.err, ERR_MMA);
+}
+
+// The tiles of a CTA one after the other, without dividing for each (four dependent divisions were a third of
+// a short tile's time).
+struct TileWalk {
+  int t, n, l, b, dn, dl, db;
+  __device__ explicit TileWalk(const ConvPlan& p)
+      : t(blockIdx.x), n(blockIdx.x % p.ntn), l((blockIdx.x / p.ntn) % p.ntl), b(blockIdx.x / (p.ntn * p.ntl)),
+        dn(gridDim.x % p.ntn), dl((gridDim.x / p.ntn) % p.ntl), db(gridDim.x / (p.ntn * p.ntl)) {}
+  __device__ void next(const ConvPlan& p) {
+    t += gridDim.x;
+    n += dn;
+    l += dl;
+    b += db;
+    if (n >= p.ntn) n -= p.ntn, ++l;
+    if (l >= p.ntl) l -= p.ntl, ++b;
+  }
+};
+
+template <int BN, bool STAGED>
+__global__ void __launch_bounds__(PTHREADS, 1)
+    conv_fwd_persistent_kernel(const __grid_constant__ ConvArgs a, const __grid_constant__ ConvPlan p) {
+  constexpr int W_BYTES = BN * BK * 2;
+  constexpr int ACCS = BN == 64 ? 8 : (BN == 128 ? 4 : 2);
+  constexpr uint32_t TCOLS = tmem_cols<ACCS * BN>();
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = align1024(smem_raw);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
-  uint64_t* empty = full + STAGES;
-  uint64_t* tfull = empty + STAGES;
-  uint64_t* tempty = tfull + 2;
-  uint64_t* done = tempty + 2;
+  uint8_t* const slots = align1024(smem_raw);
+  uint8_t* const ring = slots + p.aslots * SLOT_BYTES;
+  const int stage_bytes = W_BYTES + (p.aslots ? 0 : BM * BK * 2);
+  uint8_t* const bars = ring + p.stages * stage_bytes;
+  uint64_t* full = reinterpret_cast<uint64_t*>(bars);
+  uint64_t* empty = full + MAX_STAGES;
+  uint64_t* afull = empty + MAX_STAGES;
+  uint64_t* aempty = afull + MAX_SLOTS;
+  uint64_t* tfull = aempty + MAX_SLOTS;
+  uint64_t* tempty = tfull + 8;
+  uint64_t* done = tempty + 8;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
 
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int warp = umma::warp_index(), lane = threadIdx.x % 32;
   const int kc = a.Cin / BK;
-  const int nk = a.taps * kc;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < p.stages; ++s) {
       umma::mbar_init(&full[s], 1);
       umma::mbar_init(&empty[s], 1);
     }
-    for (int k = 0; k < 2; ++k) {
+    for (int s = 0; s < p.aslots; ++s) {
+      umma::mbar_init(&afull[s], 1);
+      umma::mbar_init(&aempty[s], 1);
+    }
+    for (int k = 0; k < ACCS; ++k) {
       umma::mbar_init(&tfull[k], 1);
-      umma::mbar_init(&tempty[k], 128);
+      umma::mbar_init(&tempty[k], 4 * (BN / 64));
     }
     umma::mbar_init(done, 1);
     umma::fence_barrier_init();
@@ -471,91 +654,97 @@ __global__ void __launch_bounds__(THREADS, 1) conv_fwd_persistent_kernel(const _
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      int s = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-        const int n0 = (t % ntn) * BN;
-        const int l0 = ((t / ntn) % ntl) * BM;
-        const int b = t / (ntn * ntl);
-        for (int kk = 0; kk < nk; ++kk, ++s) {
-          const int st = s % STAGES;
-          if (!umma::mbar_wait(&empty[st], ((s / STAGES) & 1) ^ 1, a.err, ERR_PRODUCER)) {
-            ok = false;
-            break;
+    int st = 0, issued = 0;
+    uint32_t ph = 1;  // parity of the empty barrier's phase before the first
+    bool ok = true;
+    for (TileWalk w(p); w.t < p.ntiles && ok; w.next(p)) {
+      const int n0 = w.n * BN, l0 = w.l * BM;
+      for (int tap = 0; tap < a.taps && ok; ++tap) {
+        for (int c = 0; c < kc; ++c) {
+          ok = umma::mbar_wait_warp(&empty[st], ph, a.err, ERR_PRODUCER);
+          if (!ok) break;
+          uint8_t* dst = ring + st * stage_bytes;
+          if (umma::elect()) {
+            umma::mbar_arrive_expect_tx(&full[st], stage_bytes);
+            if (!p.aslots) umma::tma_load_3d(dst + W_BYTES, &a.tm_a, &full[st], c * BK, l0 + tap - a.pad, w.b);
+            umma::tma_load_2d(dst, &a.tm_b, &full[st], tap * a.Cin + c * BK, n0);
           }
-          uint8_t* sa = smem + st * STAGE_BYTES;
-          umma::mbar_arrive_expect_tx(&full[st], STAGE_BYTES);
-          const int tap = kk / kc, c0 = (kk % kc) * BK;
-          umma::tma_load_3d(sa, &a.tm_a, &full[st], c0, l0 + tap - a.pad, b);
-          umma::tma_load_2d(sa + A_BYTES, &a.tm_b, &full[st], tap * a.Cin + c0, n0);
+          ++issued;
+          if (++st == p.stages) st = 0, ph ^= 1;
         }
       }
-      // drain: every issued copy has landed before the block can exit
-      for (int q = s > STAGES ? s - STAGES : 0; q < s; ++q)
-        umma::mbar_wait(&full[q % STAGES], (q / STAGES) & 1, a.err, ERR_PRODUCER);
+      if (p.wres) break;
     }
+    // drain: every issued copy has landed before the block can exit
+    for (int q = max(0, issued - p.stages); q < issued; ++q)
+      umma::mbar_wait_warp(&full[q % p.stages], (q / p.stages) & 1, a.err, ERR_PRODUCER);
+  } else if (warp == 2) {
+    const uint32_t bytes = (BM + a.taps - 1) * BK * 2;
+    int sl = 0, issued = 0;
+    uint32_t ph = 1;
+    bool ok = p.aslots > 0;
+    for (TileWalk w(p); w.t < p.ntiles && ok; w.next(p)) {
+      for (int c = 0; c < kc; ++c) {
+        ok = umma::mbar_wait_warp(&aempty[sl], ph, a.err, ERR_PRODUCER);
+        if (!ok) break;
+        if (umma::elect()) {
+          umma::mbar_arrive_expect_tx(&afull[sl], bytes);
+          umma::tma_load_3d(slots + sl * SLOT_BYTES, &a.tm_a, &afull[sl], c * BK, w.l * BM - a.pad, w.b);
+        }
+        ++issued;
+        if (++sl == p.aslots) sl = 0, ph ^= 1;
+      }
+    }
+    for (int q = max(0, issued - p.aslots); q < issued; ++q)
+      umma::mbar_wait_warp(&afull[q % p.aslots], (q / p.aslots) & 1, a.err, ERR_PRODUCER);
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma::idesc_bf16_f32(BM, BN, false, false);
-      int s = 0, j = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x, ++j) {
-        const int acc = j & 1;
-        if (!umma::mbar_wait(&tempty[acc], ((j >> 1) & 1) ^ 1, a.err, ERR_MMA)) break;
-        umma::fence_after_sync();
-        const uint32_t d = tmem + acc * BN;
-        for (int kk = 0; kk < nk; ++kk, ++s) {
-          const int st = s % STAGES;
-          if (!umma::mbar_wait(&full[st], (s / STAGES) & 1, a.err, ERR_MMA)) {
-            ok = false;
-            break;
-          }
-          umma::fence_after_sync();
-          const uint32_t sa = umma::smem_u32(smem + st * STAGE_BYTES);
-          const uint32_t sb = sa + A_BYTES;
-#pragma unroll
-          for (int k4 = 0; k4 < BK / 16; ++k4) {
-            umma::mma_bf16(d, umma::sdesc_sw128(sa + k4 * 32, 16, 1024), umma::sdesc_sw128(sb + k4 * 32, 16, 1024),
-                           idesc, (kk | k4) != 0);
-          }
-          umma::mma_commit(&empty[st]);
-        }
-        if (ok) umma::mma_commit(&tfull[acc]);
-      }
-      // every MMA this thread issued has completed before TMEM is released
-      umma::mma_commit(done);
-      umma::mbar_wait(done, 0, a.err, ERR_MMA);
+    const ConvSmem m{umma::smem_u32(full),  umma::smem_u32(empty),  umma::smem_u32(afull),
+                     umma::smem_u32(aempty), umma::smem_u32(tfull), umma::smem_u32(tempty),
+                     umma::smem_u32(done),  umma::smem_u32(ring),   umma::smem_u32(slots)};
+    if (p.wres) {
+      conv_mma_loop<BN, ACCS, true, true>(a, p, m, tmem, kc);
+    } else if (p.aslots) {
+      conv_mma_loop<BN, ACCS, true, false>(a, p, m, tmem, kc);
+    } else {
+      conv_mma_loop<BN, ACCS, false, false>(a, p, m, tmem, kc);
     }
-  } else {
+  } else if (warp >= 4) {
+    // the CTA's 64-column units, tile after tile, go round the groups
+    constexpr int UNITS = BN / 64;
     const int q = warp & 3;
-    int j = 0, nb = 0;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++j) {
-      const int acc = j & 1;
-      const bool ok = umma::mbar_wait(&tfull[acc], (j >> 1) & 1, a.err, ERR_EPILOGUE);
+    uint8_t* const stg = bars + 1024 + (warp - 4) * p.bufs * 4096;
+    int acc = 0, nb = 0, u = (warp - 4) >> 2;
+    uint32_t ph = 0;
+    for (TileWalk w(p);; u += p.groups) {
+      while (u >= UNITS) {
+        u -= UNITS;
+        w.next(p);
+        if (++acc == ACCS) acc = 0, ph ^= 1;
+      }
+      if (w.t >= p.ntiles) break;
+      const bool ok = umma::mbar_wait_warp(&tfull[acc], ph, a.err, ERR_EPILOGUE);
       umma::fence_after_sync();
       if (!ok) break;
-      const int n0 = (t % ntn) * BN;
-      const int y = ((t / ntn) % ntl) * BM + 32 * q;
-      const int b = t / (ntn * ntl);
+      const int col0 = w.n * BN + u * 64;
+      const int y = w.l * BM + 32 * q;
+      const uint32_t unit = tmem + (static_cast<uint32_t>(32 * q) << 16) + acc * BN + u * 64;
       if constexpr (STAGED) {
-        conv_epilogue_staged<BN>(a, tmem + (static_cast<uint32_t>(32 * q) << 16) + acc * BN,
-                                 smem + STAGES * STAGE_BYTES + 1024 + q * 8192, nb, n0, y, b);
+        conv_epilogue_unit(a, unit, stg, p.bufs, nb, col0, y, w.b);
       } else {
         const int l = y + lane;
         const bool row_ok = l < a.L;
-        const size_t row = static_cast<size_t>(b) * a.L + (row_ok ? l : 0);
+        const size_t row = static_cast<size_t>(w.b) * a.L + (row_ok ? l : 0);
 #pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
+        for (int c = 0; c < 2; ++c) {
           float v[32];
-          umma::tmem_ld32(tmem + (static_cast<uint32_t>(32 * q) << 16) + acc * BN + c * 32, v);
-          const int col0 = n0 + c * 32;
-          if (!row_ok || col0 >= a.n_valid) continue;
-          conv_epilogue_chunk(a, v, row, col0);
+          umma::tmem_ld32(unit + c * 32, v);
+          if (row_ok && col0 + c * 32 < a.n_valid) conv_epilogue_chunk(a, v, row, col0 + c * 32);
+          __syncwarp();
         }
       }
       umma::fence_before_sync();
-      umma::mbar_arrive(&tempty[acc]);
+      __syncwarp();
+      if (lane == 0) umma::mbar_arrive(&tempty[acc]);
     }
     if constexpr (STAGED) staged_drain();
   }
@@ -1488,27 +1677,19 @@ cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, int threads, int smem, cud
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
-// Once per kernel and device: the shared-memory permission and the CTAs that fit an SM (asking the runtime
-// on every launch took longer than the launch).
+// Once per kernel and device: the shared-memory permission (asking the runtime on every launch took
+// longer than the launch).
 struct KernelLimits {
-  std::atomic<int> per_sm[64] = {};
-  int get(const void* kern, int smem, int* out) {
+  std::atomic<bool> set[64] = {};
+  int get(const void* kern, int smem) {
     int dev = 0;
     int rc = cuda_ok(cudaGetDevice(&dev), "cudaGetDevice");
     if (rc) return rc;
     if (dev < 0 || dev >= 64) return fail(MSUR_ERR_UNSUPPORTED, "device %d out of range", dev);
-    int n = per_sm[dev].load(std::memory_order_acquire);
-    if (n == 0) {
-      rc = cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attribute");
-      if (!rc) rc = cuda_ok(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, THREADS, smem), "occupancy");
-      int sms = 0;
-      if (!rc) rc = cuda_ok(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
-      if (rc) return rc;
-      n = (sms << 8) | std::max(1, n);
-      per_sm[dev].store(n, std::memory_order_release);
-    }
-    *out = n;
-    return MSUR_OK;
+    if (set[dev].load(std::memory_order_acquire)) return MSUR_OK;
+    rc = cuda_ok(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), "smem attribute");
+    if (!rc) set[dev].store(true, std::memory_order_release);
+    return rc;
   }
 };
 
@@ -1517,47 +1698,122 @@ int launch_conv(const ConvArgs& a, int ntiles_n, cudaStream_t st) {
   constexpr int smem = conv_smem<BN, STAGES, STAGED>();
   auto kern = conv_fwd_kernel<BN, STAGES, STAGED>;
   static KernelLimits limits;
-  int lim = 0;
-  const int rc = limits.get(reinterpret_cast<const void*>(kern), smem, &lim);
+  const int rc = limits.get(reinterpret_cast<const void*>(kern), smem);
   if (rc) return rc;
   dim3 grid(ntiles_n, (a.L + BM - 1) / BM, a.B);
   return cuda_ok(launch_pdl(kern, grid, THREADS, smem, st, a),
                  "conv_fwd_kernel launch");
 }
 
-template <int BN, int STAGES, bool STAGED>
-int launch_conv_persistent(const ConvArgs& a, int ntn, cudaStream_t st) {
-  constexpr int smem = conv_smem<BN, STAGES, STAGED>();
-  constexpr int tcols = static_cast<int>(tmem_cols<2 * BN>());
-  auto kern = conv_fwd_persistent_kernel<BN, STAGES, STAGED>;
-  static KernelLimits limits;
-  int lim = 0;
-  const int rc = limits.get(reinterpret_cast<const void*>(kern), smem, &lim);
+int sm_count(int* out) {
+  static std::atomic<int> count[64] = {};
+  int dev = 0;
+  int rc = cuda_ok(cudaGetDevice(&dev), "cudaGetDevice");
   if (rc) return rc;
-  const int sms = lim >> 8;
-  int per_sm = lim & 255;
-  per_sm = std::max(1, std::min(per_sm, 512 / tcols));  // each resident CTA holds its accumulators in TMEM
-  const int ntl = (a.L + BM - 1) / BM;
-  const int ntiles = ntn * ntl * a.B;
-  const int grid = std::min(ntiles, sms * per_sm);
-  return cuda_ok(launch_pdl(kern, dim3(grid), THREADS, smem, st, a, ntn, ntl, ntiles),
-                 "conv_fwd_persistent_kernel launch");
+  if (dev < 0 || dev >= 64) return fail(MSUR_ERR_UNSUPPORTED, "device %d out of range", dev);
+  int n = count[dev].load(std::memory_order_relaxed);
+  if (!n) {
+    rc = cuda_ok(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev), "SM count");
+    if (rc) return rc;
+    count[dev].store(n, std::memory_order_relaxed);
+  }
+  *out = n;
+  return MSUR_OK;
 }
 
-template <int BN, int STAGES>
-int launch_conv_form(const ConvArgs& a, int ntn, bool persistent, bool staged, cudaStream_t st) {
-  if (persistent) {
-    return staged ? launch_conv_persistent<BN, STAGES, true>(a, ntn, st)
-                  : launch_conv_persistent<BN, STAGES, false>(a, ntn, st);
+// How the persistent kernel uses its shared memory (ConvPlan), in this order of preference:
+//  1. more than one tap, and all weights of an N tile fit beside the slots of one or two tiles: weights stay;
+//  2. more than one tap, and the slots fit beside at least three weight stages;
+//  3. both operands stage by stage (a single tap reads its activations once anyway: the head's convolution of
+//     256 maps took 508 us with slots, 465 without).
+// A single tile's slots do when its chunks, freed one by one in its last tap, leave the next tile's first loads
+// four K steps or more ahead (192 to 64 channels at 4000 positions, 256 maps: 128 us with one
+// tile's three slots, 92 with six).  Epilogue groups: as many as fit up to four, two without an activation.
+ConvPlan conv_plan(int bn, int cin, int taps, int cout, int L, int B, int stages, bool staged, bool heavy, int sms,
+                   int* grid, int* smem) {
+  constexpr int ROOM = 227 * 1024 - 2048;  // alignment slack and the barriers
+  const int kc = cin / BK, nk = taps * kc, w = bn * BK * 2;
+  const int group = staged ? 4 * 4096 : 0, most = heavy ? 4 : 2;
+  ConvPlan p{};
+  p.ntn = (cout + bn - 1) / bn;
+  p.ntl = (L + BM - 1) / BM;
+  p.ntiles = p.ntn * p.ntl * B;
+  *grid = std::min(p.ntiles, sms);
+  const int fixed = sms / p.ntn * p.ntn;  // a grid whose stride keeps a CTA's N tile
+  const int least = kc >= 4 ? kc : 2 * kc;
+  const bool slots = taps > 1 && taps - 1 <= 8 && least <= MAX_SLOTS;
+  int used = 0;
+  if (slots && nk <= MAX_STAGES && fixed > 0) {
+    for (int g = most; g >= 2 && !p.groups; --g) {
+      if (nk * w + least * SLOT_BYTES + g * group > ROOM) continue;
+      p.groups = g;
+      p.wres = 1;
+      p.stages = nk;
+      p.aslots = least;
+      *grid = std::min(p.ntiles, fixed);
+    }
   }
-  return staged ? launch_conv<BN, STAGES, true>(a, ntn, st) : launch_conv<BN, STAGES, false>(a, ntn, st);
+  for (int st = stages; slots && st >= std::min(3, stages) && !p.groups; --st) {
+    for (int g = most; g >= 2 && !p.groups; --g) {
+      if (st * w + least * SLOT_BYTES + g * group > ROOM) continue;
+      p.groups = g;
+      p.stages = st;
+      p.aslots = least;
+    }
+  }
+  for (int st = stages; st >= 2 && !p.groups; --st) {
+    for (int g = most; g >= 2 && !p.groups; --g) {
+      if (st * (w + BM * BK * 2) + g * group > ROOM) continue;
+      p.groups = g;
+      p.stages = st;
+    }
+  }
+  used = p.stages * (w + (p.aslots ? 0 : BM * BK * 2)) + p.aslots * SLOT_BYTES + p.groups * group;
+  if (p.aslots && p.aslots + kc <= MAX_SLOTS && used + kc * SLOT_BYTES <= ROOM) {
+    p.aslots += kc;
+    used += kc * SLOT_BYTES;
+  }
+  p.bufs = staged ? 1 : 0;
+  if (staged && used + p.groups * group <= ROOM) {
+    p.bufs = 2;
+    used += p.groups * group;
+  }
+  *smem = 2048 + used;
+  return p;
+}
+
+template <int BN, bool STAGED>
+int launch_conv_persistent(const ConvArgs& a, const ConvPlan& p, int grid, int smem, cudaStream_t st) {
+  auto kern = conv_fwd_persistent_kernel<BN, STAGED>;
+  static KernelLimits limits;
+  const int rc = limits.get(reinterpret_cast<const void*>(kern), 227 * 1024);
+  if (rc) return rc;
+  return cuda_ok(launch_pdl(kern, dim3(grid), 128 + 128 * p.groups, smem, st, a, p), "conv_fwd_persistent_kernel launch");
+}
+
+int dispatch_conv_persistent(int bn, const ConvArgs& a, const ConvPlan& p, int grid, int smem, cudaStream_t st) {
+  const bool staged = p.bufs > 0;
+  switch (bn) {
+    case 64:
+      return staged ? launch_conv_persistent<64, true>(a, p, grid, smem, st)
+                    : launch_conv_persistent<64, false>(a, p, grid, smem, st);
+    case 128:
+      return staged ? launch_conv_persistent<128, true>(a, p, grid, smem, st)
+                    : launch_conv_persistent<128, false>(a, p, grid, smem, st);
+    case 192:
+      return staged ? launch_conv_persistent<192, true>(a, p, grid, smem, st)
+                    : launch_conv_persistent<192, false>(a, p, grid, smem, st);
+    default:
+      return staged ? launch_conv_persistent<256, true>(a, p, grid, smem, st)
+                    : launch_conv_persistent<256, false>(a, p, grid, smem, st);
+  }
 }
 
 template <int BN>
-int dispatch_conv(const ConvArgs& a, int ntn, bool persistent, bool staged, int stages, cudaStream_t st) {
-  if (stages == 2) return launch_conv_form<BN, 2>(a, ntn, persistent, staged, st);
-  if (stages == 3) return launch_conv_form<BN, 3>(a, ntn, persistent, staged, st);
-  return launch_conv_form<BN, 4>(a, ntn, persistent, staged, st);
+int dispatch_conv(const ConvArgs& a, int ntn, bool staged, int stages, cudaStream_t st) {
+  if (stages == 2) return staged ? launch_conv<BN, 2, true>(a, ntn, st) : launch_conv<BN, 2, false>(a, ntn, st);
+  if (stages == 3) return staged ? launch_conv<BN, 3, true>(a, ntn, st) : launch_conv<BN, 3, false>(a, ntn, st);
+  return staged ? launch_conv<BN, 4, true>(a, ntn, st) : launch_conv<BN, 4, false>(a, ntn, st);
 }
 
 template <int BN, int NT, int STAGES>
@@ -1565,8 +1821,7 @@ int launch_wgrad(const WgradArgs& a, int splits, cudaStream_t st) {
   constexpr int smem = wgrad_region<BN, NT, STAGES>() + 1024 + 256;
   auto kern = wgrad_kernel<BN, NT, STAGES>;
   static KernelLimits limits;
-  int lim = 0;
-  const int rc = limits.get(reinterpret_cast<const void*>(kern), smem, &lim);
+  const int rc = limits.get(reinterpret_cast<const void*>(kern), smem);
   if (rc) return rc;
   dim3 grid((a.Cin + BN - 1) / BN, (a.Cout + BM - 1) / BM, splits);
   return cuda_ok(launch_pdl(kern, grid, THREADS, smem, st, a),
@@ -1628,12 +1883,24 @@ static int conv_forward_impl(const void* x, int B, int L, int Cin, const void* w
   // A tile is one CTA's chain of K steps, and a step's time is its operands' transfer, so while the tiles
   // leave SMs idle a narrower one halves the chain's time on twice the SMs (the products and their order
   // are the same).  One map: the deep levels have 2 to 16 tiles at 256 columns, 8 to 64 at 64.
+  const bool persistent = (form & 1) != 0, staged = (form & 2) != 0;
   int BN = slot == 2 ? 256 : (slot == 1 ? 128 : 64);
-  while (BN > 64 && static_cast<long long>((Cout + BN - 1) / BN) * ((L + BM - 1) / BM) * B < 152) BN /= 2;
+  if (persistent && slot == 1 && Cout % 192 == 0) BN = 192;
+  while (BN > 64 && static_cast<long long>((Cout + BN - 1) / BN) * ((L + BM - 1) / BM) * B < 152)
+    BN = BN == 192 ? 64 : BN / 2;
   ConvArgs a;
   std::memset(&a, 0, sizeof(a));
   const uint64_t dims_a[3] = {static_cast<uint64_t>(Cin), static_cast<uint64_t>(L), static_cast<uint64_t>(B)};
-  const uint32_t box_a[3] = {64, BM, 1};
+  ConvPlan plan{};
+  int grid = 0, smem = 0;
+  if (persistent) {
+    int sms = 0;
+    rc = sm_count(&sms);
+    if (rc) return rc;
+    plan = conv_plan(BN, Cin, taps, Cout, L, B, stages, staged, act == MSUR_ACT_SILU || gate,
+                     sms, &grid, &smem);
+  }
+  const uint32_t box_a[3] = {64, static_cast<uint32_t>(plan.aslots ? BM + taps - 1 : BM), 1};
   rc = make_map(&a.tm_a, x, 3, dims_a, box_a);
   if (rc) return rc;
   const uint64_t dims_b[2] = {static_cast<uint64_t>(taps) * Cin, static_cast<uint64_t>(Cout)};
@@ -1657,11 +1924,8 @@ static int conv_forward_impl(const void* x, int B, int L, int Cin, const void* w
   const int ntn = (Cout + BN - 1) / BN;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // kernel form: bit 0 the persistent kernel, bit 1 the staged epilogue (outputs through shared
-  // memory and TMA), which needs no gate: the data gradient's gate is read row by row, so that
-  // epilogue stays per thread
-  const bool persistent = (form & 1) != 0;
-  const bool staged = (form & 2) != 0 && !gate;
-  if ((out_skip || out_dup || out_pool) && !staged)
+  // memory and TMA)
+  if ((out_skip || out_dup || out_pool) && (!staged || gate))
     return fail(MSUR_ERR_UNSUPPORTED, "msur_conv_forward_fused: the fused copies need the staged form (bit 1) "
                                       "for N tile %d and no gate", BN);
   if (staged) {
@@ -1682,9 +1946,10 @@ static int conv_forward_impl(const void* x, int B, int L, int Cin, const void* w
     a.has_dup = out_dup ? 1 : 0;
     a.has_pool = out_pool ? 1 : 0;
   }
-  if (BN == 256) return dispatch_conv<256>(a, ntn, persistent, staged, stages, st);
-  if (BN == 128) return dispatch_conv<128>(a, ntn, persistent, staged, stages, st);
-  return dispatch_conv<64>(a, ntn, persistent, staged, stages, st);
+  if (persistent) return dispatch_conv_persistent(BN, a, plan, grid, smem, st);
+  if (BN == 256) return dispatch_conv<256>(a, ntn, staged, stages, st);
+  if (BN == 128) return dispatch_conv<128>(a, ntn, staged, stages, st);
+  return dispatch_conv<64>(a, ntn, staged, stages, st);
 }
 
 int msur_conv_forward(const void* x, int B, int L, int Cin, const void* w, int Cout, int taps, const float* bias,
@@ -1944,13 +2209,6 @@ int msur_run(const msur_op* ops, int n, void* stream) {
         break;
       case MSUR_OP_UPCAT_BWD:
         rc = msur_upcat_bwd(p[0], p[1], i[0], i[1], i[2], i[3], p[2], stream);
-        break;
-      case MSUR_OP_MSE:
-        rc = msur_mse(static_cast<const float*>(p[0]), i[0], static_cast<const float*>(p[1]), i[1], o.rows, i[2], p[2],
-                      i[3], o.f, static_cast<double*>(p[3]), stream);
-        break;
-      case MSUR_OP_ZERO:
-        rc = cuda_ok(cudaMemsetAsync(p[0], 0, o.rows, static_cast<cudaStream_t>(stream)), "cudaMemsetAsync");
         break;
       default:
         rc = fail(MSUR_ERR_INVALID_ARG, "msur_run: operation %d has an unknown kind %d", k, o.kind);

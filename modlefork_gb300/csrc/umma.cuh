@@ -43,14 +43,29 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+  return mbar_try_wait(smem_u32(bar), parity);
+}
+// Whether that phase has completed, without waiting for it.
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
       : "memory");
   return ok != 0;
 }
@@ -68,6 +83,38 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsign
   }
   return true;
 }
+
+// The same for a whole converged warp: control flow that depends on the result stays warp-uniform.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, unsigned* err, unsigned code,
+                                               uint64_t limit_ns = 1000000000ull) {
+  if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+  const uint64_t t0 = global_ns();
+  while (!__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) {
+    if (__any_sync(0xFFFFFFFFu, global_ns() - t0 > limit_ns)) {
+      if (err && (threadIdx.x & 31) == 0) atomicOr(err, code);
+      return false;
+    }
+  }
+  return true;
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, unsigned* err, unsigned code) {
+  return mbar_wait_warp(smem_u32(bar), parity, err, code);
+}
+// One lane of a converged warp, the same one each time.  The issuing warps keep their loops
+// warp-uniform and enter only the issue itself with one lane: descriptors and tensor-map operands then
+// stay in uniform registers (issued from a branch of a single thread, a K step without any work took
+// about 480 cycles).
+__device__ __forceinline__ bool elect() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xFFFFFFFF;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+// The warp's index as a warp-uniform value.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xFFFFFFFFu, static_cast<int>(threadIdx.x / 32), 0); }
 
 // ---- TMA --------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch(const CUtensorMap* map) {
@@ -170,11 +217,36 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Arrive on *bar once every MMA issued so far by this thread has completed.
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
+// One K step of 64 elements with 128-byte swizzled K-major operands: four products of 16, their
+// descriptors (sdesc_sw128 split into the words that change and the one that does not) 32 bytes apart.
+constexpr uint32_t SDESC_SW128_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t sdesc_sw128_lo(uint32_t saddr) { return (saddr >> 4) | (1u << 16); }
+__device__ __forceinline__ void mma_bf16_k64(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.eq.b32 q, 0, 0;\n\t"
+      "mov.b64 a, {%1, %3};\n\t"
+      "mov.b64 b, {%2, %3};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t"
+      "add.s64 a, a, 2;\n\t"
+      "add.s64 b, b, 2;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, q;\n\t"
+      "add.s64 a, a, 2;\n\t"
+      "add.s64 b, b, 2;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, q;\n\t"
+      "add.s64 a, a, 2;\n\t"
+      "add.s64 b, b, 2;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, q;\n\t}" ::"r"(d_tmem),
+      "r"(a_lo), "r"(b_lo), "r"(SDESC_SW128_HI), "r"(idesc), "r"(accumulate)
+      : "memory");
 }
+// Arrive on *bar once every MMA issued so far by this thread has completed.
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint64_t* bar) { mma_commit(smem_u32(bar)); }
 
 // 32 consecutive FP32 accumulator columns of this thread's TMEM lane.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
