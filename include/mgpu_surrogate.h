@@ -156,25 +156,23 @@ int msur_map_sums_of(unsigned which, const float* pred, uint64_t pstride_map, co
 int msur_compact_rows(const float* in, int stride, uint64_t rows, int n_valid, float* out, void* stream);
 
 /* A list of the operations above in one call, enqueued in order: a network's pass without a foreign-function
- * call per layer.  p, i and rows hold the operation's arguments in the order of its function:
+ * call per layer.  p and i hold the operation's arguments in the order of its function:
  *   CONV      p: x w bias out_pre out_post out_f32 gate out_skip out_dup out_pool;
  *             i: B L Cin Cout taps act out_stride n_valid skip_stride dup_stride pool_stride;
  *             form and stages: the kernel form and depth, -1 for the width's current settings
- *   WGRAD     p: x dz dw; i: B L Cin Cout taps splits
- *   BIAS_GRAD p: dz db; i: C stride; rows
+ *   WGRAD     p: x dz dw db; i: B L Cin Cout taps splits; the bias gradient too unless db is null
  *   POOL2     p: x y; i: B Lout C
  *   SKIP_GRAD p: dpool dcat z dz; i: Lp cat_stride cat_off B L C
  *   UPCAT     p: x skip out; i: B L C1 C2
  *   UPCAT_BWD p: dcat z dz; i: B Lh C1 C
  * Stops at the first operation that fails and returns its status. */
 enum {
-  MSUR_OP_CONV = 0, MSUR_OP_WGRAD, MSUR_OP_BIAS_GRAD, MSUR_OP_POOL2, MSUR_OP_SKIP_GRAD, MSUR_OP_UPCAT,
+  MSUR_OP_CONV = 0, MSUR_OP_WGRAD, MSUR_OP_POOL2, MSUR_OP_SKIP_GRAD, MSUR_OP_UPCAT,
   MSUR_OP_UPCAT_BWD
 };
 typedef struct msur_op {
   int kind, form, stages;
   int i[12];
-  uint64_t rows;
   void* p[10];
 } msur_op;
 int msur_run(const msur_op* ops, int n, void* stream);

@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_fwd_kernel(const __grid_const
   uint64_t* done = empty + STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
 
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int warp = umma::warp_index(), lane = threadIdx.x % 32;
   const int n0 = blockIdx.x * BN, l0 = blockIdx.y * BM, b = blockIdx.z;
   const int kc = a.Cin / BK;
   const int nk = a.taps * kc;
@@ -391,49 +391,41 @@ __global__ void __launch_bounds__(THREADS, 1) conv_fwd_kernel(const __grid_const
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      int issued = 0;
-      for (int s = 0; s < nk; ++s) {
-        const int st = s % STAGES;
-        const uint32_t ph = (s / STAGES) & 1;
-        if (!umma::mbar_wait(&empty[st], ph ^ 1, a.err, ERR_PRODUCER)) break;
-        uint8_t* sa = smem + st * STAGE_BYTES;
+    int issued = 0;
+    for (int s = 0; s < nk; ++s) {
+      const int st = s % STAGES;
+      if (!umma::mbar_wait_warp(&empty[st], ((s / STAGES) & 1) ^ 1, a.err, ERR_PRODUCER)) break;
+      uint8_t* sa = smem + st * STAGE_BYTES;
+      const int t = s / kc, c0 = (s % kc) * BK;
+      if (umma::elect()) {
         umma::mbar_arrive_expect_tx(&full[st], STAGE_BYTES);
-        const int t = s / kc, c0 = (s % kc) * BK;
         umma::tma_load_3d(sa, &a.tm_a, &full[st], c0, l0 + t - a.pad, b);
         umma::tma_load_2d(sa + A_BYTES, &a.tm_b, &full[st], t * a.Cin + c0, n0);
-        issued = s + 1;
       }
-      // drain: every issued copy has landed before the block can exit
-      for (int s = issued > STAGES ? issued - STAGES : 0; s < issued; ++s)
-        umma::mbar_wait(&full[s % STAGES], (s / STAGES) & 1, a.err, ERR_PRODUCER);
+      issued = s + 1;
     }
+    // drain: every issued copy has landed before the block can exit
+    for (int s = issued > STAGES ? issued - STAGES : 0; s < issued; ++s)
+      umma::mbar_wait_warp(&full[s % STAGES], (s / STAGES) & 1, a.err, ERR_PRODUCER);
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma::idesc_bf16_f32(BM, BN, false, false);
-      for (int s = 0; s < nk; ++s) {
-        const int st = s % STAGES;
-        const uint32_t ph = (s / STAGES) & 1;
-        if (!umma::mbar_wait(&full[st], ph, a.err, ERR_MMA)) break;
-        umma::fence_after_sync();
-        const uint32_t sa = umma::smem_u32(smem + st * STAGE_BYTES);
-        const uint32_t sb = sa + A_BYTES;
-#pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk) {
-          umma::mma_bf16(tmem, umma::sdesc_sw128(sa + kk * 32, 16, 1024), umma::sdesc_sw128(sb + kk * 32, 16, 1024),
-                         idesc, (s | kk) != 0);
-        }
+    constexpr uint32_t idesc = umma::idesc_bf16_f32(BM, BN, false, false);
+    for (int s = 0; s < nk; ++s) {
+      const int st = s % STAGES;
+      if (!umma::mbar_wait_warp(&full[st], (s / STAGES) & 1, a.err, ERR_MMA)) break;
+      const uint32_t sa = umma::smem_u32(smem + st * STAGE_BYTES);
+      if (umma::elect()) {
+        umma::mma_bf16_x4<2>(tmem, umma::sdesc_sw128_lo(sa), umma::sdesc_sw128_lo(sa + A_BYTES), idesc, s);
         umma::mma_commit(&empty[st]);
       }
-      umma::mma_commit(done);
     }
+    if (umma::elect()) umma::mma_commit(done);
   } else {
     // epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31, one output row per thread
     const int q = warp & 3;
     const int l = l0 + 32 * q + lane;
     const bool row_ok = l < a.L;
     const size_t row = static_cast<size_t>(b) * a.L + (row_ok ? l : 0);
-    const bool ok = umma::mbar_wait(done, 0, a.err, ERR_EPILOGUE);
+    const bool ok = umma::mbar_wait_warp(done, 0, a.err, ERR_EPILOGUE);
     umma::fence_after_sync();
     if constexpr (STAGED) {
       if (ok) {
@@ -526,7 +518,7 @@ __device__ __forceinline__ void conv_mma_loop(const ConvArgs& a, const ConvPlan&
       if (umma::elect()) {
         uint32_t a_lo = umma::sdesc_sw128_lo(sa), b_lo = umma::sdesc_sw128_lo(sb);
         for (int c = 0; c < kc; ++c) {
-          umma::mma_bf16_k64(d, a_lo, b_lo, idesc, 1);
+          umma::mma_bf16_x4<2>(d, a_lo, b_lo, idesc, 1);
           if (decltype(release)::value) umma::mma_commit(m.aempty + sl + 8 * c);
           a_lo += SLOT_BYTES / 16;
           b_lo += W_BYTES / 16;
@@ -548,7 +540,7 @@ __device__ __forceinline__ void conv_mma_loop(const ConvArgs& a, const ConvPlan&
       if (fb == full_end) fb = m.full, sb = m.ring, ph ^= 1;
       if (!WRES) ready = umma::mbar_test(fb, ph);
       if (umma::elect()) {
-        umma::mma_bf16_k64(d, a_lo, b_lo, idesc, accumulate);
+        umma::mma_bf16_x4<2>(d, a_lo, b_lo, idesc, accumulate);
         if (!WRES) umma::mma_commit(eb);
         if (ASLOTS && decltype(release)::value) umma::mma_commit(m.aempty + sl);
       }
@@ -761,6 +753,11 @@ __global__ void __launch_bounds__(PTHREADS, 1)
 // (b, 64-position block) range; M = output channels (128 per tile), N = input channels (BN per
 // tile), one TMEM accumulator of BN columns per tap; both operands M/N-major.
 //
+// A block's 64 (+ taps - 1) positions of X are loaded once: tap t's operand starts t rows into them.  Where
+// the bias gradient is wanted too, the epilogue warps of the first input-channel tile add up the dZ blocks as they
+// pass through shared memory (25 launches of 4 to 17 us in a network's pass).  Together with warp-uniform issue
+// loops: the backward pass of 16 maps lost 100 us of 1255 for both passes.
+//
 // The splits' partial sums meet in dw.  A thread holds one output channel's row of the accumulators;
 // adding it word by word (32 rows per warp and instruction) took longer than the products: 113 of
 // 133 us for 16 x 999 positions, 256 to 256 channels.  So the rows go to the operand stages, free by
@@ -769,13 +766,15 @@ __global__ void __launch_bounds__(PTHREADS, 1)
 // ---------------------------------------------------------------------------------------
 struct WgradArgs {
   CUtensorMap tm_dz;  // [B][L][Cout]: dims {Cout, L, B}, box {64, 64, 1}
-  CUtensorMap tm_x;   // [B][L][Cin]: dims {Cin, L, B}, box {64, 64, 1}
+  CUtensorMap tm_x;   // [B][L][Cin]: dims {Cin, L, B}, box {64, 64 + taps - 1, 1}
   int B, L, Cin, Cout, taps, pad;
   int lblocks;        // 64-position blocks per sequence
   int total;          // B * lblocks
   int per_split;      // blocks per split
   int bulk;           // dw is 16-byte aligned: bulk reductions
   float* dw;          // [Cout][taps][Cin], accumulated into
+  float* db;          // [Cout], accumulated into, or null
+  uint32_t zero;
   unsigned* err;
 };
 
@@ -785,9 +784,13 @@ template <int BN, int NT>
 __host__ __device__ constexpr int wgrad_row_bytes() {
   return NT * BN * 4 + 16;
 }
+template <int NT>
+__host__ __device__ constexpr int wgrad_box_bytes() {  // 64 + NT - 1 rows, 1 KB aligned
+  return (64 + (NT > 1 ? 8 : 0)) * 128;
+}
 template <int BN, int NT, int STAGES>
 __host__ __device__ constexpr int wgrad_region() {
-  const int stages = STAGES * (2 * 8192 + NT * (BN / 64) * 8192), rows = BM * wgrad_row_bytes<BN, NT>();
+  const int stages = STAGES * (2 * 8192 + (BN / 64) * wgrad_box_bytes<NT>()), rows = BM * wgrad_row_bytes<BN, NT>();
   return stages > rows ? stages : (rows + 1023) / 1024 * 1024;
 }
 
@@ -795,8 +798,9 @@ template <int BN, int NT, int STAGES>
 __global__ void __launch_bounds__(THREADS, 1) wgrad_kernel(const __grid_constant__ WgradArgs a) {
   constexpr int BOX = 64 * 64 * 2;  // one 64 x 64 BF16 box
   constexpr int A_BYTES = 2 * BOX;  // 128 output channels
-  constexpr int B_TAP = (BN / 64) * BOX;
-  constexpr int STAGE_BYTES = A_BYTES + NT * B_TAP;
+  constexpr int XBOX = wgrad_box_bytes<NT>();
+  constexpr int STAGE_BYTES = A_BYTES + (BN / 64) * XBOX;
+  constexpr uint32_t STAGE_LOAD = A_BYTES + (BN / 64) * (64 + NT - 1) * 128;
   constexpr uint32_t TCOLS = NT * BN <= 128 ? 128 : (NT * BN <= 256 ? 256 : 512);
   static_assert(NT * BN <= 512, "accumulators exceed tensor memory");
   extern __shared__ uint8_t smem_raw[];
@@ -805,17 +809,19 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_kernel(const __grid_constant
   uint64_t* empty = full + STAGES;
   uint64_t* done = empty + STAGES;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  float* bias_part = reinterpret_cast<float*>(full + 32);  // [4 warps][128 channels]
 
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int warp = umma::warp_index(), lane = threadIdx.x % 32;
   const int c0 = blockIdx.x * BN, n0 = blockIdx.y * BM;
   const int kb0 = blockIdx.z * a.per_split;
   const int kb1 = min(a.total, kb0 + a.per_split);
   const int nk = kb1 > kb0 ? kb1 - kb0 : 0;
+  const bool bias = a.db != nullptr && blockIdx.x == 0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       umma::mbar_init(&full[s], 1);
-      umma::mbar_init(&empty[s], 1);
+      umma::mbar_init(&empty[s], bias ? 5 : 1);  // the products, and the warps that add up dZ
     }
     umma::mbar_init(done, 1);
     umma::fence_barrier_init();
@@ -831,55 +837,84 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_kernel(const __grid_constant
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      int issued = 0;
-      for (int s = 0; s < nk; ++s) {
-        const int st = s % STAGES;
-        const uint32_t ph = (s / STAGES) & 1;
-        if (!umma::mbar_wait(&empty[st], ph ^ 1, a.err, ERR_PRODUCER)) break;
-        uint8_t* sa = smem + st * STAGE_BYTES;
-        const int kb = kb0 + s;
-        const int bb = kb / a.lblocks, l0 = (kb % a.lblocks) * 64;
-        umma::mbar_arrive_expect_tx(&full[st], STAGE_BYTES);
+    int issued = 0, st = 0;
+    uint32_t ph = 1;
+    int bb = kb0 / a.lblocks, l0 = (kb0 % a.lblocks) * 64;
+    for (int s = 0; s < nk; ++s) {
+      if (!umma::mbar_wait_warp(&empty[st], ph, a.err, ERR_PRODUCER)) break;
+      uint8_t* sa = smem + st * STAGE_BYTES;
+      if (umma::elect()) {
+        umma::mbar_arrive_expect_tx(&full[st], STAGE_LOAD);
         umma::tma_load_3d(sa, &a.tm_dz, &full[st], n0, l0, bb);
         umma::tma_load_3d(sa + BOX, &a.tm_dz, &full[st], n0 + 64, l0, bb);
 #pragma unroll
-        for (int t = 0; t < NT; ++t) {
-#pragma unroll
-          for (int j = 0; j < BN / 64; ++j)
-            umma::tma_load_3d(sa + A_BYTES + t * B_TAP + j * BOX, &a.tm_x, &full[st], c0 + 64 * j, l0 + t - a.pad, bb);
-        }
-        issued = s + 1;
+        for (int j = 0; j < BN / 64; ++j)
+          umma::tma_load_3d(sa + A_BYTES + j * XBOX, &a.tm_x, &full[st], c0 + 64 * j, l0 - a.pad, bb);
       }
-      for (int s = issued > STAGES ? issued - STAGES : 0; s < issued; ++s)
-        umma::mbar_wait(&full[s % STAGES], (s / STAGES) & 1, a.err, ERR_PRODUCER);
+      issued = s + 1;
+      if (++st == STAGES) st = 0, ph ^= 1;
+      if ((l0 += 64) >= a.lblocks * 64) l0 = 0, ++bb;
     }
+    for (int s = issued > STAGES ? issued - STAGES : 0; s < issued; ++s)
+      umma::mbar_wait_warp(&full[s % STAGES], (s / STAGES) & 1, a.err, ERR_PRODUCER);
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma::idesc_bf16_f32(BM, BN, true, true);
-      for (int s = 0; s < nk; ++s) {
-        const int st = s % STAGES;
-        const uint32_t ph = (s / STAGES) & 1;
-        if (!umma::mbar_wait(&full[st], ph, a.err, ERR_MMA)) break;
-        umma::fence_after_sync();
-        const uint32_t sa = umma::smem_u32(smem + st * STAGE_BYTES);
+    constexpr uint32_t idesc = umma::idesc_bf16_f32(BM, BN, true, true);
+    int st = 0;
+    uint32_t ph = 0;
+    for (int s = 0; s < nk; ++s) {
+      if (!umma::mbar_wait_warp(&full[st], ph, a.err, ERR_MMA)) break;
+      const uint32_t sa = umma::smem_u32(smem) + st * STAGE_BYTES;
+      const uint32_t a_lo = umma::sdesc_sw128_lo(sa, BOX), b_lo = umma::sdesc_sw128_lo(sa + A_BYTES, XBOX);
+      if (umma::elect()) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          const uint64_t ad = umma::sdesc_sw128(sa + kk * 2048, BOX, 1024);
-#pragma unroll
-          for (int t = 0; t < NT; ++t) {
-            const uint64_t bd = umma::sdesc_sw128(sa + A_BYTES + t * B_TAP + kk * 2048, BOX, 1024);
-            umma::mma_bf16(tmem + t * BN, ad, bd, idesc, (s | kk) != 0);
-          }
-        }
+        for (int t = 0; t < NT; ++t) umma::mma_bf16_x4<128>(tmem + t * BN, a_lo, b_lo + 8 * t, idesc, s);
         umma::mma_commit(&empty[st]);
       }
-      umma::mma_commit(done);
+      if (++st == STAGES) st = 0, ph ^= 1;
     }
+    if (umma::elect()) umma::mma_commit(done);
   } else if (nk > 0) {
     const int q = warp & 3;
     const int n = n0 + 32 * q + lane;
-    const bool ok = umma::mbar_wait(done, 0, a.err, ERR_EPILOGUE);
+    if (bias) {
+      // thread e: 8 channels (16-byte unit e % 16 of the two boxes), rows 8 (e / 16) .. + 7 of each block
+      const int e = threadIdx.x - 64, unit = e & 15;
+      float sum[8] = {};
+      int st = 0;
+      uint32_t ph = 0;
+      for (int s = 0; s < nk; ++s) {
+        if (!umma::mbar_wait_warp(&full[st], ph, a.err, ERR_EPILOGUE)) break;
+        const uint32_t rows = umma::smem_u32(smem) + st * STAGE_BYTES + (unit >> 3) * BOX + (e >> 4) * 1024;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          uint32_t x[4];
+          umma::ld_shared_v4(x, rows + r * 128 + (((unit & 7) ^ r) << 4));
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[h]));
+            sum[2 * h] += f.x;
+            sum[2 * h + 1] += f.y;
+          }
+        }
+        // The next copy may write here once the loads have returned, not once they are issued: the products
+        // take most of the shared memory's cycles, and loads were seen to lose rows to the copy six
+        // blocks on.  So the arrival's address depends on what was loaded (by an AND with a zero
+        // that only the launch knows).
+        const float all = ((sum[0] + sum[1]) + (sum[2] + sum[3])) + ((sum[4] + sum[5]) + (sum[6] + sum[7]));
+        __syncwarp();
+        if (lane == 0) umma::mbar_arrive(umma::smem_u32(&empty[st]) + (__float_as_uint(all) & a.zero));
+        if (++st == STAGES) st = 0, ph ^= 1;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        sum[k] += __shfl_xor_sync(0xFFFFFFFFu, sum[k], 16);
+        if (lane < 16) bias_part[(e >> 5) * 128 + 8 * unit + k] = sum[k];
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps
+      if (n0 + e < a.Cout)
+        atomicAdd(a.db + n0 + e, (bias_part[e] + bias_part[128 + e]) + (bias_part[256 + e] + bias_part[384 + e]));
+    }
+    const bool ok = umma::mbar_wait_warp(done, 0, a.err, ERR_EPILOGUE);
     umma::fence_after_sync();
     if (ok) {
 #pragma unroll 1
@@ -1818,7 +1853,7 @@ int dispatch_conv(const ConvArgs& a, int ntn, bool staged, int stages, cudaStrea
 
 template <int BN, int NT, int STAGES>
 int launch_wgrad(const WgradArgs& a, int splits, cudaStream_t st) {
-  constexpr int smem = wgrad_region<BN, NT, STAGES>() + 1024 + 256;
+  constexpr int smem = wgrad_region<BN, NT, STAGES>() + 1024 + 256 + 2048;  // alignment, barriers, bias sums
   auto kern = wgrad_kernel<BN, NT, STAGES>;
   static KernelLimits limits;
   const int rc = limits.get(reinterpret_cast<const void*>(kern), smem);
@@ -2006,8 +2041,8 @@ int msur_conv_get_stages(int bn) {
   return g_conv_stages[bn == 256 ? 2 : (bn == 128 ? 1 : 0)];
 }
 
-int msur_conv_wgrad(const void* x, const void* dz, int B, int L, int Cin, int Cout, int taps, float* dw, int splits,
-                    void* stream) {
+static int conv_wgrad_impl(const void* x, const void* dz, int B, int L, int Cin, int Cout, int taps, float* dw, float* db,
+                           int splits, void* stream) {
   if (!x || !dz || !dw || B <= 0 || L <= 0 || Cin <= 0 || Cout <= 0 || (taps != 1 && taps != 3))
     return fail(MSUR_ERR_INVALID_ARG, "msur_conv_wgrad: bad shape or null pointer (taps must be 1 or 3)");
   if ((Cin % 8) || (Cout % 8) || !aligned16(x) || !aligned16(dz))
@@ -2021,7 +2056,8 @@ int msur_conv_wgrad(const void* x, const void* dz, int B, int L, int Cin, int Co
   const uint64_t x_dims[3] = {static_cast<uint64_t>(Cin), static_cast<uint64_t>(L), static_cast<uint64_t>(B)};
   const uint32_t box[3] = {64, 64, 1};
   rc = make_map(&a.tm_dz, dz, 3, dz_dims, box);
-  if (!rc) rc = make_map(&a.tm_x, x, 3, x_dims, box);
+  const uint32_t xbox[3] = {64, static_cast<uint32_t>(64 + taps - 1), 1};
+  if (!rc) rc = make_map(&a.tm_x, x, 3, x_dims, xbox);
   if (rc) return rc;
   a.B = B;
   a.L = L;
@@ -2041,14 +2077,20 @@ int msur_conv_wgrad(const void* x, const void* dz, int B, int L, int Cin, int Co
   a.per_split = (a.total + splits - 1) / splits;
   splits = (a.total + a.per_split - 1) / a.per_split;
   a.dw = dw;
+  a.db = db;
   a.bulk = aligned16(dw) ? 1 : 0;
   a.err = err;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (taps == 3) {
-    if (Cin <= 64) return launch_wgrad<64, 3, 4>(a, splits, st);
-    return launch_wgrad<128, 3, 3>(a, splits, st);
+    if (Cin <= 64) return launch_wgrad<64, 3, 6>(a, splits, st);
+    return launch_wgrad<128, 3, 6>(a, splits, st);
   }
-  return launch_wgrad<128, 1, 4>(a, splits, st);
+  return launch_wgrad<128, 1, 6>(a, splits, st);
+}
+
+int msur_conv_wgrad(const void* x, const void* dz, int B, int L, int Cin, int Cout, int taps, float* dw, int splits,
+                    void* stream) {
+  return conv_wgrad_impl(x, dz, B, L, Cin, Cout, taps, dw, nullptr, splits, stream);
 }
 
 int msur_pool2(const void* x, int B, int Lout, int C, void* y, void* stream) {
@@ -2193,10 +2235,8 @@ int msur_run(const msur_op* ops, int n, void* stream) {
                                o.form, o.stages, stream);
         break;
       case MSUR_OP_WGRAD:
-        rc = msur_conv_wgrad(p[0], p[1], i[0], i[1], i[2], i[3], i[4], static_cast<float*>(p[2]), i[5], stream);
-        break;
-      case MSUR_OP_BIAS_GRAD:
-        rc = msur_bias_grad(p[0], o.rows, i[0], i[1], static_cast<float*>(p[1]), stream);
+        rc = conv_wgrad_impl(p[0], p[1], i[0], i[1], i[2], i[3], i[4], static_cast<float*>(p[2]),
+                             static_cast<float*>(p[3]), i[5], stream);
         break;
       case MSUR_OP_POOL2:
         rc = msur_pool2(p[0], i[0], i[1], i[2], p[1], stream);

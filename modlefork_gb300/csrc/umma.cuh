@@ -28,6 +28,14 @@ __device__ __forceinline__ uint64_t global_ns() {
   return t;
 }
 
+// A 16-byte load from shared memory that stays where it is among the barrier operations.
+__device__ __forceinline__ void ld_shared_v4(uint32_t (&x)[4], uint32_t addr) {
+  asm volatile("ld.volatile.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3])
+               : "r"(addr)
+               : "memory");
+}
+
 // ---- mbarrier ---------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
@@ -40,9 +48,10 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) { mbar_arrive(smem_u32(bar)); }
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -217,12 +226,16 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// One K step of 64 elements with 128-byte swizzled K-major operands: four products of 16, their
-// descriptors (sdesc_sw128 split into the words that change and the one that does not) 32 bytes apart.
+// Four products of 16 along K from 128-byte swizzled operands whose descriptors (sdesc_sw128 split into the word
+// that changes and the one that does not) advance by STEP 16-byte units: 2 for a K-major step of 64 elements,
+// 128 for an MN-major one of 64 rows.
 constexpr uint32_t SDESC_SW128_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
-__device__ __forceinline__ uint32_t sdesc_sw128_lo(uint32_t saddr) { return (saddr >> 4) | (1u << 16); }
-__device__ __forceinline__ void mma_bf16_k64(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
-                                             uint32_t accumulate) {
+__device__ __forceinline__ uint32_t sdesc_sw128_lo(uint32_t saddr, uint32_t lbo_bytes = 16) {
+  return (saddr >> 4) | ((lbo_bytes >> 4) << 16);
+}
+template <int STEP>
+__device__ __forceinline__ void mma_bf16_x4(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc,
+                                            uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
       "setp.ne.b32 p, %5, 0;\n\t"
@@ -230,16 +243,16 @@ __device__ __forceinline__ void mma_bf16_k64(uint32_t d_tmem, uint32_t a_lo, uin
       "mov.b64 a, {%1, %3};\n\t"
       "mov.b64 b, {%2, %3};\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t"
-      "add.s64 a, a, 2;\n\t"
-      "add.s64 b, b, 2;\n\t"
+      "add.s64 a, a, %6;\n\t"
+      "add.s64 b, b, %6;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, q;\n\t"
-      "add.s64 a, a, 2;\n\t"
-      "add.s64 b, b, 2;\n\t"
+      "add.s64 a, a, %6;\n\t"
+      "add.s64 b, b, %6;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, q;\n\t"
-      "add.s64 a, a, 2;\n\t"
-      "add.s64 b, b, 2;\n\t"
+      "add.s64 a, a, %6;\n\t"
+      "add.s64 b, b, %6;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, q;\n\t}" ::"r"(d_tmem),
-      "r"(a_lo), "r"(b_lo), "r"(SDESC_SW128_HI), "r"(idesc), "r"(accumulate)
+      "r"(a_lo), "r"(b_lo), "r"(SDESC_SW128_HI), "r"(idesc), "r"(accumulate), "n"(STEP)
       : "memory");
 }
 // Arrive on *bar once every MMA issued so far by this thread has completed.

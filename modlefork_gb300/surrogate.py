@@ -283,40 +283,39 @@ class UNet:
         return (ops.Op * len(lst))(*lst)
 
     # ---- backward ------------------------------------------------------------------------
-    def _grad_ops(self, name, x, dz):
+    def _grad_op(self, name, x, dz):
         """Weight and bias gradients of convolution `name` with input x and output gradient dz."""
         B, L, cin = x.shape
         s = self.specs[name]
-        return [ops.op(ops.OP_WGRAD, (x, dz, self.gw[name]), (B, L, cin, s.cout, s.taps, 0)),
-                ops.op(ops.OP_BIAS_GRAD, (dz, self.gb[name]), (s.cout, dz.shape[-1]), rows=B * L)]
+        return ops.op(ops.OP_WGRAD, (x, dz, self.gw[name], self.gb[name]), (B, L, cin, s.cout, s.taps, 0))
 
     def _dgrad_op(self, name, dz, out, gate=None):
         return ops.conv_op(dz, self.wt[name], post=out, gate=gate)
 
     def _backward_ops(self, B, ws):
         D = self.depth
-        lst = self._grad_ops("head", ws["ydb0"], ws["dout"])
+        lst = [self._grad_op("head", ws["ydb0"], ws["dout"])]
         lst.append(self._dgrad_op("head", ws["dout"], ws["ddb0"], gate=ws["zdb0"]))
         for i in range(D):
-            lst += self._grad_ops(f"dec{i}b", ws[f"yda{i}"], ws[f"ddb{i}"])
+            lst.append(self._grad_op(f"dec{i}b", ws[f"yda{i}"], ws[f"ddb{i}"]))
             lst.append(self._dgrad_op(f"dec{i}b", ws[f"ddb{i}"], ws[f"dda{i}"], gate=ws[f"zda{i}"]))
-            lst += self._grad_ops(f"dec{i}a", ws[f"cat{i}"], ws[f"dda{i}"])
+            lst.append(self._grad_op(f"dec{i}a", ws[f"cat{i}"], ws[f"dda{i}"]))
             lst.append(self._dgrad_op(f"dec{i}a", ws[f"dda{i}"], ws[f"dcat{i}"]))
             z, dz = (ws[f"zdb{i + 1}"], ws[f"ddb{i + 1}"]) if i + 1 < D else (ws["zmb"], ws["dmb"])
             lst.append(ops.op(ops.OP_UPCAT_BWD, (ws[f"dcat{i}"], z, dz),
                               (B, z.shape[1], z.shape[2], ws[f"dcat{i}"].shape[-1])))
-        lst += self._grad_ops("mid_b", ws["yma"], ws["dmb"])
+        lst.append(self._grad_op("mid_b", ws["yma"], ws["dmb"]))
         lst.append(self._dgrad_op("mid_b", ws["dmb"], ws["dma"], gate=ws["zma"]))
-        lst += self._grad_ops("mid_a", ws[f"p{D - 1}"], ws["dma"])
+        lst.append(self._grad_op("mid_a", ws[f"p{D - 1}"], ws["dma"]))
         lst.append(self._dgrad_op("mid_a", ws["dma"], ws[f"dp{D - 1}"]))
         for i in reversed(range(D)):
             ch = self.mid if i == D - 1 else self.widths[i + 1]
             z = ws[f"zb{i}"]
             lst.append(ops.op(ops.OP_SKIP_GRAD, (ws[f"dp{i}"], ws[f"dcat{i}"], z, ws[f"dzb{i}"]),
                               (ws[f"dp{i}"].shape[1], ws[f"dcat{i}"].shape[-1], ch, B, z.shape[1], z.shape[2])))
-            lst += self._grad_ops(f"enc{i}b", ws[f"ya{i}"], ws[f"dzb{i}"])
+            lst.append(self._grad_op(f"enc{i}b", ws[f"ya{i}"], ws[f"dzb{i}"]))
             lst.append(self._dgrad_op(f"enc{i}b", ws[f"dzb{i}"], ws[f"dza{i}"], gate=ws[f"za{i}"]))
-            lst += self._grad_ops(f"enc{i}a", ws["x"] if i == 0 else ws[f"p{i - 1}"], ws[f"dza{i}"])
+            lst.append(self._grad_op(f"enc{i}a", ws["x"] if i == 0 else ws[f"p{i - 1}"], ws[f"dza{i}"]))
             if i > 0:
                 lst.append(self._dgrad_op(f"enc{i}a", ws[f"dza{i}"], ws[f"dp{i - 1}"]))
         return (ops.Op * len(lst))(*lst)
@@ -327,7 +326,7 @@ class UNet:
         if "backward_ops" not in ws:
             ws["backward_ops"] = self._backward_ops(B, ws)
         oplist = ws["backward_ops"]
-        oplist[len(oplist) - 2].p[0] = ws["h_in0"].data_ptr()  # enc0a's weight gradient reads the input
+        oplist[len(oplist) - 1].p[0] = ws["h_in0"].data_ptr()  # enc0a's weight gradient reads the input
         ops.run(oplist)
 
     def loss_and_grad(self, x, target):

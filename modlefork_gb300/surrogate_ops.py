@@ -26,10 +26,10 @@ class Op(C.Structure):
     """msur_op: one operation of a list (run)."""
 
     _fields_ = [("kind", C.c_int), ("form", C.c_int), ("stages", C.c_int), ("i", C.c_int * 12),
-                ("rows", C.c_uint64), ("p", C.c_void_p * 10)]
+                ("p", C.c_void_p * 10)]
 
 
-OP_CONV, OP_WGRAD, OP_BIAS_GRAD, OP_POOL2, OP_SKIP_GRAD, OP_UPCAT, OP_UPCAT_BWD = range(7)
+OP_CONV, OP_WGRAD, OP_POOL2, OP_SKIP_GRAD, OP_UPCAT, OP_UPCAT_BWD = range(6)
 
 
 def load(path=LIB_PATH):
@@ -189,11 +189,10 @@ def weight_transpose(w, wt):
     _check(load().msur_weight_transpose(_p(w), N, taps, Cw, _p(wt), _stream()), "msur_weight_transpose")
 
 
-def op(kind, tensors, ints, rows=0, form=-1, stages=-1):
+def op(kind, tensors, ints, form=-1, stages=-1):
     """One Op: tensors (or None) and integers in msur_op's order.  Holds addresses only: the caller keeps the
     tensors alive for as long as the operation is run."""
     o = Op(kind, form, stages)
-    o.rows = rows
     for k, t in enumerate(tensors):
         o.p[k] = _p(t)
     for k, v in enumerate(ints):

@@ -133,8 +133,7 @@ def test_list_of_operations_equals_them_one_by_one():
                ops.op(ops.OP_UPCAT, (post2, post, cat), (B, L, C, C)),
                ops.conv_op(post, w2, post=dcat),
                ops.op(ops.OP_UPCAT_BWD, (dcat, post2, dz), (B, L // 2, C, 2 * C)),
-               ops.op(ops.OP_WGRAD, (pool, dz, dw), (B, L // 2, C, C, 3, 1)),
-               ops.op(ops.OP_BIAS_GRAD, (dz, db), (C, C), rows=B * L // 2)]
+               ops.op(ops.OP_WGRAD, (pool, dz, dw, db), (B, L // 2, C, C, 3, 1))]
         run(lst)
         torch.cuda.synchronize()
         return pre, post, pool, post2, cat, dcat, dz, dw, db
@@ -146,11 +145,8 @@ def test_list_of_operations_equals_them_one_by_one():
 
     want = chain(one_by_one)
     got = chain(lambda lst: ops.run((ops.Op * len(lst))(*lst)))
-    for k, (a, c) in enumerate(zip(got[:-1], want[:-1])):
+    for k, (a, c) in enumerate(zip(got, want)):
         assert torch.equal(a, c), k
-    # the bias gradient's blocks add in any order: 250 blocks' partial sums of FP32
-    size = want[6].float().abs().sum((0, 1))
-    assert ((got[8] - want[8]).abs() <= 250 * 2.0 ** -23 * size).all()
     bad = ops.op(99, (x,), (B,))
     with pytest.raises(ops.SurrogateKernelError):
         ops.run((ops.Op * 1)(bad))
@@ -169,3 +165,27 @@ def test_selected_map_sums():
                 assert ((part[:, k] - full[:, k]).abs() <= 1e-13 * 40_001).all(), k
             else:
                 assert not part[:, k].any(), k
+
+
+@pytest.mark.parametrize("B,L,cin,cout,taps", [(16, 999, 256, 256, 3), (3, 130, 64, 64, 3), (5, 64, 128, 600, 1),
+                                               (1, 63, 8, 8, 3), (2, 1, 192, 136, 3), (40, 65, 896, 384, 3)])
+def test_weight_and_bias_gradient_in_one(B, L, cin, cout, taps):
+    """Against FP64: products and sums of BF16 values in FP32, K terms each (error of any order of adding: at most
+    (K + 1) 2^-24 of the sum of magnitudes; 16 times its square root covers a random walk many times over), added to
+    what was there; rows and columns past the tiles' edges."""
+    x, _, _, z = _inputs(B, L, cin, cout, taps)
+    dw = torch.ones(cout, taps, cin, device=DEV)
+    db = torch.ones(cout, device=DEV)
+    o = ops.op(ops.OP_WGRAD, (x, z, dw, db), (B, L, cin, cout, taps, 0))
+    ops.run((ops.Op * 1)(o))
+    pad = (taps - 1) // 2
+    xp = torch.zeros(B, L + 2 * pad, cin, dtype=torch.float64, device=DEV)
+    xp[:, pad:pad + L] = x.double()
+    zd = z.double()
+    tol = 16 * (B * L + 2) ** 0.5 * 2.0 ** -24
+    assert ((db - 1 - zd.sum((0, 1))).abs() <= tol * (zd.abs().sum((0, 1)) + 1)).all()
+    for t in range(taps):
+        xt = xp[:, t:t + L]
+        want = torch.einsum("bln,blc->nc", zd, xt)
+        size = torch.einsum("bln,blc->nc", zd.abs(), xt.abs()) + 1
+        assert ((dw[:, t] - 1 - want).abs() <= tol * size).all()
