@@ -1808,6 +1808,9 @@ ConvPlan conv_plan(int bn, int cin, int taps, int cout, int L, int B, int stages
     p.aslots += kc;
     used += kc * SLOT_BYTES;
   }
+  // with a tile or two per CTA the ring's depth is what hides a load (one map: 200 us with four stages, 186)
+  const int stage = w + (p.aslots ? 0 : BM * BK * 2);
+  while (!p.wres && p.stages < 8 && p.stages < nk && used + stage <= ROOM) ++p.stages, used += stage;
   p.bufs = staged ? 1 : 0;
   if (staged && used + p.groups * group <= ROOM) {
     p.bufs = 2;

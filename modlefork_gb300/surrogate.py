@@ -227,7 +227,7 @@ class UNet:
         """x: [B, L, 64] BF16 input; returns the [B, L, 600] FP32 prediction: `out` when given
         (contiguous FP32 on the device), else a workspace view that the next call overwrites.
 
-        In inference (and with fuse, when fusable()) the encoder's second convolution writes its
+        With fuse, when fusable(), the encoder's second convolution writes its
         output into the skip half of its level's concatenation buffer and, pooled, into the next
         level's input, and the convolution below a decoder level writes its output upsampled into
         the other half, so no separate pooling or upsample-and-concatenate step runs; the results
@@ -235,7 +235,7 @@ class UNet:
         B = x.shape[0]
         assert tuple(x.shape[1:]) == (self.length, IN_CH) and x.dtype == torch.bfloat16
         ws = self._workspace(B, train)
-        fused = bool(fuse and not train and self.fusable())
+        fused = bool(fuse and self.fusable())
         # the pass as a list of operations on the workspace; only its input and output differ by call
         key = (fused, tuple(LAYER_CFG.items()))
         if ws.get("forward_key") != key:
@@ -257,15 +257,16 @@ class UNet:
             lst.append(self._conv_op(f"enc{i}a", h, pre=get(f"za{i}"), post=ws[f"ya{i}"]))
             if fused:
                 cat = ws[f"cat{i}"]
-                lst.append(self._conv_op(f"enc{i}b", ws[f"ya{i}"], skip=cat[:, :, cat.shape[-1] - self.widths[i]:],
-                                         pool=ws[f"p{i}"]))
+                lst.append(self._conv_op(f"enc{i}b", ws[f"ya{i}"], pre=get(f"zb{i}"),
+                                         skip=cat[:, :, cat.shape[-1] - self.widths[i]:], pool=ws[f"p{i}"]))
             else:
                 lst.append(self._conv_op(f"enc{i}b", ws[f"ya{i}"], pre=get(f"zb{i}"), post=ws[f"yb{i}"]))
                 lst.append(ops.op(ops.OP_POOL2, (ws[f"yb{i}"], ws[f"p{i}"]), (B, lens // 2, self.widths[i])))
             h = ws[f"p{i}"]
         lst.append(self._conv_op("mid_a", h, pre=get("zma"), post=ws["yma"]))
         if fused:
-            lst.append(self._conv_op("mid_b", ws["yma"], dup=ws[f"cat{self.depth - 1}"][:, :, :self.mid]))
+            lst.append(self._conv_op("mid_b", ws["yma"], pre=get("zmb"),
+                                     dup=ws[f"cat{self.depth - 1}"][:, :, :self.mid]))
         else:
             lst.append(self._conv_op("mid_b", ws["yma"], pre=get("zmb"), post=ws["ymb"]))
             h = ws["ymb"]
@@ -275,7 +276,8 @@ class UNet:
                                   (B, self.length >> i, h.shape[-1], self.widths[i])))
             lst.append(self._conv_op(f"dec{i}a", ws[f"cat{i}"], pre=get(f"zda{i}"), post=ws[f"yda{i}"]))
             if fused and i > 0:
-                lst.append(self._conv_op(f"dec{i}b", ws[f"yda{i}"], dup=ws[f"cat{i - 1}"][:, :, :self.widths[i]]))
+                lst.append(self._conv_op(f"dec{i}b", ws[f"yda{i}"], pre=get(f"zdb{i}"),
+                                         dup=ws[f"cat{i - 1}"][:, :, :self.widths[i]]))
             else:
                 lst.append(self._conv_op(f"dec{i}b", ws[f"yda{i}"], pre=get(f"zdb{i}"), post=ws[f"ydb{i}"]))
                 h = ws[f"ydb{i}"]
