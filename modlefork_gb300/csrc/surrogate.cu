@@ -761,9 +761,13 @@ __global__ void __launch_bounds__(PTHREADS, 1)
 // The splits' partial sums meet in dw.  A thread holds one output channel's row of the accumulators;
 // adding it word by word (32 rows per warp and instruction) took longer than the products: 113 of
 // 133 us for 16 x 999 positions, 256 to 256 channels.  So the rows go to the operand stages, free by
-// then (a row is padded by 16 bytes: conflict-free 16-byte stores), and each thread adds its row with
-// one bulk reduction per tap (cp.reduce.async.bulk, up to 512 contiguous bytes).
+// then (a row is padded by 16 bytes: conflict-free 16-byte stores), and each thread adds its row tap by tap
+// with bulk reductions (cp.reduce.async.bulk, up to 256 contiguous bytes).  Eight warps share the
+// columns and a tap's reductions run while the next is staged: 16 x 2000 positions, 128 to 128
+// channels, took 15.6 us with four warps and the reductions at the end, of which 4.5 and 6.3 were these two.
 // ---------------------------------------------------------------------------------------
+constexpr int WTHREADS = 320;  // warp 0 TMA, warp 1 MMA and TMEM, warps 2-9 epilogue
+
 struct WgradArgs {
   CUtensorMap tm_dz;  // [B][L][Cout]: dims {Cout, L, B}, box {64, 64, 1}
   CUtensorMap tm_x;   // [B][L][Cin]: dims {Cin, L, B}, box {64, 64 + taps - 1, 1}
@@ -795,7 +799,7 @@ __host__ __device__ constexpr int wgrad_region() {
 }
 
 template <int BN, int NT, int STAGES>
-__global__ void __launch_bounds__(THREADS, 1) wgrad_kernel(const __grid_constant__ WgradArgs a) {
+__global__ void __launch_bounds__(WTHREADS, 1) wgrad_kernel(const __grid_constant__ WgradArgs a) {
   constexpr int BOX = 64 * 64 * 2;  // one 64 x 64 BF16 box
   constexpr int A_BYTES = 2 * BOX;  // 128 output channels
   constexpr int XBOX = wgrad_box_bytes<NT>();
@@ -874,9 +878,9 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_kernel(const __grid_constant
     }
     if (umma::elect()) umma::mma_commit(done);
   } else if (nk > 0) {
-    const int q = warp & 3;
+    const int q = warp & 3, half = warp >= 6;
     const int n = n0 + 32 * q + lane;
-    if (bias) {
+    if (bias && !half) {
       // thread e: 8 channels (16-byte unit e % 16 of the two boxes), rows 8 (e / 16) .. + 7 of each block
       const int e = threadIdx.x - 64, unit = e & 15;
       float sum[8] = {};
@@ -910,45 +914,47 @@ __global__ void __launch_bounds__(THREADS, 1) wgrad_kernel(const __grid_constant
         sum[k] += __shfl_xor_sync(0xFFFFFFFFu, sum[k], 16);
         if (lane < 16) bias_part[(e >> 5) * 128 + 8 * unit + k] = sum[k];
       }
-      asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps
+      asm volatile("bar.sync 2, 128;" ::: "memory");  // the four warps that add up
       if (n0 + e < a.Cout)
         atomicAdd(a.db + n0 + e, (bias_part[e] + bias_part[128 + e]) + (bias_part[256 + e] + bias_part[384 + e]));
     }
     const bool ok = umma::mbar_wait_warp(done, 0, a.err, ERR_EPILOGUE);
     umma::fence_after_sync();
+    if (bias) asm volatile("bar.sync 1, 256;" ::: "memory");  // the stages have been added up: rows may go there
     if (ok) {
+      // tap by tap: this half's columns of the thread's row to shared memory, and on to dw while the next tap's
+      // are read
+      constexpr int HALF = BN / 2;
+      const int cc = c0 + half * HALF;
+      const bool inside = n < a.Cout && cc < a.Cin;
+      const uint32_t cols = tmem + (static_cast<uint32_t>(32 * q) << 16) + half * HALF;
+      uint8_t* const row = smem + (32 * q + lane) * wgrad_row_bytes<BN, NT>() + half * HALF * 4;
 #pragma unroll 1
       for (int t = 0; t < NT; ++t) {
-#pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
-          float v[32];
-          umma::tmem_ld32(tmem + (static_cast<uint32_t>(32 * q) << 16) + t * BN + c * 32, v);
-          const int cc = c0 + c * 32;
-          if (n >= a.Cout || cc >= a.Cin) continue;
-          if (a.bulk) {
-            float4* row = reinterpret_cast<float4*>(smem + (32 * q + lane) * wgrad_row_bytes<BN, NT>() +
-                                                    (t * BN + c * 32) * 4);
+        float v[HALF];
+        if constexpr (HALF == 64) {
+          umma::tmem_ld64(cols + t * BN, v);
+        } else {
+          umma::tmem_ld32(cols + t * BN, v);
+        }
+        if (!inside) continue;
+        float* dst = a.dw + (static_cast<size_t>(n) * a.taps + t) * a.Cin + cc;
+        if (a.bulk) {
+          float4* to = reinterpret_cast<float4*>(row + t * BN * 4);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) row[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-            continue;
-          }
-          float* dst = a.dw + (static_cast<size_t>(n) * a.taps + t) * a.Cin + cc;
-          const int nv = min(32, a.Cin - cc);
-          for (int j = 0; j < nv; ++j) atomicAdd(dst + j, v[j]);
-        }
-      }
-      if (a.bulk) {
-        if (n < a.Cout) {
-          umma::fence_async_smem();  // this thread's row, read by its own reductions
-          const uint8_t* row = smem + (32 * q + lane) * wgrad_row_bytes<BN, NT>();
-          for (int t = 0; t < NT; ++t)
-            umma::bulk_reduce_add_f32(a.dw + (static_cast<size_t>(n) * a.taps + t) * a.Cin + c0, row + t * BN * 4,
-                                      4 * min(BN, a.Cin - c0));
+          for (int k = 0; k < HALF / 4; ++k) to[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+          umma::fence_async_smem();  // this thread's values, read by its own reduction
+          umma::bulk_reduce_add_f32(dst, to, 4 * min(HALF, a.Cin - cc));
           umma::bulk_commit();
-          umma::bulk_wait_all();
+        } else {
+          const int nv = min(HALF, a.Cin - cc);
+#pragma unroll
+          for (int j = 0; j < HALF; ++j)
+            if (j < nv) atomicAdd(dst + j, v[j]);
         }
-        __syncwarp();
       }
+      umma::bulk_wait_all();
+      __syncwarp();
     }
   }
   umma::fence_before_sync();
@@ -1862,8 +1868,7 @@ int launch_wgrad(const WgradArgs& a, int splits, cudaStream_t st) {
   const int rc = limits.get(reinterpret_cast<const void*>(kern), smem);
   if (rc) return rc;
   dim3 grid((a.Cin + BN - 1) / BN, (a.Cout + BM - 1) / BM, splits);
-  return cuda_ok(launch_pdl(kern, grid, THREADS, smem, st, a),
-                 "wgrad_kernel launch");
+  return cuda_ok(launch_pdl(kern, grid, WTHREADS, smem, st, a), "wgrad_kernel launch");
 }
 
 unsigned grid_for(size_t n, unsigned block = 256) {
