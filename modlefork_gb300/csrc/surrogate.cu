@@ -1164,10 +1164,72 @@ struct PairSum {
   }
   __device__ __forceinline__ double value() const { return static_cast<double>(h) + static_cast<double>(l); }
 };
-__device__ __forceinline__ void exact_difference(float a, float b, float& h, float& l) {
-  h = __fsub_rn(a, b);
-  const float z = __fsub_rn(h, a);
-  l = __fsub_rn(__fsub_rn(a, __fsub_rn(h, z)), __fadd_rn(b, z));
+
+// Two floats in a register pair and the packed operations on them: each half rounds as the scalar operation does,
+// at half the instructions.
+struct F2 {
+  unsigned long long v = 0;
+};
+__device__ __forceinline__ F2 f2(float x, float y) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void f2_get(F2 a, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v)); }
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+  asm("add.rn.f32x2 %0, %0, %1;" : "+l"(a.v) : "l"(b.v));
+  return a;
+}
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) {
+  asm("sub.rn.f32x2 %0, %0, %1;" : "+l"(a.v) : "l"(b.v));
+  return a;
+}
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) {
+  asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(a.v) : "l"(b.v));
+  return a;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c.v) : "l"(a.v), "l"(b.v));
+  return c;
+}
+__device__ __forceinline__ F2 operator-(F2 a) {
+  a.v ^= 0x8000000080000000ull;
+  return a;
+}
+// Two running sums as pairs of floats, side by side.
+struct PairSum2 {
+  F2 h, l;
+  __device__ __forceinline__ void add(F2 x) {
+    const F2 t = h + x, z = t - h;
+    l = l + ((h - (t - z)) + (x - z));
+    h = t;
+  }
+  __device__ __forceinline__ void add(F2 x, F2 rest) {
+    add(x);
+    l = l + rest;
+  }
+  // a * b + rest, rest far smaller
+  __device__ __forceinline__ void add_product(F2 a, F2 b, F2 rest) {
+    const F2 p = a * b;
+    add(p, f2_fma(a, b, -p) + rest);
+  }
+  __device__ __forceinline__ void add_product(F2 a, F2 b) {
+    const F2 p = a * b;
+    add(p, f2_fma(a, b, -p));
+  }
+  __device__ __forceinline__ double value() const {
+    float x, y, u, w;
+    f2_get(h, x, y);
+    f2_get(l, u, w);
+    const float t = __fadd_rn(x, y), z = __fsub_rn(t, x);
+    const float e = __fadd_rn(__fsub_rn(x, __fsub_rn(t, z)), __fsub_rn(y, z));
+    return static_cast<double>(t) + static_cast<double>(__fadd_rn(__fadd_rn(u, w), e));
+  }
+};
+__device__ __forceinline__ void exact_difference(F2 a, F2 b, F2& h, F2& l) {
+  h = a - b;
+  const F2 z = h - a;
+  l = (a - (h - z)) - (b + z);
 }
 
 // The same eight channels (16 bytes) per thread: a block covers 64 channels and 32 rows at a time.  Reads at
@@ -1456,17 +1518,19 @@ __global__ void band_target_kernel(const uint32_t* band, size_t ncols, int nrows
 // the reference's Pearson (mean, then covariances of the deviations).
 //
 // FP64's accuracy at the FP32 pipes' rate (FP64 runs at 1/64 of it on sm_103a: 11 FP64 operations per
-// element took 1.7 ms for 32 maps of 2.4 M values, of which the memory needs 0.1).  Each thread sums chunks of 64
-// elements in pairs of floats: differences, products and sums with their exact rounding errors (Knuth's
+// element took 1.7 ms for 32 maps of 2.4 M values, of which the memory needs 0.1).  Each thread sums chunks of 128
+// elements in two pairs of floats: differences, products and sums with their exact rounding errors (Knuth's
 // two-sum, two-product by FMA), and adds each chunk's pair to FP64 totals.  The means are split into a float
 // m and a remainder d: the deviations from m are exact pairs, and d enters the FP64 totals,
 // sum (a - d)^2 = sum a^2 - 2 d sum a + n d^2.  A pair carries 2^-47 per operation and the chunks' errors
 // average out over the map; measured against 64-bit sums the scores are as close as before (a few 1e-16).
 // A chunk with values outside [2^-30, 2^50) in size throughout, infinities or NaN is summed in FP64.
 // WHICH: the sums wanted (bit k: sum k); MEANS: deviations from the means, raw values otherwise.
-constexpr int SUM_VECS = 16;  // float4 per thread and chunk
+// The pairs come two to a packed operation (PairSum2), and two loads of each side run ahead: both passes over
+// those maps took 406 us without, 356 with (more loads ahead, or three blocks per SM, spill).
+constexpr int SUM_VECS = 32;  // float4 per thread and chunk
 template <bool VEC, bool MEANS, unsigned WHICH>
-__global__ void __launch_bounds__(256) map_sums_pair_kernel(const float* pred, size_t pstride_map, const float* ref,
+__global__ void __launch_bounds__(256, 2) map_sums_pair_kernel(const float* pred, size_t pstride_map, const float* ref,
                                                             size_t rstride_map, size_t n, const double* means,
                                                             double* out) {
   const int m = blockIdx.y;
@@ -1479,21 +1543,36 @@ __global__ void __launch_bounds__(256) map_sums_pair_kernel(const float* pred, s
   double cnt = 0.0;
   const size_t span = static_cast<size_t>(SUM_VECS) * 256 * 4;  // elements of a block's step
   const uint32_t LO = 0x30800000u, HI = 0x58800000u;           // 2^-30, 2^50
+  auto load2 = [&](float4& x, float4& y, size_t i) {
+    if (i < n) {
+      x = __ldg(reinterpret_cast<const float4*>(p + i));
+      y = __ldg(reinterpret_cast<const float4*>(r + i));
+    }
+  };
   const bool means_ok = __float_as_uint(fabsf(fp)) < HI && __float_as_uint(fabsf(fr)) < HI;
   for (size_t base = blockIdx.x * span; base < n; base += gridDim.x * span) {
-    PairSum t[6];
+    PairSum2 t[6];
     uint32_t mxp = 0, mxr = 0;
     int k = 0;
+    const F2 fp2 = f2(fp, fp), fr2 = f2(fr, fr);
+    // two loads of each side in flight while the ones before them are summed
+    float4 qp[2], qr[2];
+    const size_t first = base + threadIdx.x * 4;
+    if constexpr (VEC) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) load2(qp[u], qr[u], first + u * 1024);
+    }
 #pragma unroll 2
     for (int v = 0; v < SUM_VECS; ++v) {
-      const size_t i = base + (static_cast<size_t>(v) * 256 + threadIdx.x) * 4;
+      const size_t i = first + static_cast<size_t>(v) * 1024;
       if (i >= n) break;
       float a[4], b[4];
       int valid = 4;
       if constexpr (VEC) {
-        const float4 pa = __ldg(reinterpret_cast<const float4*>(p + i)), rb = __ldg(reinterpret_cast<const float4*>(r + i));
+        const float4 pa = qp[v & 1], rb = qr[v & 1];
         a[0] = pa.x, a[1] = pa.y, a[2] = pa.z, a[3] = pa.w;
         b[0] = rb.x, b[1] = rb.y, b[2] = rb.z, b[3] = rb.w;
+        if (v + 2 < SUM_VECS) load2(qp[v & 1], qr[v & 1], i + 2048);
       } else {
         valid = static_cast<int>(n - i < 4 ? n - i : 4);
 #pragma unroll
@@ -1506,28 +1585,34 @@ __global__ void __launch_bounds__(256) map_sums_pair_kernel(const float* pred, s
       for (int e = 0; e < 4; ++e) {
         mxp = max(mxp, __float_as_uint(fabsf(a[e])));
         mxr = max(mxr, __float_as_uint(fabsf(b[e])));
-        float ah, al, bh, bl, h, l;
+      }
+#pragma unroll
+      for (int e = 0; e < 4; e += 2) {
+        const F2 a2 = f2(a[e], a[e + 1]), b2 = f2(b[e], b[e + 1]);
         if constexpr (MEANS) {
-          exact_difference(a[e], fp, ah, al);
-          exact_difference(b[e], fr, bh, bl);
+          F2 ah, al, bh, bl;
+          exact_difference(a2, fp2, ah, al);
+          exact_difference(b2, fr2, bh, bl);
+          if constexpr (WHICH & 1) t[0].add(ah, al);
+          if constexpr (WHICH & 2) t[1].add(bh, bl);
+          if constexpr (WHICH & 4) t[2].add_product(ah, ah, (ah + ah) * al);
+          if constexpr (WHICH & 8) t[3].add_product(bh, bh, (bh + bh) * bl);
+          if constexpr (WHICH & 16) t[4].add_product(ah, bh, f2_fma(ah, bl, al * bh));
         } else {
-          ah = a[e], al = 0.0f, bh = b[e], bl = 0.0f;
+          if constexpr (WHICH & 1) t[0].add(a2);
+          if constexpr (WHICH & 2) t[1].add(b2);
+          if constexpr (WHICH & 4) t[2].add_product(a2, a2);
+          if constexpr (WHICH & 8) t[3].add_product(b2, b2);
+          if constexpr (WHICH & 16) t[4].add_product(a2, b2);
         }
-        if constexpr (WHICH & 1) {
-          t[0].add(ah);
-          t[0].l += al;
-        }
-        if constexpr (WHICH & 2) {
-          t[1].add(bh);
-          t[1].l += bl;
-        }
-        if constexpr (WHICH & 4) t[2].add_product(ah, ah, MEANS ? 2.0f * ah * al : 0.0f);
-        if constexpr (WHICH & 8) t[3].add_product(bh, bh, MEANS ? 2.0f * bh * bl : 0.0f);
-        if constexpr (WHICH & 16) t[4].add_product(ah, bh, MEANS ? ah * bl + al * bh : 0.0f);
         if constexpr (WHICH & 32) {
-          exact_difference(a[e], b[e], h, l);
-          if (!VEC && e >= valid) h = l = 0.0f;
-          t[5].add_product(h, h, 2.0f * h * l);
+          F2 h, l;
+          if (VEC || e + 1 < valid) {
+            exact_difference(a2, b2, h, l);
+          } else {
+            exact_difference(f2(e < valid ? a[e] : 0.0f, 0.0f), f2(e < valid ? b[e] : 0.0f, 0.0f), h, l);
+          }
+          t[5].add_product(h, h, (h + h) * l);
         }
       }
       k += valid;
@@ -2337,8 +2422,8 @@ extern "C" {
 int msur_map_sums_of(unsigned which, const float* pred, uint64_t pstride_map, const float* ref, uint64_t rstride_map,
                      uint64_t n, int nmaps, const double* means, double* out, void* stream) {
   if (!pred || !ref || !out || nmaps <= 0 || nmaps > 65535) return fail(MSUR_ERR_INVALID_ARG, "msur_map_sums: bad argument");
-  // blocks of 16384 elements, about eight per SM over all maps
-  const uint64_t steps = (n + 16383) / 16384, most = std::max(1, 8 * 152 / nmaps);
+  // blocks of 32768 elements, about eight per SM over all maps
+  const uint64_t steps = (n + 32767) / 32768, most = std::max(1, 8 * 152 / nmaps);
   const dim3 grid(static_cast<unsigned>(std::min(steps, most)), nmaps);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool vec = n % 4 == 0 && pstride_map % 4 == 0 && rstride_map % 4 == 0 && aligned16(pred) && aligned16(ref);
