@@ -410,8 +410,8 @@ int mgpu_simulate_cells_ex(mgpu_ctx* ctx, int chrom_id, const uint64_t* cell_see
  * chromosome) receives the contacts, added to; missed[chrom_id] is incremented (may be NULL);
  * stats[i] is task i's outcome (may be NULL).  Results equal one mgpu_simulate_cells call per
  * chromosome.  A shared-memory budget set with mgpu_set_debug_flags applies to every cell;
- * without one, large batches use 16 KiB per cell and a 60 % shared-memory carveout, so that
- * nine cells share an SM and keep an 88 KB L1 for their arrays in global slots.
+ * without one, large batches use 16 KiB per cell and a 60 % shared-memory carveout (the cells'
+ * arrays live in global slots under an 88 KB L1).
  */
 typedef struct mgpu_batch_task {
   uint64_t seed;

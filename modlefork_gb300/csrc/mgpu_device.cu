@@ -1,7 +1,7 @@
 // mgpu_device.cu - sm_103a kernels of the loop-extrusion epoch engine.
 //
 // One thread block simulates one cell (Simulation::simulate_one_cell, src/libmodle/cpu/
-// simulation.cpp:1056-1152): 4, 8 or 16 worker warps by the number of LEFs, and one or two producer
+// simulation.cpp:1056-1152): 8 or 16 worker warps by the number of LEFs, and one or two producer
 // warps that generate the cell's random numbers.  The cell's state is structure-of-arrays of
 // 32-bit words; the host plans which per-LEF arrays fit in the cell's shared memory and places
 // the rest in a per-cell global scratch slot (large chromosomes).  The barrier track and its integer
@@ -11,7 +11,10 @@
 // Why a block per cell.  An epoch is about twenty dependent sweeps over the LEFs or barriers.  With one
 // warp per cell a sweep of 2,000 LEFs is 63 dependent rounds of loads, shared memory holds at most a
 // dozen such warps per SM, and an instruction issued on 10 % of cycles.  With 16 warps a sweep is
-// two or four rounds, the arrays stay in shared memory, and a sweep costs about one barrier.
+// two or four rounds, the arrays stay in shared memory, and a sweep costs about one barrier.  152 cells
+// of 73 Mbp (1,460 LEFs) took 843 ms with a warp per cell, 149 now; 24 chromosomes of 40-110 Mbp x 24 cells
+// 1.29 s and 0.29; 2 x 1024 cells of 20 Mbp (an instruction-fetch-bound load: several small blocks per SM
+// in different steps) 1.34 s and 0.56.
 //
 // Draw order.  Every random number of the reference comes from one sequential
 // Xoshiro256++ stream per cell, consumed in a data-dependent order.  The producer warps keep a
@@ -93,7 +96,8 @@ __device__ __forceinline__ u32 warp_excl_scan(u32 v, u32* total) {
 
 // Cell scalars (the same for every thread, kept in shared memory so thread 0's serial code can update
 // them; a value thread 0 writes is read by the others only after a barrier).
-// Per-launch profile counters (cycles per step and fallback counts), summed over cells.
+// Per-launch profile counters (cycles per step and fallback counts), summed over cells.  The two refill
+// counters stay 0: the producer warps refill the ring beside the epoch.
 enum : u32 {
   PF_BURNIN = 0, PF_BIND, PF_RANK, PF_CONTACTS, PF_MOVES, PF_ADJUST, PF_BARRIERS, PF_BOUNDARIES,
   PF_LEF_BAR, PF_PRIMARY, PF_CORRECT, PF_SECONDARY, PF_FIX, PF_EXTRUDE_RELEASE, PF_TRACE, PF_TOTAL,

@@ -1191,9 +1191,9 @@ extern "C" int mgpu_simulate_batch(mgpu_ctx* ctx, const mgpu_batch_task* tasks, 
   }
   int dev_sms = 0;
   cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device);
-  // Large batches: 16 KiB per cell and a 60 % shared-memory carveout, so that nine cells share
-  // an SM and the per-LEF arrays that live in global slots keep an 88 KB L1 (measured best on the
-  // genome workload).
+  // Large batches: 16 KiB per cell and a 60 % shared-memory carveout: the per-LEF arrays live in global slots
+  // under an 88 KB L1, and the registers, not shared memory, bound the cells per SM (the genome
+  // workload: 1.90e9 LEF-epochs/s, 1.81e9 with everything that fits on chip).
   const bool large = ntasks >= 8ull * (uint64_t)dev_sms;
   uint64_t budget = ctx->smem_budget ? ctx->smem_budget : (large ? 16384ull : 0ull);
   // a tuned table (mgpu_set_launch_table) replaces those defaults for large batches without

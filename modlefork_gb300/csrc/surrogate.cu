@@ -9,8 +9,9 @@
 // implicit GEMM:
 //   Y[b, l, n] = sum_t sum_c X[b, l + t - pad, c] * W[n][t][c]      (M = positions, N = Cout,
 //                                                                    K = taps x Cin)
-// TMA loads the A tile of tap t directly from X at row offset t - pad: rows outside [0, L)
-// come back as zeros, which is the convolution's zero padding.  The data gradient is the same
+// TMA loads the A tile of tap t directly from X at row offset t - pad, or one tile with the rows of all taps,
+// into which tap t's operand starts t rows: rows outside [0, L) come back as zeros, which is the
+// convolution's zero padding.  The data gradient is the same
 // product with the taps reversed and W transposed; the weight gradient contracts over the
 // positions (K = B x L) with both operands M/N-major.
 //
@@ -82,7 +83,7 @@ struct ConvArgs {
   bf16* out_post;      // value after the activation, or null
   float* out_f32;      // FP32 value before the activation, or null
   unsigned* err;
-  // staged epilogue (no gate): each epilogue warp writes its 32 rows of a 64-column unit to
+  // staged epilogue: each epilogue warp writes its 32 rows of a 64-column unit to
   // shared memory and stores them with TMA.  Maps over [B][L][n_valid] with row stride
   // out_stride and 128-byte swizzled boxes of 32 rows: FP32 boxes of 32 columns, BF16 of 64.
   CUtensorMap tm_f32, tm_pre, tm_post;
@@ -91,8 +92,8 @@ struct ConvArgs {
   // output row l stored at rows 2l and 2l + 1 of its buffer (two maps over the even and the odd
   // rows); out_post may then be null
   CUtensorMap tm_skip, tm_dup0, tm_dup1;
-  // and an average-pooled copy: rows 2m and 2m + 1 (lanes 2m, 2m + 1 of an epilogue warp) into
-  // row m, as msur_pool2 computes it from the BF16 values (16-row boxes)
+  // and an average-pooled copy: rows 2m and 2m + 1 of a staged box into row m, as msur_pool2 computes it
+  // from the BF16 values (16-row boxes)
   CUtensorMap tm_pool;
   int has_skip, has_dup, has_pool;
 };
@@ -760,11 +761,11 @@ __global__ void __launch_bounds__(PTHREADS, 1)
 //
 // The splits' partial sums meet in dw.  A thread holds one output channel's row of the accumulators;
 // adding it word by word (32 rows per warp and instruction) took longer than the products: 113 of
-// 133 us for 16 x 999 positions, 256 to 256 channels.  So the rows go to the operand stages, free by
-// then (a row is padded by 16 bytes: conflict-free 16-byte stores), and each thread adds its row tap by tap
-// with bulk reductions (cp.reduce.async.bulk, up to 256 contiguous bytes).  Eight warps share the
-// columns and a tap's reductions run while the next is staged: 16 x 2000 positions, 128 to 128
-// channels, took 15.6 us with four warps and the reductions at the end, of which 4.5 and 6.3 were these two.
+// 133 us for 16 x 999 positions, 256 to 256 channels.  So eight warps put half a tap's row per thread into shared
+// memory (rows padded by 16 bytes: conflict-free 16-byte stores), and each thread adds its row with one bulk
+// reduction (cp.reduce.async.bulk, up to 256 contiguous bytes) that runs while the next tap is read, or
+// the next accumulation's products.  16 x 2000 positions, 128 to 128 channels: 15.6 us with four warps and all
+// reductions at the end, of which 4.5 and 6.3 were these two.
 // ---------------------------------------------------------------------------------------
 constexpr int WTHREADS = 320;  // warp 0 TMA, warp 1 MMA and TMEM, warps 2-9 epilogue
 
@@ -775,6 +776,7 @@ struct WgradArgs {
   int lblocks;        // 64-position blocks per sequence
   int total;          // B * lblocks
   int per_split;      // blocks per split
+  int per_phase;      // blocks per accumulation: a split's accumulators are added to dw this often
   int bulk;           // dw is 16-byte aligned: bulk reductions
   float* dw;          // [Cout][taps][Cin], accumulated into
   float* db;          // [Cout], accumulated into, or null
@@ -782,20 +784,18 @@ struct WgradArgs {
   unsigned* err;
 };
 
-// Shared memory of a weight-gradient kernel before its barriers: the operand stages, later the
-// padded accumulator rows.
-template <int BN, int NT>
-__host__ __device__ constexpr int wgrad_row_bytes() {
-  return NT * BN * 4 + 16;
-}
 template <int NT>
 __host__ __device__ constexpr int wgrad_box_bytes() {  // 64 + NT - 1 rows, 1 KB aligned
   return (64 + (NT > 1 ? 8 : 0)) * 128;
 }
-template <int BN, int NT, int STAGES>
-__host__ __device__ constexpr int wgrad_region() {
-  const int stages = STAGES * (2 * 8192 + (BN / 64) * wgrad_box_bytes<NT>()), rows = BM * wgrad_row_bytes<BN, NT>();
-  return stages > rows ? stages : (rows + 1023) / 1024 * 1024;
+template <int BN, int NT>
+__host__ __device__ constexpr int wgrad_stage_bytes() {
+  return 2 * 8192 + (BN / 64) * wgrad_box_bytes<NT>();
+}
+// A thread's staging row: half a tap's columns, padded by 16 bytes.
+template <int BN>
+__host__ __device__ constexpr int wgrad_row_bytes() {
+  return BN / 2 * 4 + 16;
 }
 
 template <int BN, int NT, int STAGES>
@@ -803,16 +803,18 @@ __global__ void __launch_bounds__(WTHREADS, 1) wgrad_kernel(const __grid_constan
   constexpr int BOX = 64 * 64 * 2;  // one 64 x 64 BF16 box
   constexpr int A_BYTES = 2 * BOX;  // 128 output channels
   constexpr int XBOX = wgrad_box_bytes<NT>();
-  constexpr int STAGE_BYTES = A_BYTES + (BN / 64) * XBOX;
+  constexpr int STAGE_BYTES = wgrad_stage_bytes<BN, NT>();
   constexpr uint32_t STAGE_LOAD = A_BYTES + (BN / 64) * (64 + NT - 1) * 128;
   constexpr uint32_t TCOLS = NT * BN <= 128 ? 128 : (NT * BN <= 256 ? 256 : 512);
   static_assert(NT * BN <= 512, "accumulators exceed tensor memory");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + wgrad_region<BN, NT, STAGES>());
+  uint8_t* const staging = smem + STAGES * STAGE_BYTES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(staging + 256 * wgrad_row_bytes<BN>());
   uint64_t* empty = full + STAGES;
   uint64_t* done = empty + STAGES;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  uint64_t* drained = done + 1;  // the accumulators have been read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drained + 1);
   float* bias_part = reinterpret_cast<float*>(full + 32);  // [4 warps][128 channels]
 
   const int warp = umma::warp_index(), lane = threadIdx.x % 32;
@@ -828,6 +830,7 @@ __global__ void __launch_bounds__(WTHREADS, 1) wgrad_kernel(const __grid_constan
       umma::mbar_init(&empty[s], bias ? 5 : 1);  // the products, and the warps that add up dZ
     }
     umma::mbar_init(done, 1);
+    umma::mbar_init(drained, 8);
     umma::fence_barrier_init();
     umma::tma_prefetch(&a.tm_dz);
     umma::tma_prefetch(&a.tm_x);
@@ -863,72 +866,75 @@ __global__ void __launch_bounds__(WTHREADS, 1) wgrad_kernel(const __grid_constan
       umma::mbar_wait_warp(&full[s % STAGES], (s / STAGES) & 1, a.err, ERR_PRODUCER);
   } else if (warp == 1) {
     constexpr uint32_t idesc = umma::idesc_bf16_f32(BM, BN, true, true);
-    int st = 0;
-    uint32_t ph = 0;
+    int st = 0, in = 0;  // stage, blocks in this accumulation
+    uint32_t ph = 0, dph = 0;
     for (int s = 0; s < nk; ++s) {
+      if (in == a.per_phase) {
+        if (umma::elect()) umma::mma_commit(done);
+        if (!umma::mbar_wait_warp(drained, dph, a.err, ERR_MMA)) break;
+        umma::fence_after_sync();
+        dph ^= 1;
+        in = 0;
+      }
       if (!umma::mbar_wait_warp(&full[st], ph, a.err, ERR_MMA)) break;
       const uint32_t sa = umma::smem_u32(smem) + st * STAGE_BYTES;
       const uint32_t a_lo = umma::sdesc_sw128_lo(sa, BOX), b_lo = umma::sdesc_sw128_lo(sa + A_BYTES, XBOX);
       if (umma::elect()) {
 #pragma unroll
-        for (int t = 0; t < NT; ++t) umma::mma_bf16_x4<128>(tmem + t * BN, a_lo, b_lo + 8 * t, idesc, s);
+        for (int t = 0; t < NT; ++t) umma::mma_bf16_x4<128>(tmem + t * BN, a_lo, b_lo + 8 * t, idesc, in);
         umma::mma_commit(&empty[st]);
       }
+      ++in;
       if (++st == STAGES) st = 0, ph ^= 1;
     }
     if (umma::elect()) umma::mma_commit(done);
   } else if (nk > 0) {
+    constexpr int HALF = BN / 2;
     const int q = warp & 3, half = warp >= 6;
-    const int n = n0 + 32 * q + lane;
-    if (bias && !half) {
-      // thread e: 8 channels (16-byte unit e % 16 of the two boxes), rows 8 (e / 16) .. + 7 of each block
-      const int e = threadIdx.x - 64, unit = e & 15;
-      float sum[8] = {};
-      int st = 0;
-      uint32_t ph = 0;
-      for (int s = 0; s < nk; ++s) {
-        if (!umma::mbar_wait_warp(&full[st], ph, a.err, ERR_EPILOGUE)) break;
-        const uint32_t rows = umma::smem_u32(smem) + st * STAGE_BYTES + (unit >> 3) * BOX + (e >> 4) * 1024;
+    const int n = n0 + 32 * q + lane, cc = c0 + half * HALF;
+    const bool inside = n < a.Cout && cc < a.Cin;
+    const uint32_t cols = tmem + (static_cast<uint32_t>(32 * q) << 16) + half * HALF;
+    uint8_t* const row = staging + (threadIdx.x - 64) * wgrad_row_bytes<BN>();
+    // bias: thread e: 8 channels (16-byte unit e % 16 of the two boxes), rows 8 (e / 16) .. + 7 of each block
+    const int e = threadIdx.x - 64, unit = e & 15;
+    float sum[8] = {};
+    int st = 0;
+    uint32_t ph = 0, dph = 0;
+    bool ok = true;
+    for (int s0 = 0; s0 < nk && ok; s0 += a.per_phase, dph ^= 1) {
+      if (bias && !half) {
+        const int s1 = min(nk, s0 + a.per_phase);
+        for (int s = s0; s < s1; ++s) {
+          ok = umma::mbar_wait_warp(&full[st], ph, a.err, ERR_EPILOGUE);
+          if (!ok) break;
+          const uint32_t rows = umma::smem_u32(smem) + st * STAGE_BYTES + (unit >> 3) * BOX + (e >> 4) * 1024;
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-          uint32_t x[4];
-          umma::ld_shared_v4(x, rows + r * 128 + (((unit & 7) ^ r) << 4));
+          for (int r = 0; r < 8; ++r) {
+            uint32_t x[4];
+            umma::ld_shared_v4(x, rows + r * 128 + (((unit & 7) ^ r) << 4));
 #pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[h]));
-            sum[2 * h] += f.x;
-            sum[2 * h + 1] += f.y;
+            for (int h = 0; h < 4; ++h) {
+              const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x[h]));
+              sum[2 * h] += f.x;
+              sum[2 * h + 1] += f.y;
+            }
           }
+          // The next copy may write here once the loads have returned, not once they are issued: the products
+          // take most of the shared memory's cycles, and loads were seen to lose rows to the copy six
+          // blocks on.  So the arrival's address depends on what was loaded (by an AND with a zero
+          // that only the launch knows).
+          const float all = ((sum[0] + sum[1]) + (sum[2] + sum[3])) + ((sum[4] + sum[5]) + (sum[6] + sum[7]));
+          __syncwarp();
+          if (lane == 0) umma::mbar_arrive(umma::smem_u32(&empty[st]) + (__float_as_uint(all) & a.zero));
+          if (++st == STAGES) st = 0, ph ^= 1;
         }
-        // The next copy may write here once the loads have returned, not once they are issued: the products
-        // take most of the shared memory's cycles, and loads were seen to lose rows to the copy six
-        // blocks on.  So the arrival's address depends on what was loaded (by an AND with a zero
-        // that only the launch knows).
-        const float all = ((sum[0] + sum[1]) + (sum[2] + sum[3])) + ((sum[4] + sum[5]) + (sum[6] + sum[7]));
-        __syncwarp();
-        if (lane == 0) umma::mbar_arrive(umma::smem_u32(&empty[st]) + (__float_as_uint(all) & a.zero));
-        if (++st == STAGES) st = 0, ph ^= 1;
+        if (!ok) break;
       }
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        sum[k] += __shfl_xor_sync(0xFFFFFFFFu, sum[k], 16);
-        if (lane < 16) bias_part[(e >> 5) * 128 + 8 * unit + k] = sum[k];
-      }
-      asm volatile("bar.sync 2, 128;" ::: "memory");  // the four warps that add up
-      if (n0 + e < a.Cout)
-        atomicAdd(a.db + n0 + e, (bias_part[e] + bias_part[128 + e]) + (bias_part[256 + e] + bias_part[384 + e]));
-    }
-    const bool ok = umma::mbar_wait_warp(done, 0, a.err, ERR_EPILOGUE);
-    umma::fence_after_sync();
-    if (bias) asm volatile("bar.sync 1, 256;" ::: "memory");  // the stages have been added up: rows may go there
-    if (ok) {
+      ok = umma::mbar_wait_warp(done, dph, a.err, ERR_EPILOGUE);
+      if (!ok) break;
+      umma::fence_after_sync();
       // tap by tap: this half's columns of the thread's row to shared memory, and on to dw while the next tap's
       // are read
-      constexpr int HALF = BN / 2;
-      const int cc = c0 + half * HALF;
-      const bool inside = n < a.Cout && cc < a.Cin;
-      const uint32_t cols = tmem + (static_cast<uint32_t>(32 * q) << 16) + half * HALF;
-      uint8_t* const row = smem + (32 * q + lane) * wgrad_row_bytes<BN, NT>() + half * HALF * 4;
 #pragma unroll 1
       for (int t = 0; t < NT; ++t) {
         float v[HALF];
@@ -937,10 +943,16 @@ __global__ void __launch_bounds__(WTHREADS, 1) wgrad_kernel(const __grid_constan
         } else {
           umma::tmem_ld32(cols + t * BN, v);
         }
+        if (t == NT - 1) {
+          umma::fence_before_sync();
+          __syncwarp();
+          if (lane == 0) umma::mbar_arrive(drained);
+        }
         if (!inside) continue;
         float* dst = a.dw + (static_cast<size_t>(n) * a.taps + t) * a.Cin + cc;
         if (a.bulk) {
-          float4* to = reinterpret_cast<float4*>(row + t * BN * 4);
+          umma::bulk_wait_read<0>();  // the row's previous reduction has read it
+          float4* to = reinterpret_cast<float4*>(row);
 #pragma unroll
           for (int k = 0; k < HALF / 4; ++k) to[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
           umma::fence_async_smem();  // this thread's values, read by its own reduction
@@ -953,9 +965,19 @@ __global__ void __launch_bounds__(WTHREADS, 1) wgrad_kernel(const __grid_constan
             if (j < nv) atomicAdd(dst + j, v[j]);
         }
       }
-      umma::bulk_wait_all();
-      __syncwarp();
     }
+    if (bias && !half) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        sum[k] += __shfl_xor_sync(0xFFFFFFFFu, sum[k], 16);
+        if (lane < 16) bias_part[(e >> 5) * 128 + 8 * unit + k] = sum[k];
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");  // the four warps that add up
+      if (ok && n0 + e < a.Cout)
+        atomicAdd(a.db + n0 + e, (bias_part[e] + bias_part[128 + e]) + (bias_part[256 + e] + bias_part[384 + e]));
+    }
+    umma::bulk_wait_all();
+    __syncwarp();
   }
   umma::fence_before_sync();
   __syncthreads();
@@ -1196,34 +1218,51 @@ __device__ __forceinline__ F2 operator-(F2 a) {
   a.v ^= 0x8000000080000000ull;
   return a;
 }
-// Two running sums as pairs of floats, side by side.
+// Two running sums side by side, each as a sum h, the rounding errors l of its additions and the products' low parts,
+// and l's own rounding errors m: without m the sums of squares of a map of 2.4 M values were 1e-15 to
+// 2e-15 off, FP64 sums 1e-16 to 1e-15.
 struct PairSum2 {
-  F2 h, l;
-  __device__ __forceinline__ void add(F2 x) {
-    const F2 t = h + x, z = t - h;
-    l = l + ((h - (t - z)) + (x - z));
+  F2 h, l, m;
+  __device__ __forceinline__ F2 high(F2 x) {
+    const F2 t = h + x, z = t - h, e = (h - (t - z)) + (x - z);
     h = t;
+    return e;
   }
+  __device__ __forceinline__ void low(F2 x) {
+    const F2 t = l + x, z = t - l;
+    m = m + ((l - (t - z)) + (x - z));
+    l = t;
+  }
+  __device__ __forceinline__ void add(F2 x) { l = l + high(x); }
   __device__ __forceinline__ void add(F2 x, F2 rest) {
-    add(x);
-    l = l + rest;
-  }
-  // a * b + rest, rest far smaller
-  __device__ __forceinline__ void add_product(F2 a, F2 b, F2 rest) {
-    const F2 p = a * b;
-    add(p, f2_fma(a, b, -p) + rest);
+    l = l + high(x);
+    m = m + rest;
   }
   __device__ __forceinline__ void add_product(F2 a, F2 b) {
     const F2 p = a * b;
-    add(p, f2_fma(a, b, -p));
+    low(high(p));
+    low(f2_fma(a, b, -p));
+  }
+  // (a + al)^2 and (a + al) (b + bl)
+  __device__ __forceinline__ void add_square(F2 a, F2 al) {
+    const F2 p = a * a;
+    low(high(p));
+    low(f2_fma(a + a + al, al, f2_fma(a, a, -p)));
+  }
+  __device__ __forceinline__ void add_product(F2 a, F2 al, F2 b, F2 bl) {
+    const F2 p = a * b;
+    low(high(p));
+    low(f2_fma(al, b + bl, f2_fma(a, bl, f2_fma(a, b, -p))));
   }
   __device__ __forceinline__ double value() const {
-    float x, y, u, w;
+    float x, y, u, w, c, d;
     f2_get(h, x, y);
     f2_get(l, u, w);
+    f2_get(m, c, d);
     const float t = __fadd_rn(x, y), z = __fsub_rn(t, x);
-    const float e = __fadd_rn(__fsub_rn(x, __fsub_rn(t, z)), __fsub_rn(y, z));
-    return static_cast<double>(t) + static_cast<double>(__fadd_rn(__fadd_rn(u, w), e));
+    const float r = __fadd_rn(__fsub_rn(x, __fsub_rn(t, z)), __fsub_rn(y, z));
+    return static_cast<double>(t) + ((static_cast<double>(u) + static_cast<double>(w)) +
+                                     (static_cast<double>(r) + static_cast<double>(__fadd_rn(c, d))));
   }
 };
 __device__ __forceinline__ void exact_difference(F2 a, F2 b, F2& h, F2& l) {
@@ -1522,12 +1561,13 @@ __global__ void band_target_kernel(const uint32_t* band, size_t ncols, int nrows
 // elements in two pairs of floats: differences, products and sums with their exact rounding errors (Knuth's
 // two-sum, two-product by FMA), and adds each chunk's pair to FP64 totals.  The means are split into a float
 // m and a remainder d: the deviations from m are exact pairs, and d enters the FP64 totals,
-// sum (a - d)^2 = sum a^2 - 2 d sum a + n d^2.  A pair carries 2^-47 per operation and the chunks' errors
-// average out over the map; measured against 64-bit sums the scores are as close as before (a few 1e-16).
+// sum (a - d)^2 = sum a^2 - 2 d sum a + n d^2.  Low parts are summed with
+// their own rounding errors; measured against exact sums the scores are as close as FP64's (6e-16, 4e-16).
 // A chunk with values outside [2^-30, 2^50) in size throughout, infinities or NaN is summed in FP64.
 // WHICH: the sums wanted (bit k: sum k); MEANS: deviations from the means, raw values otherwise.
-// The pairs come two to a packed operation (PairSum2), and two loads of each side run ahead: both passes over
-// those maps took 406 us without, 356 with (more loads ahead, or three blocks per SM, spill).
+// The sums come two to a packed operation (PairSum2), and two loads of each side run ahead (more, or three blocks
+// per SM, spill): 0.61 ms for the scores of those maps, 3.4 in FP64.  With single low parts it took 0.47, but was
+// up to 9e-15 off where FP64 is 4e-16.
 constexpr int SUM_VECS = 32;  // float4 per thread and chunk
 template <bool VEC, bool MEANS, unsigned WHICH>
 __global__ void __launch_bounds__(256, 2) map_sums_pair_kernel(const float* pred, size_t pstride_map, const float* ref,
@@ -1595,9 +1635,9 @@ __global__ void __launch_bounds__(256, 2) map_sums_pair_kernel(const float* pred
           exact_difference(b2, fr2, bh, bl);
           if constexpr (WHICH & 1) t[0].add(ah, al);
           if constexpr (WHICH & 2) t[1].add(bh, bl);
-          if constexpr (WHICH & 4) t[2].add_product(ah, ah, (ah + ah) * al);
-          if constexpr (WHICH & 8) t[3].add_product(bh, bh, (bh + bh) * bl);
-          if constexpr (WHICH & 16) t[4].add_product(ah, bh, f2_fma(ah, bl, al * bh));
+          if constexpr (WHICH & 4) t[2].add_square(ah, al);
+          if constexpr (WHICH & 8) t[3].add_square(bh, bl);
+          if constexpr (WHICH & 16) t[4].add_product(ah, al, bh, bl);
         } else {
           if constexpr (WHICH & 1) t[0].add(a2);
           if constexpr (WHICH & 2) t[1].add(b2);
@@ -1612,7 +1652,7 @@ __global__ void __launch_bounds__(256, 2) map_sums_pair_kernel(const float* pred
           } else {
             exact_difference(f2(e < valid ? a[e] : 0.0f, 0.0f), f2(e < valid ? b[e] : 0.0f, 0.0f), h, l);
           }
-          t[5].add_product(h, h, (h + h) * l);
+          t[5].add_square(h, l);
         }
       }
       k += valid;
@@ -1947,7 +1987,7 @@ int dispatch_conv(const ConvArgs& a, int ntn, bool staged, int stages, cudaStrea
 
 template <int BN, int NT, int STAGES>
 int launch_wgrad(const WgradArgs& a, int splits, cudaStream_t st) {
-  constexpr int smem = wgrad_region<BN, NT, STAGES>() + 1024 + 256 + 2048;  // alignment, barriers, bias sums
+  constexpr int smem = STAGES * wgrad_stage_bytes<BN, NT>() + 256 * wgrad_row_bytes<BN>() + 1024 + 256 + 2048;  // alignment, barriers, bias sums
   auto kern = wgrad_kernel<BN, NT, STAGES>;
   static KernelLimits limits;
   const int rc = limits.get(reinterpret_cast<const void*>(kern), smem);
@@ -2160,8 +2200,9 @@ static int conv_wgrad_impl(const void* x, const void* dz, int B, int L, int Cin,
   a.pad = (taps - 1) / 2;
   a.lblocks = (L + 63) / 64;
   a.total = B * a.lblocks;
-  if (splits <= 0) {
-    // one CTA per SM and one wave: a second wave would add every accumulator to dw a second time
+  const bool automatic = splits <= 0;
+  if (automatic) {
+    // one CTA per SM and one wave
     const int bn = taps == 3 && Cin <= 64 ? 64 : 128;
     const int tiles = ((Cin + bn - 1) / bn) * ((Cout + BM - 1) / BM);
     splits = std::max(1, 152 / tiles);
@@ -2169,6 +2210,15 @@ static int conv_wgrad_impl(const void* x, const void* dz, int B, int L, int Cin,
   if (splits > a.total) splits = a.total;
   a.per_split = (a.total + splits - 1) / splits;
   splits = (a.total + a.per_split - 1) / a.per_split;
+  a.per_phase = a.per_split;
+  if (automatic) {
+    // The tensor core's sums lose accuracy with their length, so an accumulation takes no more blocks than with
+    // two waves of 128-wide tiles: 64 x 1000 positions, 256 to 256 channels, 9e-7 of the gradient's norm,
+    // 1.8e-6 with a split's blocks in one.
+    const int tiles = ((Cin + 127) / 128) * ((Cout + BM - 1) / BM);
+    const int chains = std::min(a.total, (2 * 152 + tiles - 1) / tiles);
+    a.per_phase = std::min(a.per_split, (a.total + chains - 1) / chains);
+  }
   a.dw = dw;
   a.db = db;
   a.bulk = aligned16(dw) ? 1 : 0;
@@ -2176,9 +2226,9 @@ static int conv_wgrad_impl(const void* x, const void* dz, int B, int L, int Cin,
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (taps == 3) {
     if (Cin <= 64) return launch_wgrad<64, 3, 6>(a, splits, st);
-    return launch_wgrad<128, 3, 6>(a, splits, st);
+    return launch_wgrad<128, 3, 4>(a, splits, st);
   }
-  return launch_wgrad<128, 1, 6>(a, splits, st);
+  return launch_wgrad<128, 1, 4>(a, splits, st);
 }
 
 int msur_conv_wgrad(const void* x, const void* dz, int B, int L, int Cin, int Cout, int taps, float* dw, int splits,

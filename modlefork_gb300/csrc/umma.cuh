@@ -11,6 +11,8 @@
 //  * MN-major operand (M or N contiguous): TMA boxes of 64 MN elements x 64 K rows (8 KB), one
 //    per 64 MN elements; leading byte offset = the distance between those boxes, stride byte
 //    offset = 1024 B (8 K rows); a K step of 16 rows advances the start address by 2048 B.
+//  * the swizzle follows the address bits, so an operand may start any number of whole rows (128 B) into such a
+//    tile: the taps of a convolution read one tile of positions that way.
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -78,22 +80,9 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Wait for the phase of the given parity; gives up after `limit_ns` of wall time, records
-// `code` in *err and returns false (the caller then abandons its work and drains).
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, unsigned* err, unsigned code,
-                                          uint64_t limit_ns = 1000000000ull) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = global_ns();
-  while (!mbar_try_wait(bar, parity)) {
-    if (global_ns() - t0 > limit_ns) {
-      if (err) atomicOr(err, code);
-      return false;
-    }
-  }
-  return true;
-}
-
-// The same for a whole converged warp: control flow that depends on the result stays warp-uniform.
+// A whole converged warp waits for the phase of the given parity (control flow that depends on the result stays
+// warp-uniform); gives up after `limit_ns` of wall time, records `code` in *err and returns false (the caller
+// then abandons its work and drains).
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, unsigned* err, unsigned code,
                                                uint64_t limit_ns = 1000000000ull) {
   if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
@@ -209,25 +198,9 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(uint32_t m, uint32_t n, bo
          | ((m >> 4) << 24);                // M / 16
 }
 
-// Shared-memory matrix descriptor with 128-byte swizzling.
-__device__ __forceinline__ uint64_t sdesc_sw128(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  return static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4) | (static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16) |
-         (static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFFu) << 32) | (1ull << 46)  // descriptor version
-         | (2ull << 61);                                                           // SWIZZLE_128B
-}
-
-// D (TMEM) [+]= A (smem) x B (smem), issued by one thread.
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                         uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Four products of 16 along K from 128-byte swizzled operands whose descriptors (sdesc_sw128 split into the word
-// that changes and the one that does not) advance by STEP 16-byte units: 2 for a K-major step of 64 elements,
+// Four products of 16 along K, D (TMEM) [+]= A (smem) x B (smem), issued by one thread, from 128-byte swizzled operands
+// whose shared-memory descriptors (the word that changes and the one that does not: 1024 bytes between
+// groups of eight rows, descriptor version 1, 128-byte swizzle) advance by STEP 16-byte units: 2 for a K-major step of 64 elements,
 // 128 for an MN-major one of 64 rows.
 constexpr uint32_t SDESC_SW128_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t sdesc_sw128_lo(uint32_t saddr, uint32_t lbo_bytes = 16) {

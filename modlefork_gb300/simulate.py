@@ -54,7 +54,7 @@ def prepare_chrom(eng, cfg, chrom, barriers, ncells):
 
 # Shared-memory budget per cell when several chromosome launches run at once, and the share of
 # the SM's unified memory given to shared memory (the rest is L1 for the per-LEF arrays that
-# live in global slots): six cells per SM with a 70 KB L1 measured best on the genome workload.
+# live in global slots).
 CONCURRENT_SMEM_BUDGET = 24 * 1024
 CONCURRENT_CARVEOUT = 70
 
