@@ -198,7 +198,7 @@ def run_windows(args, device, log):
             "parity_sample": {"cells": compared, "equal": equal,
                               "against": "plain per-window launches on engines with each window's configuration"},
             "note": "the first windows of the seeded 4096-window workload (a stated subset); the whole "
-                    "workload is about 2e12 LEF-epochs.  One warp advances one cell, so the launch's tail "
+                    "workload is about 2e12 LEF-epochs.  One thread block advances one cell, so the launch's tail "
                     "is the longest cell: the fourth window (170 Mbp at 1 kb bins, 6450 LEFs, about 1e4 epochs per "
                     "cell) sets this subset's time"}
 
