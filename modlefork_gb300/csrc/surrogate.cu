@@ -205,6 +205,7 @@ __device__ __forceinline__ void stage_end(const CUtensorMap* map, uint8_t* buf, 
     umma::tma_store_3d(map, buf, x, y, z);
     umma::bulk_commit();
   }
+  __syncwarp();  // a tcgen05.ld may follow, which wants the warp converged
   ++nb;
 }
 
@@ -318,6 +319,7 @@ __device__ __forceinline__ void conv_epilogue_unit(const ConvArgs& a, uint32_t t
       }
       umma::bulk_commit();
     }
+    __syncwarp();
     ++nb;
     if (out == 1 && a.has_pool) {
       // rows 2m and 2m + 1 of the staged box are averaged into row m of a 16-row box (y is a multiple of 32):
@@ -420,6 +422,7 @@ __global__ void __launch_bounds__(THREADS, 1) conv_fwd_kernel(const __grid_const
       }
     }
     if (umma::elect()) umma::mma_commit(done);
+    __syncwarp();
   } else {
     // epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31, one output row per thread
     const int q = warp & 3;
@@ -443,8 +446,8 @@ __global__ void __launch_bounds__(THREADS, 1) conv_fwd_kernel(const __grid_const
         float v[32];
         umma::tmem_ld32(tmem + (static_cast<uint32_t>(32 * q) << 16) + c * 32, v);
         const int col0 = n0 + c * 32;
-        if (!row_ok || col0 >= a.n_valid) continue;
-        conv_epilogue_chunk(a, v, row, col0);
+        if (row_ok && col0 < a.n_valid) conv_epilogue_chunk(a, v, row, col0);
+        __syncwarp();  // tcgen05.ld is .sync.aligned: the rows past the end rejoin before the next one
       }
     }
   }
@@ -888,6 +891,7 @@ __global__ void __launch_bounds__(WTHREADS, 1) wgrad_kernel(const __grid_constan
       if (++st == STAGES) st = 0, ph ^= 1;
     }
     if (umma::elect()) umma::mma_commit(done);
+    __syncwarp();
   } else if (nk > 0) {
     constexpr int HALF = BN / 2;
     const int q = warp & 3, half = warp >= 6;
@@ -948,22 +952,24 @@ __global__ void __launch_bounds__(WTHREADS, 1) wgrad_kernel(const __grid_constan
           __syncwarp();
           if (lane == 0) umma::mbar_arrive(drained);
         }
-        if (!inside) continue;
-        float* dst = a.dw + (static_cast<size_t>(n) * a.taps + t) * a.Cin + cc;
-        if (a.bulk) {
-          umma::bulk_wait_read<0>();  // the row's previous reduction has read it
-          float4* to = reinterpret_cast<float4*>(row);
+        if (inside) {
+          float* dst = a.dw + (static_cast<size_t>(n) * a.taps + t) * a.Cin + cc;
+          if (a.bulk) {
+            umma::bulk_wait_read<0>();  // the row's previous reduction has read it
+            float4* to = reinterpret_cast<float4*>(row);
 #pragma unroll
-          for (int k = 0; k < HALF / 4; ++k) to[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-          umma::fence_async_smem();  // this thread's values, read by its own reduction
-          umma::bulk_reduce_add_f32(dst, to, 4 * min(HALF, a.Cin - cc));
-          umma::bulk_commit();
-        } else {
-          const int nv = min(HALF, a.Cin - cc);
+            for (int k = 0; k < HALF / 4; ++k) to[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+            umma::fence_async_smem();  // this thread's values, read by its own reduction
+            umma::bulk_reduce_add_f32(dst, to, 4 * min(HALF, a.Cin - cc));
+            umma::bulk_commit();
+          } else {
+            const int nv = min(HALF, a.Cin - cc);
 #pragma unroll
-          for (int j = 0; j < HALF; ++j)
-            if (j < nv) atomicAdd(dst + j, v[j]);
+            for (int j = 0; j < HALF; ++j)
+              if (j < nv) atomicAdd(dst + j, v[j]);
+          }
         }
+        __syncwarp();  // channels past Cout rejoin: the next tcgen05.ld is .sync.aligned
       }
     }
     if (bias && !half) {
@@ -972,6 +978,7 @@ __global__ void __launch_bounds__(WTHREADS, 1) wgrad_kernel(const __grid_constan
         sum[k] += __shfl_xor_sync(0xFFFFFFFFu, sum[k], 16);
         if (lane < 16) bias_part[(e >> 5) * 128 + 8 * unit + k] = sum[k];
       }
+      __syncwarp();
       asm volatile("bar.sync 1, 128;" ::: "memory");  // the four warps that add up
       if (ok && n0 + e < a.Cout)
         atomicAdd(a.db + n0 + e, (bias_part[e] + bias_part[128 + e]) + (bias_part[256 + e] + bias_part[384 + e]));
