@@ -783,7 +783,6 @@ struct WgradArgs {
   int bulk;           // dw is 16-byte aligned: bulk reductions
   float* dw;          // [Cout][taps][Cin], accumulated into
   float* db;          // [Cout], accumulated into, or null
-  uint32_t zero;
   unsigned* err;
 };
 
@@ -923,13 +922,12 @@ __global__ void __launch_bounds__(WTHREADS, 1) wgrad_kernel(const __grid_constan
               sum[2 * h + 1] += f.y;
             }
           }
-          // The next copy may write here once the loads have returned, not once they are issued: the products
-          // take most of the shared memory's cycles, and loads were seen to lose rows to the copy six
-          // blocks on.  So the arrival's address depends on what was loaded (by an AND with a zero
-          // that only the launch knows).
-          const float all = ((sum[0] + sum[1]) + (sum[2] + sum[3])) + ((sum[4] + sum[5]) + (sum[6] + sum[7]));
+          // Reads through the generic proxy before a write through the async one: an arrival alone does not
+          // order them, and rows were seen to be lost to the copy that fills this stage next.  Every lane
+          // fences its own loads, then one arrives for the warp.
+          umma::fence_async_smem();
           __syncwarp();
-          if (lane == 0) umma::mbar_arrive(umma::smem_u32(&empty[st]) + (__float_as_uint(all) & a.zero));
+          if (lane == 0) umma::mbar_arrive(&empty[st]);
           if (++st == STAGES) st = 0, ph ^= 1;
         }
         if (!ok) break;

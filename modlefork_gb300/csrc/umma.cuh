@@ -160,7 +160,8 @@ __device__ __forceinline__ void fence_after_sync() {
 }
 
 // ---- TMA stores ---------------------------------------------------------------------------
-// Make this thread's shared-memory writes visible to the bulk-copy (async) proxy.
+// Order this thread's earlier shared-memory accesses before later ones of the bulk-copy (async) proxy: its writes
+// become visible to a copy out, its reads are done before a copy in.
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // Store one box from shared memory to global memory (rows and columns outside the tensor are
 // dropped); joins this thread's current bulk group.

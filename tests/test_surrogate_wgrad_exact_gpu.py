@@ -63,3 +63,19 @@ def test_unstaged_epilogue_at_ragged_lengths(L, form):
     want = sum(xp[:, t:t + L] @ w[:, t].double().T for t in range(3))
     assert torch.equal(out.double(), want)
     assert ops.take_error() == 0
+
+
+# the bias gradient's warps read the stages of a long ring while copies refill it: many blocks per split at full-rate
+# copies, the head's five output tiles, one tap and three, ragged channels, lengths that end inside a block
+@pytest.mark.parametrize("B,L,cin,cout,taps", [(64, 1000, 256, 256, 3), (32, 4000, 64, 640, 1), (64, 4000, 64, 64, 3),
+                                               (32, 2000, 384, 128, 3), (16, 999, 72, 136, 3), (256, 125, 512, 512, 3),
+                                               (300, 65, 8, 8, 1)])
+def test_bias_gradient_of_the_weight_gradient(B, L, cin, cout, taps):
+    x, dz = _inputs(B, L, cin, cout, L + cout)
+    want, wantb = _want(x, dz, taps)
+    for k in range(20):
+        dw, db = torch.zeros(cout, taps, cin, device=DEV), torch.ones(cout, device=DEV)
+        ops.run((ops.Op * 1)(ops.op(ops.OP_WGRAD, (x, dz, dw, db), (B, L, cin, cout, taps, 0))))
+        assert torch.equal(db.double() - 1, wantb), k
+        assert torch.equal(dw.double(), want), k
+    assert ops.take_error() == 0
