@@ -1,7 +1,7 @@
 // mgpu_device.cu - sm_103a kernels of the loop-extrusion epoch engine.
 //
 // One thread block simulates one cell (Simulation::simulate_one_cell, src/libmodle/cpu/
-// simulation.cpp:1056-1152): 8 or 16 worker warps by the number of LEFs, and one or two producer
+// simulation.cpp:1056-1152): 1 to 16 worker warps by the number of LEFs, and one or two producer
 // warps that generate the cell's random numbers.  The cell's state is structure-of-arrays of
 // 32-bit words; the host plans which per-LEF arrays fit in the cell's shared memory and places
 // the rest in a per-cell global scratch slot (large chromosomes).  The barrier track and its integer
@@ -1915,7 +1915,9 @@ __device__ __noinline__ u32 rank_dir_block(u32 dir, u32 n, u32 epoch, bool exact
   const u32 nt = g_bt.ntie;
   if (m > maxb) return RANK_MANY;
   if (nt > MAX_TIES) return RANK_TIE;
-  if (threadIdx.x < nt && !tie_keeps_order(kmask, nch, g_bt.tierank[threadIdx.x])) g_bt.tie2 = 1;
+#pragma unroll 1
+  for (u32 q = threadIdx.x; q < nt; q += T)
+    if (!tie_keeps_order(kmask, nch, g_bt.tierank[q])) g_bt.tie2 = 1;
   // 3: runs of 32
   if (w == W - 1) {  // removed units before each warp's range
     u32 v = lane < W ? g_bt.rem[lane] : 0u;
@@ -3261,6 +3263,11 @@ __device__ __noinline__ double ordered_sum(u32 n) {
   const u64 MANT = 0xFFFFFFFFFFFFFull, TOP = 1ull << 53;
   double s = 0.0;
   u32 i = 0;
+  if (n <= 64) {  // the first terms leave a binade each, so a short sum is cheaper as it stands (20 LEFs: 2,700 cycles)
+#pragma unroll 1
+    for (; i < n; ++i) s = s + __longlong_as_double((i64)t.at64(i));
+    return s;
+  }
 #pragma unroll 1
   while (i < n) {
     u64 sb = (u64)__double_as_longlong(s);

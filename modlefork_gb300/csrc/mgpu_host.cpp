@@ -772,8 +772,13 @@ static MoveSpec move_spec(double mean, double sd) {
   return m;
 }
 
-// Worker warps of a cell: a sweep over its LEFs takes two to four rounds of the block.
-static u32 workers_for(uint64_t nlefs) { return nlefs <= 256 ? 8 : 16; }
+// Worker warps of a cell: a thread per LEF up to 256 LEFs, 512 threads above.  Below 129 LEFs more warps only make
+// the block barriers dearer and leave fewer cells per SM: 4096 cells of 20 LEFs took 348 ms with eight warps, 306
+// with one (313 with a warp per cell and no barriers); 60 LEFs 373 and 354 with two (417); 100 LEFs 395 and
+// 379 with four (568).  With more LEFs eight pay: 4096 cells of 200 LEFs 504 ms with four, 464 with eight.
+static u32 workers_for(uint64_t nlefs) {
+  return nlefs <= 32 ? 1 : (nlefs <= 64 ? 2 : (nlefs <= 128 ? 4 : (nlefs <= 256 ? 8 : 16)));
+}
 
 static int make_kparams(const mgpu_ctx* ctx, const ChromEntry& ch, uint64_t nlefs, KParams* P,
                         uint64_t budget_override = 0, u32 workers = 0) {
@@ -1221,7 +1226,8 @@ extern "C" int mgpu_simulate_batch(mgpu_ctx* ctx, const mgpu_batch_task* tasks, 
     }
     budget = tuned->smem_budget;
   }
-  // one block size for the launch: the LEF-weighted median cell's
+  // one block size for the launch: the LEF-weighted median cell's, but below eight warps only what the largest cell
+  // would get (a large cell among many small ones is the launch's tail)
   u32 workers = 0;
   {
     std::vector<uint64_t> nl(ntasks);
@@ -1235,6 +1241,7 @@ extern "C" int mgpu_simulate_batch(mgpu_ctx* ctx, const mgpu_batch_task* tasks, 
         break;
       }
     }
+    if (workers < 8) workers = std::min<u32>(8, workers_for(nl.back()));
   }
   std::vector<BatchPlan> plans(keys.size());
   u32 smem_bytes = 0;
@@ -1291,7 +1298,8 @@ extern "C" int mgpu_simulate_batch(mgpu_ctx* ctx, const mgpu_batch_task* tasks, 
   // tuning switches (mgpu_set_debug_flags bits 8-15: carveout percent, 16-23: blocks per SM cap)
   u32 carveout = (ctx->debug_flags >> 8) & 0xFFu;
   u32 max_per_sm = (ctx->debug_flags >> 16) & 0xFFu;
-  if (!carveout && large && !ctx->smem_budget) carveout = 60;
+  // (blocks of fewer than eight workers: shared memory bounds the cells per SM, and little lies in global slots)
+  if (!carveout && large && !ctx->smem_budget) carveout = workers < 8 ? 100 : 60;
   if (tuned) {
     carveout = tuned->carveout_pct;
     max_per_sm = tuned->max_cells_per_sm;

@@ -21,7 +21,7 @@ typedef int32_t i32;
 // Unbound unit / LEF sentinel for the 32-bit device encodings.
 constexpr u32 UNBOUND = 0xFFFFFFFFu;
 
-// A cell's thread block: 8 or 16 worker warps (the plan's choice) and one producer warp per 256
+// A cell's thread block: 1, 2, 4, 8 or 16 worker warps (the plan's choice) and one producer warp per 256
 // worker threads.  Each producer lane generates RNG_S consecutive draws of the cell's single
 // Xoshiro256++ stream per refill; the ring holds two refills.  A refill is at least four draws per
 // worker thread: a step consumes up to two per thread and window and gives them back one window later.
