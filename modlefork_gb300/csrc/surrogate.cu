@@ -1174,24 +1174,6 @@ __global__ void bias_grad_kernel(const bf16* dz, size_t rows, int C, int stride,
   }
 }
 
-// A running sum as a pair of floats (see map_sums_pair_kernel).
-struct PairSum {
-  float h = 0.0f, l = 0.0f;
-  __device__ __forceinline__ void add(float x) {
-    const float t = __fadd_rn(h, x), z = __fsub_rn(t, h);
-    l = __fadd_rn(l, __fadd_rn(__fsub_rn(h, __fsub_rn(t, z)), __fsub_rn(x, z)));
-    h = t;
-  }
-  // a * b + rest, rest far smaller
-  __device__ __forceinline__ void add_product(float a, float b, float rest) {
-    const float p = __fmul_rn(a, b);
-    const float e = __fmaf_rn(a, b, -p);
-    add(p);
-    l = __fadd_rn(l, __fadd_rn(e, rest));
-  }
-  __device__ __forceinline__ double value() const { return static_cast<double>(h) + static_cast<double>(l); }
-};
-
 // Two floats in a register pair and the packed operations on them: each half rounds as the scalar operation does,
 // at half the instructions.
 struct F2 {
@@ -1343,8 +1325,10 @@ __global__ void mse_kernel(const float* pred, int pstride, const float* target, 
   }
 }
 
-// Four channels per thread (counts and strides multiples of 4, aligned buffers), the squares summed in pairs of
-// floats (PairSum) per 64 values and then in FP64.  I: 32-bit indexes where they reach.
+// Four channels per thread (counts and strides multiples of 4, aligned buffers), the squares summed as floats with
+// their errors (PairSum2) per 64 values and then in FP64.  Sums of 64 squares are 5e-17 off (a loop in FP64
+// 3e-16); a single low part, without the errors of its own sums, left 1.4e-14, of which 1.2e-15 had one
+// sign and stayed in the total.  I: 32-bit indexes where they reach.
 template <typename I>
 __global__ void __launch_bounds__(256) mse_v4_kernel(const float* __restrict__ pred, int pstride,
                                                      const float* __restrict__ target, int tstride, size_t rows,
@@ -1356,7 +1340,7 @@ __global__ void __launch_bounds__(256) mse_v4_kernel(const float* __restrict__ p
   double acc = 0.0;
   I i = blockIdx.x * static_cast<I>(blockDim.x) + threadIdx.x;
   while (i < n) {
-    PairSum t;
+    PairSum2 t;
     uint32_t mx = 0;
     const I first = i;
     for (int k = 0; k < 16 && i < n; ++k, i += step) {
@@ -1369,9 +1353,11 @@ __global__ void __launch_bounds__(256) mse_v4_kernel(const float* __restrict__ p
         const float4 b = __ldg(reinterpret_cast<const float4*>(target + r * tstride + c));
         d[0] = a.x - b.x, d[1] = a.y - b.y, d[2] = a.z - b.z, d[3] = a.w - b.w;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          mx = max(mx, __float_as_uint(fabsf(d[e])));
-          t.add_product(d[e], d[e], 0.0f);
+        for (int e = 0; e < 4; ++e) mx = max(mx, __float_as_uint(fabsf(d[e])));
+#pragma unroll
+        for (int e = 0; e < 4; e += 2) {
+          const F2 d2 = f2(d[e], d[e + 1]);
+          t.add_product(d2, d2);
         }
       }
       if (dp)
