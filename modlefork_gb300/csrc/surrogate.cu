@@ -1230,16 +1230,19 @@ struct PairSum2 {
     low(high(p));
     low(f2_fma(a, b, -p));
   }
-  // (a + al)^2 and (a + al) (b + bl)
+  // (a + al)^2 and (a + al) (b + bl).  The products of the low parts are below half a unit of everything in l and
+  // would round away there, al^2 always downwards: they go to m.
   __device__ __forceinline__ void add_square(F2 a, F2 al) {
     const F2 p = a * a;
     low(high(p));
-    low(f2_fma(a + a + al, al, f2_fma(a, a, -p)));
+    low(f2_fma(a + a, al, f2_fma(a, a, -p)));
+    m = f2_fma(al, al, m);
   }
   __device__ __forceinline__ void add_product(F2 a, F2 al, F2 b, F2 bl) {
     const F2 p = a * b;
     low(high(p));
-    low(f2_fma(al, b + bl, f2_fma(a, bl, f2_fma(a, b, -p))));
+    low(f2_fma(al, b, f2_fma(a, bl, f2_fma(a, b, -p))));
+    m = f2_fma(al, bl, m);
   }
   __device__ __forceinline__ double value() const {
     float x, y, u, w, c, d;
@@ -1552,13 +1555,15 @@ __global__ void band_target_kernel(const uint32_t* band, size_t ncols, int nrows
 // elements in two pairs of floats: differences, products and sums with their exact rounding errors (Knuth's
 // two-sum, two-product by FMA), and adds each chunk's pair to FP64 totals.  The means are split into a float
 // m and a remainder d: the deviations from m are exact pairs, and d enters the FP64 totals,
-// sum (a - d)^2 = sum a^2 - 2 d sum a + n d^2.  Low parts are summed with
-// their own rounding errors; measured against exact sums the scores are as close as FP64's (6e-16, 4e-16).
+// sum (a - d)^2 = sum a^2 - 2 d sum a + n d^2.  Low parts are summed with their own rounding errors and the
+// products of two low parts apart from the rest, so that nothing an element loses adds up: emulated against exact
+// sums for maps of 2.4 M values, the threads' sums are 1e-17 to 3e-17 off (FP64 sums 5e-17 to 7e-17), r 3e-16 (5e-16)
+// and the relative L2 3e-16 (7e-16); most of both is the blocks' FP64 additions.
 // A chunk with values outside [2^-30, 2^50) in size throughout, infinities or NaN is summed in FP64.
 // WHICH: the sums wanted (bit k: sum k); MEANS: deviations from the means, raw values otherwise.
 // The sums come two to a packed operation (PairSum2), and two loads of each side run ahead (more, or three blocks
-// per SM, spill): 0.61 ms for the scores of those maps, 3.4 in FP64.  With single low parts it took 0.47, but was
-// up to 9e-15 off where FP64 is 4e-16.
+// per SM, spill): 0.62 ms for the scores of those maps, 3.4 in FP64.  With single low parts it took 0.47, but was
+// up to 9e-15 off.
 constexpr int SUM_VECS = 32;  // float4 per thread and chunk
 template <bool VEC, bool MEANS, unsigned WHICH>
 __global__ void __launch_bounds__(256, 2) map_sums_pair_kernel(const float* pred, size_t pstride_map, const float* ref,

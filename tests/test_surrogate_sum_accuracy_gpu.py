@@ -1,4 +1,4 @@
-"""The loss's sums are as exact as FP64 sums, bias included, against exact integer arithmetic."""
+"""The loss's and the scores' sums are as exact as FP64 sums, bias included, against exact integer arithmetic."""
 
 import numpy as np
 import pytest
@@ -9,6 +9,12 @@ from modlefork_gb300 import surrogate_ops as ops  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
+
+
+def _exact(x):
+    """Sum of an int64 array of values below 2^54 in size, as a Python integer."""
+    pad = np.concatenate([x, np.zeros(-x.size % 256, dtype=np.int64)])
+    return sum(pad.reshape(-1, 256).sum(axis=1).tolist())
 
 
 def test_loss_of_one_thread():
@@ -32,3 +38,51 @@ def test_loss_of_one_thread():
         want = sum(x * x for x in q)
         got = int(loss.item() * 2.0 ** 60) << 40
         assert abs(got - want) * 2 ** 50 <= want, abs(got - want) / want  # 8 * 2^-53
+
+
+def _maps(n, maps, seed):
+    """Float maps in [1, 16), whole multiples of 2^-23, and means that leave no deviation exact in a float."""
+    rng = np.random.default_rng(seed)
+    ref = np.clip(np.exp(rng.normal(1.2, 0.5, (maps, n))), 1.0, 15.5).astype(np.float32)
+    pred = np.clip(ref + 0.1 * rng.standard_normal(ref.shape), 1.0, 15.5).astype(np.float32)
+    return pred, ref, np.array([1.3700001, 1.7300003], dtype=np.float32)
+
+
+@pytest.mark.parametrize("n,maps", [(2_400_000, 16), (700_001, 16)])
+def test_map_sums_are_unbiased(n, maps):
+    """Sums about float means.  The blocks' FP64 sums meet in some 40 additions in any order, a random walk of
+    about 2e-16 per map; what each element loses must not add up: 1.5e-15 for one map, 2e-16 for the mean of 16
+    (dropping the squares of the deviations' low parts lost 4e-16 to 7e-16 of every map)."""
+    pred, ref, mean = _maps(n, maps, n)
+    out = torch.zeros(maps, 6, dtype=torch.float64, device=DEV)
+    ops.map_sums(torch.from_numpy(pred).to(DEV), torch.from_numpy(ref).to(DEV), n, maps, out,
+                 means=torch.from_numpy(np.tile(mean.astype(np.float64), (maps, 1))).to(DEV))
+    got = out.cpu().numpy()
+    unit = 2.0 ** 23
+    mp, mr = (int(float(m) * unit) for m in mean)
+    err = np.zeros((maps, 6))
+    for k in range(maps):
+        p, r = ((x[k].astype(np.float64) * unit).astype(np.int64) for x in (pred, ref))
+        a, b, d = p - mp, r - mr, p - r
+        for j, v in enumerate((a, b, a * a, b * b, a * b, d * d)):
+            want, scale = _exact(v), unit if j < 2 else unit * unit
+            err[k, j] = (int(got[k, j] * scale * 2 ** 20) - (want << 20)) / (want << 20)
+    assert np.abs(err).max() <= 1.5e-15, np.abs(err).max(axis=0)
+    assert np.abs(err.mean(axis=0)).max() <= 2e-16, err.mean(axis=0)
+
+
+def test_scores_of_whole_maps():
+    """Pearson r and relative L2 of 4000 x 600 maps against exact sums: 2e-15 (FP64 sums: up to 1e-15)."""
+    from fractions import Fraction as F
+
+    n, maps = 2_400_000, 8
+    pred, ref, _ = _maps(n, maps, 5)
+    r, l2 = ops.map_scores(torch.from_numpy(pred).to(DEV), torch.from_numpy(ref).to(DEV), n, maps)
+    for k in range(maps):
+        p, q = ((x[k].astype(np.float64) * 2.0 ** 23).astype(np.int64) for x in (pred, ref))
+        sp, sq = _exact(p), _exact(q)
+        spp, sqq, spq, sdd = _exact(p * p), _exact(q * q), _exact(p * q), _exact((p - q) ** 2)
+        cov, vp, vq = F(spq) - F(sp * sq, n), F(spp) - F(sp * sp, n), F(sqq) - F(sq * sq, n)
+        # r^2 and l2^2 are ratios of integers: compare the squares, whose relative error is twice as large
+        assert abs(F(float(r[k])) ** 2 / (cov * cov / (vp * vq)) - 1) <= 4e-15
+        assert abs(F(float(l2[k])) ** 2 / F(sdd, sqq) - 1) <= 4e-15
