@@ -1576,7 +1576,6 @@ __global__ void __launch_bounds__(256, 2) map_sums_pair_kernel(const float* pred
   const float fp = static_cast<float>(mp), fr = static_cast<float>(mr);
   const double dp = mp - fp, dr = mr - fr;
   double s[6] = {0, 0, 0, 0, 0, 0};
-  double cnt = 0.0;
   const size_t span = static_cast<size_t>(SUM_VECS) * 256 * 4;  // elements of a block's step
   const uint32_t LO = 0x30800000u, HI = 0x58800000u;           // 2^-30, 2^50
   auto load2 = [&](float4& x, float4& y, size_t i) {
@@ -1655,34 +1654,30 @@ __global__ void __launch_bounds__(256, 2) map_sums_pair_kernel(const float* pred
     }
     const bool plain = means_ok && mxp < HI && mxr < HI && (mxp >= LO || (mxp == 0 && fp == 0.0f)) &&
                        (mxr >= LO || (mxr == 0 && fr == 0.0f));
-    if (plain || k == 0) {
+    if (plain) {
       const double sa = t[0].value(), sb = t[1].value(), c = k;
-      s[0] += sa;
-      s[1] += sb;
+      s[0] += sa - c * dp;
+      s[1] += sb - c * dr;
       s[2] += t[2].value() - 2.0 * dp * sa + c * dp * dp;
       s[3] += t[3].value() - 2.0 * dr * sb + c * dr * dr;
       s[4] += t[4].value() - dr * sa - dp * sb + c * dp * dr;
       s[5] += t[5].value();
-      cnt += c;
-    } else {
+    } else if (k > 0) {  // nothing of fp, fr, dp, dr, which are infinite or NaN for means outside float's range
       for (int v = 0; v < SUM_VECS; ++v) {
         for (int e = 0; e < 4; ++e) {
           const size_t i = base + (static_cast<size_t>(v) * 256 + threadIdx.x) * 4 + e;
           if (i >= n) break;
           const double a = p[i] - mp, b = r[i] - mr, d = static_cast<double>(p[i]) - r[i];
-          s[0] += a + dp;  // the totals of s[0] and s[1] are relative to fp and fr
-          s[1] += b + dr;
+          s[0] += a;
+          s[1] += b;
           s[2] += a * a;
           s[3] += b * b;
           s[4] += a * b;
           s[5] += d * d;
-          cnt += 1.0;
         }
       }
     }
   }
-  s[0] -= cnt * dp;
-  s[1] -= cnt * dr;
   __shared__ double red[6][8];
   for (int k = 0; k < 6; ++k) {
     double x = s[k];

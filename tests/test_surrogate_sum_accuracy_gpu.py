@@ -86,3 +86,25 @@ def test_scores_of_whole_maps():
         # r^2 and l2^2 are ratios of integers: compare the squares, whose relative error is twice as large
         assert abs(F(float(r[k])) ** 2 / (cov * cov / (vp * vq)) - 1) <= 4e-15
         assert abs(F(float(l2[k])) ** 2 / F(sdd, sqq) - 1) <= 4e-15
+
+
+@pytest.mark.parametrize("mean", [1e39, -3e300, np.inf, -np.inf, np.nan, 2.0 ** 60])
+@pytest.mark.parametrize("n", [5000, 40_001])
+def test_map_sums_about_means_beyond_floats(n, mean):
+    """Deviations from means that no float holds, as FP64 numpy gives them (1e-13 of each sum, infinities and NaN
+    as they come); threads without elements add nothing."""
+    rng = np.random.default_rng(n)
+    p, r = (rng.random(n).astype(np.float32) for _ in range(2))
+    out = torch.zeros(1, 6, dtype=torch.float64, device=DEV)
+    ops.map_sums(torch.from_numpy(p).to(DEV), torch.from_numpy(r).to(DEV), n, 1, out,
+                 means=torch.tensor([[mean, 0.5]], dtype=torch.float64, device=DEV))
+    with np.errstate(all="ignore"):
+        a, b, d = p.astype(np.float64) - mean, r.astype(np.float64) - 0.5, p.astype(np.float64) - r
+        want = np.array([a.sum(), b.sum(), (a * a).sum(), (b * b).sum(), (a * b).sum(), (d * d).sum()])
+        size = np.array([np.abs(x).sum() for x in (a, b, a * a, b * b, a * b, d * d)])
+    got = out.cpu().numpy()[0]
+    for k in range(6):
+        if np.isfinite(size[k]):
+            assert abs(got[k] - want[k]) <= 1e-13 * size[k], (k, got[k], want[k])
+        else:
+            assert got[k] == want[k] or (np.isnan(got[k]) and np.isnan(want[k])), (k, got[k], want[k])
