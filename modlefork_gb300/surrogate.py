@@ -77,6 +77,10 @@ def conv_specs(widths, mid):
     return specs
 
 
+# entries of a workspace that hold addresses
+OP_LISTS = ("forward_ops", "forward_key", "backward_ops")
+
+
 class UNet:
     """Parameters, optimiser state and per-batch-size workspaces of the surrogate network."""
 
@@ -118,6 +122,12 @@ class UNet:
         self.step_count = 0
         self._ws = {}
         self._init(seed, head_bias)
+
+    def __getstate__(self):
+        """Copies and pickles leave the lists of operations out: they hold addresses of this network's tensors."""
+        state = dict(self.__dict__)
+        state["_ws"] = {key: {k: t for k, t in ws.items() if k not in OP_LISTS} for key, ws in self._ws.items()}
+        return state
 
     # ---- parameters ----------------------------------------------------------------------
     def _init(self, seed, head_bias):

@@ -225,15 +225,24 @@ class TransposeList:
 
     def __init__(self, pairs):
         self.pairs = list(pairs)
-        self.calls = []
+        self.calls = None
+
+    def __getstate__(self):
+        return {"pairs": self.pairs, "calls": None}  # a copy has tensors, and so addresses, of its own
+
+    def _arguments(self):
+        calls = []
         for k in range(0, len(self.pairs), MAX_TRANSPOSES):
             part = self.pairs[k:k + MAX_TRANSPOSES]
             n = len(part)
             dims = [(C.c_int * n)(*(w.shape[d] for w, _ in part)) for d in range(3)]
-            self.calls.append((n, (C.c_void_p * n)(*(w.data_ptr() for w, _ in part)), *dims,
-                               (C.c_void_p * n)(*(t.data_ptr() for _, t in part))))
+            calls.append((n, (C.c_void_p * n)(*(w.data_ptr() for w, _ in part)), *dims,
+                          (C.c_void_p * n)(*(t.data_ptr() for _, t in part))))
+        return calls
 
     def run(self):
+        if self.calls is None:
+            self.calls = self._arguments()
         for call in self.calls:
             _check(load().msur_weight_transpose_list(*call, _stream()), "msur_weight_transpose_list")
 
