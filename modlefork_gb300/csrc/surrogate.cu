@@ -1521,9 +1521,10 @@ __global__ void __launch_bounds__(256) assemble_input_v8_kernel(const float* tra
     uint4 u = make_uint4(0, 0, 0, 0);
     if (i - bl * C8 == 0) {
       const I b = bl / L, l = bl - b * L;
-      const float* t = track + static_cast<size_t>(b) * 4 * L + l;
+      const size_t S = L;  // a channel's stride: three of them may be past 2^31
+      const float* t = track + static_cast<size_t>(b) * 4 * S + l;
       const float4 q = make_float4(params[b * 4], params[b * 4 + 1], params[b * 4 + 2], params[b * 4 + 3]);
-      u = make_uint4(pack_bf16x2(t[0], t[L]), pack_bf16x2(t[2 * L], t[3 * L]), pack_bf16x2(q.x, q.y), pack_bf16x2(q.z, q.w));
+      u = make_uint4(pack_bf16x2(t[0], t[S]), pack_bf16x2(t[2 * S], t[3 * S]), pack_bf16x2(q.x, q.y), pack_bf16x2(q.z, q.w));
     }
     x[i] = u;
   }
