@@ -52,7 +52,7 @@ def parse_args():
                     help="plain path one launch at a time over every n-th chromosome (0 = skip)")
     ap.add_argument("--workers", type=int, default=24, help="concurrent engine contexts")
     ap.add_argument("--wave", type=int, default=24, help="chromosome launches per step")
-    ap.add_argument("--smem-budget", type=int, default=None, help="shared memory per cell (bytes)")
+    ap.add_argument("--smem-budget", type=int, default=None, help="what a cell keeps in shared memory at most (bytes)")
     ap.add_argument("--carveout", type=int, default=None, help="shared-memory carveout percent")
     ap.add_argument("--wave-steps", type=int, default=1,
                     help="timed steps of the plain path (one-chromosome launches from concurrent contexts)")

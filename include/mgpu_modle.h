@@ -231,18 +231,21 @@ int mgpu_last_kernel_ms(mgpu_ctx* ctx, double* ms);
 /* Test and tuning switches (no counterpart in the reference).  flags: bit 0 ranks, bit 1
  * move adjustment, bit 2 collision processing, bit 3 contact sampling use the exact serial
  * restatement instead of the warp-parallel form (results are identical either way); bit 4
- * collects the per-step cycle counters of mgpu_last_profile;
- * smem_budget caps the shared memory one cell may use (0 = device limit), placing the
- * remaining per-LEF arrays in global scratch.  Flags bits 8-15 give the shared-memory carveout
+ * collects the per-step cycle counters of mgpu_last_profile.  Flags bits 8-15 give the shared-memory carveout
  * preference in percent and bits 16-23 cap the cells per SM (0 = the CUDA driver's default and the
- * occupancy limit). */
+ * occupancy limit).
+ * smem_budget limits what a cell keeps on chip (0 = as much as fits): its burn-in history, barrier bits and per-LEF
+ * arrays get the budget less 8,448 bytes, the rest goes to global scratch; a budget too small for the history
+ * and the bits is refused.  The cell's block takes more shared memory than its budget: the budget
+ * counts 8 KiB for the ring of random numbers, which takes 16 KiB (32 in blocks of 16 worker warps: cells above
+ * 256 LEFs), and not the 9.5 KiB of fixed scratch.  Size residency with bits 16-23, not with the budget. */
 int mgpu_set_debug_flags(mgpu_ctx* ctx, uint32_t flags, uint64_t smem_budget);
 
 /* Tuned settings of large batched launches (no counterpart in the reference): entries in
  * increasing max_lefs; a batch of at least 8 tasks per SM, on a context without explicit
  * mgpu_set_debug_flags budget or carveout, takes the first entry whose max_lefs is at least the
- * LEF count of its LEF-weighted median task (the last entry beyond).  smem_budget is the shared
- * memory per cell (0 = the device limit), carveout_pct the shared-memory carveout preference
+ * LEF count of its LEF-weighted median task (the last entry beyond).  smem_budget is that of
+ * mgpu_set_debug_flags (0 = as much as fits), carveout_pct the shared-memory carveout preference
  * (0 = the CUDA driver's default), max_cells_per_sm a cap on resident cells per SM (0 = the
  * occupancy limit).  The settings move arrays between shared memory and global slots; results
  * do not depend on them.  modlefork_gb300/autotune.py measures a table per device; n = 0 clears. */
@@ -410,8 +413,8 @@ int mgpu_simulate_cells_ex(mgpu_ctx* ctx, int chrom_id, const uint64_t* cell_see
  * chromosome) receives the contacts, added to; missed[chrom_id] is incremented (may be NULL);
  * stats[i] is task i's outcome (may be NULL).  Results equal one mgpu_simulate_cells call per
  * chromosome.  A shared-memory budget set with mgpu_set_debug_flags applies to every cell;
- * without one, large batches use 16 KiB per cell and a 60 % shared-memory carveout (the cells'
- * arrays live in global slots under an 88 KB L1).
+ * without one, large batches use a budget of 16 KiB per cell and a 60 % shared-memory carveout (the
+ * cells' arrays live in global slots under an 88 KB L1), or the whole carveout when no cell has more than 128 LEFs.
  */
 typedef struct mgpu_batch_task {
   uint64_t seed;

@@ -586,8 +586,9 @@ struct mgpu_ctx {
   u32* d_work = nullptr;
   std::vector<ChromEntry> chroms;
   std::mutex mu;
-  u64 smem_limit = 0;
-  u64 smem_budget = 0;     // per-cell shared memory the layout planner may use (0 = limit)
+  u64 smem_limit = 0;      // dynamic shared memory a block may request
+  u64 smem_optin = 0;      // shared memory a block may have, static included
+  u64 smem_budget = 0;     // what the layout planner may place on chip per cell (0 = limit)
   uint32_t debug_flags = 0;
   char* d_scratch = nullptr;  // per-cell global slots for arrays that do not fit on chip
   u64 scratch_bytes = 0;
@@ -642,6 +643,9 @@ extern "C" int mgpu_create(int device, const mgpu_config* cfg, mgpu_ctx** out) {
     return rc;
   }
   ctx->smem_limit = max_smem_per_block();
+  int optin = 0;
+  cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device);
+  ctx->smem_optin = (u64)optin;
   *out = ctx;
   return MGPU_OK;
 }
@@ -867,11 +871,13 @@ static int make_kparams(const mgpu_ctx* ctx, const ChromEntry& ch, uint64_t nlef
   P->occ_bins = (ch.chrom.size + c.bin_size - 1) / c.bin_size;
   // Layout: the PRNG ring is always on chip (the scalars are static shared memory); the burn-in history, the barrier bits
   // and then the per-LEF arrays go on chip in priority order while they fit, the rest into a global
-  // slot.  A budget counts the ring as BUDGET_RING_BYTES whatever the block's own takes.
+  // slot.  A budget counts the ring as BUDGET_RING_BYTES whatever the block's own takes.  A cell whose
+  // history and bits exceed the budget, or all of a block's shared memory, is refused, as where nothing else could
+  // hold them: a budget that is too small for its cells is an error of the caller's.
   P->workers = workers ? workers : workers_for(nlefs);
   const u64 header = cell_header_bytes(ch.nb, P->hist_cap);
   const u64 budget = budget_override ? budget_override : ctx->smem_budget;
-  const u64 limit = std::min<u64>(ctx->smem_limit, budget ? budget : ctx->smem_limit);
+  const u64 limit = std::min<u64>(ctx->smem_optin, budget ? budget : ctx->smem_optin);
   if (header > limit)
     return fail(MGPU_ERR_UNSUPPORTED, "%u barriers need %llu B of shared memory (limit %llu)", ch.nb,
                 (unsigned long long)header, (unsigned long long)limit);
@@ -1196,8 +1202,8 @@ extern "C" int mgpu_simulate_batch(mgpu_ctx* ctx, const mgpu_batch_task* tasks, 
   }
   int dev_sms = 0;
   cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, ctx->device);
-  // Large batches: 16 KiB per cell and a 60 % shared-memory carveout: the per-LEF arrays live in global slots
-  // under an 88 KB L1, and the registers, not shared memory, bound the cells per SM (the genome
+  // Large batches: a budget of 16 KiB per cell and a 60 % shared-memory carveout: the per-LEF arrays live in global
+  // slots under an 88 KB L1, and the registers, not shared memory, bound the cells per SM (the genome
   // workload: 1.90e9 LEF-epochs/s, 1.81e9 with everything that fits on chip).
   const bool large = ntasks >= 8ull * (uint64_t)dev_sms;
   uint64_t budget = ctx->smem_budget ? ctx->smem_budget : (large ? 16384ull : 0ull);

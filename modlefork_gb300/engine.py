@@ -434,7 +434,8 @@ class Engine:
     def set_debug_flags(self, flags=0, smem_budget=0):
         """Force the serial restatement of some steps (bit 0 rank, 1 adjust, 2 collisions,
         3 contacts), collect the step profile (bit 4), set the carveout (bits 8-15) and the
-        cells-per-SM cap (bits 16-23), and/or cap a cell's shared memory (bytes, 0 = limit)."""
+        cells-per-SM cap (bits 16-23), and/or limit what a cell keeps on chip (bytes, 0 = as much as fits; the block's random-number
+        ring and fixed scratch come on top, see the header)."""
         _check(self.lib.mgpu_set_debug_flags(self.h, flags, smem_budget), "mgpu_set_debug_flags")
 
     PROFILE_NAMES = ("burnin", "bind", "rank", "contacts", "moves", "adjust", "barriers",

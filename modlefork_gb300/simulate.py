@@ -66,7 +66,7 @@ def simulate_genome(cfg, genome, ncells=None, device=0, simulate_wo_barriers=Fal
     With ``workers`` > 1, that many host threads each drive their own engine context (own
     CUDA stream), taking chromosomes from a queue largest first, so several one-chromosome
     launches share the GPU at once, as the reference's worker threads share its cores.
-    ``smem_budget`` caps each cell's shared memory (bytes; default: the device limit with one
+    ``smem_budget`` limits what each cell keeps on chip (bytes; default: as much as fits with one
     worker, CONCURRENT_SMEM_BUDGET with several)."""
     import queue
     import threading
@@ -254,7 +254,7 @@ def _main(argv=None):
     ap.add_argument("--device", type=int, default=0)
     ap.add_argument("--workers", type=int, default=1, help="concurrent chromosome launches")
     ap.add_argument("--batched", action="store_true", help="all chromosomes in one batched launch")
-    ap.add_argument("--smem-budget", type=int, default=None, help="shared memory per cell (bytes)")
+    ap.add_argument("--smem-budget", type=int, default=None, help="what a cell keeps in shared memory at most (bytes)")
     ap.add_argument("--carveout", type=int, default=None,
                     help="batched launch: percent of the SM's unified memory used as shared memory")
     ap.add_argument("--pixels", default=None, help="write the pixel table (bin1_id, bin2_id, count) as TSV")
