@@ -1988,9 +1988,16 @@ int launch_wgrad(const WgradArgs& a, int splits, cudaStream_t st) {
   return cuda_ok(launch_pdl(kern, grid, WTHREADS, smem, st, a), "wgrad_kernel launch");
 }
 
+// The current device's SMs, for grids that any number suits (a GB300's where the query fails: the launch then
+// reports what is wrong).
+unsigned sms() {
+  int n = 0;
+  return sm_count(&n) == MSUR_OK && n > 0 ? static_cast<unsigned>(n) : 152u;
+}
+
 unsigned grid_for(size_t n, unsigned block = 256) {
-  const size_t g = (n + block - 1) / block;
-  return static_cast<unsigned>(g < 152 * 32 ? (g ? g : 1) : 152 * 32);
+  const size_t g = (n + block - 1) / block, most = 32 * sms();
+  return static_cast<unsigned>(g < most ? (g ? g : 1) : most);
 }
 
 }  // namespace
@@ -2044,22 +2051,20 @@ static int conv_forward_impl(const void* x, int B, int L, int Cin, const void* w
   // leave SMs idle a narrower one halves the chain's time on twice the SMs (the products and their order
   // are the same).  One map: the deep levels have 2 to 16 tiles at 256 columns, 8 to 64 at 64.
   const bool persistent = (form & 1) != 0, staged = (form & 2) != 0;
+  int nsm = 0;
+  rc = sm_count(&nsm);
+  if (rc) return rc;
   int BN = slot == 2 ? 256 : (slot == 1 ? 128 : 64);
   if (persistent && slot == 1 && Cout % 192 == 0) BN = 192;
-  while (BN > 64 && static_cast<long long>((Cout + BN - 1) / BN) * ((L + BM - 1) / BM) * B < 152)
+  while (BN > 64 && static_cast<long long>((Cout + BN - 1) / BN) * ((L + BM - 1) / BM) * B < nsm)
     BN = BN == 192 ? 64 : BN / 2;
   ConvArgs a;
   std::memset(&a, 0, sizeof(a));
   const uint64_t dims_a[3] = {static_cast<uint64_t>(Cin), static_cast<uint64_t>(L), static_cast<uint64_t>(B)};
   ConvPlan plan{};
   int grid = 0, smem = 0;
-  if (persistent) {
-    int sms = 0;
-    rc = sm_count(&sms);
-    if (rc) return rc;
-    plan = conv_plan(BN, Cin, taps, Cout, L, B, stages, staged, act == MSUR_ACT_SILU || gate,
-                     sms, &grid, &smem);
-  }
+  if (persistent)
+    plan = conv_plan(BN, Cin, taps, Cout, L, B, stages, staged, act == MSUR_ACT_SILU || gate, nsm, &grid, &smem);
   const uint32_t box_a[3] = {64, static_cast<uint32_t>(plan.aslots ? BM + taps - 1 : BM), 1};
   rc = make_map(&a.tm_a, x, 3, dims_a, box_a);
   if (rc) return rc;
@@ -2197,7 +2202,7 @@ static int conv_wgrad_impl(const void* x, const void* dz, int B, int L, int Cin,
     // one CTA per SM and one wave
     const int bn = taps == 3 && Cin <= 64 ? 64 : 128;
     const int tiles = ((Cin + bn - 1) / bn) * ((Cout + BM - 1) / BM);
-    splits = std::max(1, 152 / tiles);
+    splits = std::max(1, static_cast<int>(sms()) / tiles);
   }
   if (splits > a.total) splits = a.total;
   a.per_split = (a.total + splits - 1) / splits;
@@ -2205,7 +2210,7 @@ static int conv_wgrad_impl(const void* x, const void* dz, int B, int L, int Cin,
   a.per_phase = a.per_split;
   if (automatic) {
     // The tensor core's sums lose accuracy with their length, so an accumulation takes no more blocks than with
-    // two waves of 128-wide tiles: 64 x 1000 positions, 256 to 256 channels, 9e-7 of the gradient's norm,
+    // two waves of 128-wide tiles on 152 SMs (the accuracy does not follow the device's): 64 x 1000 positions, 256 to 256 channels, 9e-7 of the gradient's norm,
     // 1.8e-6 with a split's blocks in one.
     const int tiles = ((Cin + 127) / 128) * ((Cout + BM - 1) / BM);
     const int chains = std::min(a.total, (2 * 152 + tiles - 1) / tiles);
@@ -2294,7 +2299,7 @@ int msur_bias_grad(const void* dz, uint64_t rows, int C, int stride, float* db, 
     // four blocks per SM, but at least four rows per thread
     const unsigned gx = (C + 63) / 64;
     const uint64_t most = (rows + 127) / 128;
-    const unsigned gy = static_cast<unsigned>(std::min<uint64_t>(std::max(1u, 4 * 152 / gx), most ? most : 1));
+    const unsigned gy = static_cast<unsigned>(std::min<uint64_t>(std::max(1u, 4 * sms() / gx), most ? most : 1));
     return cuda_ok(launch_pdl(bias_grad_v8_kernel, dim3(gx, gy), 256, 0, static_cast<cudaStream_t>(stream),
                               static_cast<const bf16*>(dz), rows, C, stride, db),
                    "bias_grad_v8_kernel launch");
@@ -2314,7 +2319,7 @@ int msur_mse(const float* pred, int pstride, const float* target, int tstride, u
   const size_t n = rows * static_cast<size_t>(dstride);
   if (n_valid % 4 == 0 && pstride % 4 == 0 && tstride % 4 == 0 && dstride % 4 == 0 && aligned16(pred) &&
       aligned16(target) && (!dp || (reinterpret_cast<uintptr_t>(dp) & 7u) == 0)) {
-    const unsigned blocks = std::min(grid_for(n / 4), 152u * 8u);
+    const unsigned blocks = std::min(grid_for(n / 4), 8 * sms());
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (n / 4 < (1ull << 31)) {
       return cuda_ok(launch_pdl(mse_v4_kernel<unsigned>, dim3(blocks), 256, 0, st, pred, pstride, target,
@@ -2465,7 +2470,7 @@ int msur_map_sums_of(unsigned which, const float* pred, uint64_t pstride_map, co
                      uint64_t n, int nmaps, const double* means, double* out, void* stream) {
   if (!pred || !ref || !out || nmaps <= 0 || nmaps > 65535) return fail(MSUR_ERR_INVALID_ARG, "msur_map_sums: bad argument");
   // blocks of 32768 elements, about eight per SM over all maps
-  const uint64_t steps = (n + 32767) / 32768, most = std::max(1, 8 * 152 / nmaps);
+  const uint64_t steps = (n + 32767) / 32768, most = std::max(1, 8 * static_cast<int>(sms()) / nmaps);
   const dim3 grid(static_cast<unsigned>(std::min(steps, most)), nmaps);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool vec = n % 4 == 0 && pstride_map % 4 == 0 && rstride_map % 4 == 0 && aligned16(pred) && aligned16(ref);
