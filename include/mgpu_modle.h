@@ -547,7 +547,8 @@ void mgpu_prng_seed(uint64_t seed, uint64_t state[4]);
  * compare it with the host, bit for bit, on the argument streams the loop feeds it.
  *
  * mgpu_probe_samplers: per_stream samples from each of nstreams seeded streams (seed as for
- * mgpu_prng_seed) through the serial samplers the epoch loop uses; out[s * per_stream + i] is
+ * mgpu_prng_seed) through the samplers the epoch loop uses: its serial ones, and with the last two kinds the
+ * fixed-point forms of its parallel steps, which take the serial ones where they cannot tell; out[s * per_stream + i] is
  * sample i of stream s and draws[s] the raw 64-bit draws stream s consumed (UINT64_MAX if a
  * sampler hit its iteration limit).  Kinds and parameters:
  *   MGPU_PROBE_NORMAL              normal(a0, a1): move lengths (simulation.cpp:264-290)
@@ -557,6 +558,9 @@ void mgpu_prng_seed(uint64_t seed, uint64_t state[4]);
  *                                  with (1 - p)^t taken from the host, as in a full epoch
  *   MGPU_PROBE_BINOMIAL_DEVICE_POW the same with (1 - p)^t evaluated on the device (last epoch)
  *   MGPU_PROBE_GEV                 genextreme(0, a0, a1) noise (genextreme_value_distribution.hpp:87-105)
+ *   MGPU_PROBE_MOVE                the moves round(max(0, normal(a0, a1))); -1 for one above 32 bits
+ *   MGPU_PROBE_POSITION            the whole base pairs that 2^31 - noise and 2^31 + noise (in turn, genextreme(0, a0,
+ *                                  a1), clamped to [-1, 2^32]) fall into
  * mgpu_probe_libm: out[i] = f(x[i], y[i]) on the device for
  *   MGPU_PROBE_LOG log x, MGPU_PROBE_EXP exp x, MGPU_PROBE_POW pow(x, y),
  *   MGPU_PROBE_GEV_NOISE the GEV noise of a uniform x with (mu, sigma, xi),
@@ -569,6 +573,8 @@ void mgpu_prng_seed(uint64_t seed, uint64_t state[4]);
 #define MGPU_PROBE_BINOMIAL 3
 #define MGPU_PROBE_BINOMIAL_DEVICE_POW 4
 #define MGPU_PROBE_GEV 5
+#define MGPU_PROBE_MOVE 6
+#define MGPU_PROBE_POSITION 7
 #define MGPU_PROBE_LOG 0
 #define MGPU_PROBE_EXP 1
 #define MGPU_PROBE_POW 2

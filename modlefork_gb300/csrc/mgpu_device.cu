@@ -3519,6 +3519,24 @@ __device__ __noinline__ bool gev_fixed(u64 u, i64* n) {
   return true;
 }
 
+// The whole base pairs that a contact's noised positions rev - noise(u1) and fwd + noise(u2) fall into.
+__device__ __forceinline__ void noised_positions(u64 rev, u64 fwd, u64 u1, u64 u2, i64* ia, i64* ib) {
+  i64 n1, n2;
+  bool exact = !g_P.gev_fixed || !gev_fixed(u1, &n1) || !gev_fixed(u2, &n2);
+  if (!exact) {
+    const i64 a = ((i64)rev << 25) - n1, d = ((i64)fwd << 25) + n2;
+    const u32 near = 1u << 12, one = 1u << 25;  // fractions within 2^-13 of a whole number
+    exact = (((u32)a + near) & (one - 1)) <= 2 * near || (((u32)d + near) & (one - 1)) <= 2 * near;
+    *ia = a >> 25;
+    *ib = d >> 25;
+  }
+  if (exact) {
+    // positions outside [0, 2^32) fail a contact's bounds in any case
+    *ia = (i64)floor(fmin(fmax((double)rev - gev_noise(u1), -1.0), 4294967296.0));
+    *ib = (i64)floor(fmin(fmax((double)fwd + gev_noise(u2), -1.0), 4294967296.0));
+  }
+}
+
 // One contact attempt read from draws at `at` (register_contacts.cpp:129-198).  Returns the
 // draws it takes; *ok tells whether it registers a contact; *regular is false when the attempt
 // hit a bucket rejection (exact handling needs the serial path).
@@ -3545,20 +3563,7 @@ __device__ __forceinline__ u32 contact_attempt(u64 at, bool tad,
   if (P.noisify) {
     const u64 u1 = ring_at(c.rmask, at + used), u2 = ring_at(c.rmask, at + used + 1);
     used += 2;
-    i64 n1, n2;
-    bool exact = !P.gev_fixed || !gev_fixed(u1, &n1) || !gev_fixed(u2, &n2);
-    if (!exact) {
-      const i64 a = ((i64)rp << 25) - n1, d = ((i64)fp << 25) + n2;
-      const u32 near = 1u << 12, one = 1u << 25;  // fractions within 2^-13 of a whole number
-      exact = (((u32)a + near) & (one - 1)) <= 2 * near || (((u32)d + near) & (one - 1)) <= 2 * near;
-      ia = a >> 25;
-      ib = d >> 25;
-    }
-    if (exact) {
-      // positions outside [0, 2^32) fail the bounds below in any case
-      ia = (i64)floor(fmin(fmax((double)rp - gev_noise(u1), -1.0), 4294967296.0));
-      ib = (i64)floor(fmin(fmax((double)fp + gev_noise(u2), -1.0), 4294967296.0));
-    }
+    noised_positions(rp, fp, u1, u2, &ia, &ib);
   }
   const i64 p1 = min(ia, ib), p2 = max(ia, ib);
   if (!(p1 >= (i64)start && p2 < (i64)end)) return used;
@@ -4574,6 +4579,46 @@ __global__ void __launch_bounds__(32) sampler_probe_kernel(const __grid_constant
   }
 }
 
+// The same for what the epoch's parallel steps evaluate themselves: kind 5 the moves of P.rev_move[0]
+// (move_sample), kind 6 the whole base pairs of 2^31 - noise and 2^31 + noise in turn (noised_positions), one
+// draw each.  A ring of the stream's draws in shared memory, as the producer warps keep one.
+constexpr u32 PROBE_DRAWS = 512;
+__global__ void __launch_bounds__(32) step_probe_kernel(const __grid_constant__ KParams P, int kind, const u64* states,
+                                                        u64 nstreams, u64 per, double* out, u64* draws,
+                                                        const ulonglong2* jt) {
+  load_layers(jt);
+  load_plan(P);
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  u64* ring = reinterpret_cast<u64*>(dyn_smem);
+  for (u64 s = blockIdx.x; s < nstreams; s += gridDim.x) {
+    u64 st[4];
+    for (int k = 0; k < 4; ++k) st[k] = states[4 * s + k];
+    u64 pos = 0, filled = 0;
+    bool ok = true;
+    for (u64 i = 0; i < per; ++i) {
+      for (; filled - pos < PROBE_DRAWS / 2; ++filled) ring[filled & (PROBE_DRAWS - 1)] = xo_next(st);
+      double r = 0.0;
+      if (kind == 5) {
+        RingSrc g{PROBE_DRAWS - 1, (u32)pos, (u32)filled, 0};
+        u32 v = 0;
+        bool range = false;
+        ok &= move_sample(g, g_P.rev_move[0], &v, &range) == SMP_OK;
+        pos += g.n;
+        r = range ? -1.0 : (double)v;
+      } else {
+        const u64 u = ring[pos & (PROBE_DRAWS - 1)];
+        ++pos;
+        i64 ia, ib;
+        noised_positions(1ull << 31, 1ull << 31, u, u, &ia, &ib);
+        r = (double)((i & 1) ? ib : ia);
+      }
+      out[s * per + i] = r;
+    }
+    draws[s] = ok ? pos : ~0ull;
+  }
+}
+
 // out[i] = f(x[i], y[i]) for f = 0: log x, 1: exp x, 2: pow(x, y), 3: the GEV noise of
 // register_contacts.cpp:48-64 from u = x (mu, sigma, xi), 4: below_exp(x, y) as 0 or 1.
 __global__ void libm_probe_kernel(int kind, const double* x, const double* y, u64 n, double mu, double sigma,
@@ -4600,6 +4645,15 @@ int launch_sampler_probe(const KParams& P, int kind, const u64* states, u64 nstr
   sampler_probe_kernel<<<(unsigned)blocks, 32, 0, (cudaStream_t)stream>>>(P, kind, states, nstreams, per, a0, a1,
                                                                           out, draws);
   return cuda_fail(cudaGetLastError(), "sampler_probe_kernel launch", errbuf, errlen);
+}
+
+int launch_step_probe(const KParams& P, int kind, const u64* states, u64 nstreams, u64 per, double* out, u64* draws,
+                      const void* tables, void* stream, char* errbuf, int errlen) {
+  if (nstreams == 0) return MGPU_OK;
+  const u64 blocks = nstreams < 65535 ? nstreams : 65535;
+  step_probe_kernel<<<(unsigned)blocks, 32, PROBE_DRAWS * sizeof(u64), (cudaStream_t)stream>>>(
+      P, kind, states, nstreams, per, out, draws, (const ulonglong2*)tables);
+  return cuda_fail(cudaGetLastError(), "step_probe_kernel launch", errbuf, errlen);
 }
 
 int launch_libm_probe(int kind, const double* x, const double* y, u64 n, double mu, double sigma, double xi,

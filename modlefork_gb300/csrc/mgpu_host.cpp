@@ -513,7 +513,7 @@ static void build_layer(int i, uint64_t* e) {
   e[1] = (uint64_t)(x * 1152921504606846976.0);
 }
 
-static std::vector<uint64_t> build_tables() {
+static std::vector<uint64_t> make_tables() {
   std::vector<uint64_t> t(MAX_PRODUCERS * JUMP_TABLE_ENTRIES * 4 + (NORMAL_LAYERS + LOG_PARTS) * 2, 0);
   for (u32 p = 1; p <= MAX_PRODUCERS; ++p) build_jump_table(jump_distance(p), &t[(p - 1) * JUMP_TABLE_ENTRIES * 4]);
   for (u32 i = 0; i < NORMAL_LAYERS; ++i) build_layer((int)i, &t[MAX_PRODUCERS * JUMP_TABLE_ENTRIES * 4 + 2 * i]);
@@ -525,6 +525,12 @@ static std::vector<uint64_t> build_tables() {
     e[0] = inv << 32;
     e[1] = (uint64_t)(-logl((long double)inv / 4294967296.0L) * 9223372036854775808.0L);
   }
+  return t;
+}
+
+// The tables, built once per process.
+static const std::vector<uint64_t>& constant_tables() {
+  static const std::vector<uint64_t> t = make_tables();
   return t;
 }
 
@@ -631,7 +637,7 @@ extern "C" int mgpu_create(int device, const mgpu_config* cfg, mgpu_ctx** out) {
   ctx->device = device;
   ctx->cfg = *cfg;
   rc = cuda_check(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking), "cudaStreamCreate");
-  static const std::vector<uint64_t> jt = build_tables();
+  const std::vector<uint64_t>& jt = constant_tables();
   if (!rc) rc = cuda_check(cudaMalloc(&ctx->d_jump, jt.size() * 8), "cudaMalloc(jump table)");
   if (!rc) rc = cuda_check(cudaMemcpy(ctx->d_jump, jt.data(), jt.size() * 8, cudaMemcpyHostToDevice), "copy jump table");
   if (!rc) rc = cuda_check(cudaMalloc(&ctx->d_work, sizeof(u32)), "cudaMalloc(work counter)");
@@ -776,6 +782,22 @@ static MoveSpec move_spec(double mean, double sd) {
   return m;
 }
 
+// The contact noise: in fixed point for the parameters its error bound covers (xi == 0 has a formula of its own).
+static void set_noise(KParams* P, double mu, double sigma, double xi) {
+  P->gev_mu = mu;
+  P->gev_sigma = sigma;
+  P->gev_xi = xi;
+  const double scale = xi == 0.0 ? mu - sigma : -sigma;
+  const double base = xi == 0.0 ? 0.0 : mu;
+  P->gev_fixed = std::fabs(scale) < 32768.0 && std::fabs(base) < 1e9 && std::fabs(xi) <= 0.0014;
+  if (P->gev_fixed) {
+    P->gev_base = (int64_t)std::llround(base * 33554432.0);
+    P->gev_scale = (uint64_t)(std::fabs(scale) * 4294967296.0);
+    P->gev_scale_neg = scale < 0.0;
+    P->gev_xiq = (uint64_t)(std::fabs(xi) * 18446744073709551616.0);
+  }
+}
+
 // Worker warps of a cell: a thread per LEF up to 256 LEFs, 512 threads above.  Below 129 LEFs more warps only make
 // the block barriers dearer and leave fewer cells per SM: 4096 cells of 20 LEFs took 348 ms with eight warps, 306
 // with one (313 with a warp per cell and no barriers); 60 LEFs 373 and 354 with two (417); 100 LEFs 395 and
@@ -841,21 +863,7 @@ static int make_kparams(const mgpu_ctx* ctx, const ChromEntry& ch, uint64_t nlef
   P->ratio_mode = ratio == 0 ? 0 : (!std::isfinite(ratio) ? 1 : 2);
   P->p_loop = 1.0 / (ratio + 1.0);
   P->noisify = (c.contact_sampling_strategy & MGPU_CS_NOISIFY) ? 1 : 0;
-  P->gev_mu = c.genextreme_mu;
-  P->gev_sigma = c.genextreme_sigma;
-  P->gev_xi = c.genextreme_xi;
-  // fixed-point noise for the parameters its error bound covers (xi == 0 has a formula of its own)
-  {
-    const double scale = c.genextreme_xi == 0.0 ? c.genextreme_mu - c.genextreme_sigma : -c.genextreme_sigma;
-    const double base = c.genextreme_xi == 0.0 ? 0.0 : c.genextreme_mu;
-    P->gev_fixed = std::fabs(scale) < 32768.0 && std::fabs(base) < 1e9 && std::fabs(c.genextreme_xi) <= 0.0014;
-    if (P->gev_fixed) {
-      P->gev_base = (int64_t)std::llround(base * 33554432.0);
-      P->gev_scale = (uint64_t)(std::fabs(scale) * 4294967296.0);
-      P->gev_scale_neg = scale < 0.0;
-      P->gev_xiq = (uint64_t)(std::fabs(c.genextreme_xi) * 18446744073709551616.0);
-    }
-  }
+  set_noise(P, c.genextreme_mu, c.genextreme_sigma, c.genextreme_xi);
   {
     const double p = (0.5 < P->p_loop) ? (1 - P->p_loop) : P->p_loop;
     P->bin_q_n = std::pow((1 - p), (double)(int64_t)P->spe);
@@ -1663,7 +1671,7 @@ extern "C" int mgpu_run_phase(mgpu_ctx* ctx, int chrom_id, int phase, mgpu_phase
 // ===========================================================================================
 extern "C" int mgpu_probe_samplers(int device, int kind, const uint64_t* seeds, uint64_t nstreams,
                                    uint64_t per_stream, double a0, double a1, double* out, uint64_t* draws) {
-  if ((nstreams && (!seeds || !out || !draws)) || kind < 0 || kind > MGPU_PROBE_GEV)
+  if ((nstreams && (!seeds || !out || !draws)) || kind < 0 || kind > MGPU_PROBE_POSITION)
     return fail(MGPU_ERR_INVALID_ARG, "mgpu_probe_samplers: bad argument");
   if (nstreams == 0 || per_stream == 0) return MGPU_OK;
   CK(cudaSetDevice(device));
@@ -1701,6 +1709,14 @@ extern "C" int mgpu_probe_samplers(int device, int kind, const uint64_t* seeds, 
       P.gev_sigma = a0;
       P.gev_xi = a1;
       break;
+    case MGPU_PROBE_MOVE:
+      dev_kind = 5;
+      P.rev_move[0] = move_spec(a0, a1);
+      break;
+    case MGPU_PROBE_POSITION:
+      dev_kind = 6;
+      set_noise(&P, 0.0, a0, a1);
+      break;
   }
   std::vector<uint64_t> states(4 * nstreams);
   for (uint64_t s = 0; s < nstreams; ++s) mgpu_prng_seed(seeds[s], &states[4 * s]);
@@ -1712,7 +1728,17 @@ extern "C" int mgpu_probe_samplers(int device, int kind, const uint64_t* seeds, 
   if (!rc) rc = cuda_check(cudaMalloc(&d_draws, nstreams * 8), "cudaMalloc(draws)");
   if (!rc) rc = cuda_check(cudaMemcpy(d_states, states.data(), states.size() * 8, cudaMemcpyHostToDevice), "copy");
   char err[256] = {0};
-  if (!rc) {
+  u64* d_tables = nullptr;
+  if (!rc && dev_kind >= 5) {
+    const std::vector<uint64_t>& t = constant_tables();
+    rc = cuda_check(cudaMalloc(&d_tables, t.size() * 8), "cudaMalloc(tables)");
+    if (!rc) rc = cuda_check(cudaMemcpy(d_tables, t.data(), t.size() * 8, cudaMemcpyHostToDevice), "copy tables");
+    if (!rc) {
+      rc = launch_step_probe(P, dev_kind, d_states, nstreams, per_stream, d_out, d_draws, d_tables, nullptr, err,
+                             sizeof(err));
+      if (rc) rc = fail(rc, "%s", err);
+    }
+  } else if (!rc) {
     rc = launch_sampler_probe(P, dev_kind, d_states, nstreams, per_stream, a0, a1, d_out, d_draws, nullptr, err,
                               sizeof(err));
     if (rc) rc = fail(rc, "%s", err);
@@ -1723,6 +1749,7 @@ extern "C" int mgpu_probe_samplers(int device, int kind, const uint64_t* seeds, 
   cudaFree(d_states);
   cudaFree(d_out);
   cudaFree(d_draws);
+  cudaFree(d_tables);
   return rc;
 }
 

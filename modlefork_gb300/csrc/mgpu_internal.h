@@ -253,6 +253,9 @@ int launch_band_pixels(const u32* band, u64 nrows, u64 ncols, u64 bin_offset, co
 // with P.gev_*) and the device's log / exp / pow / GEV noise / below_exp on arguments.
 int launch_sampler_probe(const KParams& P, int kind, const u64* states, u64 nstreams, u64 per, double a0,
                          double a1, double* out, u64* draws, void* stream, char* errbuf, int errlen);
+// What the parallel steps evaluate themselves: kind 5 moves of P.rev_move[0], 6 noised positions (P.gev_*).
+int launch_step_probe(const KParams& P, int kind, const u64* states, u64 nstreams, u64 per, double* out, u64* draws,
+                      const void* tables, void* stream, char* errbuf, int errlen);
 int launch_libm_probe(int kind, const double* x, const double* y, u64 n, double mu, double sigma, double xi,
                       double* out, void* stream, char* errbuf, int errlen);
 

@@ -158,12 +158,13 @@ def barriers_from_bed(chrom, records, default_stp_active, default_stp_inactive):
     return out
 
 
-PROBE_NORMAL, PROBE_EXPONENTIAL, PROBE_POISSON, PROBE_BINOMIAL, PROBE_BINOMIAL_DEVICE_POW, PROBE_GEV = range(6)
+(PROBE_NORMAL, PROBE_EXPONENTIAL, PROBE_POISSON, PROBE_BINOMIAL, PROBE_BINOMIAL_DEVICE_POW, PROBE_GEV, PROBE_MOVE,
+ PROBE_POSITION) = range(8)
 PROBE_LOG, PROBE_EXP, PROBE_POW, PROBE_GEV_NOISE, PROBE_BELOW_EXP = range(5)
 
 
 def probe_samplers(kind, seeds, per_stream, a0=0.0, a1=0.0, device=0):
-    """The epoch loop's serial samplers on the device (test hook mgpu_probe_samplers):
+    """The epoch loop's samplers on the device (test hook mgpu_probe_samplers):
     (samples[nstreams, per_stream], draws[nstreams])."""
     seeds = np.ascontiguousarray(seeds, dtype=np.uint64)
     out = np.empty((len(seeds), per_stream), dtype=np.float64)
