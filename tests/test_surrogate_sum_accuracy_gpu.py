@@ -108,3 +108,27 @@ def test_map_sums_about_means_beyond_floats(n, mean):
             assert abs(got[k] - want[k]) <= 1e-13 * size[k], (k, got[k], want[k])
         else:
             assert got[k] == want[k] or (np.isnan(got[k]) and np.isnan(want[k])), (k, got[k], want[k])
+
+
+@pytest.mark.parametrize("B,L,cin,cout,taps,splits", [(64, 1000, 256, 256, 3, (76, 38)), (64, 4000, 64, 64, 3, (304, 152)),
+                                                      (64, 2000, 128, 128, 1, (304, 152))])
+def test_weight_gradient_accumulation_length(B, L, cin, cout, taps, splits):
+    """The automatic split adds its accumulations to dw often enough: its error (norm against FP64) is that of as many
+    splits as give each accumulation two waves' share of the positions (76, 304), not that of one wave of splits with a
+    single accumulation each (38, 152), which is about twice as large."""
+    g = torch.Generator(device=DEV).manual_seed(B + L)
+    x = torch.nn.functional.silu(torch.randn(B, L, cin, generator=g, device=DEV)).to(torch.bfloat16)
+    dz = (torch.randn(B, L, cout, generator=g, device=DEV) * 1e-2).to(torch.bfloat16)
+    pad = (taps - 1) // 2
+    xp = torch.zeros(B, L + 2 * pad, cin, dtype=torch.float64, device=DEV)
+    xp[:, pad:pad + L] = x.double()
+    zd = dz.double().reshape(B * L, cout)
+    want = torch.stack([zd.T @ xp[:, t:t + L].reshape(B * L, cin) for t in range(taps)], dim=1)
+
+    def error(k):
+        dw = torch.zeros(cout, taps, cin, device=DEV)
+        ops.conv_wgrad(x, dz, dw, splits=k)
+        return float((dw.double() - want).norm() / want.norm())
+
+    auto, short, long = error(0), error(splits[0]), error(splits[1])
+    assert auto <= 1.15 * short and auto <= 0.85 * long, (auto, short, long)
