@@ -1331,9 +1331,11 @@ __global__ void mse_kernel(const float* pred, int pstride, const float* target, 
 // Four channels per thread (counts and strides multiples of 4, aligned buffers), the squares summed as floats with
 // their errors (PairSum2) per 64 values and then in FP64.  Sums of 64 squares are 5e-17 off (a loop in FP64
 // 3e-16); a single low part, without the errors of its own sums, left 1.4e-14, of which 1.2e-15 had one
-// sign and stayed in the total.  I: 32-bit indexes where they reach.
+// sign and stayed in the total.  32 registers, so that the eight blocks per SM of the grid are there at once: 65 us for
+// 16 maps (81 with the 40 that the compiler takes, 60 with the single low part; the memory needs 60).  I:
+// 32-bit indexes where they reach.
 template <typename I>
-__global__ void __launch_bounds__(256) mse_v4_kernel(const float* __restrict__ pred, int pstride,
+__global__ void __launch_bounds__(256, 8) mse_v4_kernel(const float* __restrict__ pred, int pstride,
                                                      const float* __restrict__ target, int tstride, size_t rows,
                                                      int n_valid, bf16* dp, int dstride, float scale, double* loss) {
   umma::pdl_wait();
