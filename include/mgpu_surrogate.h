@@ -74,18 +74,21 @@ int msur_conv_forward_fused(const void* x, int B, int L, int Cin, const void* w,
                             int n_valid, void* stream);
 
 /* Pipeline depth of msur_conv_forward for one N tile width (64, 128 or 256 output channels per
- * tile, chosen by Cout): 2 to 4 shared-memory stages.  Fewer stages let 2-4 CTAs share an SM,
- * so that one tile's epilogue overlaps another's main loop; the autotuner
- * (modlefork_gb300/autotune.py) picks the depths per device.  Defaults 4 (64), 3 (128), 4 (256).
+ * tile, chosen by Cout): 2 to 4.  With one CTA per tile it is the number of shared-memory stages; fewer let
+ * 2-4 CTAs share an SM, so that one tile's epilogue overlaps another's main loop.  The persistent form plans its
+ * shared memory itself: there it is the depth of the operand ring that the plan starts from, which goes
+ * before more than two groups of epilogue warps (a smaller depth leaves room for more groups), and what
+ * is left over deepens the ring up to eight stages.  The autotuner (modlefork_gb300/autotune.py) picks the
+ * depths per device.  Defaults 4 (64), 3 (128), 4 (256).
  * msur_conv_get_stages returns the current depth (negative on a bad width). */
 int msur_conv_set_stages(int bn, int stages);
 int msur_conv_get_stages(int bn);
 /* Kernel form of msur_conv_forward for one N tile width, two bits:
- *   bit 0: a persistent kernel (CTAs walk the tiles with a double-buffered TMEM accumulator, so
- *          a tile's epilogue overlaps the next tile's MMAs) instead of one CTA per output tile;
+ *   bit 0: a persistent kernel (CTAs walk the tiles with two to eight TMEM accumulators, so a
+ *          tile's epilogue overlaps the next tiles' MMAs) instead of one CTA per output tile; it also
+ *          uses 192-column tiles and narrower ones where tiles would leave SMs idle;
  *   bit 1: the staged epilogue: each epilogue warp writes 32 rows x 64 columns of output to
- *          shared memory and stores them with a TMA store, instead of one row per thread
- *          (calls with a gate always take the per-thread epilogue).
+ *          shared memory and stores them with a TMA store, instead of one row per thread.
  * Results are identical in every form; the default is 2 and the autotuner picks per device and
  * per layer.  The getter returns the current form (negative on a bad width).
  * msur_conv_set_persistent / msur_conv_get_persistent set and read bit 0 alone. */
@@ -96,8 +99,9 @@ int msur_conv_get_persistent(int bn);
 
 /* Weight gradient of that convolution, ADDED to dw [Cout][taps][Cin] (FP32):
  *   dw[n][t][c] += sum_{b, l} dz[b, l, n] * x[b, l + t - (taps - 1) / 2, c]
- * taps 1 or 3; the position range is split over `splits` CTAs per tile (0 = enough to fill the
- * GPU), whose partial sums are added with atomics. */
+ * taps 1 or 3; the position range is split over `splits` CTAs per tile (0 = one wave of the GPU, each with
+ * accumulations short enough for FP32), whose partial sums are added to dw in any order: by bulk reductions when
+ * dw is 16-byte aligned, word by word otherwise. */
 int msur_conv_wgrad(const void* x, const void* dz, int B, int L, int Cin, int Cout, int taps, float* dw, int splits,
                     void* stream);
 

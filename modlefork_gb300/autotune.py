@@ -11,13 +11,15 @@
    which case the default stays.  The settings only move per-LEF arrays between
    shared memory and global slots, so every candidate simulates the same cells.
 2. Surrogate convolutions: the kernel form (one CTA per tile or persistent, outputs per thread or
-   staged through shared memory and TMA stores) and pipeline depth (2-4 stages) per N tile width
+   staged through shared memory and TMA stores) and pipeline depth (2-4: the stages of a tile's CTA, or
+   where the persistent kernel's plan of its shared memory starts) per N tile width
    of msur_conv_forward, then per forward layer of the network, by coordinate descent on the
    network's inference time at batch 256.
 
 The result is a JSON file keyed by the device's name and SM count; ``load_table`` and
 ``apply_all`` read it back (engine contexts and the surrogate library take it from there).  The
-tuned table measured on a GB300 ships as modlefork_gb300/data/tuning_gb300.json.
+tuned table measured on a GB300 ships as modlefork_gb300/data/tuning_gb300.json; its rates and times are those of
+the kernels it was measured on (a warp per cell, four epilogue warps per convolution), slower than today's.
 """
 
 import argparse

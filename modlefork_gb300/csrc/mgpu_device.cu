@@ -12,9 +12,10 @@
 // warp per cell a sweep of 2,000 LEFs is 63 dependent rounds of loads, shared memory holds at most a
 // dozen such warps per SM, and an instruction issued on 10 % of cycles.  With 16 warps a sweep is
 // two or four rounds, the arrays stay in shared memory, and a sweep costs about one barrier.  152 cells
-// of 73 Mbp (1,460 LEFs) took 843 ms with a warp per cell, 149 now; 24 chromosomes of 40-110 Mbp x 24 cells
+// of 73 Mbp (1,460 LEFs) took 843 ms with a warp per cell, 147-165 now; 24 chromosomes of 40-110 Mbp x 24 cells
 // 1.29 s and 0.29; 2 x 1024 cells of 20 Mbp (an instruction-fetch-bound load: several small blocks per SM
-// in different steps) 1.34 s and 0.56.
+// in different steps) 1.2-1.34 s and 0.57-0.63.  Cells of a few dozen LEFs get a warp or two (workers_for): there the
+// barriers would cost more than the rounds they save.
 //
 // Draw order.  Every random number of the reference comes from one sequential
 // Xoshiro256++ stream per cell, consumed in a data-dependent order.  The producer warps keep a
@@ -34,7 +35,7 @@
 //    the offsets they would have if every earlier item took its usual count; the offsets are then
 //    corrected from the items that deviate, or the workers resume after the first of them;
 //  * sequential sweeps are replaced by closed forms: rank_lefs by a merge of the units that moved
-//    into the still-sorted order of the others, adjust_moves by walks from the units that push a
+//    into the still-sorted order of the others, the adjustment of moves by walks from the units that push a
 //    neighbour, the LEF-BAR and primary LEF-LEF sweeps by searches over the ranked positions.
 // Where a closed form's precondition does not hold (full ties in the ranking, a chain that
 // reaches a chromosome end, unsorted caller input), the step falls back to an exact restatement run

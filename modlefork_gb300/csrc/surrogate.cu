@@ -51,10 +51,10 @@ enum : unsigned { ERR_PRODUCER = 1u, ERR_MMA = 2u, ERR_EPILOGUE = 4u };
 __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
   return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
 }
-// The logistic function as two hardware approximations (relative error about 2^-22), SiLU and its
-// derivative: the epilogues evaluate one per output element.  Flushing subnormals loses nothing here: added to 1
-// a subnormal exponential vanishes, and the reciprocal of a sum above 2^126 is 0, the limit (as in
-// __fdividef, whose results these are bit for bit at a third of the instructions of __fdividef(z, 1 + __expf(-z))).
+// The logistic function 1 / (1 + 2^(-z log2 e)) as two hardware approximations (relative error about 2^-22), SiLU
+// and its derivative: the epilogues evaluate one per output element.  Flushing subnormals loses nothing here:
+// added to 1 a subnormal exponential vanishes, and the reciprocal of a sum above 2^126 is 0, the limit.  SiLU
+// compared over all 2^32 arguments with z times the fast division 1 / (1 + __expf(-z)): the same outputs.
 __device__ __forceinline__ float logistic(float z) {
   float e, r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.44269504088896340736f));
@@ -1716,10 +1716,11 @@ thread_local char g_err[512];
 std::mutex g_mu;
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 unsigned* g_dev_err[64] = {};
-// pipeline stages of the forward/data-gradient convolution per N tile width (64, 128, 256):
-// fewer stages let more CTAs share an SM, so one tile's epilogue overlaps another's main loop
+// pipeline depth of the forward/data-gradient convolution per N tile width (64, 128, 256): with one CTA
+// per tile its stages (fewer let more CTAs share an SM, so one tile's epilogue overlaps another's main loop), in
+// the persistent form where conv_plan starts
 int g_conv_stages[3] = {4, 3, 4};
-// kernel form per N tile width: bit 0 the persistent kernel (double-buffered TMEM accumulator),
+// kernel form per N tile width: bit 0 the persistent kernel (two to eight TMEM accumulators),
 // bit 1 the staged epilogue (outputs through shared memory and TMA stores)
 int g_conv_form[3] = {2, 2, 2};
 
